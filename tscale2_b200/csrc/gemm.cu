@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(GATED ? NUM_THREADS_GATED : NUM_THREADS, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
     const int tiles = p.m_tiles * p.n_tiles;
@@ -750,6 +751,7 @@ __global__ void __launch_bounds__(GATED ? NUM_THREADS_GATED : NUM_THREADS, 1)
 template <int BN>
 __global__ void reduce_splitk_kernel(const GemmParams p)
 {
+    grid_dep_wait();
     const int tiles = p.m_tiles * p.n_tiles;
     const int vec_per_tile = BM * BN / 4;
     const long long total = (long long)tiles * vec_per_tile;
@@ -1034,13 +1036,11 @@ static int launch(const GemmArgs &a, const Plan &pl, const CUtensorMap &tmA, con
     // SMs left to kernels that run beside this one (the data-parallel exchange): a persistent CTA that finds its SM
     // taken starts only when another CTA of the grid has finished all of its units, which can double the launch's time
     const int grid = std::max(1, std::min(pl.grid, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)));
-    kern<<<grid, GATED ? NUM_THREADS_GATED : NUM_THREADS, SmemLayout<BN>::TOTAL, a.stream>>>(tmA, tmB, tmC, p);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((kern), grid, GATED ? NUM_THREADS_GATED : NUM_THREADS, SmemLayout<BN>::TOTAL, a.stream, tmA, tmB, tmC, p);
     if (pl.splits > 1) {
         const long long total = (long long)pl.m_tiles * pl.n_tiles * BM * BN / 4;
         int blocks = (int)std::min<long long>(ceil_div(total, 256), 4 * sm_count(a.device));
-        reduce_splitk_kernel<BN><<<blocks, 256, 0, a.stream>>>(p);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((reduce_splitk_kernel<BN>), blocks, 256, 0, a.stream, p);
     }
     return TS2_OK;
 }

@@ -48,6 +48,7 @@ __host__ __device__ inline float att_dot_scale() { return sqrtf(1.0f / 128) * (0
 // rope[t][2i] = cos(t * theta^(-2i/128)), rope[t][2i+1] = sin(...)   (TRopeComputer, src/gpt/att/rope.cpp:4-24)
 __global__ void fill_rope_kernel(float *__restrict__ rope, int T)
 {
+    grid_dep_wait();
     const long long total = (long long)T * 64;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int t = (int)(i / 64), k = (int)(i % 64);
@@ -60,8 +61,7 @@ __global__ void fill_rope_kernel(float *__restrict__ rope, int T)
 
 int fill_rope(const Ctx &c, float *rope, int T)
 {
-    fill_rope_kernel<<<std::max(1, std::min(T, 1024)), 64, 0, c.stream>>>(rope, T);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((fill_rope_kernel), std::max(1, std::min(T, 1024)), 64, 0, c.stream, rope, T);
     return TS2_OK;
 }
 
@@ -76,6 +76,7 @@ __global__ void att_post_forward_kernel(const __half *__restrict__ qkvg, const f
                                         __half *__restrict__ q, __half *__restrict__ k, __half *__restrict__ v,
                                         float *__restrict__ qscale, float *__restrict__ vscale)
 {
+    grid_dep_wait();
     const int Q = H * TILE;
     constexpr int R = 2; // two (node, head) items in flight per warp
     WARP_BATCH_LOOP((long long)T * H, R)
@@ -116,8 +117,8 @@ __global__ void att_post_forward_kernel(const __half *__restrict__ qkvg, const f
 int att_post_forward(const Ctx &c, const __half *qkvg, const float *rope, int T, int H, __half *q, __half *k, __half *v, float *qscale,
                      float *vscale)
 {
-    att_post_forward_kernel<<<grid_for(c, att_post_forward_kernel, (long long)T * H), THREADS, 0, c.stream>>>(qkvg, rope, T, H, q, k, v, qscale, vscale);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((att_post_forward_kernel), grid_for(c, att_post_forward_kernel, (long long)T * H), THREADS, 0, c.stream, qkvg, rope, T, H,
+               q, k, v, qscale, vscale);
     return TS2_OK;
 }
 
@@ -141,6 +142,7 @@ __global__ void att_post_backward_kernel(const GT *__restrict__ dq, const GT *__
                                          const float *__restrict__ vscale, const float *__restrict__ rope,
                                          const float *__restrict__ sko_k, int T, int H, void *__restrict__ d4)
 {
+    grid_dep_wait();
     const int Q = H * TILE;
     const float kfold = __ldg(sko_k);
     constexpr int R = 2;
@@ -193,9 +195,8 @@ int att_post_backward(const Ctx &c, const void *dq, const void *dk, const void *
                       const float *qscale, const float *vscale, const float *rope, const float *sko_k, int T, int H, void *d4)
 {
 #define TS2_POST_BWD(FT_, GT_)                                                                                          \
-    att_post_backward_kernel<FT_, GT_><<<grid_for(c, att_post_backward_kernel<FT_, GT_>, (long long)T * H), THREADS, 0, \
-                                         c.stream>>>((const GT_ *)dq, (const GT_ *)dk, (const GT_ *)dv, q, v, qscale, vscale, \
-                                                     rope, sko_k, T, H, d4)
+    TS2_LAUNCH((att_post_backward_kernel<FT_, GT_>), grid_for(c, att_post_backward_kernel<FT_, GT_>, (long long)T * H), THREADS, 0, c.stream, \
+               (const GT_ *)dq, (const GT_ *)dk, (const GT_ *)dv, q, v, qscale, vscale, rope, sko_k, T, H, d4)
     if (c.ft == 0 && grads16)
         TS2_POST_BWD(0, __half);
     else if (c.ft == 0)
@@ -205,7 +206,6 @@ int att_post_backward(const Ctx &c, const void *dq, const void *dk, const void *
     else
         TS2_POST_BWD(1, float);
 #undef TS2_POST_BWD
-    TS2_CHECK_LAUNCH();
     return TS2_OK;
 }
 
@@ -216,6 +216,7 @@ __global__ void attention_forward_kernel(const __half *__restrict__ q, const __h
                                          const int *__restrict__ span_start, const int *__restrict__ span_finish, int T, int H,
                                          float slope, __half *__restrict__ o, float *__restrict__ lse)
 {
+    grid_dep_wait();
     const int Q = H * TILE;
     const float ds = att_dot_scale();
     WARP_ITEM_LOOP((long long)T * H)
@@ -247,8 +248,8 @@ __global__ void attention_forward_kernel(const __half *__restrict__ q, const __h
 int attention_forward_rowwise(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start,
                               const int *span_finish, int T, int H, float slope, __half *o, float *lse)
 {
-    attention_forward_kernel<<<grid_for(c, (long long)T * H), THREADS, 0, c.stream>>>(q, k, v, span_start, span_finish, T, H, slope, o, lse);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((attention_forward_kernel), grid_for(c, (long long)T * H), THREADS, 0, c.stream, q, k, v, span_start, span_finish, T, H,
+               slope, o, lse);
     return TS2_OK;
 }
 
@@ -257,6 +258,7 @@ __global__ void attention_dq_kernel(const __half *__restrict__ q, const __half *
                                     const int *__restrict__ span_start, const int *__restrict__ span_finish, int T, int H, float slope,
                                     float *__restrict__ dq)
 {
+    grid_dep_wait();
     const int Q = H * TILE;
     const float ds = att_dot_scale(), c2 = ds * 0.693147f;
     WARP_ITEM_LOOP((long long)T * H)
@@ -283,6 +285,7 @@ __global__ void attention_dkv_kernel(const __half *__restrict__ q, const __half 
                                      const int *__restrict__ rev_first, const int *__restrict__ rev_last, int T, int H, float slope,
                                      float *__restrict__ dk, float *__restrict__ dv)
 {
+    grid_dep_wait();
     const int Q = H * TILE;
     const float ds = att_dot_scale(), c2 = ds * 0.693147f;
     WARP_ITEM_LOOP((long long)T * H)
@@ -311,11 +314,9 @@ int attention_backward_rowwise(const Ctx &c, const __half *q, const __half *k, c
                                const int *rev_last, int T, int H, float slope, float *dq, float *dk, float *dv)
 {
     const int grid = grid_for(c, (long long)T * H);
-    attention_dq_kernel<<<grid, THREADS, 0, c.stream>>>(q, k, v, dout, lse, dscale, span_start, span_finish, T, H, slope, dq);
-    TS2_CHECK_LAUNCH();
-    attention_dkv_kernel<<<grid, THREADS, 0, c.stream>>>(q, k, v, dout, lse, dscale, span_start, span_finish, rev_first, rev_last, T, H,
-                                                         slope, dk, dv);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((attention_dq_kernel), grid, THREADS, 0, c.stream, q, k, v, dout, lse, dscale, span_start, span_finish, T, H, slope, dq);
+    TS2_LAUNCH((attention_dkv_kernel), grid, THREADS, 0, c.stream, q, k, v, dout, lse, dscale, span_start, span_finish, rev_first,
+               rev_last, T, H, slope, dk, dv);
     return TS2_OK;
 }
 

@@ -66,6 +66,11 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int T = p.T, H = p.H, h = blockIdx.y, r0 = blockIdx.x * TC_BM;
 
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), 512);
+        tmem_relinquish();
+    }
+    grid_dep_wait();
     // range of nodes that see any of this block's keys
     if (threadIdx.x == 0) {
         rng[0] = 0x7fffffff;
@@ -98,10 +103,6 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
         prefetch_tmap(&tmV);
         prefetch_tmap(&tmQ);
         prefetch_tmap(&tmDO);
-    }
-    if (warp == 1) {
-        tmem_alloc(smem_u32(tmem_slot), 512);
-        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
@@ -360,10 +361,9 @@ int attention_backward_kv_tc(const Ctx &c, const __half *q, const __half *k, con
         return fail(TS2_ERR_CUDA, "attention: no device status word");
     dim3 grid((unsigned)ceil_div(T, TC_BM), (unsigned)H);
     if (out16)
-        att_bwd_kv_tc_kernel<true><<<grid, KV_THREADS, KV_SMEM, c.stream>>>(tK, tV, tQ, tDO, tDK, tDV, p);
+        TS2_LAUNCH((att_bwd_kv_tc_kernel<true>), grid, KV_THREADS, KV_SMEM, c.stream, tK, tV, tQ, tDO, tDK, tDV, p);
     else
-        att_bwd_kv_tc_kernel<false><<<grid, KV_THREADS, KV_SMEM, c.stream>>>(tK, tV, tQ, tDO, tDK, tDV, p);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((att_bwd_kv_tc_kernel<false>), grid, KV_THREADS, KV_SMEM, c.stream, tK, tV, tQ, tDO, tDK, tDV, p);
     return TS2_OK;
 }
 

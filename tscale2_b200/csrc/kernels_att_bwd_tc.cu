@@ -46,6 +46,7 @@ static_assert(BwdLayout::SMEM <= 232448, "shared memory budget");
 __global__ void att_pack_meta_kernel(const float *__restrict__ lse, const float *__restrict__ dscale, const int *__restrict__ span_start,
                                      const int *__restrict__ span_finish, int T, int Tpad, int H, float c2, float4 *__restrict__ meta)
 {
+    grid_dep_wait();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= Tpad * H)
         return;
@@ -86,6 +87,11 @@ __global__ void __launch_bounds__(BW_THREADS, 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int T = p.T, H = p.H, h = blockIdx.y, r0 = blockIdx.x * BW_ROWS;
 
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), 512);
+        tmem_relinquish();
+    }
+    grid_dep_wait();
     // range of streamed rows each block has to visit
     if (threadIdx.x < 4)
         rng[threadIdx.x] = (threadIdx.x & 1) ? -1 : 0x7fffffff;
@@ -114,10 +120,6 @@ __global__ void __launch_bounds__(BW_THREADS, 1)
         prefetch_tmap(&tmA1);
         prefetch_tmap(&tmB1);
         prefetch_tmap(&tmB2);
-    }
-    if (warp == 1) {
-        tmem_alloc(smem_u32(tmem_slot), 512);
-        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
@@ -377,8 +379,7 @@ static int launch_bwd_dq(const Ctx &c, const __half *a1, const __half *a2, const
     if ((rc = make_tensor_map(&tOut, p.out, out16 ? 2 : 4, Q, p.T, Q, 32)) != TS2_OK) // boxes of 128 bytes x 32 rows
         return rc;
     dim3 grid((unsigned)ceil_div(p.T, BW_ROWS), (unsigned)p.H);
-    kern<<<grid, BW_THREADS, BwdLayout::SMEM, c.stream>>>(tA1, tA2, tB1, tB2, tOut, p);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((kern), grid, BW_THREADS, BwdLayout::SMEM, c.stream, tA1, tA2, tB1, tB2, tOut, p);
     return TS2_OK;
 }
 
@@ -427,9 +428,8 @@ int attention_backward_tc(const Ctx &c, const __half *q, const __half *k, const 
         return rc;
     {
         const int total = Tpad * H;
-        att_pack_meta_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, c.stream>>>(lse, dscale, span_start, span_finish, T, Tpad, H,
-                                                                                  att_dot_scale_tc() * 0.693147f, meta);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((att_pack_meta_kernel), (unsigned)ceil_div(total, 256), 256, 0, c.stream, lse, dscale, span_start, span_finish, T,
+                   Tpad, H, att_dot_scale_tc() * 0.693147f, meta);
     }
     p.out = dq;
     if ((rc = launch_bwd_dq(c, q, dout, k, v, p, grads16)) != TS2_OK)

@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(ATT_THREADS)
                        const int *__restrict__ span_start, const int *__restrict__ span_finish, int T, int H, float slope,
                        __half *__restrict__ o, float *__restrict__ lse)
 {
+    grid_dep_wait();
     extern __shared__ __align__(1024) uint8_t att_smem[];
     __shared__ int s_lo, s_hi;
     const uint32_t sQ = smem_u32(att_smem), sK = sQ + TILE_BYTES, sV = sK + 2 * TILE_BYTES; // K and V double-buffered
@@ -289,6 +290,7 @@ __global__ void __launch_bounds__(ATT_THREADS)
                       const int *__restrict__ span_start, const int *__restrict__ span_finish, int T, int H, float slope,
                       float *__restrict__ dq)
 {
+    grid_dep_wait();
     extern __shared__ __align__(1024) uint8_t att_smem[];
     __shared__ int s_lo, s_hi;
     const uint32_t sQ = smem_u32(att_smem), sDO = sQ + TILE_BYTES, sK = sDO + TILE_BYTES, sV = sK + 2 * TILE_BYTES;
@@ -380,6 +382,7 @@ __global__ void __launch_bounds__(ATT_THREADS)
                        const int *__restrict__ span_start, const int *__restrict__ span_finish, const int *__restrict__ rev_first,
                        const int *__restrict__ rev_last, int T, int H, float slope, float *__restrict__ dk, float *__restrict__ dv)
 {
+    grid_dep_wait();
     extern __shared__ __align__(1024) uint8_t att_smem[];
     __shared__ int s_lo, s_hi;
     __shared__ int s_st[2][BLK], s_fi[2][BLK];
@@ -496,8 +499,7 @@ int attention_forward_mma(const Ctx &c, const __half *q, const __half *k, const 
     if (rc != TS2_OK)
         return rc;
     dim3 grid((unsigned)ceil_div(T, BLK), (unsigned)H);
-    att_fwd_mma_kernel<<<grid, ATT_THREADS, 5 * TILE_BYTES, c.stream>>>(q, k, v, span_start, span_finish, T, H, slope, o, lse);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((att_fwd_mma_kernel), grid, ATT_THREADS, 5 * TILE_BYTES, c.stream, q, k, v, span_start, span_finish, T, H, slope, o, lse);
     return TS2_OK;
 }
 
@@ -509,11 +511,10 @@ int attention_backward_mma(const Ctx &c, const __half *q, const __half *k, const
     if (rc != TS2_OK)
         return rc;
     dim3 grid((unsigned)ceil_div(T, BLK), (unsigned)H);
-    att_dq_mma_kernel<<<grid, ATT_THREADS, 6 * TILE_BYTES, c.stream>>>(q, k, v, dout, lse, dscale, span_start, span_finish, T, H, slope, dq);
-    TS2_CHECK_LAUNCH();
-    att_dkv_mma_kernel<<<grid, ATT_THREADS, 6 * TILE_BYTES, c.stream>>>(q, k, v, dout, lse, dscale, span_start, span_finish, rev_first,
-                                                                        rev_last, T, H, slope, dk, dv);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((att_dq_mma_kernel), grid, ATT_THREADS, 6 * TILE_BYTES, c.stream, q, k, v, dout, lse, dscale, span_start, span_finish, T,
+               H, slope, dq);
+    TS2_LAUNCH((att_dkv_mma_kernel), grid, ATT_THREADS, 6 * TILE_BYTES, c.stream, q, k, v, dout, lse, dscale, span_start, span_finish,
+               rev_first, rev_last, T, H, slope, dk, dv);
     return TS2_OK;
 }
 

@@ -58,6 +58,11 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int T = p.T, H = p.H, h = blockIdx.y, t0 = blockIdx.x * TC_BM;
 
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), 256);
+        tmem_relinquish();
+    }
+    grid_dep_wait();
     // key range of the block: [min start, max finish] over its rows
     {
         if (threadIdx.x == 0) {
@@ -89,10 +94,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
         prefetch_tmap(&tmQ);
         prefetch_tmap(&tmK);
         prefetch_tmap(&tmV);
-    }
-    if (warp == 1) {
-        tmem_alloc(smem_u32(tmem_slot), 256);
-        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
@@ -384,8 +385,7 @@ int attention_forward_tc(const Ctx &c, const __half *q, const __half *k, const _
     if (!p.status)
         return fail(TS2_ERR_CUDA, "attention: no device status word");
     dim3 grid((unsigned)ceil_div(T, TC_BM), (unsigned)H);
-    att_fwd_tc_kernel<<<grid, TC_THREADS, FWD_SMEM, c.stream>>>(tmQ, tmK, tmV, tmO, p);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((att_fwd_tc_kernel), grid, TC_THREADS, FWD_SMEM, c.stream, tmQ, tmK, tmV, tmO, p);
     return TS2_OK;
 }
 

@@ -34,6 +34,7 @@ __device__ __forceinline__ void batch_fail(int *status, int code, int where, int
 __global__ void span_expand_kernel(const int *__restrict__ span_ptr, const int *__restrict__ csr_start, const int *__restrict__ csr_finish,
                                    int T, int n_spans, int *__restrict__ start, int *__restrict__ finish, int *status)
 {
+    grid_dep_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T)
         return;
@@ -62,6 +63,7 @@ __global__ void span_expand_kernel(const int *__restrict__ span_ptr, const int *
 __global__ void __launch_bounds__(1024) span_block_reduce_kernel(const int *__restrict__ start, const int *__restrict__ finish, int T,
                                                                  int *__restrict__ blk_max, int *__restrict__ blk_min)
 {
+    grid_dep_wait();
     __shared__ int s_max[32], s_min[32];
     const int t = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int mx = -1, mn = T;
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(1024) span_scan_kernel(const int *__restrict__
                                                          const int *__restrict__ blk_max, const int *__restrict__ blk_min,
                                                          int *__restrict__ run_max, int *__restrict__ suf_min)
 {
+    grid_dep_wait();
     __shared__ int s_max[32], s_min[32];
     const int t = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int mx = -1, mn = T;
@@ -147,6 +150,7 @@ __global__ void __launch_bounds__(1024) span_scan_kernel(const int *__restrict__
 __global__ void span_reverse_kernel(const int *__restrict__ run_max, const int *__restrict__ suf_min, int T, int *__restrict__ rev_first,
                                     int *__restrict__ rev_last)
 {
+    grid_dep_wait();
     const int to = blockIdx.x * blockDim.x + threadIdx.x;
     if (to >= T)
         return;
@@ -177,6 +181,7 @@ __global__ void span_reverse_kernel(const int *__restrict__ run_max, const int *
 __global__ void target_scatter_kernel(const int *__restrict__ node, const int *__restrict__ id, int n, int T, int V, int *__restrict__ target,
                                       int *status)
 {
+    grid_dep_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
@@ -194,6 +199,7 @@ __global__ void target_scatter_kernel(const int *__restrict__ node, const int *_
 __global__ void label_entries_kernel(uint32_t *__restrict__ label_arr, uint32_t *__restrict__ label_ptr, int T, uint32_t n_labels,
                                      uint32_t label_count, uint32_t *__restrict__ key, uint32_t *__restrict__ val, int *status)
 {
+    grid_dep_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T)
         return;
@@ -220,6 +226,7 @@ __global__ void label_entries_kernel(uint32_t *__restrict__ label_arr, uint32_t 
 // stay inside label_arr whatever the input held)
 __global__ void label_ptr_clamp_kernel(uint32_t *__restrict__ label_ptr, int T, uint32_t n_labels)
 {
+    grid_dep_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t <= T)
         label_ptr[t] = min(label_ptr[t], n_labels);
@@ -233,6 +240,7 @@ __global__ void __launch_bounds__(BP_THREADS) radix_pass_kernel(const uint32_t *
                                                                 uint32_t n, int shift, uint32_t *__restrict__ hist, uint32_t nblocks,
                                                                 uint32_t *__restrict__ key_out, uint32_t *__restrict__ val_out)
 {
+    grid_dep_wait();
     __shared__ uint32_t cnt[BP_WARPS][256];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int i = tid; i < BP_WARPS * 256; i += BP_THREADS)
@@ -267,6 +275,7 @@ __global__ void __launch_bounds__(BP_THREADS) radix_pass_kernel(const uint32_t *
 // counters on top of the sums of the blocks before it
 __global__ void __launch_bounds__(1024) scan_block_sums_kernel(const uint32_t *__restrict__ x, uint32_t total, uint32_t *__restrict__ blk_sum)
 {
+    grid_dep_wait();
     __shared__ uint32_t s_sum[32];
     const uint32_t i = blockIdx.x * 1024 + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -287,6 +296,7 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(const uint32_t *_
 
 __global__ void __launch_bounds__(1024) exclusive_scan_kernel(uint32_t *__restrict__ x, uint32_t total, const uint32_t *__restrict__ blk_sum)
 {
+    grid_dep_wait();
     __shared__ uint32_t s_sum[32];
     const uint32_t i = blockIdx.x * 1024 + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -341,6 +351,7 @@ __global__ void __launch_bounds__(BP_THREADS) embed_runs_kernel(const float *__r
                                                                 const uint32_t *__restrict__ val, uint32_t n, int D,
                                                                 float *__restrict__ dE, float *__restrict__ partial)
 {
+    grid_dep_wait();
     const int tiles = D / TILE, lane = threadIdx.x & 31;
     const uint32_t nchunks = (n + EMB_CHUNK - 1) / EMB_CHUNK;
     const unsigned long long items = (unsigned long long)nchunks * tiles;
@@ -399,6 +410,7 @@ __global__ void __launch_bounds__(BP_THREADS) embed_runs_kernel(const float *__r
 __global__ void __launch_bounds__(BP_THREADS) embed_chain_kernel(const uint32_t *__restrict__ key, uint32_t n, int D,
                                                                  const float *__restrict__ partial, float *__restrict__ dE)
 {
+    grid_dep_wait();
     const int tiles = D / TILE, lane = threadIdx.x & 31;
     const uint32_t nchunks = (n + EMB_CHUNK - 1) / EMB_CHUNK;
     const unsigned long long items = (unsigned long long)nchunks * tiles;
@@ -438,8 +450,8 @@ int blocks_for(long long n)
 int batch_span_tables(const Ctx &c, const int *span_ptr, const int *csr_start, const int *csr_finish, int T, int n_spans, int *start,
                       int *finish, int *scan_tmp, int *rev_first, int *rev_last, int *status)
 {
-    span_expand_kernel<<<blocks_for(T), BP_THREADS, 0, c.stream>>>(span_ptr, csr_start, csr_finish, T, n_spans, start, finish, status);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((span_expand_kernel), blocks_for(T), BP_THREADS, 0, c.stream, span_ptr, csr_start, csr_finish, T, n_spans, start, finish,
+               status);
     return batch_reverse_ranges(c, start, finish, T, scan_tmp, rev_first, rev_last);
 }
 
@@ -447,12 +459,9 @@ int batch_reverse_ranges(const Ctx &c, const int *start, const int *finish, int 
 {
     const int nb = (T + 1023) / 1024;
     int *blk = scan_tmp + 2 * (size_t)T;
-    span_block_reduce_kernel<<<nb, 1024, 0, c.stream>>>(start, finish, T, blk, blk + nb);
-    TS2_CHECK_LAUNCH();
-    span_scan_kernel<<<nb, 1024, 0, c.stream>>>(start, finish, T, blk, blk + nb, scan_tmp, scan_tmp + T);
-    TS2_CHECK_LAUNCH();
-    span_reverse_kernel<<<blocks_for(T), BP_THREADS, 0, c.stream>>>(scan_tmp, scan_tmp + T, T, rev_first, rev_last);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((span_block_reduce_kernel), nb, 1024, 0, c.stream, start, finish, T, blk, blk + nb);
+    TS2_LAUNCH((span_scan_kernel), nb, 1024, 0, c.stream, start, finish, T, blk, blk + nb, scan_tmp, scan_tmp + T);
+    TS2_LAUNCH((span_reverse_kernel), blocks_for(T), BP_THREADS, 0, c.stream, scan_tmp, scan_tmp + T, T, rev_first, rev_last);
     return TS2_OK;
 }
 
@@ -460,8 +469,7 @@ int batch_targets(const Ctx &c, const int *node, const int *id, int n, int T, in
 {
     TS2_CUDA(cudaMemsetAsync(target, 0xff, (size_t)T * 4, c.stream));
     if (n > 0) {
-        target_scatter_kernel<<<blocks_for(n), BP_THREADS, 0, c.stream>>>(node, id, n, T, V, target, status);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((target_scatter_kernel), blocks_for(n), BP_THREADS, 0, c.stream, node, id, n, T, V, target, status);
     }
     return TS2_OK;
 }
@@ -492,11 +500,9 @@ int label_index_entries(const Ctx &c, uint32_t *label_arr, uint32_t *label_ptr, 
         TS2_CUDA(cudaMemsetAsync(ix.key[0], 0, (size_t)n_labels * 4, c.stream));
         TS2_CUDA(cudaMemsetAsync(ix.val[0], 0, (size_t)n_labels * 4, c.stream));
     }
-    label_entries_kernel<<<blocks_for(T), BP_THREADS, 0, c.stream>>>(label_arr, label_ptr, T, n_labels, label_count, ix.key[0], ix.val[0],
-                                                                     status);
-    TS2_CHECK_LAUNCH();
-    label_ptr_clamp_kernel<<<blocks_for(T + 1), BP_THREADS, 0, c.stream>>>(label_ptr, T, n_labels);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((label_entries_kernel), blocks_for(T), BP_THREADS, 0, c.stream, label_arr, label_ptr, T, n_labels, label_count, ix.key[0],
+               ix.val[0], status);
+    TS2_LAUNCH((label_ptr_clamp_kernel), blocks_for(T + 1), BP_THREADS, 0, c.stream, label_ptr, T, n_labels);
     return TS2_OK;
 }
 
@@ -511,17 +517,13 @@ int label_index_sort(const Ctx &c, uint32_t label_count, LabelIndex &ix)
     int cur = 0;
     for (int shift = 0; shift < bits; shift += 8) {
         const int out = cur ^ 1;
-        radix_pass_kernel<true><<<nblocks, BP_THREADS, 0, c.stream>>>(ix.key[cur], ix.val[cur], ix.n, shift, ix.hist, nblocks, nullptr,
-                                                                     nullptr);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((radix_pass_kernel<true>), nblocks, BP_THREADS, 0, c.stream, ix.key[cur], ix.val[cur], ix.n, shift, ix.hist, nblocks,
+                   nullptr, nullptr);
         const uint32_t total = 256 * nblocks, nb = (total + 1023) / 1024;
-        scan_block_sums_kernel<<<nb, 1024, 0, c.stream>>>(ix.hist, total, ix.hist + total);
-        TS2_CHECK_LAUNCH();
-        exclusive_scan_kernel<<<nb, 1024, 0, c.stream>>>(ix.hist, total, ix.hist + total);
-        TS2_CHECK_LAUNCH();
-        radix_pass_kernel<false><<<nblocks, BP_THREADS, 0, c.stream>>>(ix.key[cur], ix.val[cur], ix.n, shift, ix.hist, nblocks, ix.key[out],
-                                                                      ix.val[out]);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((scan_block_sums_kernel), nb, 1024, 0, c.stream, ix.hist, total, ix.hist + total);
+        TS2_LAUNCH((exclusive_scan_kernel), nb, 1024, 0, c.stream, ix.hist, total, ix.hist + total);
+        TS2_LAUNCH((radix_pass_kernel<false>), nblocks, BP_THREADS, 0, c.stream, ix.key[cur], ix.val[cur], ix.n, shift, ix.hist, nblocks,
+                   ix.key[out], ix.val[out]);
         cur = out;
     }
     ix.sorted = cur;
@@ -535,10 +537,8 @@ int embed_backward_indexed(const Ctx &c, const float *g, const LabelIndex &ix, i
     const uint32_t nchunks = (ix.n + EMB_CHUNK - 1) / EMB_CHUNK;
     const long long items = (long long)nchunks * (D / TILE);
     const int grid = (int)std::max<long long>(1, std::min<long long>((items + BP_WARPS - 1) / BP_WARPS, (long long)sm_count(c.device) * 8));
-    embed_runs_kernel<<<grid, BP_THREADS, 0, c.stream>>>(g, ix.key[ix.sorted], ix.val[ix.sorted], ix.n, D, dE, ix.partial);
-    TS2_CHECK_LAUNCH();
-    embed_chain_kernel<<<grid, BP_THREADS, 0, c.stream>>>(ix.key[ix.sorted], ix.n, D, ix.partial, dE);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((embed_runs_kernel), grid, BP_THREADS, 0, c.stream, g, ix.key[ix.sorted], ix.val[ix.sorted], ix.n, D, dE, ix.partial);
+    TS2_LAUNCH((embed_chain_kernel), grid, BP_THREADS, 0, c.stream, ix.key[ix.sorted], ix.n, D, ix.partial, dE);
     return TS2_OK;
 }
 

@@ -46,6 +46,7 @@ __global__ void embed_forward_kernel(const __half *__restrict__ embed, const flo
                                      const uint32_t *__restrict__ label_arr, const uint32_t *__restrict__ label_ptr, int T, int D,
                                      float *__restrict__ state)
 {
+    grid_dep_wait();
     const int tiles = D / TILE;
     const float scale = __ldg(sko) * (1.f / 32);
     WARP_ITEM_LOOP((long long)T * tiles)
@@ -70,8 +71,8 @@ __global__ void embed_forward_kernel(const __half *__restrict__ embed, const flo
 int embed_forward(const Ctx &c, const __half *embed, const float *sko, const uint32_t *label_arr, const uint32_t *label_ptr, int T,
                   int D, float *state)
 {
-    embed_forward_kernel<<<grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream>>>(embed, sko, label_arr, label_ptr, T, D, state);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((embed_forward_kernel), grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream, embed, sko, label_arr, label_ptr, T,
+               D, state);
     return TS2_OK;
 }
 
@@ -80,6 +81,7 @@ template <int FT>
 __global__ void tilenorm_forward_kernel(const float *__restrict__ x, int T, int D, float s_act, void *__restrict__ n_fast,
                                         __half *__restrict__ n16)
 {
+    grid_dep_wait();
     const int tiles = D / TILE;
     constexpr int R = 2;
     WARP_BATCH_LOOP((long long)T * tiles, R)
@@ -113,12 +115,11 @@ int tilenorm_forward(const Ctx &c, const float *x, int T, int D, void *n_fast, _
                      : c.ft == 1 ? grid_for(c, tilenorm_forward_kernel<1>, (long long)T * (D / TILE))
                                  : grid_for(c, tilenorm_forward_kernel<2>, (long long)T * (D / TILE));
     if (c.ft == 0)
-        tilenorm_forward_kernel<0><<<grid, THREADS, 0, c.stream>>>(x, T, D, c.s_act, n_fast, n16);
+        TS2_LAUNCH((tilenorm_forward_kernel<0>), grid, THREADS, 0, c.stream, x, T, D, c.s_act, n_fast, n16);
     else if (c.ft == 1)
-        tilenorm_forward_kernel<1><<<grid, THREADS, 0, c.stream>>>(x, T, D, c.s_act, n_fast, n16);
+        TS2_LAUNCH((tilenorm_forward_kernel<1>), grid, THREADS, 0, c.stream, x, T, D, c.s_act, n_fast, n16);
     else
-        tilenorm_forward_kernel<2><<<grid, THREADS, 0, c.stream>>>(x, T, D, c.s_act, n_fast, n16);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((tilenorm_forward_kernel<2>), grid, THREADS, 0, c.stream, x, T, D, c.s_act, n_fast, n16);
     return TS2_OK;
 }
 
@@ -126,6 +127,7 @@ __global__ void tilenorm_backward_kernel(const float *__restrict__ x, const floa
                                          float dn_alpha, int T, int D, float *__restrict__ g, int add, unsigned *__restrict__ absmax,
                                          unsigned *__restrict__ health, unsigned step_no)
 {
+    grid_dep_wait();
     const int tiles = D / TILE;
     const float a = dn_alpha * (dyn ? __ldg(dyn) : 1.f);
     float local_max = 0.f;
@@ -186,9 +188,8 @@ __global__ void tilenorm_backward_kernel(const float *__restrict__ x, const floa
 int tilenorm_backward(const Ctx &c, const float *x, const float *dn, const float *dyn, float dn_alpha, int T, int D, float *g, bool add,
                       unsigned *absmax, unsigned *health, unsigned step_no)
 {
-    tilenorm_backward_kernel<<<grid_for(c, tilenorm_backward_kernel, (long long)T * (D / TILE)), THREADS, 0, c.stream>>>(
-        x, dn, dyn, dn_alpha, T, D, g, add ? 1 : 0, absmax, health, step_no);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((tilenorm_backward_kernel), grid_for(c, tilenorm_backward_kernel, (long long)T * (D / TILE)), THREADS, 0, c.stream, x, dn,
+               dyn, dn_alpha, T, D, g, add ? 1 : 0, absmax, health, step_no);
     return TS2_OK;
 }
 
@@ -208,6 +209,7 @@ template <int FT>
 __global__ void cast_grad_kernel(const float *__restrict__ g, size_t n4, const unsigned *__restrict__ absmax, void *__restrict__ out,
                                  float *__restrict__ ginv, float f_static, const float *__restrict__ sko, float *__restrict__ fscale)
 {
+    grid_dep_wait();
     const float mult = grad_mult(*absmax, 128.f);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *ginv = 1.f / mult;
@@ -234,10 +236,9 @@ int cast_grad(const Ctx &c, const float *g, size_t n, const unsigned *absmax, vo
     const int per_sm = resident_blocks(c.device, c.ft == 0 ? (const void *)cast_grad_kernel<0> : (const void *)cast_grad_kernel<1>, THREADS);
     const int grid = (int)std::min<size_t>(ceil_div(n4, THREADS), (size_t)sm_count(c.device) * per_sm);
     if (c.ft == 0)
-        cast_grad_kernel<0><<<grid, THREADS, 0, c.stream>>>(g, n4, absmax, g_fast, ginv, f_static, sko, fscale);
+        TS2_LAUNCH((cast_grad_kernel<0>), grid, THREADS, 0, c.stream, g, n4, absmax, g_fast, ginv, f_static, sko, fscale);
     else
-        cast_grad_kernel<1><<<grid, THREADS, 0, c.stream>>>(g, n4, absmax, g_fast, ginv, f_static, sko, fscale);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((cast_grad_kernel<1>), grid, THREADS, 0, c.stream, g, n4, absmax, g_fast, ginv, f_static, sko, fscale);
     return TS2_OK;
 }
 
@@ -277,6 +278,7 @@ __global__ void rowquant_i8_kernel(const SRC *__restrict__ src, int T, int D, co
                                    int8_t *__restrict__ q, float *__restrict__ row_scale, __half *__restrict__ x16,
                                    float *__restrict__ ginv, float f_static, const float *__restrict__ sko, float *__restrict__ fscale)
 {
+    grid_dep_wait();
     extern __shared__ int8_t rq_rows[]; // [WARPS][D]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float mult = absmax ? grad_mult(*absmax, target) : 1.f;
@@ -334,8 +336,7 @@ static int rowquant_launch(const Ctx &c, const SRC *src, int T, int D, const uns
         configured[c.device & 15] = true;
     }
     const int grid = (int)std::max<long long>(1, std::min<long long>(ceil_div(T, WARPS), (long long)sm_count(c.device) * 4));
-    kern<<<grid, THREADS, smem, c.stream>>>(src, T, D, absmax, 128.f, q, row_scale, x16, ginv, f_static, sko, fscale);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((kern), grid, THREADS, smem, c.stream, src, T, D, absmax, 128.f, q, row_scale, x16, ginv, f_static, sko, fscale);
     return TS2_OK;
 }
 
@@ -352,6 +353,7 @@ int rowquant_half(const Ctx &c, const __half *x, int T, int D, int8_t *q, float 
 
 __global__ void i8_to_half_kernel(const char4 *__restrict__ src, size_t n4, uint2 *__restrict__ dst)
 {
+    grid_dep_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
         const char4 v = src[i];
         const __half2 a = __floats2half2_rn((float)v.x, (float)v.y), b = __floats2half2_rn((float)v.z, (float)v.w);
@@ -363,8 +365,7 @@ int i8_to_half(const Ctx &c, const void *src, size_t n, __half *dst)
 {
     const size_t n4 = n / 4;
     const int grid = (int)std::max<size_t>(1, std::min<size_t>(ceil_div(n4, 256 * 4), (size_t)sm_count(c.device) * 8));
-    i8_to_half_kernel<<<grid, 256, 0, c.stream>>>((const char4 *)src, n4, (uint2 *)dst);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((i8_to_half_kernel), grid, 256, 0, c.stream, (const char4 *)src, n4, (uint2 *)dst);
     return TS2_OK;
 }
 
@@ -374,6 +375,7 @@ template <int FT>
 __global__ void ffn_act_backward_kernel(const __half *__restrict__ drg, const __half *__restrict__ wg, const __half *__restrict__ what,
                                         int what_ld, const float *__restrict__ wscale, int T, int F, void *__restrict__ d2)
 {
+    grid_dep_wait();
     const int tiles = F / TILE;
     constexpr int R = 2;
     WARP_BATCH_LOOP((long long)T * tiles, R)
@@ -419,6 +421,7 @@ __global__ void ffn_act_backward_kernel(const __half *__restrict__ drg, const __
 __global__ void ffn_act_backward_e4m3_kernel(const __half *__restrict__ drg, const __half *__restrict__ wg, const __half *__restrict__ what,
                                              int what_ld, const float *__restrict__ wscale, int T, int F, uint8_t *__restrict__ d2)
 {
+    grid_dep_wait();
     const int tiles = F / TILE;
     constexpr int R = 2;
     WARP_BATCH_LOOP((long long)T * tiles, R)
@@ -467,18 +470,16 @@ int ffn_act_backward(const Ctx &c, const __half *drg, const __half *wg, const __
                      void *d2)
 {
     if (c.ft == 0) {
-        ffn_act_backward_e4m3_kernel<<<grid_for(c, ffn_act_backward_e4m3_kernel, (long long)T * (F / TILE)), THREADS, 0, c.stream>>>(
-            drg, wg, what, what_ld, wscale, T, F, (uint8_t *)d2);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((ffn_act_backward_e4m3_kernel), grid_for(c, ffn_act_backward_e4m3_kernel, (long long)T * (F / TILE)), THREADS, 0,
+                   c.stream, drg, wg, what, what_ld, wscale, T, F, (uint8_t *)d2);
         return TS2_OK;
     }
     const int grid = c.ft == 0 ? grid_for(c, ffn_act_backward_kernel<0>, (long long)T * (F / TILE))
                                : grid_for(c, ffn_act_backward_kernel<1>, (long long)T * (F / TILE));
     if (c.ft == 0)
-        ffn_act_backward_kernel<0><<<grid, THREADS, 0, c.stream>>>(drg, wg, what, what_ld, wscale, T, F, d2);
+        TS2_LAUNCH((ffn_act_backward_kernel<0>), grid, THREADS, 0, c.stream, drg, wg, what, what_ld, wscale, T, F, d2);
     else
-        ffn_act_backward_kernel<1><<<grid, THREADS, 0, c.stream>>>(drg, wg, what, what_ld, wscale, T, F, d2);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((ffn_act_backward_kernel<1>), grid, THREADS, 0, c.stream, drg, wg, what, what_ld, wscale, T, F, d2);
     return TS2_OK;
 }
 
@@ -487,6 +488,7 @@ template <int FT>
 __global__ void att_gate_forward_kernel(const __half *__restrict__ qkvg, const __half *__restrict__ o, int T, int Q, float s_act,
                                         void *__restrict__ rg)
 {
+    grid_dep_wait();
     const int tiles = Q / TILE;
     constexpr int R = 2;
     WARP_BATCH_LOOP((long long)T * tiles, R)
@@ -518,6 +520,7 @@ __global__ void att_gate_forward_kernel(const __half *__restrict__ qkvg, const _
 __global__ void att_gate_forward_e4m3_kernel(const __half *__restrict__ qkvg, const __half *__restrict__ o, int T, int Q, float s_act,
                                              uint8_t *__restrict__ rg)
 {
+    grid_dep_wait();
     const int tiles = Q / TILE;
     constexpr int R = 4;
     const __half2 sa = __float2half2_rn(s_act);
@@ -551,21 +554,19 @@ __global__ void att_gate_forward_e4m3_kernel(const __half *__restrict__ qkvg, co
 int att_gate_forward(const Ctx &c, const __half *qkvg, const __half *o, int T, int Q, void *rg)
 {
     if (c.ft == 0) {
-        att_gate_forward_e4m3_kernel<<<grid_for(c, att_gate_forward_e4m3_kernel, (long long)T * (Q / TILE)), THREADS, 0, c.stream>>>(
-            qkvg, o, T, Q, c.s_act, (uint8_t *)rg);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((att_gate_forward_e4m3_kernel), grid_for(c, att_gate_forward_e4m3_kernel, (long long)T * (Q / TILE)), THREADS, 0,
+                   c.stream, qkvg, o, T, Q, c.s_act, (uint8_t *)rg);
         return TS2_OK;
     }
     const int grid = c.ft == 0   ? grid_for(c, att_gate_forward_kernel<0>, (long long)T * (Q / TILE))
                      : c.ft == 1 ? grid_for(c, att_gate_forward_kernel<1>, (long long)T * (Q / TILE))
                                  : grid_for(c, att_gate_forward_kernel<2>, (long long)T * (Q / TILE));
     if (c.ft == 0)
-        att_gate_forward_kernel<0><<<grid, THREADS, 0, c.stream>>>(qkvg, o, T, Q, c.s_act, rg);
+        TS2_LAUNCH((att_gate_forward_kernel<0>), grid, THREADS, 0, c.stream, qkvg, o, T, Q, c.s_act, rg);
     else if (c.ft == 1)
-        att_gate_forward_kernel<1><<<grid, THREADS, 0, c.stream>>>(qkvg, o, T, Q, c.s_act, rg);
+        TS2_LAUNCH((att_gate_forward_kernel<1>), grid, THREADS, 0, c.stream, qkvg, o, T, Q, c.s_act, rg);
     else
-        att_gate_forward_kernel<2><<<grid, THREADS, 0, c.stream>>>(qkvg, o, T, Q, c.s_act, rg);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((att_gate_forward_kernel<2>), grid, THREADS, 0, c.stream, qkvg, o, T, Q, c.s_act, rg);
     return TS2_OK;
 }
 
@@ -573,6 +574,7 @@ template <int FT>
 __global__ void att_gate_backward_kernel(const __half *__restrict__ drg, const __half *__restrict__ qkvg, const __half *__restrict__ o,
                                          int T, int Q, void *__restrict__ d4, __half *__restrict__ dout, float *__restrict__ dscale)
 {
+    grid_dep_wait();
     const int tiles = Q / TILE; // = heads
     constexpr int R = 2;
     WARP_BATCH_LOOP((long long)T * tiles, R)
@@ -613,6 +615,7 @@ __global__ void att_gate_backward_kernel(const __half *__restrict__ drg, const _
 __global__ void att_gate_backward_e4m3_kernel(const __half *__restrict__ drg, const __half *__restrict__ qkvg, const __half *__restrict__ o,
                                               int T, int Q, uint8_t *__restrict__ d4, __half *__restrict__ dout, float *__restrict__ dscale)
 {
+    grid_dep_wait();
     const int tiles = Q / TILE; // = heads
     constexpr int R = 2;
     WARP_BATCH_LOOP((long long)T * tiles, R)
@@ -659,18 +662,16 @@ int att_gate_backward(const Ctx &c, const __half *drg, const __half *qkvg, const
                       float *dscale)
 {
     if (c.ft == 0) {
-        att_gate_backward_e4m3_kernel<<<grid_for(c, att_gate_backward_e4m3_kernel, (long long)T * (Q / TILE)), THREADS, 0, c.stream>>>(
-            drg, qkvg, o, T, Q, (uint8_t *)d4, dout, dscale);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((att_gate_backward_e4m3_kernel), grid_for(c, att_gate_backward_e4m3_kernel, (long long)T * (Q / TILE)), THREADS, 0,
+                   c.stream, drg, qkvg, o, T, Q, (uint8_t *)d4, dout, dscale);
         return TS2_OK;
     }
     const int grid = c.ft == 0 ? grid_for(c, att_gate_backward_kernel<0>, (long long)T * (Q / TILE))
                                : grid_for(c, att_gate_backward_kernel<1>, (long long)T * (Q / TILE));
     if (c.ft == 0)
-        att_gate_backward_kernel<0><<<grid, THREADS, 0, c.stream>>>(drg, qkvg, o, T, Q, d4, dout, dscale);
+        TS2_LAUNCH((att_gate_backward_kernel<0>), grid, THREADS, 0, c.stream, drg, qkvg, o, T, Q, d4, dout, dscale);
     else
-        att_gate_backward_kernel<1><<<grid, THREADS, 0, c.stream>>>(drg, qkvg, o, T, Q, d4, dout, dscale);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((att_gate_backward_kernel<1>), grid, THREADS, 0, c.stream, drg, qkvg, o, T, Q, d4, dout, dscale);
     return TS2_OK;
 }
 
@@ -683,6 +684,7 @@ __global__ void __launch_bounds__(512, 2)
     softmax_ce_kernel(__half *__restrict__ logits, int rows, int V, const float *__restrict__ bias, const int *__restrict__ target,
                       float gscale, float *__restrict__ logp_sum, int write_grad)
 {
+    grid_dep_wait();
     extern __shared__ uint4 row_s4[];
     __shared__ float red[32];
     __shared__ float x_tgt_s;
@@ -800,6 +802,7 @@ __global__ void __launch_bounds__(1024, 1)
         fence_barrier_init();
     }
     __syncthreads();
+    grid_dep_wait();
     volatile int *abort_flag = &abort_s;
     const int first = blockIdx.x, step = gridDim.x;
     if (tid == 0 && first < rows) {
@@ -948,6 +951,7 @@ __global__ void __launch_bounds__(1024, 1)
 // of the largest finite |x| as fp32).
 __global__ void checksum_kernel(const uint32_t *__restrict__ p, size_t nwords, int kind, unsigned long long *__restrict__ out)
 {
+    grid_dep_wait();
     unsigned long long sum = 0, bad = 0;
     float mx = 0.f;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nwords; i += (size_t)gridDim.x * blockDim.x) {
@@ -988,8 +992,7 @@ int checksum(const Ctx &c, const void *p, size_t bytes, int kind, unsigned long 
 {
     const size_t nwords = bytes / 4;
     const int grid = (int)std::max<size_t>(1, std::min<size_t>(ceil_div(nwords, 256 * 8), (size_t)sm_count(c.device) * 8));
-    checksum_kernel<<<grid, 256, 0, c.stream>>>((const uint32_t *)p, nwords, kind, out);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((checksum_kernel), grid, 256, 0, c.stream, (const uint32_t *)p, nwords, kind, out);
     return TS2_OK;
 }
 
@@ -1009,8 +1012,8 @@ int softmax_ce(const Ctx &c, __half *logits, int rows, int V, const float *bias,
         if (!status)
             return fail(TS2_ERR_CUDA, "softmax_ce: no device status word");
         const int grid = std::min(rows, sm_count(c.device));
-        softmax_ce_pipe_kernel<<<grid, 1024, two_rows, c.stream>>>(logits, rows, V, bias, target, gscale, logp_sum, write_grad ? 1 : 0, status);
-        TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((softmax_ce_pipe_kernel), grid, 1024, two_rows, c.stream, logits, rows, V, bias, target, gscale, logp_sum,
+                   write_grad ? 1 : 0, status);
         return TS2_OK;
     }
     const size_t smem = (size_t)V * sizeof(__half);
@@ -1022,8 +1025,7 @@ int softmax_ce(const Ctx &c, __half *logits, int rows, int V, const float *bias,
     if (smem > 200 * 1024)
         return fail(TS2_ERR_TOO_LARGE, "softmax_ce: vocabulary %d does not fit the shared-memory row buffer", V);
     const int grid = std::min(rows, sm_count(c.device) * 2);
-    softmax_ce_kernel<<<grid, 512, smem, c.stream>>>(logits, rows, V, bias, target, gscale, logp_sum, write_grad ? 1 : 0);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((softmax_ce_kernel), grid, 512, smem, c.stream, logits, rows, V, bias, target, gscale, logp_sum, write_grad ? 1 : 0);
     return TS2_OK;
 }
 

@@ -35,6 +35,7 @@ static int grid_for(const Ctx &c, long long warp_items)
 __global__ void moe_route_kernel(const float *__restrict__ logits, int ld, int T, int E, int k, int *__restrict__ ids,
                                  float *__restrict__ weights)
 {
+    grid_dep_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T)
         return;
@@ -74,8 +75,7 @@ int moe_route(const Ctx &c, const float *logits, int ld, int T, int E, int k, in
 {
     if (k < 1 || k > 8 || E < k || E > 128)
         return fail(TS2_ERR_UNSUPPORTED, "moe_route: need 1 <= selected <= 8 and selected <= experts <= 128 (got %d of %d)", k, E);
-    moe_route_kernel<<<(T + 127) / 128, 128, 0, c.stream>>>(logits, ld, T, E, k, ids, weights);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((moe_route_kernel), (T + 127) / 128, 128, 0, c.stream, logits, ld, T, E, k, ids, weights);
     return TS2_OK;
 }
 
@@ -83,6 +83,7 @@ int moe_route(const Ctx &c, const float *logits, int ld, int T, int E, int k, in
 // slot tables in three steps: per-block histograms, one-block scan, in-order assignment
 __global__ void moe_count_kernel(const int *__restrict__ ids, int n_pairs, int k, int E, int *__restrict__ hist)
 {
+    grid_dep_wait();
     extern __shared__ int sh[];
     for (int e = threadIdx.x; e < E; e += blockDim.x)
         sh[e] = 0;
@@ -101,6 +102,7 @@ __global__ void moe_scan_kernel(const int *__restrict__ hist, int n_blocks, int 
                                 int *__restrict__ block_base, int *__restrict__ tile_group, int *__restrict__ token_of,
                                 int *__restrict__ counts)
 {
+    grid_dep_wait();
     __shared__ int total[128], start[129];
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         int run = 0;
@@ -143,6 +145,7 @@ __global__ void moe_assign_kernel(const int *__restrict__ ids, const float *__re
                                   const int *__restrict__ block_base, int *__restrict__ slot_of, int *__restrict__ token_of,
                                   float *__restrict__ weight_of)
 {
+    grid_dep_wait();
     // thread e walks the block's (token, choice) pairs in order and hands out expert e's slots
     const int p0 = blockIdx.x * ROUTE_BLOCK * k, p1 = min(n_pairs, p0 + ROUTE_BLOCK * k);
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
@@ -162,13 +165,11 @@ int moe_build_slots(const Ctx &c, const int *ids, const float *weights, int T, i
                     int *block_base_scratch, int *seg_ptr, int *tile_group, int *slot_of, int *token_of, float *weight_of, int *counts)
 {
     const int n_pairs = T * k, n_blocks = (T + ROUTE_BLOCK - 1) / ROUTE_BLOCK;
-    moe_count_kernel<<<n_blocks, 256, E * sizeof(int), c.stream>>>(ids, n_pairs, k, E, hist_scratch);
-    TS2_CHECK_LAUNCH();
-    moe_scan_kernel<<<1, 1024, 0, c.stream>>>(hist_scratch, n_blocks, E, max_rows, seg_ptr, block_base_scratch, tile_group, token_of,
-                                               counts);
-    TS2_CHECK_LAUNCH();
-    moe_assign_kernel<<<n_blocks, 128, 0, c.stream>>>(ids, weights, n_pairs, k, E, block_base_scratch, slot_of, token_of, weight_of);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((moe_count_kernel), n_blocks, 256, E * sizeof(int), c.stream, ids, n_pairs, k, E, hist_scratch);
+    TS2_LAUNCH((moe_scan_kernel), 1, 1024, 0, c.stream, hist_scratch, n_blocks, E, max_rows, seg_ptr, block_base_scratch, tile_group,
+               token_of, counts);
+    TS2_LAUNCH((moe_assign_kernel), n_blocks, 128, 0, c.stream, ids, weights, n_pairs, k, E, block_base_scratch, slot_of, token_of,
+               weight_of);
     return TS2_OK;
 }
 
@@ -180,6 +181,7 @@ int moe_build_slots(const Ctx &c, const int *ids, const float *weights, int T, i
 __global__ void moe_ep_tables_kernel(const int *__restrict__ seg, const int *__restrict__ valid, int E, int max_rows,
                                      int *__restrict__ tile_group, int *__restrict__ token_of)
 {
+    grid_dep_wait();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= max_rows)
         return;
@@ -196,14 +198,14 @@ __global__ void moe_ep_tables_kernel(const int *__restrict__ seg, const int *__r
 
 int moe_ep_tables(const Ctx &c, const int *seg, const int *valid, int E, int max_rows, int *tile_group, int *token_of)
 {
-    moe_ep_tables_kernel<<<(max_rows + 255) / 256, 256, 0, c.stream>>>(seg, valid, E, max_rows, tile_group, token_of);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((moe_ep_tables_kernel), (max_rows + 255) / 256, 256, 0, c.stream, seg, valid, E, max_rows, tile_group, token_of);
     return TS2_OK;
 }
 
 // zeroes the padding rows of a received buffer (a contraction over an expert's segment reads them)
 __global__ void moe_zero_pad_rows_kernel(uint8_t *__restrict__ buf, int row_bytes, const int *__restrict__ seg, const int *__restrict__ valid)
 {
+    grid_dep_wait();
     const int e = blockIdx.x;
     const int r0 = seg[e] + valid[e], r1 = seg[e + 1];
     const long long chunks = (long long)(r1 - r0) * (row_bytes / 16);
@@ -216,8 +218,7 @@ int moe_zero_pad_rows(const Ctx &c, void *buf, int row_bytes, const int *seg, co
 {
     if (row_bytes % 16)
         return fail(TS2_ERR_INVALID_ARG, "moe_zero_pad_rows: row size must be a multiple of 16 bytes");
-    moe_zero_pad_rows_kernel<<<E, 256, 0, c.stream>>>((uint8_t *)buf, row_bytes, seg, valid);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((moe_zero_pad_rows_kernel), E, 256, 0, c.stream, (uint8_t *)buf, row_bytes, seg, valid);
     return TS2_OK;
 }
 
@@ -233,6 +234,7 @@ template <int V>
 __global__ void __launch_bounds__(256) moe_pull_rows_kernel(const int4 *__restrict__ moves, int n_moves, uint8_t *const *__restrict__ bases,
                                                             uint8_t *__restrict__ local, int row_bytes, int to_owner)
 {
+    grid_dep_wait();
     __shared__ int first_chunk[PULL_MAX_MOVES + 1];
     using VT = typename std::conditional<V == 16, uint4, uint32_t>::type;
     if (threadIdx.x == 0) {
@@ -283,10 +285,10 @@ int moe_pull_rows(const Ctx &c, const int4 *moves, int n_moves, uint8_t *const *
     const long long chunks = total_bytes / PULL_CHUNK + n_moves;
     const int grid = (int)std::max<long long>(1, std::min<long long>(chunks, (long long)sm_count(c.device) * 8));
     if (row_bytes % 16 == 0)
-        moe_pull_rows_kernel<16><<<grid, 256, 0, c.stream>>>(moves, n_moves, bases, (uint8_t *)local, row_bytes, to_owner ? 1 : 0);
+        TS2_LAUNCH((moe_pull_rows_kernel<16>), grid, 256, 0, c.stream, moves, n_moves, bases, (uint8_t *)local, row_bytes,
+                   to_owner ? 1 : 0);
     else
-        moe_pull_rows_kernel<4><<<grid, 256, 0, c.stream>>>(moves, n_moves, bases, (uint8_t *)local, row_bytes, to_owner ? 1 : 0);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((moe_pull_rows_kernel<4>), grid, 256, 0, c.stream, moves, n_moves, bases, (uint8_t *)local, row_bytes, to_owner ? 1 : 0);
     return TS2_OK;
 }
 
@@ -295,6 +297,7 @@ int moe_pull_rows(const Ctx &c, const int4 *moves, int n_moves, uint8_t *const *
 __global__ void moe_gather_rows_kernel(const uint8_t *__restrict__ src, const int *__restrict__ token_of, int rows, int row_bytes,
                                        uint8_t *__restrict__ dst)
 {
+    grid_dep_wait();
     const int chunks = row_bytes / 16;
     const long long total = (long long)rows * chunks;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -313,8 +316,8 @@ int moe_gather_rows(const Ctx &c, const void *src, const int *token_of, int rows
         return fail(TS2_ERR_INVALID_ARG, "moe_gather_rows: row size must be a multiple of 16 bytes");
     const long long total = (long long)rows * (row_bytes / 16);
     const int grid = (int)std::min<long long>(ceil_div(total, 256), (long long)sm_count(c.device) * 8);
-    moe_gather_rows_kernel<<<std::max(grid, 1), 256, 0, c.stream>>>((const uint8_t *)src, token_of, rows, row_bytes, (uint8_t *)dst);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((moe_gather_rows_kernel), std::max(grid, 1), 256, 0, c.stream, (const uint8_t *)src, token_of, rows, row_bytes,
+               (uint8_t *)dst);
     return TS2_OK;
 }
 
@@ -325,6 +328,7 @@ __global__ void moe_act_forward_kernel(const __half *__restrict__ cat, const int
                                        const float *__restrict__ weight_of, int rows, int X, float s_act, __half *__restrict__ what,
                                        float *__restrict__ wscale, void *__restrict__ rg)
 {
+    grid_dep_wait();
     const int tiles = X / TILE;
     WARP_ITEM_LOOP((long long)rows * tiles)
     {
@@ -352,10 +356,9 @@ int moe_act_forward(const Ctx &c, const __half *cat, const int *token_of, const 
 {
     const int grid = grid_for(c, (long long)rows * (X / TILE));
     if (c.ft == 0)
-        moe_act_forward_kernel<0><<<grid, THREADS, 0, c.stream>>>(cat, token_of, weight_of, rows, X, c.s_act, what, wscale, rg);
+        TS2_LAUNCH((moe_act_forward_kernel<0>), grid, THREADS, 0, c.stream, cat, token_of, weight_of, rows, X, c.s_act, what, wscale, rg);
     else
-        moe_act_forward_kernel<1><<<grid, THREADS, 0, c.stream>>>(cat, token_of, weight_of, rows, X, c.s_act, what, wscale, rg);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((moe_act_forward_kernel<1>), grid, THREADS, 0, c.stream, cat, token_of, weight_of, rows, X, c.s_act, what, wscale, rg);
     return TS2_OK;
 }
 
@@ -367,6 +370,7 @@ __global__ void moe_act_backward_kernel(const __half *__restrict__ drg, const __
                                         const float *__restrict__ weight_of, int rows, int X, void *__restrict__ dcat,
                                         float *__restrict__ dmoe_part)
 {
+    grid_dep_wait();
     const int tiles = X / TILE;
     WARP_ITEM_LOOP((long long)rows * tiles)
     {
@@ -403,10 +407,11 @@ int moe_act_backward(const Ctx &c, const __half *drg, const __half *cat, const _
 {
     const int grid = grid_for(c, (long long)rows * (X / TILE));
     if (c.ft == 0)
-        moe_act_backward_kernel<0><<<grid, THREADS, 0, c.stream>>>(drg, cat, what, wscale, token_of, weight_of, rows, X, dcat, dmoe_part);
+        TS2_LAUNCH((moe_act_backward_kernel<0>), grid, THREADS, 0, c.stream, drg, cat, what, wscale, token_of, weight_of, rows, X, dcat,
+                   dmoe_part);
     else
-        moe_act_backward_kernel<1><<<grid, THREADS, 0, c.stream>>>(drg, cat, what, wscale, token_of, weight_of, rows, X, dcat, dmoe_part);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((moe_act_backward_kernel<1>), grid, THREADS, 0, c.stream, drg, cat, what, wscale, token_of, weight_of, rows, X, dcat,
+                   dmoe_part);
     return TS2_OK;
 }
 
@@ -415,6 +420,7 @@ int moe_act_backward(const Ctx &c, const __half *drg, const __half *cat, const _
 __global__ void moe_combine_kernel(const float *__restrict__ y, const int *__restrict__ slot_of, int T, int k, int D,
                                    const float *__restrict__ in, float *__restrict__ out)
 {
+    grid_dep_wait();
     const int tiles = D / TILE;
     WARP_ITEM_LOOP((long long)T * tiles)
     {
@@ -433,6 +439,7 @@ __global__ void moe_combine_kernel(const float *__restrict__ y, const int *__res
 __global__ void moe_combine_half_kernel(const __half *__restrict__ y, const int *__restrict__ slot_of, int T, int k, int D,
                                         const float *__restrict__ in, float *__restrict__ out)
 {
+    grid_dep_wait();
     const int tiles = D / TILE;
     WARP_ITEM_LOOP((long long)T * tiles)
     {
@@ -449,15 +456,13 @@ __global__ void moe_combine_half_kernel(const __half *__restrict__ y, const int 
 
 int moe_combine_half(const Ctx &c, const __half *y, const int *slot_of, int T, int k, int D, const float *in, float *out)
 {
-    moe_combine_half_kernel<<<grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream>>>(y, slot_of, T, k, D, in, out);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((moe_combine_half_kernel), grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream, y, slot_of, T, k, D, in, out);
     return TS2_OK;
 }
 
 int moe_combine(const Ctx &c, const float *y, const int *slot_of, int T, int k, int D, const float *in, float *out)
 {
-    moe_combine_kernel<<<grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream>>>(y, slot_of, T, k, D, in, out);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((moe_combine_kernel), grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream, y, slot_of, T, k, D, in, out);
     return TS2_OK;
 }
 
@@ -469,6 +474,7 @@ __global__ void moe_router_backward_kernel(const float *__restrict__ dmoe_part, 
                                            const float *__restrict__ weights, const int *__restrict__ slot_of, int T, int k, int E,
                                            int ld, void *__restrict__ dl)
 {
+    grid_dep_wait();
     using QT = typename std::conditional<FT == 0, __nv_fp8_e4m3, __half>::type;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T)
@@ -495,10 +501,11 @@ int moe_router_backward(const Ctx &c, const float *dmoe_part, int tiles, const i
                         int k, int E, int ld, void *dl)
 {
     if (c.ft == 0)
-        moe_router_backward_kernel<0><<<(T + 127) / 128, 128, 0, c.stream>>>(dmoe_part, tiles, ids, weights, slot_of, T, k, E, ld, dl);
+        TS2_LAUNCH((moe_router_backward_kernel<0>), (T + 127) / 128, 128, 0, c.stream, dmoe_part, tiles, ids, weights, slot_of, T, k, E,
+                   ld, dl);
     else
-        moe_router_backward_kernel<1><<<(T + 127) / 128, 128, 0, c.stream>>>(dmoe_part, tiles, ids, weights, slot_of, T, k, E, ld, dl);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((moe_router_backward_kernel<1>), (T + 127) / 128, 128, 0, c.stream, dmoe_part, tiles, ids, weights, slot_of, T, k, E,
+                   ld, dl);
     return TS2_OK;
 }
 

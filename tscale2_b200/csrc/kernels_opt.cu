@@ -13,6 +13,7 @@ static constexpr int THREADS = WARPS * 32;
 
 __global__ void fill_vector_kernel(float *dst, int n, float value, const float *dyn, int reciprocal)
 {
+    grid_dep_wait();
     float v = value;
     if (dyn)
         v = reciprocal ? value / *dyn : value * *dyn;
@@ -57,6 +58,7 @@ __device__ __forceinline__ void seg_row_cols(const OptSeg &sg, int r, long long 
 __global__ void opt_row_sum2_kernel(const OptSeg *__restrict__ segs, int nseg, int nitems, const float *__restrict__ grad,
                                     float *__restrict__ rowsum)
 {
+    grid_dep_wait();
     const int lane = threadIdx.x & 31;
     for (int item = blockIdx.x * WARPS + (threadIdx.x >> 5); item < nitems; item += gridDim.x * WARPS) {
         const OptSeg sg = segs[find_seg(segs, nseg, item)];
@@ -80,6 +82,7 @@ __global__ void opt_row_sum2_kernel(const OptSeg *__restrict__ segs, int nseg, i
 __global__ void opt_disp_kernel(const OptMat *__restrict__ mats, const float *__restrict__ rowsum, float disp_decay,
                                 float *__restrict__ row_scale)
 {
+    grid_dep_wait();
     __shared__ float red[32];
     __shared__ float bcast;
     const OptMat mt = mats[blockIdx.x];
@@ -131,6 +134,7 @@ __global__ void opt_update_kernel(const OptSeg *__restrict__ segs, int nseg, int
                                   const float *__restrict__ row_scale, ts2_training_step step, float *__restrict__ avg,
                                   float *__restrict__ w, double *__restrict__ roww2)
 {
+    grid_dep_wait();
     const int lane = threadIdx.x & 31;
     for (int item = blockIdx.x * WARPS + (threadIdx.x >> 5); item < nitems; item += gridDim.x * WARPS) {
         const OptSeg sg = segs[find_seg(segs, nseg, item)];
@@ -179,6 +183,7 @@ __global__ void opt_update_kernel(const OptSeg *__restrict__ segs, int nseg, int
 // one block per matrix: sko = sqrt(sum of squares / (x y)), rows summed in a fixed order
 __global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__restrict__ roww2, float *__restrict__ skos)
 {
+    grid_dep_wait();
     __shared__ double red[32];
     const OptMat mt = mats[blockIdx.x];
     double s = 0.0;
@@ -201,6 +206,7 @@ __global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__
 __global__ void opt_quant_kernel(const OptSeg *__restrict__ segs, int nseg, int nitems, const float *__restrict__ w,
                                  const float *__restrict__ skos)
 {
+    grid_dep_wait();
     const int lane = threadIdx.x & 31;
     for (int item = blockIdx.x * WARPS + (threadIdx.x >> 5); item < nitems; item += gridDim.x * WARPS) {
         const OptSeg sg = segs[find_seg(segs, nseg, item)];
@@ -239,15 +245,13 @@ int opt_row_sum2(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const f
 {
     if (nitems <= 0)
         return TS2_OK;
-    opt_row_sum2_kernel<<<opt_grid(c, nitems), THREADS, 0, c.stream>>>(segs, nseg, nitems, grad, rowsum);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((opt_row_sum2_kernel), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, nitems, grad, rowsum);
     return TS2_OK;
 }
 
 int opt_disp(const Ctx &c, const OptMat *mats, int n_mats, const float *rowsum, float disp_decay, float *row_scale)
 {
-    opt_disp_kernel<<<n_mats, 1024, 0, c.stream>>>(mats, rowsum, disp_decay, row_scale);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((opt_disp_kernel), n_mats, 1024, 0, c.stream, mats, rowsum, disp_decay, row_scale);
     return TS2_OK;
 }
 
@@ -257,18 +261,17 @@ int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const flo
     if (nitems <= 0)
         return TS2_OK;
     if (step)
-        opt_update_kernel<true><<<opt_grid(c, nitems), THREADS, 0, c.stream>>>(segs, nseg, nitems, grad, row_scale, *step, avg, w, roww2);
+        TS2_LAUNCH((opt_update_kernel<true>), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, nitems, grad, row_scale, *step, avg,
+                   w, roww2);
     else
-        opt_update_kernel<false><<<opt_grid(c, nitems), THREADS, 0, c.stream>>>(segs, nseg, nitems, nullptr, nullptr, ts2_training_step(),
-                                                                                 nullptr, w, roww2);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((opt_update_kernel<false>), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, nitems, nullptr, nullptr,
+                   ts2_training_step(), nullptr, w, roww2);
     return TS2_OK;
 }
 
 int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos)
 {
-    opt_sko_kernel<<<n_mats, 1024, 0, c.stream>>>(mats, roww2, skos);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((opt_sko_kernel), n_mats, 1024, 0, c.stream, mats, roww2, skos);
     return TS2_OK;
 }
 
@@ -276,8 +279,7 @@ int opt_quantize(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const f
 {
     if (nitems <= 0)
         return TS2_OK;
-    opt_quant_kernel<<<opt_grid(c, nitems), THREADS, 0, c.stream>>>(segs, nseg, nitems, w, skos);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((opt_quant_kernel), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, nitems, w, skos);
     return TS2_OK;
 }
 
@@ -288,6 +290,7 @@ template <int ES, int TH>
 __global__ void qcopy_kernel(const void *__restrict__ src, long long x, long long y, long long ld_src, void *__restrict__ dst,
                              long long ld, void *__restrict__ dstT, long long ldT)
 {
+    grid_dep_wait();
     using QT = typename std::conditional<ES == 1, uint8_t, uint16_t>::type;
     using TT = typename std::conditional<TH != 0, uint16_t, QT>::type;
     __shared__ QT tile[32][33];
@@ -326,14 +329,13 @@ int qcopy_block(const Ctx &c, const void *src, int64_t x, int64_t y, int64_t ld_
 {
     dim3 g((unsigned)ceil_div(x, 32), (unsigned)ceil_div(y, 32)), b(32, 8);
     if (elem_size == 1 && transposed_as_half == 1)
-        qcopy_kernel<1, 1><<<g, b, 0, c.stream>>>(src, x, y, ld_src, dst, ld, dstT, ldT);
+        TS2_LAUNCH((qcopy_kernel<1, 1>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
     else if (elem_size == 1 && transposed_as_half == 2)
-        qcopy_kernel<1, 2><<<g, b, 0, c.stream>>>(src, x, y, ld_src, dst, ld, dstT, ldT);
+        TS2_LAUNCH((qcopy_kernel<1, 2>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
     else if (elem_size == 1)
-        qcopy_kernel<1, 0><<<g, b, 0, c.stream>>>(src, x, y, ld_src, dst, ld, dstT, ldT);
+        TS2_LAUNCH((qcopy_kernel<1, 0>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
     else
-        qcopy_kernel<2, 0><<<g, b, 0, c.stream>>>(src, x, y, ld_src, dst, ld, dstT, ldT);
-    TS2_CHECK_LAUNCH();
+        TS2_LAUNCH((qcopy_kernel<2, 0>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
     return TS2_OK;
 }
 
@@ -343,6 +345,7 @@ int qcopy_block(const Ctx &c, const void *src, int64_t x, int64_t y, int64_t ld_
 __global__ void layer_scales_kernel(float *__restrict__ fwd_col, float *__restrict__ bwd_row, int W, int ncat, int is_att, float a,
                                     const float *__restrict__ skos)
 {
+    grid_dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncat * W; i += gridDim.x * blockDim.x) {
         const int j = i / W;
         fwd_col[i] = (is_att && j == 1) ? a * skos[1] : a;
@@ -353,16 +356,15 @@ __global__ void layer_scales_kernel(float *__restrict__ fwd_col, float *__restri
 
 int layer_scales(const Ctx &c, float *fwd_col, float *bwd_row, int W, int ncat, bool is_att, float a, const float *skos)
 {
-    layer_scales_kernel<<<std::max(1, std::min(64, (ncat * W + 255) / 256)), 256, 0, c.stream>>>(fwd_col, bwd_row, W, ncat, is_att ? 1 : 0,
-                                                                                              a, skos);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((layer_scales_kernel), std::max(1, std::min(64, (ncat * W + 255) / 256)), 256, 0, c.stream, fwd_col, bwd_row, W, ncat,
+               is_att ? 1 : 0, a, skos);
     return TS2_OK;
 }
 
 int fill_vector(const Ctx &c, float *dst, int n, float value, const float *dyn, bool reciprocal_dyn)
 {
-    fill_vector_kernel<<<std::max(1, std::min(64, (n + 255) / 256)), 256, 0, c.stream>>>(dst, n, value, dyn, reciprocal_dyn ? 1 : 0);
-    TS2_CHECK_LAUNCH();
+    TS2_LAUNCH((fill_vector_kernel), std::max(1, std::min(64, (n + 255) / 256)), 256, 0, c.stream, dst, n, value, dyn,
+               reciprocal_dyn ? 1 : 0);
     return TS2_OK;
 }
 
