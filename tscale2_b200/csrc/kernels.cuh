@@ -33,6 +33,13 @@ enum {
     BATCH_BAD_LABEL_PTR = 6, // where = node
     BATCH_BAD_LABEL = 7,     // where = entry of label_arr, details = label, node
 };
+// what the host wants to know when it waits, in pinned host memory
+struct HostReport {
+    int32_t device_status, static_status; // the device's status words (common.cuh)
+    int batch[4];                         // {code, where, detail, detail} of the first malformed batch element
+    float scalar;
+};
+int queue_report(const Ctx &c, const int *batch_status, const float *scalar, HostReport *report);
 // per-node span tables from the CSR form (at most one span per node), and per key the range [rev_first, rev_last] of
 // nodes that may attend to it ((T, -1) = none; a superset, the kernels test each node's own span).
 // scan_tmp: batch_scan_tmp_elems(T) ints.

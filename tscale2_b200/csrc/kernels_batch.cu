@@ -30,6 +30,18 @@ __device__ __forceinline__ void batch_fail(int *status, int code, int where, int
     }
 }
 
+// ---- what a waiting host reads ---------------------------------------------------------
+__global__ void report_kernel(const int32_t *device_status, const int32_t *static_status, const int *batch_status, const float *scalar,
+                              HostReport *report)
+{
+    grid_dep_wait();
+    report->device_status = device_status ? *device_status : 0;
+    report->static_status = static_status ? *static_status : 0;
+    for (int i = 0; i < 4; ++i)
+        report->batch[i] = batch_status[i];
+    report->scalar = scalar ? *scalar : 0.f;
+}
+
 // ---- spans ---------------------------------------------------------------------------
 __global__ void span_expand_kernel(const int *__restrict__ span_ptr, const int *__restrict__ csr_start, const int *__restrict__ csr_finish,
                                    int T, int n_spans, int *__restrict__ start, int *__restrict__ finish, int *status)
@@ -446,6 +458,13 @@ int blocks_for(long long n)
 }
 
 } // namespace
+
+int queue_report(const Ctx &c, const int *batch_status, const float *scalar, HostReport *report)
+{
+    TS2_LAUNCH((report_kernel), 1, 1, 0, c.stream, device_status_word(c.device), static_status_word_if_ready(c.device), batch_status, scalar,
+               report);
+    return TS2_OK;
+}
 
 int batch_span_tables(const Ctx &c, const int *span_ptr, const int *csr_start, const int *csr_finish, int T, int n_spans, int *start,
                       int *finish, int *scan_tmp, int *rev_first, int *rev_last, int *status)

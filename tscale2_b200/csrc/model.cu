@@ -214,7 +214,8 @@ struct ts2_model {
     BatchDev batch;
     void *pinned = nullptr;
     size_t pinned_bytes = 0;
-    int *h_batch_status = nullptr; // pinned copy of batch.status, refreshed by every ts2_set_batch
+    HostReport *report = nullptr;  // pinned; written by the kernel that every wait queues (queue_report)
+    bool unreported = false;       // work was queued since the last wait
     bool grads_dirty = false; // the flat gradient holds an accumulated, not yet applied gradient
     bool reduce_in_backward = false; // this backward pass is followed by apply(): all-reduce every layer's gradient as soon as it is complete
     int gemm_tag = 0; // class of the contractions being queued (timing statistics)
@@ -1040,10 +1041,10 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
     }
     M_TRY(dalloc(m, &b.ix.hist, label_index_hist_elems(b.label_cap)));
     M_TRY(dalloc(m, &b.ix.partial, label_index_partial_elems(b.label_cap, D)));
-    m->pinned_bytes = 2 * b.raw_cap * 4 + 16;
+    m->pinned_bytes = 2 * b.raw_cap * 4 + sizeof(HostReport);
     TS2_CUDA(cudaMallocHost(&m->pinned, m->pinned_bytes));
-    m->h_batch_status = (int *)((uint32_t *)m->pinned + 2 * b.raw_cap);
-    memset(m->h_batch_status, 0, 16);
+    m->report = (HostReport *)((uint32_t *)m->pinned + 2 * b.raw_cap);
+    memset(m->report, 0, sizeof(HostReport));
     for (int i = 0; i < 2; ++i)
         TS2_CUDA(cudaEventCreateWithFlags(&b.slot_ev[i], cudaEventDisableTiming));
 
@@ -1697,7 +1698,6 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
         M_TRY(batch_span_tables(c, (const int *)b.raw + o_ptr[a], (const int *)b.raw + o_start[a], (const int *)b.raw + o_finish[a], T,
                                 n_spans[a], b.span_start[a], b.span_finish[a], b.scan_tmp, b.rev_first[a], b.rev_last[a], b.status));
     M_TRY(batch_targets(c, (const int *)b.raw + o_tnode, (const int *)b.raw + o_tid, n_targets, T, m->V, b.target, b.status));
-    TS2_CUDA(cudaMemcpyAsync(m->h_batch_status, b.status, 16, cudaMemcpyDeviceToHost, s));
     b.node_count = T;
     b.target_count = n_targets;
     return TS2_OK;
@@ -1706,8 +1706,8 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
 // what the device found wrong with a batch, if anything; clears the record
 int report_batch_status(ts2_model *m)
 {
-    int *h = m->h_batch_status;
-    if (!h || h[0] == BATCH_OK)
+    int *h = m->report->batch;
+    if (h[0] == BATCH_OK)
         return TS2_OK;
     const int code = h[0], where = h[1], d0 = h[2], d1 = h[3];
     h[0] = BATCH_OK;
@@ -1731,21 +1731,37 @@ int report_batch_status(ts2_model *m)
     return fail(TS2_ERR_INVALID_ARG, "batch: malformed (code %d)", code);
 }
 
-int wait_stream(ts2_model *m)
+// bounded wait: poll the stream for up to 120 s of wall time, then report a timeout
+int poll_stream(ts2_model *m)
 {
-    // bounded wait: poll the stream for up to 120 s of wall time, then report a timeout
     cudaError_t e;
     const auto t0 = std::chrono::steady_clock::now();
     while ((e = cudaStreamQuery(m->stream)) == cudaErrorNotReady) {
-        if (std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > 120.0)
+        const double waited = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        if (waited > 120.0)
             return fail(TS2_ERR_TIMEOUT, "the device did not finish within 120 s");
-        if (std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > 0.002)
+        if (waited > 0.02) // a sleep takes 100 us with the kernel's timer slack: not worth it in steps of a few ms
             std::this_thread::sleep_for(std::chrono::microseconds(50));
     }
     if (e != cudaSuccess)
         return fail(TS2_ERR_CUDA, "stream failed: %s", cudaGetErrorString(e));
-    M_TRY(collect_device_status(m->device));
-    return report_batch_status(m);
+    return TS2_OK;
+}
+
+// Waits for everything queued and reports what the device recorded.  One small kernel at the end of the queue writes the
+// status words, the batch record and, if asked for, a scalar into pinned memory, so that a wait needs no copy of its
+// own: three blocking 4-byte copies after the stream had drained took as long as several kernels of a small step.
+int wait_stream(ts2_model *m, const float *scalar = nullptr, float *value = nullptr)
+{
+    M_TRY(queue_report(ctx_of(m), m->batch.status, scalar, m->report));
+    M_TRY(poll_stream(m));
+    m->unreported = false;
+    if (m->report->device_status | m->report->static_status)
+        M_TRY(collect_device_status(m->device)); // clears the words and reports them
+    M_TRY(report_batch_status(m));
+    if (value)
+        *value = m->report->scalar;
+    return TS2_OK;
 }
 
 } // namespace
@@ -1887,8 +1903,11 @@ int ts2_set_batch(ts2_model *m, const ts2_batch_nodes *nodes)
     if (!m || !nodes)
         return fail(TS2_ERR_INVALID_ARG, "null argument");
     TS2_CUDA(cudaSetDevice(m->device));
-    // the staging buffer is reused: the previous copy must have left it
-    M_TRY(wait_stream(m));
+    // The batch queues up behind the step that is running (stage_batch waits only for a staging slot, two batches back),
+    // so the device does not idle between steps while the host prepares the next one.  A step that is over is reported.
+    if (m->unreported && cudaStreamQuery(m->stream) == cudaSuccess)
+        M_TRY(wait_stream(m));
+    m->unreported = true;
     M_TRY(stage_batch(m, nodes));
     return TS2_OK;
 }
@@ -1900,6 +1919,7 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
     if (m->batch.node_count <= 0)
         return mfail(m, fail(TS2_ERR_INVALID_ARG, "ts2_backprop before ts2_set_batch"));
     TS2_CUDA(cudaSetDevice(m->device));
+    m->unreported = true;
     TS2_CUDA(cudaEventRecord(m->ev_start, m->stream));
     ++m->step_no;
     m->logp = m->logp_ring + m->step_no % ts2_model::LOSS_RING; // final_layer() clears and fills this step's slot
@@ -1960,9 +1980,8 @@ int ts2_forward_score(ts2_model *m, float *out_score)
     m->trace_on = tr;
     if (rc != TS2_OK)
         return rc;
-    M_TRY(wait_stream(m));
     float s = 0;
-    TS2_CUDA(cudaMemcpy(&s, score_slot, 4, cudaMemcpyDeviceToHost));
+    M_TRY(wait_stream(m, score_slot, &s));
     *out_score = m->batch.target_count ? s / m->batch.target_count : 0.f;
     return TS2_OK;
 }
@@ -1972,9 +1991,8 @@ int ts2_avg_train_err(ts2_model *m, float *out_err)
     if (!m || !out_err)
         return fail(TS2_ERR_INVALID_ARG, "null argument");
     TS2_CUDA(cudaSetDevice(m->device));
-    M_TRY(wait_stream(m));
     float s = 0;
-    TS2_CUDA(cudaMemcpy(&s, m->logp, 4, cudaMemcpyDeviceToHost));
+    M_TRY(wait_stream(m, m->logp, &s));
     *out_err = m->last_targets ? -s / m->last_targets : 0.f;
     return TS2_OK;
 }
@@ -1987,15 +2005,35 @@ int ts2_get_params(ts2_model *m, int what, ts2_matrix_view *mats_out, int n_mats
     if (what != TS2_PARAM_GRADIENT)
         M_TRY(sync_master(m));
     M_TRY(wait_stream(m));
+    // matrices that follow one another on both sides leave in one copy, all copies are queued before any is waited for
+    const float *src0 = nullptr;
+    float *dst0 = nullptr;
+    size_t run = 0;
+    auto flush = [&]() {
+        const cudaError_t e = run ? cudaMemcpyAsync(dst0, src0, run * 4, cudaMemcpyDeviceToHost, m->stream) : cudaSuccess;
+        run = 0;
+        return e;
+    };
     for (int i = 0; i < n_mats; ++i) {
         Matrix &mt = m->mats[i];
         if (!mats_out[i].data)
             continue;
-        if (mats_out[i].x_size != mt.x || mats_out[i].y_size != mt.y)
+        if (mats_out[i].x_size != mt.x || mats_out[i].y_size != mt.y) {
+            cudaStreamSynchronize(m->stream); // earlier matrices may be on their way
             return mfail(m, fail(TS2_ERR_INVALID_ARG, "matrix %d: shape mismatch", i));
+        }
         const float *src = what == TS2_PARAM_WEIGHTS ? mt.w : what == TS2_PARAM_MOMENTUM ? mt.avg : mt.grad;
-        TS2_CUDA(cudaMemcpy(mats_out[i].data, src, (size_t)mt.x * mt.y * 4, cudaMemcpyDeviceToHost));
+        const size_t n = (size_t)mt.x * mt.y;
+        if (run && (src != src0 + run || mats_out[i].data != dst0 + run))
+            TS2_CUDA(flush());
+        if (!run) {
+            src0 = src;
+            dst0 = mats_out[i].data;
+        }
+        run += n;
     }
+    TS2_CUDA(flush());
+    M_TRY(poll_stream(m));
     return TS2_OK;
 }
 
