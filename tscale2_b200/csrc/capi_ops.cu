@@ -35,7 +35,11 @@ int ts2_dev_alloc(int device, size_t bytes, void **ptr)
     if (!ptr)
         return fail(TS2_ERR_INVALID_ARG, "ts2_dev_alloc: null out pointer");
     TS2_CUDA(cudaSetDevice(device));
-    TS2_CUDA(cudaMalloc(ptr, bytes ? bytes : 16));
+    if (cudaMalloc(ptr, bytes ? bytes : 16) != cudaSuccess) {
+        cudaGetLastError();
+        scratch_trim(device);
+        TS2_CUDA(cudaMalloc(ptr, bytes ? bytes : 16));
+    }
     return TS2_OK;
 }
 
@@ -122,15 +126,16 @@ int ts2_gemm_tn(int device, void *stream, int prec, int out_kind, int64_t M, int
     a.epi.out_kind = out_kind;
     if (gemm_splits(device, a.kind, false, M, N, K) > 1) {
         // few output tiles and a long K: the scheduler splits K and needs scratch for the partial
-        // tiles; this entry point takes it from the stream-ordered allocator for the call.
+        // tiles; this entry point takes it from the library's stream-ordered scratch pool for the call.
         size_t need = gemm_workspace_bytes(device, a.kind, false, M, N, K);
         void *ws = nullptr;
         TS2_CUDA(cudaSetDevice(device));
-        TS2_CUDA(cudaMallocAsync(&ws, need, a.stream));
+        if (int rc = scratch_alloc(device, need, a.stream, &ws))
+            return rc;
         a.workspace = ws;
         a.workspace_bytes = need;
         int rc = gemm(a);
-        cudaFreeAsync(ws, a.stream);
+        scratch_free(a.stream, ws);
         return rc;
     }
     return gemm(a);
@@ -319,6 +324,32 @@ int ts2_op_rowquant_i8(int device, void *stream, const float *x, int T, int D, i
     return rowquant_grad(op_ctx(device, stream, TS2_PREC_INT8), x, T, D, nullptr, q, row_scale, nullptr, nullptr, 1.f, nullptr, nullptr);
 }
 
+// device copies of a call's host span arrays (start at d, finish at d + T) and whatever scratch follows them
+struct SpanScratch {
+    int *d = nullptr;
+    int rc = TS2_OK;
+    cudaStream_t stream;
+    SpanScratch(const Ctx &c, const int32_t *start, const int32_t *finish, int T, size_t elems) : stream(c.stream)
+    {
+        rc = fill(c, start, finish, T, elems);
+    }
+    int fill(const Ctx &c, const int32_t *start, const int32_t *finish, int T, size_t elems)
+    {
+        if (int r = scratch_alloc(c.device, elems * 4, stream, (void **)&d))
+            return r;
+        TS2_CUDA(cudaMemcpyAsync(d, start, (size_t)T * 4, cudaMemcpyHostToDevice, stream));
+        TS2_CUDA(cudaMemcpyAsync(d + T, finish, (size_t)T * 4, cudaMemcpyHostToDevice, stream));
+        return TS2_OK;
+    }
+    ~SpanScratch()
+    {
+        if (d)
+            scratch_free(stream, d);
+    }
+    SpanScratch(const SpanScratch &) = delete;
+    SpanScratch &operator=(const SpanScratch &) = delete;
+};
+
 // attention core on device arrays; span_start / span_finish are host arrays of T ints
 int ts2_attention_forward(int device, void *stream, int variant, const void *q, const void *k, const void *v, const int32_t *span_start,
                           const int32_t *span_finish, int T, int head_count, float alibi_slope, void *o, float *lse)
@@ -326,13 +357,13 @@ int ts2_attention_forward(int device, void *stream, int variant, const void *q, 
     if (T <= 0 || head_count <= 0 || !q || !k || !v || !o || !lse || !span_start || !span_finish)
         return fail(TS2_ERR_INVALID_ARG, "ts2_attention_forward: bad arguments");
     TS2_CUDA(cudaSetDevice(device));
-    int *d = nullptr;
-    TS2_CUDA(cudaMalloc(&d, (size_t)T * 8));
-    TS2_CUDA(cudaMemcpy(d, span_start, (size_t)T * 4, cudaMemcpyHostToDevice));
-    TS2_CUDA(cudaMemcpy(d + T, span_finish, (size_t)T * 4, cudaMemcpyHostToDevice));
     Ctx c;
     c.device = device;
     c.stream = (cudaStream_t)stream;
+    SpanScratch spans(c, span_start, span_finish, T, 2 * (size_t)T);
+    if (spans.rc != TS2_OK)
+        return spans.rc;
+    int *d = spans.d;
     int rc = variant == 2 ? attention_forward_tc(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,
                                                  alibi_slope, (__half *)o, lse)
              : variant == 0 ? attention_forward_mma(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,
@@ -340,7 +371,6 @@ int ts2_attention_forward(int device, void *stream, int variant, const void *q, 
                             : attention_forward_rowwise(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,
                                                       alibi_slope, (__half *)o, lse);
     cudaStreamSynchronize(c.stream);
-    cudaFree(d);
     return rc;
 }
 
@@ -351,17 +381,16 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
     if (T <= 0 || head_count <= 0 || !q || !k || !v || !dout || !lse || !dscale || !span_start || !span_finish || !dq || !dk || !dv)
         return fail(TS2_ERR_INVALID_ARG, "ts2_attention_backward: bad arguments");
     TS2_CUDA(cudaSetDevice(device));
-    int *d = nullptr; // start | finish | rev_first | rev_last | scan scratch (2T)
-    TS2_CUDA(cudaMalloc(&d, (4 * (size_t)T + batch_scan_tmp_elems(T)) * 4));
-    TS2_CUDA(cudaMemcpy(d, span_start, (size_t)T * 4, cudaMemcpyHostToDevice));
-    TS2_CUDA(cudaMemcpy(d + T, span_finish, (size_t)T * 4, cudaMemcpyHostToDevice));
     Ctx c;
     c.device = device;
     c.stream = (cudaStream_t)stream;
-    if (int rc0 = batch_reverse_ranges(c, d, d + T, T, d + 4 * (size_t)T, d + 2 * (size_t)T, d + 3 * (size_t)T)) {
-        cudaFree(d);
+    // start | finish | rev_first | rev_last | scan scratch
+    SpanScratch spans(c, span_start, span_finish, T, 4 * (size_t)T + batch_scan_tmp_elems(T));
+    if (spans.rc != TS2_OK)
+        return spans.rc;
+    int *d = spans.d;
+    if (int rc0 = batch_reverse_ranges(c, d, d + T, T, d + 4 * (size_t)T, d + 2 * (size_t)T, d + 3 * (size_t)T))
         return rc0;
-    }
     const __half *Q = (const __half *)q, *K = (const __half *)k, *V = (const __half *)v, *DO = (const __half *)dout;
     float *fq = (float *)dq, *fk = (float *)dk, *fv = (float *)dv;
     int rc = variant == 2 || variant == 3
@@ -372,7 +401,6 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
                           : attention_backward_rowwise(c, Q, K, V, DO, lse, dscale, d, d + T, d + 2 * T, d + 3 * T, T, head_count,
                                                        alibi_slope, fq, fk, fv);
     cudaStreamSynchronize(c.stream);
-    cudaFree(d);
     return rc;
 }
 
@@ -382,13 +410,13 @@ int ts2_op_attention_reverse_ranges(int device, void *stream, const int32_t *spa
     if (T <= 0 || !span_start || !span_finish || !rev_first || !rev_last)
         return fail(TS2_ERR_INVALID_ARG, "ts2_op_attention_reverse_ranges: bad arguments");
     TS2_CUDA(cudaSetDevice(device));
-    int *d = nullptr;
-    TS2_CUDA(cudaMalloc(&d, (4 * (size_t)T + batch_scan_tmp_elems(T)) * 4));
-    TS2_CUDA(cudaMemcpy(d, span_start, (size_t)T * 4, cudaMemcpyHostToDevice));
-    TS2_CUDA(cudaMemcpy(d + T, span_finish, (size_t)T * 4, cudaMemcpyHostToDevice));
     Ctx c;
     c.device = device;
     c.stream = (cudaStream_t)stream;
+    SpanScratch spans(c, span_start, span_finish, T, 4 * (size_t)T + batch_scan_tmp_elems(T));
+    if (spans.rc != TS2_OK)
+        return spans.rc;
+    int *d = spans.d;
     int rc = batch_reverse_ranges(c, d, d + T, T, d + 4 * (size_t)T, d + 2 * (size_t)T, d + 3 * (size_t)T);
     if (rc == TS2_OK && cudaStreamSynchronize(c.stream) != cudaSuccess)
         rc = fail(TS2_ERR_CUDA, "ts2_op_attention_reverse_ranges: the stream failed");
@@ -396,7 +424,6 @@ int ts2_op_attention_reverse_ranges(int device, void *stream, const int32_t *spa
         cudaMemcpy(rev_first, d + 2 * (size_t)T, (size_t)T * 4, cudaMemcpyDeviceToHost);
         cudaMemcpy(rev_last, d + 3 * (size_t)T, (size_t)T * 4, cudaMemcpyDeviceToHost);
     }
-    cudaFree(d);
     return rc;
 }
 

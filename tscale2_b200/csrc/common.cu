@@ -101,4 +101,42 @@ int collect_device_status(int device)
     return TS2_OK;
 }
 
+static cudaMemPool_t scratch_pool(int device, bool create)
+{
+    static cudaMemPool_t pools[16] = {};
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaMemPool_t &p = pools[device & 15];
+    if (!p && create) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+            p = nullptr;
+            return nullptr;
+        }
+        uint64_t keep = 64ull << 20;
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    return p;
+}
+
+int scratch_alloc(int device, size_t bytes, cudaStream_t stream, void **ptr)
+{
+    cudaMemPool_t p = scratch_pool(device, true);
+    if (!p)
+        return fail(TS2_ERR_CUDA, "no scratch pool");
+    TS2_CUDA(cudaMallocFromPoolAsync(ptr, bytes, p, stream));
+    return TS2_OK;
+}
+
+void scratch_free(cudaStream_t stream, void *ptr) { cudaFreeAsync(ptr, stream); }
+
+void scratch_trim(int device)
+{
+    if (cudaMemPool_t p = scratch_pool(device, false))
+        cudaMemPoolTrimTo(p, 0);
+}
+
 } // namespace ts2

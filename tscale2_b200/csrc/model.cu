@@ -266,6 +266,11 @@ int dalloc(ts2_model *m, T **p, size_t count)
     void *q = nullptr;
     size_t bytes = std::max<size_t>(count * sizeof(T), 256);
     cudaError_t e = cudaMalloc(&q, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        scratch_trim(m->device);
+        e = cudaMalloc(&q, bytes);
+    }
     if (e != cudaSuccess)
         return fail(TS2_ERR_CUDA, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     m->allocs.push_back(q);
