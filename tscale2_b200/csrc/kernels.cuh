@@ -58,6 +58,20 @@ struct LabelIndex {
     uint32_t n = 0;
     int sorted = 0; // which of key[] / val[] holds the sorted entries
 };
+// every table of a batch: the kernels above, or, for a small batch, one launch that also sorts the inverse index (*sorted)
+struct BatchTables {
+    int T, V, n_targets;
+    uint32_t n_labels, label_count;
+    uint32_t *label_arr, *label_ptr;
+    const int *target_node, *target_id;
+    int *target, *scan_tmp, *status;
+};
+struct BatchSpans {
+    const int *ptr, *csr_start, *csr_finish;
+    int n_spans;
+    int *start, *finish, *rev_first, *rev_last;
+};
+int batch_prepare(const Ctx &c, const BatchTables &b, const BatchSpans *att, int n_types, LabelIndex &ix, bool *sorted);
 size_t label_index_hist_elems(size_t label_cap);
 size_t label_index_partial_elems(size_t label_cap, int D);
 // validates label_arr / label_ptr in place (bad labels become label 0, label_ptr is clamped to n_labels) and writes the

@@ -159,13 +159,8 @@ __global__ void __launch_bounds__(1024) span_scan_kernel(const int *__restrict__
 
 // nodes that may attend to key `to`: none before the first node whose running maximum of span ends reaches `to`, none
 // after the last node whose suffix minimum of span starts is at most `to`.  (T, -1) when there is none.
-__global__ void span_reverse_kernel(const int *__restrict__ run_max, const int *__restrict__ suf_min, int T, int *__restrict__ rev_first,
-                                    int *__restrict__ rev_last)
+__device__ __forceinline__ void reverse_range(const int *run_max, const int *suf_min, int T, int to, int &first, int &last)
 {
-    grid_dep_wait();
-    const int to = blockIdx.x * blockDim.x + threadIdx.x;
-    if (to >= T)
-        return;
     int lo = 0, hi = T; // first t with run_max[t] >= to
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -174,7 +169,7 @@ __global__ void span_reverse_kernel(const int *__restrict__ run_max, const int *
         else
             lo = mid + 1;
     }
-    const int first = lo;
+    first = lo;
     lo = 0, hi = T; // first t with suf_min[t] > to
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -183,10 +178,24 @@ __global__ void span_reverse_kernel(const int *__restrict__ run_max, const int *
         else
             lo = mid + 1;
     }
-    const int last = lo - 1;
-    const bool any = first <= last;
-    rev_first[to] = any ? first : T;
-    rev_last[to] = any ? last : -1;
+    last = lo - 1;
+    if (first > last) {
+        first = T;
+        last = -1;
+    }
+}
+
+__global__ void span_reverse_kernel(const int *__restrict__ run_max, const int *__restrict__ suf_min, int T, int *__restrict__ rev_first,
+                                    int *__restrict__ rev_last)
+{
+    grid_dep_wait();
+    const int to = blockIdx.x * blockDim.x + threadIdx.x;
+    if (to >= T)
+        return;
+    int first, last;
+    reverse_range(run_max, suf_min, T, to, first, last);
+    rev_first[to] = first;
+    rev_last[to] = last;
 }
 
 // ---- targets -------------------------------------------------------------------------
@@ -334,12 +343,191 @@ __global__ void __launch_bounds__(1024) exclusive_scan_kernel(uint32_t *__restri
         x[i] = carry + before + v - own;
 }
 
+// ---- a small batch in one launch -----------------------------------------------------------
+// Up to SB_MAX nodes and labels everything above is work for one block per table: block 0 validates the labels and sorts
+// the inverse index (a bitonic sort of (label, position) pairs: positions differ, so it is stable), block 1 fills the
+// targets, block 2 + a the spans of attention type a.  The launches above took 45 us of a 512-token step, mostly
+// latency between them; this takes 12.
+constexpr int SB_MAX = 4096, SB_TYPES = 8, SB_THREADS = 1024, SB_PER = SB_MAX / SB_THREADS;
+struct SmallBatch {
+    int T, V, n_targets;
+    uint32_t n_labels, label_count;
+    uint32_t *label_arr, *label_ptr, *key, *val;
+    const int *target_node, *target_id;
+    int *target, *status;
+    struct {
+        const int *ptr, *csr_start, *csr_finish;
+        int n_spans;
+        int *start, *finish, *rev_first, *rev_last;
+    } att[SB_TYPES];
+};
+
+__global__ void __launch_bounds__(SB_THREADS) small_batch_kernel(const SmallBatch p)
+{
+    grid_dep_wait();
+    __shared__ unsigned long long pairs[SB_MAX]; // block 0: label << 32 | position; span blocks: run_max and suf_min
+    __shared__ int w_max[32], w_min[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = p.T;
+    if (blockIdx.x == 0) {
+        const uint32_t n = p.n_labels;
+        for (uint32_t k = tid; k < n; k += SB_THREADS) { // entries that no node owns count as label 0 of node 0
+            pairs[k] = k;
+            p.val[k] = 0;
+        }
+        __syncthreads();
+        for (int t = tid; t < T; t += SB_THREADS) {
+            uint32_t p0 = p.label_ptr[t], p1 = p.label_ptr[t + 1];
+            if (p0 > p1 || p1 > n) {
+                batch_fail(p.status, BATCH_BAD_LABEL_PTR, t, (int)p0, (int)p1);
+                p0 = min(p0, n);
+                p1 = min(max(p1, p0), n);
+            }
+            for (uint32_t k = p0; k < p1; ++k) {
+                const uint32_t raw = p.label_arr[k];
+                uint32_t label = raw & TS2_LABEL_MASK;
+                if (label >= p.label_count) {
+                    batch_fail(p.status, BATCH_BAD_LABEL, (int)k, (int)label, t);
+                    label = 0;
+                    p.label_arr[k] = raw & TS2_LABEL_NEGATIVE;
+                }
+                pairs[k] = (unsigned long long)label << 32 | k;
+                p.val[k] = (uint32_t)t | (raw & TS2_LABEL_NEGATIVE);
+            }
+        }
+        uint32_t n2 = 64;
+        while (n2 < n)
+            n2 *= 2;
+        for (uint32_t k = n + tid; k < n2; k += SB_THREADS)
+            pairs[k] = ~0ull;
+        __syncthreads();
+        for (int t = tid; t <= T; t += SB_THREADS)
+            p.label_ptr[t] = min(p.label_ptr[t], n);
+        for (uint32_t k = 2; k <= n2; k <<= 1)
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                for (uint32_t i = tid; i < n2 / 2; i += SB_THREADS) {
+                    const uint32_t a = 2 * i - (i & (j - 1)), b = a + j;
+                    const unsigned long long x = pairs[a], y = pairs[b];
+                    if ((x > y) == ((a & k) == 0)) {
+                        pairs[a] = y;
+                        pairs[b] = x;
+                    }
+                }
+                // up to a distance of 32 a warp's 32 exchanges stay inside 64 entries of its own
+                if (j > 32 || (j == 1 && k >= 64))
+                    __syncthreads();
+                else
+                    __syncwarp();
+            }
+        uint32_t v[SB_PER];
+        int c = 0;
+        for (uint32_t k = tid; k < n; k += SB_THREADS)
+            v[c++] = p.val[(uint32_t)pairs[k]];
+        __syncthreads();
+        c = 0;
+        for (uint32_t k = tid; k < n; k += SB_THREADS) {
+            p.key[k] = (uint32_t)(pairs[k] >> 32);
+            p.val[k] = v[c++];
+        }
+        return;
+    }
+    if (blockIdx.x == 1) {
+        for (int t = tid; t < T; t += SB_THREADS)
+            p.target[t] = -1;
+        __syncthreads();
+        for (int i = tid; i < p.n_targets; i += SB_THREADS) {
+            const int t = p.target_node[i], v = p.target_id[i];
+            if (t < 0 || t >= T || v < 0 || v >= p.V)
+                batch_fail(p.status, BATCH_BAD_TARGET, i, t, v);
+            else if (atomicExch(&p.target[t], v) != -1)
+                batch_fail(p.status, BATCH_DUP_TARGET, t, v, 0);
+        }
+        return;
+    }
+    const auto &at = p.att[blockIdx.x - 2];
+    int *run_max = (int *)pairs, *suf_min = run_max + SB_MAX;
+    // a thread takes SB_PER consecutive nodes: its own prefix maximum and suffix minimum, then the warp's, then the block's
+    int mx[SB_PER], mn[SB_PER], t0 = tid * SB_PER;
+#pragma unroll
+    for (int i = 0; i < SB_PER; ++i) {
+        const int t = t0 + i;
+        mx[i] = -1, mn[i] = T;
+        if (t < T) {
+            const int p0 = at.ptr[t], n = at.ptr[t + 1] - p0;
+            int s = 0, f = -1;
+            if (n < 0 || p0 < 0 || p0 + n > at.n_spans) {
+                batch_fail(p.status, BATCH_BAD_SPAN_PTR, t, p0, n);
+            } else if (n > 1) {
+                batch_fail(p.status, BATCH_MULTI_SPAN, t, n, 0);
+            } else if (n == 1) {
+                s = at.csr_start[p0];
+                f = at.csr_finish[p0];
+                if (s < 0 || f >= T || f < s) {
+                    batch_fail(p.status, BATCH_BAD_SPAN, t, s, f);
+                    s = 0;
+                    f = -1;
+                }
+            }
+            at.start[t] = s;
+            at.finish[t] = f;
+            if (f >= s)
+                mx[i] = f, mn[i] = s;
+        }
+    }
+#pragma unroll
+    for (int i = 1; i < SB_PER; ++i) {
+        mx[i] = max(mx[i], mx[i - 1]);
+        mn[SB_PER - 1 - i] = min(mn[SB_PER - 1 - i], mn[SB_PER - i]);
+    }
+    int wmx = mx[SB_PER - 1], wmn = mn[0]; // inclusive over the warp's lanes
+    for (int d = 1; d < 32; d <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, wmx, d), b = __shfl_down_sync(0xffffffffu, wmn, d);
+        if (lane >= d)
+            wmx = max(wmx, a);
+        if (lane + d < 32)
+            wmn = min(wmn, b);
+    }
+    if (lane == 31)
+        w_max[warp] = wmx;
+    if (lane == 0)
+        w_min[warp] = wmn;
+    int before = __shfl_up_sync(0xffffffffu, wmx, 1), after = __shfl_down_sync(0xffffffffu, wmn, 1);
+    before = lane > 0 ? before : -1;
+    after = lane < 31 ? after : T;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w)
+        before = max(before, w_max[w]);
+    for (int w = warp + 1; w < 32; ++w)
+        after = min(after, w_min[w]);
+#pragma unroll
+    for (int i = 0; i < SB_PER; ++i) {
+        run_max[t0 + i] = max(mx[i], before);
+        suf_min[t0 + i] = min(mn[i], after);
+    }
+    __syncthreads();
+    for (int to = tid; to < T; to += SB_THREADS) {
+        int first, last;
+        reverse_range(run_max, suf_min, T, to, first, last);
+        at.rev_first[to] = first;
+        at.rev_last[to] = last;
+    }
+}
+
 // ---- embedding gradient through the inverse index ----------------------------------------
-// The sorted entries are cut into chunks of EMB_CHUNK; one warp walks one chunk for one 128-wide tile of the state and
+// The sorted entries are cut into chunks (of 64; fewer where that leaves SMs idle); one warp walks one chunk for one 128-wide tile of the state and
 // sums the runs of equal labels in entry order.  A run that lies inside its chunk is added to its row of dE by that
 // warp alone.  A run that crosses a chunk border leaves partial sums (slot 1: the run leaves the chunk at its end and
 // did not enter it at the start; slot 0: the run entered at the start), which embed_chain_kernel adds up chunk by chunk.
-constexpr int EMB_CHUNK = 64;
+// What bounds it: a big batch, the bytes of g (read once); a small one, the latency of a warp's walk.  With chunks of 64
+// a batch of 512 tokens x 2 tiles gave work to 16 warps, each of which waited for 64 rows of dE in turn (29 us).
+constexpr int EMB_CHUNK = 64, EMB_CHUNK_MIN = 8;
+constexpr unsigned EMB_ITEMS = 148 * 16; // warps that fill the device
+static unsigned emb_chunk(size_t n, int tiles)
+{
+    unsigned chunk = EMB_CHUNK;
+    while (chunk > EMB_CHUNK_MIN && (n + chunk - 1) / chunk * tiles < EMB_ITEMS)
+        chunk /= 2;
+    return chunk;
+}
 
 __device__ __forceinline__ void add4(float4 &a, const float4 &g, float w)
 {
@@ -349,28 +537,24 @@ __device__ __forceinline__ void add4(float4 &a, const float4 &g, float w)
     a.w += g.w * w;
 }
 
+// row += a without waiting for the row: each kernel has one writer per row, so the order of the additions is fixed
 __device__ __forceinline__ void accumulate_row(float *row, const float4 &a)
 {
-    float4 v = *(float4 *)row;
-    v.x += a.x;
-    v.y += a.y;
-    v.z += a.z;
-    v.w += a.w;
-    *(float4 *)row = v;
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w) : "memory");
 }
 
 __global__ void __launch_bounds__(BP_THREADS) embed_runs_kernel(const float *__restrict__ g, const uint32_t *__restrict__ key,
-                                                                const uint32_t *__restrict__ val, uint32_t n, int D,
+                                                                const uint32_t *__restrict__ val, uint32_t n, uint32_t chunk, int D,
                                                                 float *__restrict__ dE, float *__restrict__ partial)
 {
     grid_dep_wait();
     const int tiles = D / TILE, lane = threadIdx.x & 31;
-    const uint32_t nchunks = (n + EMB_CHUNK - 1) / EMB_CHUNK;
+    const uint32_t nchunks = (n + chunk - 1) / chunk;
     const unsigned long long items = (unsigned long long)nchunks * tiles;
     for (unsigned long long item = blockIdx.x * BP_WARPS + (threadIdx.x >> 5); item < items; item += (unsigned long long)gridDim.x * BP_WARPS) {
         const uint32_t c = (uint32_t)(item / tiles);
         const int off = (int)(item % tiles) * TILE + lane * 4;
-        const uint32_t k0 = c * EMB_CHUNK, k1 = min(n, k0 + EMB_CHUNK);
+        const uint32_t k0 = c * chunk, k1 = min(n, k0 + chunk);
         const bool entered = k0 > 0 && key[k0 - 1] == key[k0]; // the first run began in an earlier chunk
         uint32_t run_label = key[k0];
         bool first_run = true;
@@ -379,12 +563,12 @@ __global__ void __launch_bounds__(BP_THREADS) embed_runs_kernel(const float *__r
             const uint32_t kk = kb + lane;
             const uint32_t my_key = kk < k1 ? key[kk] : 0, my_val = kk < k1 ? val[kk] : 0;
             const int cnt = (int)min(32u, k1 - kb);
-            for (int j0 = 0; j0 < cnt; j0 += 4) {
-                float4 gv[4];
-                uint32_t lab[4];
-                float w[4];
+            for (int j0 = 0; j0 < cnt; j0 += 8) {
+                float4 gv[8];
+                uint32_t lab[8];
+                float w[8];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < 8; ++u) {
                     const int j = min(j0 + u, cnt - 1);
                     lab[u] = __shfl_sync(0xffffffffu, my_key, j);
                     const uint32_t v = __shfl_sync(0xffffffffu, my_val, j);
@@ -392,7 +576,7 @@ __global__ void __launch_bounds__(BP_THREADS) embed_runs_kernel(const float *__r
                     gv[u] = *(const float4 *)(g + (size_t)(v & TS2_LABEL_MASK) * D + off);
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < 8; ++u) {
                     if (j0 + u >= cnt)
                         break;
                     if (lab[u] != run_label) {
@@ -419,17 +603,17 @@ __global__ void __launch_bounds__(BP_THREADS) embed_runs_kernel(const float *__r
     }
 }
 
-__global__ void __launch_bounds__(BP_THREADS) embed_chain_kernel(const uint32_t *__restrict__ key, uint32_t n, int D,
+__global__ void __launch_bounds__(BP_THREADS) embed_chain_kernel(const uint32_t *__restrict__ key, uint32_t n, uint32_t chunk, int D,
                                                                  const float *__restrict__ partial, float *__restrict__ dE)
 {
     grid_dep_wait();
     const int tiles = D / TILE, lane = threadIdx.x & 31;
-    const uint32_t nchunks = (n + EMB_CHUNK - 1) / EMB_CHUNK;
+    const uint32_t nchunks = (n + chunk - 1) / chunk;
     const unsigned long long items = (unsigned long long)nchunks * tiles;
     for (unsigned long long item = blockIdx.x * BP_WARPS + (threadIdx.x >> 5); item < items; item += (unsigned long long)gridDim.x * BP_WARPS) {
         const uint32_t c = (uint32_t)(item / tiles);
         const int off = (int)(item % tiles) * TILE + lane * 4;
-        const uint32_t k0 = c * EMB_CHUNK, k1 = min(n, k0 + EMB_CHUNK);
+        const uint32_t k0 = c * chunk, k1 = min(n, k0 + chunk);
         if (k1 >= n)
             continue;
         const uint32_t label = key[k1 - 1];
@@ -437,16 +621,29 @@ __global__ void __launch_bounds__(BP_THREADS) embed_chain_kernel(const uint32_t 
             continue; // nothing leaves this chunk
         if (k0 > 0 && key[k0 - 1] == label && key[k0] == label)
             continue; // the run that leaves also entered: an earlier chunk heads the chain
+        // the last chunk of the chain: the one that holds the label's last entry (the entries are sorted)
+        uint32_t lo = k1, hi = n; // first entry with a larger label
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (key[mid] > label)
+                hi = mid;
+            else
+                lo = mid + 1;
+        }
+        const uint32_t c_end = (lo - 1) / chunk;
         float4 sum = *(const float4 *)(partial + ((size_t)c * 2 + 1) * D + off);
-        for (uint32_t cc = c + 1; cc < nchunks; ++cc) {
-            const float4 p = *(const float4 *)(partial + ((size_t)cc * 2 + 0) * D + off);
-            sum.x += p.x;
-            sum.y += p.y;
-            sum.z += p.z;
-            sum.w += p.w;
-            const uint32_t e1 = min(n, (cc + 1) * EMB_CHUNK);
-            if (!(key[e1 - 1] == label && e1 < n && key[e1] == label))
-                break;
+        for (uint32_t c0 = c + 1; c0 <= c_end; c0 += 8) { // eight partial sums in flight, added in chunk order
+            float4 p[8];
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u)
+                p[u] = c0 + u <= c_end ? *(const float4 *)(partial + ((size_t)(c0 + u) * 2) * D + off) : make_float4(0, 0, 0, 0);
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u) {
+                sum.x += p[u].x;
+                sum.y += p[u].y;
+                sum.z += p[u].z;
+                sum.w += p[u].w;
+            }
         }
         accumulate_row(dE + (size_t)label * D + off, sum);
     }
@@ -461,7 +658,8 @@ int blocks_for(long long n)
 
 int queue_report(const Ctx &c, const int *batch_status, const float *scalar, HostReport *report)
 {
-    TS2_LAUNCH((report_kernel), 1, 1, 0, c.stream, device_status_word(c.device), static_status_word_if_ready(c.device), batch_status, scalar,
+    TS2_LAUNCH((report_kernel), 1, 1, 0, c.stream, device_status_word(c.device), static_status_word_if_ready(c.device), batch_status,
+               scalar,
                report);
     return TS2_OK;
 }
@@ -493,6 +691,39 @@ int batch_targets(const Ctx &c, const int *node, const int *id, int n, int T, in
     return TS2_OK;
 }
 
+static bool batch_prepare_small(const BatchTables &b, int n_types)
+{
+    return b.T <= SB_MAX && b.n_labels <= (uint32_t)SB_MAX && n_types <= SB_TYPES;
+}
+
+int batch_prepare(const Ctx &c, const BatchTables &b, const BatchSpans *att, int n_types, LabelIndex &ix, bool *sorted)
+{
+    *sorted = batch_prepare_small(b, n_types);
+    if (!*sorted) {
+        if (int rc = label_index_entries(c, b.label_arr, b.label_ptr, b.T, b.n_labels, b.label_count, ix, b.status))
+            return rc;
+        for (int a = 0; a < n_types; ++a)
+            if (int rc = batch_span_tables(c, att[a].ptr, att[a].csr_start, att[a].csr_finish, b.T, att[a].n_spans, att[a].start,
+                                           att[a].finish, b.scan_tmp, att[a].rev_first, att[a].rev_last, b.status))
+                return rc;
+        return batch_targets(c, b.target_node, b.target_id, b.n_targets, b.T, b.V, b.target, b.status);
+    }
+    ix.n = b.n_labels;
+    ix.sorted = 0;
+    SmallBatch s;
+    s.T = b.T, s.V = b.V, s.n_targets = b.n_targets;
+    s.n_labels = b.n_labels, s.label_count = b.label_count;
+    s.label_arr = b.label_arr, s.label_ptr = b.label_ptr, s.key = ix.key[0], s.val = ix.val[0];
+    s.target_node = b.target_node, s.target_id = b.target_id, s.target = b.target, s.status = b.status;
+    for (int a = 0; a < n_types; ++a) {
+        auto &x = s.att[a];
+        x.ptr = att[a].ptr, x.csr_start = att[a].csr_start, x.csr_finish = att[a].csr_finish, x.n_spans = att[a].n_spans;
+        x.start = att[a].start, x.finish = att[a].finish, x.rev_first = att[a].rev_first, x.rev_last = att[a].rev_last;
+    }
+    TS2_LAUNCH((small_batch_kernel), 2 + n_types, SB_THREADS, 0, c.stream, s);
+    return TS2_OK;
+}
+
 size_t batch_scan_tmp_elems(int T)
 {
     return 2 * (size_t)T + 2 * (((size_t)T + 1023) / 1024);
@@ -506,7 +737,9 @@ size_t label_index_hist_elems(size_t label_cap)
 
 size_t label_index_partial_elems(size_t label_cap, int D)
 {
-    return ((label_cap + EMB_CHUNK - 1) / EMB_CHUNK) * 2 * (size_t)D;
+    // smaller chunks are only taken while twice their size gives fewer than EMB_ITEMS items
+    const size_t tiles = D / TILE, small = std::min((label_cap + EMB_CHUNK_MIN - 1) / EMB_CHUNK_MIN, 2 * (size_t)EMB_ITEMS / tiles + 2);
+    return std::max((label_cap + EMB_CHUNK - 1) / EMB_CHUNK, small) * 2 * (size_t)D;
 }
 
 int label_index_entries(const Ctx &c, uint32_t *label_arr, uint32_t *label_ptr, int T, uint32_t n_labels, uint32_t label_count,
@@ -553,11 +786,11 @@ int embed_backward_indexed(const Ctx &c, const float *g, const LabelIndex &ix, i
 {
     if (ix.n == 0)
         return TS2_OK;
-    const uint32_t nchunks = (ix.n + EMB_CHUNK - 1) / EMB_CHUNK;
+    const uint32_t chunk = emb_chunk(ix.n, D / TILE), nchunks = (ix.n + chunk - 1) / chunk;
     const long long items = (long long)nchunks * (D / TILE);
     const int grid = (int)std::max<long long>(1, std::min<long long>((items + BP_WARPS - 1) / BP_WARPS, (long long)sm_count(c.device) * 8));
-    TS2_LAUNCH((embed_runs_kernel), grid, BP_THREADS, 0, c.stream, g, ix.key[ix.sorted], ix.val[ix.sorted], ix.n, D, dE, ix.partial);
-    TS2_LAUNCH((embed_chain_kernel), grid, BP_THREADS, 0, c.stream, ix.key[ix.sorted], ix.n, D, ix.partial, dE);
+    TS2_LAUNCH((embed_runs_kernel), grid, BP_THREADS, 0, c.stream, g, ix.key[ix.sorted], ix.val[ix.sorted], ix.n, chunk, D, dE, ix.partial);
+    TS2_LAUNCH((embed_chain_kernel), grid, BP_THREADS, 0, c.stream, ix.key[ix.sorted], ix.n, chunk, D, ix.partial, dE);
     return TS2_OK;
 }
 

@@ -1697,12 +1697,18 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
     b.label_arr = b.raw + o_labels;
     b.label_ptr = b.raw + o_label_ptr;
     b.n_labels = (uint32_t)n_labels;
-    b.ix_sorted = false;
-    M_TRY(label_index_entries(c, b.label_arr, b.label_ptr, T, b.n_labels, (uint32_t)m->descr.label_count, b.ix, b.status));
-    for (int a = 0; a < na; ++a)
-        M_TRY(batch_span_tables(c, (const int *)b.raw + o_ptr[a], (const int *)b.raw + o_start[a], (const int *)b.raw + o_finish[a], T,
-                                n_spans[a], b.span_start[a], b.span_finish[a], b.scan_tmp, b.rev_first[a], b.rev_last[a], b.status));
-    M_TRY(batch_targets(c, (const int *)b.raw + o_tnode, (const int *)b.raw + o_tid, n_targets, T, m->V, b.target, b.status));
+    BatchTables bt;
+    bt.T = T, bt.V = m->V, bt.n_targets = n_targets;
+    bt.n_labels = b.n_labels, bt.label_count = (uint32_t)m->descr.label_count;
+    bt.label_arr = b.label_arr, bt.label_ptr = b.label_ptr;
+    bt.target_node = (const int *)b.raw + o_tnode, bt.target_id = (const int *)b.raw + o_tid;
+    bt.target = b.target, bt.scan_tmp = b.scan_tmp, bt.status = b.status;
+    std::vector<BatchSpans> spans(na);
+    for (int a = 0; a < na; ++a) {
+        const int *raw = (const int *)b.raw;
+        spans[a] = {raw + o_ptr[a], raw + o_start[a], raw + o_finish[a], n_spans[a], b.span_start[a], b.span_finish[a], b.rev_first[a], b.rev_last[a]};
+    }
+    M_TRY(batch_prepare(c, bt, spans.data(), na, b.ix, &b.ix_sorted));
     b.node_count = T;
     b.target_count = n_targets;
     return TS2_OK;
