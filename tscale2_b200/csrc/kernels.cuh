@@ -18,8 +18,9 @@ struct Ctx {
 
 // ---- kernels_elem.cu ---------------------------------------------------------------
 // state0[t] = sum over the node's labels of +-E[label] * (sko/32)   (ComputeEmbedding, cpu_transformer.cpp:66-90)
+// zero: n_zero words that the step accumulates into later, cleared by the way (its first launch)
 int embed_forward(const Ctx &c, const __half *embed, const float *sko, const uint32_t *label_arr, const uint32_t *label_ptr, int T,
-                  int D, float *state);
+                  int D, float *state, unsigned *zero, int n_zero, float *zero_scalar);
 
 // ---- kernels_batch.cu: batch preparation on the device -------------------------------
 // codes of the batch status record {code, where, detail, detail}; 0 = the batch was well formed
@@ -193,8 +194,6 @@ int moe_router_backward(const Ctx &c, const float *dmoe_part, int tiles, const i
                         int k, int E, int ld, void *dl);
 
 // ---- kernels_opt.cu ----------------------------------------------------------------
-int fill_vector(const Ctx &c, float *dst, int n, float value, const float *dyn, bool reciprocal_dyn);
-
 // ---- flat, sharded optimizer + requantiser (kernels_opt.cu) -------------------------
 // the part [a, b) (elements inside the matrix, multiples of 4) of one matrix that a rank owns
 struct OptSeg {
@@ -220,11 +219,26 @@ int opt_disp(const Ctx &c, const OptMat *mats, int n_mats, const float *rowsum, 
 // step == nullptr: no update, only the per-row sums of squares of the weights
 int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const float *grad, const float *row_scale,
                const ts2_training_step *step, float *avg, float *w, double *roww2);
-int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos);
+// disp_decay: the step's, or negative when no step was applied
+int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos, float disp_decay);
 int opt_quantize(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const float *w, const float *skos);
-// copy / transposed copy of quantized values; dst or dstT may be null; transposed_as_half: 0 no, 1 e4m3 -> fp16, 2 int8 -> fp16
-int qcopy_block(const Ctx &c, const void *src, int64_t x, int64_t y, int64_t ld_src, int elem_size, void *dst, int64_t ld, void *dstT,
-                int64_t ldT, int transposed_as_half);
-int layer_scales(const Ctx &c, float *fwd_col, float *bwd_row, int W, int ncat, bool is_att, float a, const float *skos);
+// copy (dst) and / or transposed copy (dstT) of a block of quantized values [y][x], x a multiple of 128; pitches in bytes
+enum { QCOPY_1BYTE = 0, QCOPY_E4M3_HALF = 1, QCOPY_I8_HALF = 2, QCOPY_2BYTE = 3 }; // _HALF: the transpose is widened to fp16
+struct CopyJob {
+    const uint8_t *src;
+    uint8_t *dst, *dstT;
+    long long ld_src, ld, ldT;
+    int x, y, kind;
+    int tile0, tiles_x; // first tile of the job among all jobs' tiles
+};
+int qcopy_tiles(CopyJob &job); // fills tiles_x, returns the number of tiles
+int qcopy(const Ctx &c, const CopyJob *jobs, int n_jobs, int tiles);
+enum { SCALES_ATT = 0, SCALES_FFN = 1, SCALES_MOE = 2 };
+struct ScaleJob {
+    float *fwd_col, *bwd_row;
+    const float *skos;
+    int W, ncat, kind;
+};
+int layer_scales(const Ctx &c, const ScaleJob *jobs, int n_jobs, float a);
 
 } // namespace ts2

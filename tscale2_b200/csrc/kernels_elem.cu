@@ -44,9 +44,15 @@ static int grid_for(const Ctx &c, K kernel, long long warp_items)
 // ---------------------------------------------------------------------------------
 __global__ void embed_forward_kernel(const __half *__restrict__ embed, const float *__restrict__ sko,
                                      const uint32_t *__restrict__ label_arr, const uint32_t *__restrict__ label_ptr, int T, int D,
-                                     float *__restrict__ state)
+                                     float *__restrict__ state, unsigned *__restrict__ zero, int n_zero, float *__restrict__ zero_scalar)
 {
     grid_dep_wait();
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < n_zero; i += THREADS)
+            zero[i] = 0u;
+        if (threadIdx.x == 0)
+            *zero_scalar = 0.f;
+    }
     const int tiles = D / TILE;
     const float scale = __ldg(sko) * (1.f / 32);
     WARP_ITEM_LOOP((long long)T * tiles)
@@ -69,10 +75,11 @@ __global__ void embed_forward_kernel(const __half *__restrict__ embed, const flo
 }
 
 int embed_forward(const Ctx &c, const __half *embed, const float *sko, const uint32_t *label_arr, const uint32_t *label_ptr, int T,
-                  int D, float *state)
+                  int D, float *state, unsigned *zero, int n_zero, float *zero_scalar)
 {
     TS2_LAUNCH((embed_forward_kernel), grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream, embed, sko, label_arr, label_ptr, T,
-               D, state);
+               D, state,
+               zero, n_zero, zero_scalar);
     return TS2_OK;
 }
 

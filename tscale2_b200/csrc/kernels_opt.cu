@@ -11,16 +11,6 @@ namespace ts2 {
 static constexpr int WARPS = 8;
 static constexpr int THREADS = WARPS * 32;
 
-__global__ void fill_vector_kernel(float *dst, int n, float value, const float *dyn, int reciprocal)
-{
-    grid_dep_wait();
-    float v = value;
-    if (dyn)
-        v = reciprocal ? value / *dyn : value * *dyn;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        dst[i] = v;
-}
-
 // ---------------------------------------------------------------------------------
 // Flat, sharded form of the optimizer and the requantiser.  All matrices live in flat buffers (weights, momentum,
 // gradient) in matrix order, grouped into buckets (embedding, final layer, one per layer).  A rank owns one
@@ -78,7 +68,9 @@ __global__ void opt_row_sum2_kernel(const OptSeg *__restrict__ segs, int nseg, i
     }
 }
 
-// one block per matrix: dispersion EMA -> row scale for every row of the matrix (UpdateGlobalRowDisp)
+// dispersion EMA -> row scale for every row of a matrix (UpdateGlobalRowDisp).  blockIdx.x = matrix; rows with a dispersion
+// of their own are divided over blockIdx.y (one block took 43 us for a 50 k-row embedding, these 5), a matrix with one is
+// the first block's.  The weight of the average is advanced by opt_sko_kernel, when no block reads the old one any more.
 __global__ void opt_disp_kernel(const OptMat *__restrict__ mats, const float *__restrict__ rowsum, float disp_decay,
                                 float *__restrict__ row_scale)
 {
@@ -92,13 +84,13 @@ __global__ void opt_disp_kernel(const OptMat *__restrict__ mats, const float *__
     const float sw = *mt.sum_weight * disp_decay + 1.f;
     const float norm = 1.f / sw;
     if (step == 1) {
-        for (long long r = threadIdx.x; r < mt.y; r += blockDim.x) {
+        for (long long r = blockIdx.y * blockDim.x + threadIdx.x; r < mt.y; r += gridDim.y * blockDim.x) {
             const float rd = mt.row_disp[r] * disp_decay + sum2[r] / (float)mt.x;
             mt.row_disp[r] = rd;
             const float d = rd * norm;
             rs_out[r] = d > 0.f ? 1.f / sqrtf(d) : 0.f;
         }
-    } else {
+    } else if (blockIdx.y == 0) {
         for (int b = 0; b < mt.row_disp_size; ++b) {
             float s = 0.f;
             for (long long k = threadIdx.x; k < step; k += blockDim.x)
@@ -123,9 +115,6 @@ __global__ void opt_disp_kernel(const OptMat *__restrict__ mats, const float *__
             __syncthreads();
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0)
-        *mt.sum_weight = sw;
 }
 
 // AddGradientKernel on the rows of the range (UPDATE) and the sum of squares of the (new) weights per row part
@@ -181,7 +170,8 @@ __global__ void opt_update_kernel(const OptSeg *__restrict__ segs, int nseg, int
 }
 
 // one block per matrix: sko = sqrt(sum of squares / (x y)), rows summed in a fixed order
-__global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__restrict__ roww2, float *__restrict__ skos)
+// (disp_decay >= 0: a step was applied, the weight of the dispersion average moves on)
+__global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__restrict__ roww2, float *__restrict__ skos, float disp_decay)
 {
     grid_dep_wait();
     __shared__ double red[32];
@@ -199,6 +189,8 @@ __global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__
         for (int i = 0; i < (int)blockDim.x / 32; ++i)
             tot += red[i];
         skos[blockIdx.x] = sqrtf((float)tot / (float)(mt.x * mt.y));
+        if (disp_decay >= 0.f)
+            *mt.sum_weight = *mt.sum_weight * disp_decay + 1.f;
     }
 }
 
@@ -251,7 +243,7 @@ int opt_row_sum2(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const f
 
 int opt_disp(const Ctx &c, const OptMat *mats, int n_mats, const float *rowsum, float disp_decay, float *row_scale)
 {
-    TS2_LAUNCH((opt_disp_kernel), n_mats, 1024, 0, c.stream, mats, rowsum, disp_decay, row_scale);
+    TS2_LAUNCH((opt_disp_kernel), dim3(n_mats, 8), 1024, 0, c.stream, mats, rowsum, disp_decay, row_scale);
     return TS2_OK;
 }
 
@@ -269,9 +261,9 @@ int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const flo
     return TS2_OK;
 }
 
-int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos)
+int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos, float disp_decay)
 {
-    TS2_LAUNCH((opt_sko_kernel), n_mats, 1024, 0, c.stream, mats, roww2, skos);
+    TS2_LAUNCH((opt_sko_kernel), n_mats, 1024, 0, c.stream, mats, roww2, skos, disp_decay);
     return TS2_OK;
 }
 
@@ -283,88 +275,171 @@ int opt_quantize(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const f
     return TS2_OK;
 }
 
-// Copy of a block of already quantized values (ES bytes per element) into another row-major place and / or its
-// transpose: 32x32 tiles, both sides coalesced.  TH: the transposed copy holds the value widened to fp16 (1: from e4m3,
-// 2: from int8), 0: copied as it is.
-template <int ES, int TH>
-__global__ void qcopy_kernel(const void *__restrict__ src, long long x, long long y, long long ld_src, void *__restrict__ dst,
-                             long long ld, void *__restrict__ dstT, long long ldT)
+// Copies of already quantized blocks into another row-major place and / or their transpose, all of a model's in one
+// launch.  A tile is 128 bytes of 128 rows (64 rows of 2-byte values): it comes in as 16-byte vectors, lies in shared
+// memory with its 16-byte pieces rotated by the row group (so that both the vector writes and the word reads of eight
+// row groups are free of bank conflicts), is transposed in registers by byte permutes and leaves in 16-byte vectors.
+// Bound by its bytes (read once, written once or twice): 4 transposes of [16384 x 2048] bytes and their like took 52 us
+// each with 32 x 32 byte tiles (1.3 TB/s) and a launch of their own; an expert layer of 32 experts was 97 launches.
+__device__ __forceinline__ void transpose4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t (&c)[4])
+{
+    const uint32_t l01 = __byte_perm(a0, a1, 0x5140), h01 = __byte_perm(a0, a1, 0x7362);
+    const uint32_t l23 = __byte_perm(a2, a3, 0x5140), h23 = __byte_perm(a2, a3, 0x7362);
+    c[0] = __byte_perm(l01, l23, 0x5410), c[1] = __byte_perm(l01, l23, 0x7632);
+    c[2] = __byte_perm(h01, h23, 0x5410), c[3] = __byte_perm(h01, h23, 0x7632);
+}
+
+// four bytes of the operand format as four halves
+__device__ __forceinline__ uint2 widen4(uint32_t w, int kind)
+{
+    if (kind == QCOPY_I8_HALF) {
+        const __half2 a = __floats2half2_rn((float)(int8_t)w, (float)(int8_t)(w >> 8)),
+                      b = __floats2half2_rn((float)(int8_t)(w >> 16), (float)(int8_t)(w >> 24));
+        return make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
+    }
+    const __half2_raw a = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w & 0xffff), __NV_E4M3),
+                      b = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> 16), __NV_E4M3);
+    return make_uint2((uint32_t)a.x | (uint32_t)a.y << 16, (uint32_t)b.x | (uint32_t)b.y << 16);
+}
+
+__global__ void __launch_bounds__(256) qcopy_kernel(const CopyJob *__restrict__ jobs, int n_jobs, int tiles)
 {
     grid_dep_wait();
-    using QT = typename std::conditional<ES == 1, uint8_t, uint16_t>::type;
-    using TT = typename std::conditional<TH != 0, uint16_t, QT>::type;
-    __shared__ QT tile[32][33];
-    const long long x0 = (long long)blockIdx.x * 32, y0 = (long long)blockIdx.y * 32;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const long long yy = y0 + r, xx = x0 + threadIdx.x;
-        QT qv = QT();
-        if (yy < y && xx < x) {
-            qv = ((const QT *)src)[yy * ld_src + xx];
-            if (dst)
-                ((QT *)dst)[yy * ld + xx] = qv;
+    __shared__ uint4 tile_s[128 * 8];
+    const int tid = threadIdx.x;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        int lo = 0, hi = n_jobs - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (jobs[mid].tile0 <= tile)
+                lo = mid;
+            else
+                hi = mid - 1;
         }
-        tile[r][threadIdx.x] = qv;
-    }
-    if (!dstT)
-        return;
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const long long xx = x0 + r, yy = y0 + threadIdx.x;
-        if (xx < x && yy < y) {
-            const QT qv = tile[threadIdx.x][r];
-            if constexpr (TH == 1 && ES == 1) {
-                __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)qv, __NV_E4M3);
-                ((uint16_t *)dstT)[xx * ldT + yy] = h2.x;
-            } else if constexpr (TH == 2 && ES == 1) {
-                ((uint16_t *)dstT)[xx * ldT + yy] = __half_as_ushort(__float2half_rn((float)(int8_t)qv));
+        const CopyJob jb = jobs[lo];
+        const int two = jb.kind == QCOPY_2BYTE, rows = two ? 64 : 128, shift = two ? 3 : 4;
+        const int t = tile - jb.tile0, tx = t % jb.tiles_x, y0 = (t / jb.tiles_x) * rows;
+        const long long xb = (long long)tx * 128; // byte offset of the tile in a source row
+        for (int v = tid; v < rows * 8; v += 256) {
+            const int r = v >> 3, c = v & 7;
+            uint4 q = make_uint4(0, 0, 0, 0);
+            if (y0 + r < jb.y) {
+                q = *(const uint4 *)(jb.src + (y0 + r) * jb.ld_src + xb + c * 16);
+                if (jb.dst)
+                    *(uint4 *)(jb.dst + (y0 + r) * jb.ld + xb + c * 16) = q;
+            }
+            tile_s[r * 8 + (c ^ ((r >> shift) & 7))] = q;
+        }
+        if (jb.dstT) { // the same for the whole block
+            __syncthreads();
+            const uint32_t *words = (const uint32_t *)tile_s;
+            const int rg = tid & 7, cg = tid >> 3, wc = cg ^ (rg << 2);
+            if (two) {
+                const int row0 = y0 + rg * 8;
+                uint32_t w[8], c0[4], c1[4];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    w[i] = words[(rg * 8 + i) * 32 + wc];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    c0[i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x5410);
+                    c1[i] = __byte_perm(w[2 * i], w[2 * i + 1], 0x7632);
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const uint32_t *c = j ? c1 : c0;
+                    uint8_t *d = jb.dstT + ((long long)tx * 64 + cg * 2 + j) * jb.ldT + (long long)row0 * 2;
+                    if (row0 + 8 <= jb.y)
+                        *(uint4 *)d = make_uint4(c[0], c[1], c[2], c[3]);
+                    else
+                        for (int i = 0; row0 + i < jb.y; ++i)
+                            ((uint16_t *)d)[i] = (uint16_t)(c[i >> 1] >> (16 * (i & 1)));
+                }
             } else {
-                ((TT *)dstT)[xx * ldT + yy] = qv;
+                const int row0 = y0 + rg * 16;
+                uint32_t out[4][4]; // [column][four rows]
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    uint32_t w[4], c[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        w[i] = words[(rg * 16 + 4 * b + i) * 32 + wc];
+                    transpose4(w[0], w[1], w[2], w[3], c);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        out[j][b] = c[j];
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const long long col = xb + cg * 4 + j;
+                    if (jb.kind == QCOPY_1BYTE) {
+                        uint8_t *d = jb.dstT + col * jb.ldT + row0;
+                        if (row0 + 16 <= jb.y)
+                            *(uint4 *)d = make_uint4(out[j][0], out[j][1], out[j][2], out[j][3]);
+                        else
+                            for (int i = 0; row0 + i < jb.y; ++i)
+                                d[i] = (uint8_t)(out[j][i >> 2] >> (8 * (i & 3)));
+                    } else {
+                        uint8_t *d = jb.dstT + col * jb.ldT + (long long)row0 * 2;
+                        uint2 h[4];
+#pragma unroll
+                        for (int b = 0; b < 4; ++b)
+                            h[b] = widen4(out[j][b], jb.kind);
+                        if (row0 + 16 <= jb.y) {
+                            *(uint4 *)d = make_uint4(h[0].x, h[0].y, h[1].x, h[1].y);
+                            *((uint4 *)d + 1) = make_uint4(h[2].x, h[2].y, h[3].x, h[3].y);
+                        } else {
+                            for (int i = 0; row0 + i < jb.y; ++i) {
+                                const uint32_t w = (i & 2) ? h[i >> 2].y : h[i >> 2].x;
+                                ((uint16_t *)d)[i] = (uint16_t)(w >> (16 * (i & 1)));
+                            }
+                        }
+                    }
+                }
             }
         }
+        __syncthreads();
     }
 }
 
-int qcopy_block(const Ctx &c, const void *src, int64_t x, int64_t y, int64_t ld_src, int elem_size, void *dst, int64_t ld, void *dstT,
-                int64_t ldT, int transposed_as_half)
+int qcopy_tiles(CopyJob &job)
 {
-    dim3 g((unsigned)ceil_div(x, 32), (unsigned)ceil_div(y, 32)), b(32, 8);
-    if (elem_size == 1 && transposed_as_half == 1)
-        TS2_LAUNCH((qcopy_kernel<1, 1>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
-    else if (elem_size == 1 && transposed_as_half == 2)
-        TS2_LAUNCH((qcopy_kernel<1, 2>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
-    else if (elem_size == 1)
-        TS2_LAUNCH((qcopy_kernel<1, 0>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
-    else
-        TS2_LAUNCH((qcopy_kernel<2, 0>), g, b, 0, c.stream, src, x, y, ld_src, dst, ld, dstT, ldT);
+    const int es = job.kind == QCOPY_2BYTE ? 2 : 1;
+    job.tiles_x = (int)((int64_t)job.x * es / 128);
+    return job.tiles_x * (int)ceil_div(job.y, es == 2 ? 64 : 128);
+}
+
+int qcopy(const Ctx &c, const CopyJob *jobs, int n_jobs, int tiles)
+{
+    if (tiles > 0)
+        TS2_LAUNCH((qcopy_kernel), std::min(tiles, sm_count(c.device) * 8), 256, 0, c.stream, jobs, n_jobs, tiles);
     return TS2_OK;
 }
 
-// the scale vectors of one dense layer from its matrix scales (skos of the layer's matrices, in matrix order):
-// forward column scales a (x sko_k for the K block of an attention layer), dW row scales 1 / sko for the matrices
-// that are followed by a normalisation (Q, K, V; Expand), 1 elsewhere
-__global__ void layer_scales_kernel(float *__restrict__ fwd_col, float *__restrict__ bwd_row, int W, int ncat, int is_att, float a,
-                                    const float *__restrict__ skos)
+// The scale vectors of every layer from its matrices' scales (skos, in matrix order): forward column scales a (x sko_k for
+// the K block of an attention layer), dW row scales 1 / sko for the matrices that are followed by a normalisation (Q, K,
+// V; Expand), 1 elsewhere.  An expert layer has no K block and one row vector, for Expand.  blockIdx.y = layer.
+__global__ void layer_scales_kernel(const ScaleJob *__restrict__ jobs, float a)
 {
     grid_dep_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ncat * W; i += gridDim.x * blockDim.x) {
-        const int j = i / W;
-        fwd_col[i] = (is_att && j == 1) ? a * skos[1] : a;
-        const bool scaled = is_att ? j < 3 : j == 0;
-        bwd_row[i] = scaled ? 1.f / skos[j] : 1.f;
+    const ScaleJob jb = jobs[blockIdx.y];
+    const bool att = jb.kind == SCALES_ATT;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < jb.ncat * jb.W; i += gridDim.x * blockDim.x) {
+        const int j = i / jb.W;
+        jb.fwd_col[i] = (att && j == 1) ? a * jb.skos[1] : a;
+        if (jb.kind == SCALES_MOE) {
+            if (j == 0)
+                jb.bwd_row[i] = 1.f / jb.skos[0];
+            continue;
+        }
+        jb.bwd_row[i] = (att ? j < 3 : j == 0) ? 1.f / jb.skos[j] : 1.f;
     }
 }
 
-int layer_scales(const Ctx &c, float *fwd_col, float *bwd_row, int W, int ncat, bool is_att, float a, const float *skos)
+int layer_scales(const Ctx &c, const ScaleJob *jobs, int n_jobs, float a)
 {
-    TS2_LAUNCH((layer_scales_kernel), std::max(1, std::min(64, (ncat * W + 255) / 256)), 256, 0, c.stream, fwd_col, bwd_row, W, ncat,
-               is_att ? 1 : 0, a, skos);
-    return TS2_OK;
-}
-
-int fill_vector(const Ctx &c, float *dst, int n, float value, const float *dyn, bool reciprocal_dyn)
-{
-    TS2_LAUNCH((fill_vector_kernel), std::max(1, std::min(64, (n + 255) / 256)), 256, 0, c.stream, dst, n, value, dyn,
-               reciprocal_dyn ? 1 : 0);
+    if (n_jobs > 0)
+        TS2_LAUNCH((layer_scales_kernel), dim3(8, n_jobs), 256, 0, c.stream, jobs, a);
     return TS2_OK;
 }
 

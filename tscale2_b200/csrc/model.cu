@@ -148,6 +148,9 @@ struct ts2_model {
     OptMat *d_optmats = nullptr;
     OptSeg *d_segs_full = nullptr, *d_segs_shard = nullptr;
     int nseg_full = 0, nitems_full = 0, nseg_shard = 0, nitems_shard = 0;
+    CopyJob *d_copies = nullptr; // what post_quantize does
+    ScaleJob *d_scales = nullptr;
+    int n_copies = 0, copy_tiles = 0, n_scales = 0;
     bool master_stale = false; // data parallel: the fp32 weights / momentum outside this rank's parts are out of date
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr, ev_grads = nullptr, ev_reduced = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     std::string error;
@@ -217,6 +220,8 @@ struct ts2_model {
     HostReport *report = nullptr;  // pinned; written by the kernel that every wait queues (queue_report)
     bool unreported = false;       // work was queued since the last wait
     bool grads_dirty = false; // the flat gradient holds an accumulated, not yet applied gradient
+    // dense dW contractions write their whole matrix: the first of an accumulation overwrites what is there
+    int dense_dw_out() const { return grads_dirty ? TS2_OUT_F32_ADD : TS2_OUT_F32; }
     bool reduce_in_backward = false; // this backward pass is followed by apply(): all-reduce every layer's gradient as soon as it is complete
     int gemm_tag = 0; // class of the contractions being queued (timing statistics)
     bool debug_taps = false;
@@ -741,15 +746,27 @@ int ep_exchange(ts2_model *m, const Layer &ly, bool to_owner, void *own, void *x
     return TS2_OK;
 }
 
-// transposed copies, per-expert layouts and scale vectors from the row-major quantized matrices and their scales
-int post_quantize(ts2_model *m)
+// the copies and scale vectors that post_quantize makes, as tables on the device (built once: no pointer in them moves)
+int build_post_quantize(ts2_model *m)
 {
-    Ctx c = ctx_of(m);
     const int D = m->D;
     const size_t fs = fast_size(m);
+    std::vector<CopyJob> copies;
+    std::vector<ScaleJob> scales;
+    m->copy_tiles = 0;
+    auto add = [&](const void *src, int64_t x, int64_t y, int64_t ld_src, void *dst, int64_t ld, void *dstT, int64_t ldT, int kind) {
+        const bool wide = kind == QCOPY_E4M3_HALF || kind == QCOPY_I8_HALF;
+        CopyJob j;
+        j.src = (const uint8_t *)src, j.dst = (uint8_t *)dst, j.dstT = (uint8_t *)dstT;
+        j.ld_src = ld_src * fs, j.ld = ld * fs, j.ldT = ldT * (wide ? 2 : fs);
+        j.x = (int)x, j.y = (int)y, j.kind = kind;
+        j.tile0 = m->copy_tiles;
+        m->copy_tiles += qcopy_tiles(j);
+        copies.push_back(j);
+    };
+    const int plain = fs == 2 ? QCOPY_2BYTE : QCOPY_1BYTE;
     // final layer: fp16 transposed copy of the same quantized values for the dX contraction
-    M_TRY(qcopy_block(c, m->Wf, D, m->V, D, (int)fs, nullptr, 0, m->WfT16, m->V, m->ft == 0 ? 1 : m->ft == 2 ? 2 : 0));
-    const float a = sqrtf(1.0f / D) / (m->s_act * 32.f);
+    add(m->Wf, D, m->V, D, nullptr, 0, m->WfT16, m->V, m->ft == 0 ? QCOPY_E4M3_HALF : m->ft == 2 ? QCOPY_I8_HALF : QCOPY_2BYTE);
     for (Layer &ly : m->layers) {
         const int W = ly.wide, n = ly.ncat;
         auto qsrc = [&](int mat) {
@@ -762,24 +779,38 @@ int post_quantize(ts2_model *m)
             const int E = m->E, X = m->X;
             for (int e = 0; e < E; ++e) {
                 uint8_t *cat = (uint8_t *)ly.Wcat + (size_t)e * 2 * X * D * fs, *catT = (uint8_t *)ly.WcatT + (size_t)e * D * 2 * X * fs;
-                M_TRY(qcopy_block(c, qsrc(ly.mat0) + (size_t)e * X * D * fs, D, X, D, (int)fs, cat, D, catT, 2 * X, 0));
-                M_TRY(qcopy_block(c, qsrc(ly.mat0 + 1) + (size_t)e * X * D * fs, D, X, D, (int)fs, cat + (size_t)X * D * fs, D,
-                                  catT + (size_t)X * fs, 2 * X, 0));
-                M_TRY(qcopy_block(c, qsrc(ly.mat0 + 2) + (size_t)e * D * X * fs, X, D, X, (int)fs, (uint8_t *)ly.Wc + (size_t)e * D * X * fs, X,
-                                  (uint8_t *)ly.WcT + (size_t)e * X * D * fs, D, 0));
+                add(qsrc(ly.mat0) + (size_t)e * X * D * fs, D, X, D, cat, D, catT, 2 * X, plain);
+                add(qsrc(ly.mat0 + 1) + (size_t)e * X * D * fs, D, X, D, cat + (size_t)X * D * fs, D, catT + (size_t)X * fs, 2 * X, plain);
+                add(qsrc(ly.mat0 + 2) + (size_t)e * D * X * fs, X, D, X, (uint8_t *)ly.Wc + (size_t)e * D * X * fs, X,
+                    (uint8_t *)ly.WcT + (size_t)e * X * D * fs, D, plain);
             }
-            M_TRY(qcopy_block(c, qsrc(ly.mat0 + 3), D, E, D, (int)fs, ly.Wsel, D, ly.WselT, m->epad, 0));
-            M_TRY(fill_vector(c, ly.fwd_col, 2 * X, a, nullptr, false));
-            M_TRY(fill_vector(c, ly.bwd_row_e, X, 1.f, m->mats[ly.mat0].sko, true));
+            add(qsrc(ly.mat0 + 3), D, E, D, ly.Wsel, D, ly.WselT, m->epad, plain);
+            scales.push_back({ly.fwd_col, ly.bwd_row_e, m->skos + ly.mat0, X, 2, SCALES_MOE});
             continue;
         }
         // the concatenated block [n W][D] transposes in one pass: its row blocks become the column blocks of WcatT
-        M_TRY(qcopy_block(c, ly.Wcat, D, (int64_t)n * W, D, (int)fs, nullptr, 0, ly.WcatT, (int64_t)n * W, 0));
-        M_TRY(qcopy_block(c, ly.Wc, W, D, W, (int)fs, nullptr, 0, ly.WcT, D, 0));
+        add(ly.Wcat, D, (int64_t)n * W, D, nullptr, 0, ly.WcatT, (int64_t)n * W, plain);
+        add(ly.Wc, W, D, W, nullptr, 0, ly.WcT, D, plain);
         // forward column scales: matrices followed by a normalisation (Q, V, Expand) and the gates use the unit-RMS
         // matrix q/32 (GetDataNoScale), K carries its matrix scale; dW rows of Q, K, V / Expand are divided by theirs
-        M_TRY(layer_scales(c, ly.fwd_col, ly.bwd_row, W, n, ly.type == TS2_LAYER_ATT, a, m->skos + ly.mat0));
+        scales.push_back({ly.fwd_col, ly.bwd_row, m->skos + ly.mat0, W, n, ly.type == TS2_LAYER_ATT ? SCALES_ATT : SCALES_FFN});
     }
+    m->n_copies = (int)copies.size();
+    m->n_scales = (int)scales.size();
+    M_TRY(dalloc(m, &m->d_copies, copies.size()));
+    M_TRY(dalloc(m, &m->d_scales, scales.size() + 1));
+    TS2_CUDA(cudaMemcpyAsync(m->d_copies, copies.data(), copies.size() * sizeof(CopyJob), cudaMemcpyHostToDevice, m->stream));
+    TS2_CUDA(cudaMemcpyAsync(m->d_scales, scales.data(), scales.size() * sizeof(ScaleJob), cudaMemcpyHostToDevice, m->stream));
+    TS2_CUDA(cudaStreamSynchronize(m->stream)); // the host vectors go away
+    return TS2_OK;
+}
+
+// transposed copies, per-expert layouts and scale vectors from the row-major quantized matrices and their scales
+int post_quantize(ts2_model *m)
+{
+    Ctx c = ctx_of(m);
+    M_TRY(qcopy(c, m->d_copies, m->n_copies, m->copy_tiles));
+    M_TRY(layer_scales(c, m->d_scales, m->n_scales, sqrtf(1.0f / m->D) / (m->s_act * 32.f)));
     return TS2_OK;
 }
 
@@ -788,7 +819,7 @@ int requantize_all(ts2_model *m)
 {
     Ctx c = ctx_of(m);
     M_TRY(opt_update(c, m->d_segs_full, m->nseg_full, m->nitems_full, nullptr, nullptr, nullptr, nullptr, m->w_flat, m->roww2));
-    M_TRY(opt_sko(c, m->d_optmats, (int)m->mats.size(), m->roww2, m->skos));
+    M_TRY(opt_sko(c, m->d_optmats, (int)m->mats.size(), m->roww2, m->skos, -1.f));
     M_TRY(opt_quantize(c, m->d_segs_full, m->nseg_full, m->nitems_full, m->w_flat, m->skos));
     M_TRY(post_quantize(m));
     return TS2_OK;
@@ -1095,6 +1126,7 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
         m->nseg_shard = m->nseg_full;
         m->nitems_shard = m->nitems_full;
     }
+    M_TRY(build_post_quantize(m));
     M_TRY(requantize_all(m));
     TS2_CUDA(cudaStreamSynchronize(m->stream));
     return TS2_OK;
@@ -1124,7 +1156,7 @@ int forward(ts2_model *m)
     const BatchDev &b = m->batch;
     const size_t fsz = fast_size(m);
     m->gemm_tag = GEMM_TAG_FWD;
-    M_TRY(embed_forward(c, m->embed16, m->mats[0].sko, b.label_arr, b.label_ptr, T, D, m->states[0]));
+    M_TRY(embed_forward(c, m->embed16, m->mats[0].sko, b.label_arr, b.label_ptr, T, D, m->states[0], m->absmax, m->L + 2, m->logp));
     TRACE("state", 0, m->states[0], (size_t)T * D * 4, TR_F32);
     for (int l = 0; l < m->L; ++l) {
         Layer &ly = m->layers[l];
@@ -1252,7 +1284,6 @@ int final_layer(ts2_model *m, bool backward)
     const float gs = (1.f / LOG2F) * LOG2F;                // CalcFinalLayerMult() * LOG2, cpu_transformer.cpp:159
     const bool tune_final = !(m->descr.flags & TS2_MPF_DISABLE_TUNE_FINAL_LAYER);
     m->gemm_tag = GEMM_TAG_FINAL;
-    TS2_CUDA(cudaMemsetAsync(m->logp, 0, 4, m->stream));
     for (int r0 = 0; r0 < T; r0 += m->chunk) {
         const int rows = std::min(m->chunk, T - r0);
         Epilogue e;
@@ -1276,7 +1307,7 @@ int final_layer(ts2_model *m, bool backward)
             // dWf += g^T . nF   (SumRankOne, cpu_transformer.cpp:168)
             Epilogue ew;
             ew.alpha = gs / gscale;
-            ew.out_kind = TS2_OUT_F32_ADD;
+            ew.out_kind = m->grads_dirty || r0 ? TS2_OUT_F32_ADD : TS2_OUT_F32;
             M_TRY(gemm_dw(m, KIND_F16, V, D, rows, m->logits, V, m->nF16 + (size_t)r0 * D, D, m->mats[1].grad, ew));
         }
     }
@@ -1349,7 +1380,7 @@ int backward_dense_int8(ts2_model *m, int l)
         Epilogue e6;
         e6.alpha = 1.f / m->s_act;
         e6.dyn_scale = m->ginv;
-        e6.out_kind = TS2_OUT_F32_ADD;
+        e6.out_kind = m->dense_dw_out();
         M_TRY(gemm_dw(m, KIND_F16, D, W, T, m->g16, D, m->x16, W, mc.grad, e6));
         TRACE("dW_c", l, mc.grad, (size_t)D * W * 4, TR_F32);
     }
@@ -1376,9 +1407,32 @@ int backward_dense_int8(ts2_model *m, int l)
         e5.alpha = 1.f / m->s_act;
         e5.dyn_scale = m->fscale;
         e5.row_scale = ly.bwd_row;
-        e5.out_kind = TS2_OUT_F32_ADD;
+        e5.out_kind = m->dense_dw_out();
         M_TRY(gemm_dw(m, KIND_F16, C, D, T, m->dcat16, C, m->x16, D, m->mats[ly.mat0].grad, e5));
         TRACE("dW_cat", l, m->mats[ly.mat0].grad, (size_t)C * D * 4, TR_F32);
+    }
+    return TS2_OK;
+}
+
+// Zeroes what an accumulation adds to from its first call on: the embedding (only the rows of the batch's labels are
+// written), expert matrices (an expert without rows is not), and what the model's flags keep from being written at all.
+// The rest, most of the bytes, is overwritten by its first dW contraction.
+int clear_gradient(ts2_model *m)
+{
+    const bool tune_final = !(m->descr.flags & TS2_MPF_DISABLE_TUNE_FINAL_LAYER), tune_layers = !(m->descr.flags & TS2_MPF_DISABLE_TUNE_LAYERS);
+    size_t lo = 0, hi = 0; // adjacent buckets go together
+    for (size_t b = 0; b <= m->buckets.size(); ++b) {
+        const bool end = b == m->buckets.size();
+        if (!end && !(b == 0 || m->buckets[b].expert_matrix || !(b == 1 ? tune_final : tune_layers)))
+            continue;
+        if (end || m->buckets[b].off != hi) {
+            if (hi > lo)
+                TS2_CUDA(cudaMemsetAsync(m->grad_flat + lo, 0, (hi - lo) * 4, m->stream));
+            if (end)
+                break;
+            lo = m->buckets[b].off;
+        }
+        hi = m->buckets[b].off + m->buckets[b].elems;
     }
     return TS2_OK;
 }
@@ -1389,7 +1443,6 @@ int backward(ts2_model *m)
     const int T = m->batch.node_count, D = m->D, H = m->H, L = m->L;
     const BatchDev &b = m->batch;
     const bool tune_layers = !(m->descr.flags & TS2_MPF_DISABLE_TUNE_LAYERS);
-    TS2_CUDA(cudaMemsetAsync(m->absmax, 0, (L + 2) * 4, m->stream));
     M_TRY(final_layer(m, true));
     m->gemm_tag = GEMM_TAG_DX;
     M_TRY(reduce_matrices(m, 1, 2));
@@ -1453,7 +1506,7 @@ int backward(ts2_model *m)
                 Epilogue ew;
                 ew.alpha = 1.f / m->s_act;
                 ew.dyn_scale = m->fscale;
-                ew.out_kind = TS2_OUT_F32_ADD;
+                ew.out_kind = m->dense_dw_out();
                 M_TRY(gemm_dw(m, m->kind, E, D, T, m->moe_dl, m->epad, ly.n_fast, D, m->mats[ly.mat0 + 3].grad, ew));
             }
             Epilogue e4;
@@ -1511,7 +1564,7 @@ int backward(ts2_model *m)
             Epilogue e6;
             e6.alpha = 1.f / m->s_act;
             e6.dyn_scale = m->ginv;
-            e6.out_kind = TS2_OUT_F32_ADD;
+            e6.out_kind = m->dense_dw_out();
             M_TRY(gemm_dw(m, m->kind, D, W, T, m->g_fast, D, ly.rg, W, mc.grad, e6));
             TRACE("dW_c", l, mc.grad, (size_t)D * W * 4, TR_F32);
         }
@@ -1542,7 +1595,7 @@ int backward(ts2_model *m)
             e5.alpha = 1.f / m->s_act;
             e5.dyn_scale = m->fscale;
             e5.row_scale = ly.bwd_row;
-            e5.out_kind = TS2_OUT_F32_ADD;
+            e5.out_kind = m->dense_dw_out();
             M_TRY(gemm_dw(m, m->kind, C, D, T, m->dcat, C, ly.n_fast, D, m->mats[ly.mat0].grad, e5));
             TRACE("dW_cat", l, m->mats[ly.mat0].grad, (size_t)C * D * 4, TR_F32);
         }
@@ -1591,7 +1644,7 @@ int apply(ts2_model *m, const ts2_training_step *step)
                      m->roww2));
     if (dp)
         M_NCCL(ncclAllReduce(m->roww2, m->roww2, (size_t)m->n_rows_total, ncclDouble, ncclSum, m->comm, m->stream));
-    M_TRY(opt_sko(c, m->d_optmats, n_mats, m->roww2, m->skos));
+    M_TRY(opt_sko(c, m->d_optmats, n_mats, m->roww2, m->skos, step->disp_decay));
     M_TRY(opt_quantize(c, m->d_segs_shard, m->nseg_shard, m->nitems_shard, m->w_flat, m->skos));
     if (dp) {
         M_NCCL(ncclGroupStart());
@@ -1940,7 +1993,7 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
         TS2_CUDA(cudaMemsetAsync(m->trace_dev, 0, (size_t)ts2_model::TRACE_MAX * 32, m->stream));
     }
     if (!m->grads_dirty)
-        TS2_CUDA(cudaMemsetAsync(m->grad_flat, 0, m->flat_elems * 4, m->stream));
+        M_TRY(clear_gradient(m));
     M_TRY(forward(m));
     // an accumulated gradient of earlier calls sits in the same buffer: the per-layer sums below then cover it too
     m->reduce_in_backward = add_to_model == TS2_GRADIENT_APPLY && m->comm && m->world > 1;
