@@ -157,7 +157,7 @@ struct SmemLayout {
     static constexpr int A_BYTES = BM * STAGE_ROW_BYTES;
     static constexpr int B_BYTES = BN * STAGE_ROW_BYTES;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int STAGES = (BN == 256) ? 4 : 6;
+    static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
     static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
     static constexpr int STAGING_OFFSET = BAR_OFFSET + 1024;     // epilogue staging: 8 warps x 4 KB
     static constexpr int TOTAL = STAGING_OFFSET + 4 * 2 * 4096 + 1024; // + alignment slack
@@ -869,32 +869,75 @@ static uint32_t instr_desc(int kind, bool mn, int bn)
     return d;
 }
 
-static int pick_bn(int64_t N) { return (N % 256 == 0 || N > 1024) ? 256 : 128; }
-
 struct Plan {
     int bn, m_tiles, n_tiles, k_blocks, splits, kb_per_split, grid;
 };
 
-static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int group_mode = 0, int groups = 1)
+static void finish_plan(Plan &pl, int sms, int splits, int group_mode, int groups)
 {
-    Plan pl;
-    const int es = elem_size(kind);
-    const int bk = STAGE_ROW_BYTES / es;
-    pl.bn = pick_bn(N);
-    pl.m_tiles = (int)ceil_div(M, BM);
-    pl.n_tiles = (int)ceil_div(N, pl.bn);
-    pl.k_blocks = (int)ceil_div(K, bk);
-    const int sms = sm_count(device);
-    const int tiles = std::max(1, pl.m_tiles * pl.n_tiles); // an empty problem is rejected by gemm(); keep the arithmetic defined
-    int splits = 1;
-    if (group_mode == 0 && tiles * 2 <= sms) { // fewer than half the SMs would have work: split K
-        splits = sms / tiles;
-        splits = std::min(splits, std::max(1, pl.k_blocks / 8)); // keep at least 8 K blocks per unit
-    }
     pl.kb_per_split = std::max(1, (int)ceil_div(pl.k_blocks, splits));
     pl.splits = std::max(1, (int)ceil_div(pl.k_blocks, pl.kb_per_split));
-    pl.grid = std::min(sms, tiles * pl.splits * (group_mode == 2 ? std::max(1, groups) : 1));
+    pl.grid = std::min(sms, pl.m_tiles * pl.n_tiles * pl.splits * (group_mode == 2 ? std::max(1, groups) : 1));
+}
+
+// 256-column tiles (128 for a narrow output), K split when fewer than half the SMs would have a tile: what
+// ts2_gemm_dw_noalloc promises its callers to fit into its fixed scratch depends on this rule
+static Plan fixed_plan(int device, int kind, int64_t M, int64_t N, int64_t K)
+{
+    Plan pl;
+    pl.bn = (N % 256 == 0 || N > 1024) ? 256 : 128;
+    pl.m_tiles = (int)ceil_div(M, BM);
+    pl.n_tiles = (int)ceil_div(N, pl.bn);
+    pl.k_blocks = (int)ceil_div(K, STAGE_ROW_BYTES / elem_size(kind));
+    const int sms = sm_count(device), tiles = pl.m_tiles * pl.n_tiles;
+    int splits = 1;
+    if (tiles * 2 <= sms)
+        splits = std::min(sms / tiles, std::max(1, pl.k_blocks / 8)); // keep at least 8 K blocks per unit
+    finish_plan(pl, sms, splits, 0, 1);
     return pl;
+}
+
+// Tile width and K split with the smallest estimated time.  The estimate follows measurements of single launches (us):
+//  * a K block of 128 bytes takes about the same at every width, 0.28 (0.30 at 256 columns, where the tensor pipe is
+//    busy): few tiles in flight are bound by the latency of the copies in the ring, many by the pipe;
+//  * the epilogue of a tile takes 2.4 / 1.3 / 0.8 at 256 / 128 / 64 columns, behind the main loop of the next tile
+//    where a CTA has several; start and end take 4.5, and a split another launch (3) and its partial tiles' bytes.
+// 512 x 256 x 2048 fp16 14.6 -> 9.1, 512 x 256 x 4096 23.5 -> 9.6, 3001 x 768 x 3072 int8 18.3 -> 11.5,
+// dW 4096 x 256 from 512 tokens 8.6 -> 6.5, dW 768 x 3072 from 4000 tokens 20.6 -> 17.7.  A unit keeps at least 4 K
+// blocks, and split units stay within two waves, which bounds the scratch (ts2_create reserves as much).
+static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int group_mode = 0, int groups = 1)
+{
+    Plan best;
+    double best_t = 1e30;
+    const int es = elem_size(kind), sms = sm_count(device);
+    for (int bn : {256, 128, 64}) {
+        if (bn == 64 && (group_mode || (mn && es == 1))) // a token-major one-byte operand comes in boxes of 128 columns
+            continue;
+        if (group_mode && bn != ((N % 256 == 0 || N > 1024) ? 256 : 128))
+            continue;
+        Plan pl;
+        pl.bn = bn;
+        pl.m_tiles = (int)ceil_div(M, BM);
+        pl.n_tiles = (int)ceil_div(N, bn);
+        pl.k_blocks = (int)ceil_div(K, STAGE_ROW_BYTES / es);
+        const long long tiles = std::max(1, pl.m_tiles * pl.n_tiles); // an empty problem is rejected by gemm(); keep the arithmetic defined
+        const double tk = bn == 256 ? 0.30 : 0.28, te = bn == 256 ? 2.4 : bn == 128 ? 1.3 : 0.8;
+        const int most = group_mode ? 1 : (int)std::min<long long>(2 * sms / tiles, pl.k_blocks / 4);
+        for (int splits = 1; splits <= std::max(1, most); ++splits) {
+            finish_plan(pl, sms, splits, group_mode, groups);
+            if (pl.splits != splits)
+                continue;
+            const double loop = pl.kb_per_split * tk, waves = (double)ceil_div(tiles * splits, sms);
+            double t = 4.5 + loop + te + (waves - 1) * std::max(loop, te);
+            if (splits > 1)
+                t += 3.0 + tiles * BM * bn * 4.0 * (splits + 1) / 6e6;
+            if (t < best_t) {
+                best_t = t;
+                best = pl;
+            }
+        }
+    }
+    return best;
 }
 
 int gemm_splits(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K) { return make_plan(device, kind, mn, M, N, K).splits; }
@@ -1072,8 +1115,7 @@ int gemm(const GemmArgs &a)
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad gated-activation arguments");
     Plan pl = make_plan(a.device, a.kind, a.mn_major, a.M, a.N, a.K, a.group_mode, a.groups);
     if (paired) { // one tile = 128 wide + 128 gate columns, never split along K (the epilogue needs whole sums)
-        if (pl.bn != 256)
-            return fail(TS2_ERR_UNSUPPORTED, "gemm: the gated-activation form needs 256-column tiles");
+        pl.bn = 256;
         pl.n_tiles = (int)(a.epi.pair_stride / 128);
         pl.splits = 1;
         pl.kb_per_split = pl.k_blocks;
@@ -1177,6 +1219,10 @@ int gemm(const GemmArgs &a)
         else if (es == 1 && mma == 2)
             rc = launch<256, 1, 2, false, true>(a, pl, tmA, tmB, tmC, p);
     } else {
+    TS2_GEMM_CASE(64, 1, 0, false)
+    TS2_GEMM_CASE(64, 2, 1, false)
+    TS2_GEMM_CASE(64, 1, 2, false)
+    TS2_GEMM_CASE(64, 2, 1, true)
     TS2_GEMM_CASE(256, 1, 0, false)
     TS2_GEMM_CASE(128, 1, 0, false)
     TS2_GEMM_CASE(256, 1, 0, true)
@@ -1295,7 +1341,7 @@ extern "C" int ts2_gemm_dw_noalloc(int device, void *stream, int prec, int out_k
     int rc = static_setup(device, &st);
     if (rc != TS2_OK)
         return rc;
-    const Plan pl = make_plan(device, kind, true, out_dim, in_dim, T);
+    const Plan pl = fixed_plan(device, kind, out_dim, in_dim, T);
     const size_t need = pl.splits > 1 ? (size_t)pl.m_tiles * pl.n_tiles * pl.splits * BM * pl.bn * sizeof(float) : 0;
     if (need > STATIC_SCRATCH_BYTES)
         return fail(TS2_ERR_TOO_LARGE,
