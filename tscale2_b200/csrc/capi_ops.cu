@@ -124,10 +124,9 @@ int ts2_gemm_tn(int device, void *stream, int prec, int out_kind, int64_t M, int
     a.epi.row_scale = row_scale;
     a.epi.col_scale = col_scale;
     a.epi.out_kind = out_kind;
-    if (gemm_splits(device, a.kind, false, M, N, K) > 1) {
+    if (const size_t need = gemm_workspace_bytes(device, a.kind, false, M, N, K, out_kind)) {
         // few output tiles and a long K: the scheduler splits K and needs scratch for the partial
         // tiles; this entry point takes it from the library's stream-ordered scratch pool for the call.
-        size_t need = gemm_workspace_bytes(device, a.kind, false, M, N, K);
         void *ws = nullptr;
         TS2_CUDA(cudaSetDevice(device));
         if (int rc = scratch_alloc(device, need, a.stream, &ws))

@@ -18,7 +18,7 @@
 // Fp16MatMul (src/lib/cuda/cuda_fp16.cuh:49-164), and, because the dW operands are read
 // token-major through MN-major shared-memory descriptors, also the per-step transposes
 // (src/gpt/compute/matmul_fwdbwd.cuh:149-162,169-280).
-#include "gemm.cuh"
+#include "gemm_params.cuh"
 #include "fast_types.cuh"
 #include <cuda.h>
 #include <vector>
@@ -27,47 +27,8 @@
 
 namespace ts2 {
 
-static constexpr int BM = 128;
-static constexpr int STAGE_ROW_BYTES = 128; // one swizzle row
 static constexpr int NUM_THREADS = 320; // TMA warp, MMA warp, 8 epilogue warps (two per TMEM lane quarter)
 static constexpr int NUM_THREADS_GATED = 576; // the gated-activation epilogue does more per element: 16 epilogue warps
-
-struct GemmParams {
-    int M, N;
-    int m_tiles, n_tiles, splits;
-    int n_fast;        // tile order: consecutive tiles walk N first (the CTAs of a wave share A rows) or M first (share B rows)
-    int k_blocks;      // total K blocks (one block = one pipeline stage)
-    int kb_per_split;
-    uint32_t idesc;
-    void *C;
-    long long ldc;
-    float alpha;
-    const float *dyn_scale, *dyn_scale2, *row_scale, *col_scale, *c_in;
-    int out_kind;
-    float *workspace;
-    int32_t *status;
-    // dynamic unit scheduler: {next unit, finished CTAs}, both zero between launches (the last CTA to finish resets
-    // them); null: unit i of CTA b is b + i * gridDim.x
-    int *sched = nullptr;
-    // grouped forms (mixture-of-experts): 0 none; 1 every 128-row M tile belongs to one group (tile_group[m_tile],
-    // negative: skip) and reads B rows [group * group_rows_b + n]; 2 the K range of a unit is the row segment of
-    // its group (group_kptr[g] .. group_kptr[g+1], multiples of the K block) and C moves by c_group_stride per group
-    int group_mode, groups;
-    const int *tile_group;
-    int group_rows_b;
-    const int *group_kptr;
-    long long c_group_stride;
-    int bk;
-    int tma_store; // the epilogue stages 32-row blocks in shared memory and writes them with TMA (tmC)
-    // gated-activation form (see Epilogue in gemm.cuh): a tile is 128 "wide" columns [nt * 128, +128) and the 128
-    // "gate" columns pair_stride further on
-    int pair_stride = 0;
-    void *act_out = nullptr;
-    long long act_ld = 0;
-    float *act_scale = nullptr;
-    float act_mult = 1.f;
-    int act_kind = 0; // format of act_out: 0 e4m3, 1 fp16, 2 int8
-};
 
 struct Unit {
     int m0, n0, nt, kb0, kb1, b_row_off;
@@ -748,12 +709,12 @@ __global__ void __launch_bounds__(GATED ? NUM_THREADS_GATED : NUM_THREADS, 1)
 }
 
 // Sums the K-split partial tiles in split order and applies the epilogue.
-template <int BN>
+template <int BM_, int BN>
 __global__ void reduce_splitk_kernel(const GemmParams p)
 {
     grid_dep_wait();
     const int tiles = p.m_tiles * p.n_tiles;
-    const int vec_per_tile = BM * BN / 4;
+    const int vec_per_tile = BM_ * BN / 4;
     const long long total = (long long)tiles * vec_per_tile;
     float alpha = p.alpha;
     if (p.dyn_scale)
@@ -765,13 +726,13 @@ __global__ void reduce_splitk_kernel(const GemmParams p)
         const int r = e / (BN / 4), c = (e % (BN / 4)) * 4;
         int mt, nt;
         tile_coords(p, tile, mt, nt);
-        const long long row = (long long)mt * BM + r;
+        const long long row = (long long)mt * BM_ + r;
         const int col = nt * BN + c;
         if (row >= p.M || col >= p.N)
             continue;
         float4 s = make_float4(0, 0, 0, 0);
         for (int sp = 0; sp < p.splits; ++sp) {
-            float4 v = *(const float4 *)(p.workspace + ((size_t)(tile * p.splits + sp) * BM + r) * BN + c);
+            float4 v = *(const float4 *)(p.workspace + ((size_t)(tile * p.splits + sp) * BM_ + r) * BN + c);
             s.x += v.x;
             s.y += v.y;
             s.z += v.z;
@@ -849,7 +810,7 @@ int make_tensor_map(::CUtensorMap_st *tm, const void *base, int es, int64_t inne
 
 static int elem_size(int kind) { return (kind == KIND_F16 || kind == KIND_BF16) ? 2 : 1; }
 
-static uint32_t instr_desc(int kind, bool mn, int bn)
+static uint32_t instr_desc(int kind, bool mn, int bm, int bn)
 {
     uint32_t c_fmt, ab_fmt;
     switch (kind) {
@@ -865,19 +826,23 @@ static uint32_t instr_desc(int kind, bool mn, int bn)
     d |= (mn ? 1u : 0u) << 15; // A is MN-major
     d |= (mn ? 1u : 0u) << 16; // B is MN-major
     d |= (uint32_t)(bn >> 3) << 17;
-    d |= (uint32_t)(BM >> 4) << 24;
+    d |= (uint32_t)(bm >> 4) << 24;
     return d;
 }
 
 struct Plan {
-    int bn, m_tiles, n_tiles, k_blocks, splits, kb_per_split, grid;
+    int bm = BM, bn; // 256 x 256: on pairs of CTAs (gemm_pair.cu)
+    int m_tiles, n_tiles, k_blocks, splits, kb_per_split, grid;
+    bool pair() const { return bm == 2 * BM; }
+    size_t workspace() const { return splits > 1 ? (size_t)m_tiles * n_tiles * splits * bm * bn * sizeof(float) : 0; }
 };
 
 static void finish_plan(Plan &pl, int sms, int splits, int group_mode, int groups)
 {
     pl.kb_per_split = std::max(1, (int)ceil_div(pl.k_blocks, splits));
     pl.splits = std::max(1, (int)ceil_div(pl.k_blocks, pl.kb_per_split));
-    pl.grid = std::min(sms, pl.m_tiles * pl.n_tiles * pl.splits * (group_mode == 2 ? std::max(1, groups) : 1));
+    const int units = pl.m_tiles * pl.n_tiles * pl.splits * (group_mode == 2 ? std::max(1, groups) : 1);
+    pl.grid = pl.pair() ? 2 * std::min(sms / 2, units) : std::min(sms, units);
 }
 
 // 256-column tiles (128 for a narrow output), K split when fewer than half the SMs would have a tile: what
@@ -897,40 +862,56 @@ static Plan fixed_plan(int device, int kind, int64_t M, int64_t N, int64_t K)
     return pl;
 }
 
-// Tile width and K split with the smallest estimated time.  The estimate follows measurements of single launches (us):
+enum { FORM_F32, FORM_ADD, FORM_16, FORM_GATED };
+static int form_of(const Epilogue &e)
+{
+    return e.pair_stride ? FORM_GATED : e.out_kind == TS2_OUT_F32_ADD ? FORM_ADD : e.out_kind == TS2_OUT_F32 ? FORM_F32 : FORM_16;
+}
+
+// Tile and K split with the smallest estimated time.  The estimate follows measurements of single launches (us):
 //  * a K block of 128 bytes takes about the same at every width, 0.28 (0.30 at 256 columns, where the tensor pipe is
 //    busy): few tiles in flight are bound by the latency of the copies in the ring, many by the pipe;
-//  * the epilogue of a tile takes 2.4 / 1.3 / 0.8 at 256 / 128 / 64 columns, behind the main loop of the next tile
-//    where a CTA has several; start and end take 4.5, and a split another launch (3) and its partial tiles' bytes.
+//  * the epilogue of a tile takes 2.4 / 1.3 / 0.8 at 256 / 128 / 64 columns, 2.5 times as much where it adds a residual
+//    input, behind the main loop of the next tile where a CTA has several; start and end take 4.5, and a split another
+//    launch (3) and its partial tiles' bytes;
+//  * a pair of CTAs (gemm_pair.cu) starts later (7.5) and then takes 0.85 of that per tile, residual input or not.
 // 512 x 256 x 2048 fp16 14.6 -> 9.1, 512 x 256 x 4096 23.5 -> 9.6, 3001 x 768 x 3072 int8 18.3 -> 11.5,
-// dW 4096 x 256 from 512 tokens 8.6 -> 6.5, dW 768 x 3072 from 4000 tokens 20.6 -> 17.7.  A unit keeps at least 4 K
-// blocks, and split units stay within two waves, which bounds the scratch (ts2_create reserves as much).
-static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int group_mode = 0, int groups = 1)
+// dW 4096 x 256 from 512 tokens 8.6 -> 6.5, dW 768 x 3072 from 4000 tokens 20.6 -> 17.7; pairs: 65536 x 768 x 1536 e4m3
+// with residual input 142 -> 112, 32768 x 2048 x 2048 211 -> 152, dX + dW of 16384 x 4096 x 4096 482 -> 466.  A unit keeps
+// at least 4 K blocks, and split units stay within two waves, which bounds the scratch (ts2_create reserves as much).
+static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int form, int group_mode = 0, int groups = 1)
 {
     Plan best;
     double best_t = 1e30;
     const int es = elem_size(kind), sms = sm_count(device);
-    for (int bn : {256, 128, 64}) {
-        if (bn == 64 && (group_mode || (mn && es == 1))) // a token-major one-byte operand comes in boxes of 128 columns
-            continue;
-        if (group_mode && bn != ((N % 256 == 0 || N > 1024) ? 256 : 128))
-            continue;
+    const struct {
+        int bm, bn;
+        double start, block, epilogue;
+    } tiles_of[] = {{2 * BM, 256, 7.5, 0.255, 2.0}, {BM, 256, 4.5, 0.30, 2.4}, {BM, 128, 4.5, 0.28, 1.3}, {BM, 64, 4.5, 0.28, 0.8}};
+    for (const auto &shape : tiles_of) {
         Plan pl;
-        pl.bn = bn;
-        pl.m_tiles = (int)ceil_div(M, BM);
-        pl.n_tiles = (int)ceil_div(N, bn);
+        pl.bm = shape.bm;
+        pl.bn = shape.bn;
+        if (group_mode && (pl.pair() || pl.bn != ((N % 256 == 0 || N > 1024) ? 256 : 128)))
+            continue;
+        // a token-major one-byte operand comes in boxes of 128 columns; the gated form takes 128 wide and 128 gate columns
+        if ((pl.bn == 64 && mn && es == 1) || (form == FORM_GATED && pl.bn != 256))
+            continue;
+        pl.m_tiles = (int)ceil_div(M, pl.bm);
+        pl.n_tiles = (int)ceil_div(N, pl.bn);
         pl.k_blocks = (int)ceil_div(K, STAGE_ROW_BYTES / es);
+        const int workers = pl.pair() ? sms / 2 : sms;
         const long long tiles = std::max(1, pl.m_tiles * pl.n_tiles); // an empty problem is rejected by gemm(); keep the arithmetic defined
-        const double tk = bn == 256 ? 0.30 : 0.28, te = bn == 256 ? 2.4 : bn == 128 ? 1.3 : 0.8;
-        const int most = group_mode ? 1 : (int)std::min<long long>(2 * sms / tiles, pl.k_blocks / 4);
+        const double te = shape.epilogue * (form == FORM_ADD && !pl.pair() ? 2.5 : 1.0);
+        const int most = group_mode || form == FORM_GATED ? 1 : (int)std::min<long long>(2 * workers / tiles, pl.k_blocks / 4);
         for (int splits = 1; splits <= std::max(1, most); ++splits) {
             finish_plan(pl, sms, splits, group_mode, groups);
             if (pl.splits != splits)
                 continue;
-            const double loop = pl.kb_per_split * tk, waves = (double)ceil_div(tiles * splits, sms);
-            double t = 4.5 + loop + te + (waves - 1) * std::max(loop, te);
+            const double loop = pl.kb_per_split * shape.block, waves = (double)ceil_div(tiles * splits, workers);
+            double t = shape.start + loop + te + (waves - 1) * std::max(loop, te);
             if (splits > 1)
-                t += 3.0 + tiles * BM * bn * 4.0 * (splits + 1) / 6e6;
+                t += 3.0 + tiles * pl.bm * pl.bn * 4.0 * (splits + 1) / 6e6;
             if (t < best_t) {
                 best_t = t;
                 best = pl;
@@ -940,14 +921,16 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
     return best;
 }
 
-int gemm_splits(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K) { return make_plan(device, kind, mn, M, N, K).splits; }
-
-size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K)
+size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int out_kind)
 {
-    Plan pl = make_plan(device, kind, mn, M, N, K);
-    if (pl.splits == 1)
-        return 0;
-    return (size_t)pl.m_tiles * pl.n_tiles * pl.splits * BM * pl.bn * sizeof(float);
+    size_t need = 0;
+    for (int out : {TS2_OUT_F32, TS2_OUT_F32_ADD, TS2_OUT_F16, TS2_OUT_BF16}) {
+        Epilogue e;
+        e.out_kind = out;
+        if (out_kind < 0 || out == out_kind)
+            need = std::max(need, make_plan(device, kind, mn, M, N, K, form_of(e)).workspace());
+    }
+    return need;
 }
 
 // Counters of the dynamic unit scheduler: SCHED_SLOTS pairs {next unit, finished CTAs} per device, zero between
@@ -1066,6 +1049,15 @@ static cudaEvent_t pooled_event()
     return e;
 }
 
+template <int BM_, int BN>
+static int reduce_splits(const GemmArgs &a, const Plan &pl, const GemmParams &p)
+{
+    const long long total = (long long)pl.m_tiles * pl.n_tiles * BM_ * BN / 4;
+    const int blocks = (int)std::min<long long>(ceil_div(total, 256), 4 * sm_count(a.device));
+    TS2_LAUNCH((reduce_splitk_kernel<BM_, BN>), blocks, 256, 0, a.stream, p);
+    return TS2_OK;
+}
+
 template <int BN, int ES, int MMA, bool MN, bool GATED = false>
 static int launch(const GemmArgs &a, const Plan &pl, const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmC,
                   const GemmParams &p)
@@ -1080,11 +1072,8 @@ static int launch(const GemmArgs &a, const Plan &pl, const CUtensorMap &tmA, con
     // taken starts only when another CTA of the grid has finished all of its units, which can double the launch's time
     const int grid = std::max(1, std::min(pl.grid, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)));
     TS2_LAUNCH((kern), grid, GATED ? NUM_THREADS_GATED : NUM_THREADS, SmemLayout<BN>::TOTAL, a.stream, tmA, tmB, tmC, p);
-    if (pl.splits > 1) {
-        const long long total = (long long)pl.m_tiles * pl.n_tiles * BM * BN / 4;
-        int blocks = (int)std::min<long long>(ceil_div(total, 256), 4 * sm_count(a.device));
-        TS2_LAUNCH((reduce_splitk_kernel<BN>), blocks, 256, 0, a.stream, p);
-    }
+    if (pl.splits > 1)
+        return reduce_splits<BM, BN>(a, pl, p);
     return TS2_OK;
 }
 
@@ -1113,16 +1102,13 @@ int gemm(const GemmArgs &a)
                    a.epi.act_kind < 0 || a.epi.act_kind > 2 || (a.epi.act_ld * (a.epi.act_kind == 1 ? 2 : 1)) % 16 ||
                    ((uintptr_t)a.epi.act_out & 15)))
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad gated-activation arguments");
-    Plan pl = make_plan(a.device, a.kind, a.mn_major, a.M, a.N, a.K, a.group_mode, a.groups);
+    Plan pl = make_plan(a.device, a.kind, a.mn_major, a.M, a.N, a.K, form_of(a.epi), a.group_mode, a.groups);
     if (paired) { // one tile = 128 wide + 128 gate columns, never split along K (the epilogue needs whole sums)
-        pl.bn = 256;
         pl.n_tiles = (int)(a.epi.pair_stride / 128);
-        pl.splits = 1;
-        pl.kb_per_split = pl.k_blocks;
-        pl.grid = std::min(sm_count(a.device), pl.m_tiles * pl.n_tiles);
+        finish_plan(pl, sm_count(a.device), 1, 0, 1);
     }
     if (pl.splits > 1) {
-        size_t need = (size_t)pl.m_tiles * pl.n_tiles * pl.splits * BM * pl.bn * sizeof(float);
+        const size_t need = pl.workspace();
         if (!a.workspace || a.workspace_bytes < need)
             return fail(TS2_ERR_INVALID_ARG, "gemm: split-K needs %zu workspace bytes, got %zu", need, a.workspace_bytes);
     }
@@ -1132,7 +1118,8 @@ int gemm(const GemmArgs &a)
     if (!a.mn_major) {
         if ((rc = make_tmap(&tmA, a.A, es, a.K, a.M, a.lda, BM)) != TS2_OK)
             return rc;
-        if ((rc = make_tmap(&tmB, a.B, es, a.K, a.group_mode == 1 ? a.N * a.groups : a.N, a.ldb, paired ? pl.bn / 2 : pl.bn)) != TS2_OK)
+        if ((rc = make_tmap(&tmB, a.B, es, a.K, a.group_mode == 1 ? a.N * a.groups : a.N, a.ldb,
+                            paired || pl.pair() ? pl.bn / 2 : pl.bn)) != TS2_OK)
             return rc;
     } else {
         if ((rc = make_tmap(&tmA, a.A, es, a.M, a.K, a.lda, bk)) != TS2_OK)
@@ -1149,7 +1136,7 @@ int gemm(const GemmArgs &a)
     p.splits = pl.splits;
     p.k_blocks = pl.k_blocks;
     p.kb_per_split = pl.kb_per_split;
-    p.idesc = instr_desc(a.kind, a.mn_major, pl.bn);
+    p.idesc = instr_desc(a.kind, a.mn_major, pl.bm, pl.bn);
     p.C = a.C;
     p.ldc = a.ldc;
     p.alpha = a.epi.alpha;
@@ -1185,9 +1172,18 @@ int gemm(const GemmArgs &a)
     p.act_kind = a.epi.act_kind;
     // coalesced TMA-store epilogue (the accumulate form adds its residual input first; split units go to the workspace;
     // per-group C offsets of mode 2 are not expressible as one 2-D map)
-    CUtensorMap tmC = tmA;
+    CUtensorMap tmC = tmA, tmCin = tmA;
     p.tma_store = 0;
-    if (pl.splits == 1 && a.group_mode != 2) {
+    if (pl.pair()) { // every output leaves by TMA, partial tiles as rows of 256 in the workspace
+        if (pl.splits > 1)
+            rc = make_tmap(&tmC, a.workspace, 4, pl.bn, (int64_t)pl.m_tiles * pl.n_tiles * pl.splits * pl.bm, pl.bn, 32);
+        else
+            rc = make_tmap(&tmC, a.C, out_es, a.N, a.M, a.ldc, 32, paired ? 64 : STAGE_ROW_BYTES);
+        if (rc == TS2_OK && pl.splits == 1 && a.epi.out_kind == TS2_OUT_F32_ADD)
+            rc = make_tmap(&tmCin, p.c_in, 4, a.N, a.M, a.ldc, 32);
+        if (rc != TS2_OK)
+            return rc;
+    } else if (pl.splits == 1 && a.group_mode != 2) {
         if ((rc = make_tmap(&tmC, a.C, out_es, a.N, a.M, a.ldc, 32, 64)) != TS2_OK)
             return rc;
         p.tma_store = 1;
@@ -1211,7 +1207,12 @@ int gemm(const GemmArgs &a)
     if (pl.bn == BN_ && es == ES_ && mma == MMA_ && a.mn_major == MN_)       \
         rc = launch<BN_, ES_, MMA_, MN_>(a, pl, tmA, tmB, tmC, p);
     rc = TS2_ERR_UNSUPPORTED;
-    if (paired) {
+    if (pl.pair()) {
+        const int sms = std::max(2, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)) & ~1;
+        rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, paired, std::min(pl.grid, sms), tmA, tmB, tmC, tmCin, p);
+        if (rc == TS2_OK && pl.splits > 1)
+            rc = reduce_splits<2 * BM, 256>(a, pl, p);
+    } else if (paired) {
         if (es == 1 && mma == 0)
             rc = launch<256, 1, 0, false, true>(a, pl, tmA, tmB, tmC, p);
         else if (es == 2 && mma == 1)
@@ -1363,7 +1364,7 @@ extern "C" int ts2_gemm_dw_noalloc(int device, void *stream, int prec, int out_k
     p.splits = pl.splits;
     p.k_blocks = pl.k_blocks;
     p.kb_per_split = pl.kb_per_split;
-    p.idesc = instr_desc(kind, true, pl.bn);
+    p.idesc = instr_desc(kind, true, BM, pl.bn);
     p.C = dW;
     p.ldc = in_dim;
     p.alpha = alpha;

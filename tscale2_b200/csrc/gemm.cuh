@@ -57,9 +57,8 @@ struct GemmArgs {
     size_t workspace_bytes = 0;
 };
 
-// number of K splits the scheduler will use for this shape (1 = no workspace needed)
-int gemm_splits(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_t K);
-size_t gemm_workspace_bytes(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_t K);
+// bytes of scratch this shape needs for its K splits (0: none); out_kind < 0: whatever the output
+size_t gemm_workspace_bytes(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_t K, int out_kind = -1);
 int gemm(const GemmArgs &a);
 
 // 2-D TMA descriptor over a row-major [rows][ld] array of es-byte elements: box = 128 bytes x box_rows, 128-byte swizzle,
