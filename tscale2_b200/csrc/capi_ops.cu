@@ -383,8 +383,10 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
     Ctx c;
     c.device = device;
     c.stream = (cudaStream_t)stream;
-    // start | finish | rev_first | rev_last | scan scratch
-    SpanScratch spans(c, span_start, span_finish, T, 4 * (size_t)T + batch_scan_tmp_elems(T));
+    const bool tc = variant == 2 || variant == 3;
+    // start | finish | rev_first | rev_last | scan scratch, then the backward kernels' layout and records
+    const size_t tables = ((4 * (size_t)T + batch_scan_tmp_elems(T)) * 4 + 255) / 256 * 256, layout = (att_layout_bytes(T) + 255) / 256 * 256;
+    SpanScratch spans(c, span_start, span_finish, T, (tables + (tc ? layout + att_bwd_scratch_bytes(T, head_count) : 0)) / 4);
     if (spans.rc != TS2_OK)
         return spans.rc;
     int *d = spans.d;
@@ -392,13 +394,23 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
         return rc0;
     const __half *Q = (const __half *)q, *K = (const __half *)k, *V = (const __half *)v, *DO = (const __half *)dout;
     float *fq = (float *)dq, *fk = (float *)dk, *fv = (float *)dv;
-    int rc = variant == 2 || variant == 3
-                 ? attention_backward_tc(c, Q, K, V, DO, lse, dscale, d, d + T, d + 2 * T, d + 3 * T, T, head_count, alibi_slope, dq, dk, dv,
-                                         variant == 3)
-             : variant == 0 ? attention_backward_mma(c, Q, K, V, DO, lse, dscale, d, d + T, d + 2 * T, d + 3 * T, T, head_count, alibi_slope,
-                                                   fq, fk, fv)
-                          : attention_backward_rowwise(c, Q, K, V, DO, lse, dscale, d, d + T, d + 2 * T, d + 3 * T, T, head_count,
-                                                       alibi_slope, fq, fk, fv);
+    int rc = TS2_OK;
+    if (tc) {
+        AttBwdPlan plan;
+        plan.layout = (uint8_t *)d + tables;
+        plan.scratch = (uint8_t *)d + tables + layout;
+        plan.ds_bytes = att_ds_bytes(T, nullptr, span_start, span_finish) * head_count;
+        if (plan.ds_bytes == 0 || plan.ds_bytes > ATT_DS_MAX_BYTES || scratch_alloc(device, plan.ds_bytes, c.stream, &plan.ds) != TS2_OK)
+            plan.ds = nullptr, plan.ds_bytes = 0;
+        if ((rc = att_layout(c, d, d + T, d + 2 * (size_t)T, d + 3 * (size_t)T, T, plan.layout)) == TS2_OK)
+            rc = attention_backward(c, Q, K, V, DO, lse, dscale, d, d + T, plan, T, head_count, alibi_slope, dq, dk, dv, variant == 3);
+        if (plan.ds)
+            scratch_free(c.stream, plan.ds);
+    } else {
+        rc = variant == 0 ? attention_backward_mma(c, Q, K, V, DO, lse, dscale, d, d + T, d + 2 * T, d + 3 * T, T, head_count, alibi_slope, fq, fk, fv)
+                          : attention_backward_rowwise(c, Q, K, V, DO, lse, dscale, d, d + T, d + 2 * T, d + 3 * T, T, head_count, alibi_slope,
+                                                       fq, fk, fv);
+    }
     cudaStreamSynchronize(c.stream);
     return rc;
 }

@@ -116,7 +116,7 @@ static cudaMemPool_t scratch_pool(int device, bool create)
             p = nullptr;
             return nullptr;
         }
-        uint64_t keep = 64ull << 20;
+        uint64_t keep = 2ull << 30;
         cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     return p;

@@ -93,7 +93,7 @@ int32_t *static_status_word_if_ready(int device);
 int collect_device_status(int device);
 
 // Scratch of the operator-level calls, stream-ordered, from a pool of the library's own on each device that keeps up to
-// 64 MB between calls (a default pool keeps nothing: after every synchronisation the next call mapped its scratch anew,
+// 2 GB between calls (what the largest attention call of a few tens of thousand nodes takes) (a default pool keeps nothing: after every synchronisation the next call mapped its scratch anew,
 // 0.3 - 0.5 ms).  Any thread and stream; scratch_trim gives what is unused back (called when an allocation fails).
 int scratch_alloc(int device, size_t bytes, cudaStream_t stream, void **ptr);
 void scratch_free(cudaStream_t stream, void *ptr);

@@ -61,9 +61,9 @@ struct GemmArgs {
 size_t gemm_workspace_bytes(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_t K, int out_kind = -1);
 int gemm(const GemmArgs &a);
 
-// 2-D TMA descriptor over a row-major [rows][ld] array of es-byte elements: box = 128 bytes x box_rows, 128-byte swizzle,
-// out-of-range elements read as zero
-int make_tensor_map(::CUtensorMap_st *tm, const void *base, int es, int64_t inner, int64_t rows, int64_t ld, int box_rows);
+// 2-D TMA descriptor over a row-major [rows][ld] array of es-byte elements: box = row_bytes (128 or 64, swizzled alike) x
+// box_rows, out-of-range elements read as zero
+int make_tensor_map(::CUtensorMap_st *tm, const void *base, int es, int64_t inner, int64_t rows, int64_t ld, int box_rows, int row_bytes = 128);
 
 // SMs the contraction's persistent grid leaves free (for communication kernels that run beside it); process-wide
 void gemm_reserve_sms(int n);

@@ -145,9 +145,25 @@ int fill_rope(const Ctx &c, float *rope, int T);
 // o [T][Q] fp16, lse [T][H] = maxDP + log2(sumWeight); dq, dk, dv fp32, or fp16 with grads16
 int attention_forward(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
                       int T, int H, float slope, __half *o, float *lse);
+// What the backward kernels need besides the layer's tensors.
+//  layout (att_layout_bytes): the batch's spans in the form they read, made once per batch by att_layout
+//  scratch (att_bwd_scratch_bytes): per-node records of the call
+//  ds: the score gradients between the dK / dV and the dQ kernel, 16 KB per (128-key block, 64-node tile, head) that meet;
+//      att_ds_bytes bounds it for a batch.  Too small (null): dQ recomputes the scores instead.
+struct AttBwdPlan {
+    void *layout = nullptr, *scratch = nullptr, *ds = nullptr;
+    size_t ds_bytes = 0;
+};
+constexpr size_t ATT_DS_MAX_BYTES = (size_t)4 << 30; // most that is set aside for dS
+size_t att_layout_bytes(int T);
+size_t att_bwd_scratch_bytes(int T, int H);
+int att_layout(const Ctx &c, const int *span_start, const int *span_finish, const int *rev_first, const int *rev_last, int T, void *layout);
+// bytes of dS per head for a batch given by its raw span arrays (host; span_ptr null: one span per node, empty where
+// finish < start), an upper bound; with no arrays at all, the bound for any spans over T nodes
+size_t att_ds_bytes(int T, const int *span_ptr, const int *span_start, const int *span_finish);
 int attention_backward(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,
-                       const float *dscale, const int *span_start, const int *span_finish, const int *rev_first, const int *rev_last,
-                       int T, int H, float slope, void *dq, void *dk, void *dv, bool grads16 = false);
+                       const float *dscale, const int *span_start, const int *span_finish, const AttBwdPlan &plan, int T, int H, float slope,
+                       void *dq, void *dk, void *dv, bool grads16 = false);
 
 // the two formulations behind attention_forward / attention_backward
 int attention_forward_mma(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
@@ -157,9 +173,6 @@ int attention_backward_mma(const Ctx &c, const __half *q, const __half *k, const
                            const int *rev_last, int T, int H, float slope, float *dq, float *dk, float *dv);
 int attention_forward_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
                          int T, int H, float slope, __half *o, float *lse);
-int attention_backward_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,
-                          const float *dscale, const int *span_start, const int *span_finish, const int *rev_first, const int *rev_last,
-                          int T, int H, float slope, void *dq, void *dk, void *dv, bool grads16 = false);
 int attention_forward_rowwise(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start,
                               const int *span_finish, int T, int H, float slope, __half *o, float *lse);
 int attention_backward_rowwise(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,

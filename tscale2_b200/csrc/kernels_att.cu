@@ -326,12 +326,4 @@ int attention_forward(const Ctx &c, const __half *q, const __half *k, const __ha
     return attention_forward_tc(c, q, k, v, span_start, span_finish, T, H, slope, o, lse);
 }
 
-int attention_backward(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,
-                       const float *dscale, const int *span_start, const int *span_finish, const int *rev_first, const int *rev_last,
-                       int T, int H, float slope, void *dq, void *dk, void *dv, bool grads16)
-{
-    return attention_backward_tc(c, q, k, v, dout, lse, dscale, span_start, span_finish, rev_first, rev_last, T, H, slope, dq, dk, dv,
-                                 grads16);
-}
-
 } // namespace ts2

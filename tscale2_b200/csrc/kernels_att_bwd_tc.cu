@@ -1,7 +1,8 @@
-// tcgen05 attention backward for head width 128 (sm_100a): dQ, the packing of the per-node records, and the entry
-// point of the backward pass (dK and dV come from kernels_att_bwd_kv_tc.cu).  Same math, inputs and outputs as the
-// mma.sync formulation in kernels_att_mma.cu (see there for the references into
-// src/gpt/compute/layer_att_reference.h and gpu_att_fp16.cu).
+// tcgen05 attention backward for head width 128 (sm_100a): the entry point (dK, dV and the score gradients come from
+// kernels_att_bwd_kv_tc.cu, dQ from kernels_att_bwd_dq_tc.cu), and the dQ kernel for batches whose score gradients do not
+// fit the memory set aside for them, which recomputes the scores.  Same math, inputs and outputs as the mma.sync
+// formulation in kernels_att_mma.cu (see there for the references into src/gpt/compute/layer_att_reference.h and
+// gpu_att_fp16.cu).
 //
 // dQ: a CTA owns 256 resident nodes (Q and dO rows) as two blocks of 128, and streams 64-key tiles of K and V once
 // for both blocks (half the L2 traffic of one block per CTA):
@@ -13,7 +14,8 @@
 // CTA with two S / dP pairs, the structure of the dK / dV kernel, was measured slower here: twice the CTAs and twice
 // the streamed bytes.)  Every wait is bounded (see mbar_wait); a give-up raises the status word.
 #include "att_tc.cuh"
-#include <mutex>
+#include <algorithm>
+#include <vector>
 
 namespace ts2 {
 
@@ -40,25 +42,6 @@ struct BwdLayout {
     static constexpr int SMEM = BAR_OFF + 256;
 };
 static_assert(BwdLayout::SMEM <= 232448, "shared memory budget");
-
-// {-lse, -dscale * c2, start, finish - start} per (head, node); nodes past T and nodes with an empty span get a
-// start no key index reaches
-__global__ void att_pack_meta_kernel(const float *__restrict__ lse, const float *__restrict__ dscale, const int *__restrict__ span_start,
-                                     const int *__restrict__ span_finish, int T, int Tpad, int H, float c2, float4 *__restrict__ meta)
-{
-    grid_dep_wait();
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= Tpad * H)
-        return;
-    const int h = idx / Tpad, t = idx - h * Tpad;
-    float4 m = make_float4(0.f, 0.f, __int_as_float(0x40000000), __int_as_float(0));
-    if (t < T) {
-        const int st = span_start[t], fi = span_finish[t];
-        if (fi >= st)
-            m = make_float4(-lse[(size_t)t * H + h], -dscale[(size_t)t * H + h] * c2, __int_as_float(st), __int_as_float(fi - st));
-    }
-    meta[idx] = m;
-}
 
 // OUT16: dQ is written as fp16 (what the engine feeds its next kernel with) instead of fp32
 template <bool OUT16>
@@ -383,59 +366,63 @@ static int launch_bwd_dq(const Ctx &c, const __half *a1, const __half *a2, const
     return TS2_OK;
 }
 
-// per-device buffer of the packed per-node quantities, grown on demand (never inside a steady-state step:
-// the node count of a model is fixed)
-static int meta_buffer(int device, size_t bytes, float4 **out)
+size_t att_ds_bytes(int T, const int *span_ptr, const int *span_start, const int *span_finish)
 {
-    static std::mutex mu;
-    static float4 *buf[16] = {};
-    static size_t cap[16] = {};
-    std::lock_guard<std::mutex> lock(mu);
-    const int d = device & 15;
-    if (cap[d] < bytes) {
-        if (buf[d]) {
-            TS2_CUDA(cudaDeviceSynchronize());
-            TS2_CUDA(cudaFree(buf[d]));
-            buf[d] = nullptr;
-            cap[d] = 0;
+    const size_t nb = (size_t)ceil_div(T, TC_BM), tile = (size_t)TC_BM * TC_BN * 2;
+    if (!span_start || !span_finish)
+        return nb * nb * 2 * tile;
+    // as the device derives it: prefix maximum of the span ends, suffix minimum of the span starts, two searches per block
+    std::vector<int> run_max(T), suf_min(T);
+    int mx = -1, mn = T;
+    for (int t = 0; t < T; ++t) {
+        int at = t;
+        bool has = true;
+        if (span_ptr) {
+            at = span_ptr[t];
+            has = span_ptr[t + 1] == at + 1 && at >= 0 && at < span_ptr[T];
         }
-        TS2_CUDA(cudaMalloc(&buf[d], bytes));
-        cap[d] = bytes;
+        const int s = has ? span_start[at] : 0, f = has ? span_finish[at] : -1;
+        has = has && s >= 0 && f < T && f >= s;
+        mx = std::max(mx, has ? f : -1);
+        run_max[t] = mx;
+        suf_min[t] = has ? s : T;
     }
-    *out = buf[d];
-    return TS2_OK;
+    for (int t = T - 1; t >= 0; --t)
+        suf_min[t] = mn = std::min(mn, suf_min[t]);
+    size_t tiles = 0;
+    for (int k0 = 0; k0 < T; k0 += TC_BM) {
+        const int k1 = std::min(T, k0 + TC_BM) - 1;
+        const int first = (int)(std::lower_bound(run_max.begin(), run_max.end(), k0) - run_max.begin());
+        const int last = (int)(std::upper_bound(suf_min.begin(), suf_min.end(), k1) - suf_min.begin()) - 1;
+        if (first <= last)
+            tiles += (size_t)(last / TC_BM - first / TC_BM + 1) * 2;
+    }
+    return tiles * tile;
 }
 
-int attention_backward_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,
-                          const float *dscale, const int *span_start, const int *span_finish, const int *rev_first, const int *rev_last,
-                          int T, int H, float slope, void *dq, void *dk, void *dv, bool grads16)
+// With room for the score gradients: dK, dV and dS from one kernel, then dQ = dS . K.  Without, dQ recomputes the scores
+// (the kernel above).
+int attention_backward(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,
+                       const float *dscale, const int *span_start, const int *span_finish, const AttBwdPlan &plan, int T, int H, float slope,
+                       void *dq, void *dk, void *dv, bool grads16)
 {
+    if (int rc = attention_backward_kv_tc(c, q, k, v, dout, lse, dscale, plan, T, H, slope, dk, dv, grads16))
+        return rc;
+    if (plan.ds)
+        return attention_backward_dq_ds(c, k, plan, span_start, span_finish, T, H, dq, grads16);
     AttBwdParams p;
     p.T = T;
     p.H = H;
-    const int Tpad = (int)ceil_div(T, TC_BN) * TC_BN;
     p.slope = slope;
     p.span_start = span_start;
     p.span_finish = span_finish;
     p.lse = lse;
     p.dscale = dscale;
+    p.out = dq;
     p.status = device_status_word(c.device);
     if (!p.status)
         return fail(TS2_ERR_CUDA, "attention: no device status word");
-    int rc;
-    float4 *meta = nullptr;
-    if ((rc = meta_buffer(c.device, (size_t)Tpad * H * sizeof(float4), &meta)) != TS2_OK)
-        return rc;
-    {
-        const int total = Tpad * H;
-        TS2_LAUNCH((att_pack_meta_kernel), (unsigned)ceil_div(total, 256), 256, 0, c.stream, lse, dscale, span_start, span_finish, T,
-                   Tpad, H, att_dot_scale_tc() * 0.693147f, meta);
-    }
-    p.out = dq;
-    if ((rc = launch_bwd_dq(c, q, dout, k, v, p, grads16)) != TS2_OK)
-        return rc;
-    // dK and dV from one kernel that shares S and the streamed tiles (kernels_att_bwd_kv_tc.cu)
-    return attention_backward_kv_tc(c, q, k, v, dout, meta, Tpad, rev_first, rev_last, T, H, slope, dk, dv, grads16);
+    return launch_bwd_dq(c, q, dout, k, v, p, grads16);
 }
 
 } // namespace ts2

@@ -112,6 +112,8 @@ struct BatchDev {
     uint32_t n_labels = 0;
     int *target = nullptr;
     std::vector<int *> span_start, span_finish, rev_first, rev_last;
+    std::vector<void *> att_layout; // per attention type, see AttBwdPlan
+    std::vector<bool> ds_fits;      // per attention type: the batch's score gradients fit the model's buffer
     int *scan_tmp = nullptr; // batch_scan_tmp_elems(max_nodes)
     int *status = nullptr;   // {code, where, detail, detail}: the first malformed element seen since it was last reported
     LabelIndex ix;
@@ -176,6 +178,7 @@ struct ts2_model {
     __half *drg = nullptr, *dout = nullptr;
     void *dcat = nullptr;
     float *dscale = nullptr;
+    AttBwdPlan att_bwd; // of the model: records, score gradients
     __half *dq = nullptr, *dk = nullptr, *dv = nullptr; // attention gradients, fp16 between the attention core and its post-kernel
     // int8 pipeline: the gradient operands of the dX contractions are row-quantized int8 (+ one fp32 scale per row), the
     // dW contractions read fp16: the state gradient and the first-contraction output gradients as fp16, and the int8
@@ -1039,6 +1042,11 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
     M_TRY(dalloc(m, &m->dq, (size_t)T * m->Q));
     M_TRY(dalloc(m, &m->dk, (size_t)T * m->Q));
     M_TRY(dalloc(m, &m->dv, (size_t)T * m->Q));
+    if (m->Q) {
+        M_TRY(dalloc(m, (uint8_t **)&m->att_bwd.scratch, att_bwd_scratch_bytes(T, m->H)));
+        m->att_bwd.ds_bytes = std::min(ATT_DS_MAX_BYTES, att_ds_bytes(T, nullptr, nullptr, nullptr) * m->H);
+        M_TRY(dalloc(m, (uint8_t **)&m->att_bwd.ds, m->att_bwd.ds_bytes));
+    }
     M_TRY(dalloc(m, &m->rope, (size_t)T * 128));
     M_TRY(dalloc(m, &m->absmax, L + 2));
     M_TRY(dalloc(m, &m->ginv, 4));
@@ -1062,11 +1070,14 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
     b.span_finish.resize(na);
     b.rev_first.resize(na);
     b.rev_last.resize(na);
+    b.att_layout.resize(na);
+    b.ds_fits.assign(na, true);
     for (int a = 0; a < na; ++a) {
         M_TRY(dalloc(m, &b.span_start[a], (size_t)T));
         M_TRY(dalloc(m, &b.span_finish[a], (size_t)T));
         M_TRY(dalloc(m, &b.rev_first[a], (size_t)T));
         M_TRY(dalloc(m, &b.rev_last[a], (size_t)T));
+        M_TRY(dalloc(m, (uint8_t **)&b.att_layout[a], att_layout_bytes(T)));
     }
     M_TRY(dalloc(m, &b.scan_tmp, batch_scan_tmp_elems(T)));
     M_TRY(dalloc(m, &b.status, 4));
@@ -1346,6 +1357,15 @@ static int reduce_matrices(ts2_model *m, int m0, int m1)
     return TS2_OK;
 }
 
+AttBwdPlan att_plan(const ts2_model *m, const Layer &ly)
+{
+    AttBwdPlan p = m->att_bwd;
+    p.layout = m->batch.att_layout[ly.att_type];
+    if (!m->batch.ds_fits[ly.att_type])
+        p.ds = nullptr;
+    return p;
+}
+
 // Backward pass of one dense layer in the int8 pipeline (the reference's default build: FWD / BWD_MATMUL_TYPE =
 // MATMUL_INT8, cfg_precision.h:21-26).  Same chain as the e4m3 / fp16 pipelines with these differences:
 //  * the gradient operand of each dX contraction is quantized per row to int8 with the reference's stochastic rounding
@@ -1387,7 +1407,7 @@ int backward_dense_int8(ts2_model *m, int l)
     if (ly.type == TS2_LAYER_ATT) {
         M_TRY(att_gate_backward(c16, m->drg, ly.cat16, ly.o, T, W, m->dcat16, m->dout, m->dscale));
         M_TRY(attention_backward(c, ly.q, ly.k, ly.v, m->dout, ly.lse, m->dscale, b.span_start[ly.att_type], b.span_finish[ly.att_type],
-                                 b.rev_first[ly.att_type], b.rev_last[ly.att_type], T, H, ly.slope, m->dq, m->dk, m->dv, true));
+                                 att_plan(m, ly), T, H, ly.slope, m->dq, m->dk, m->dv, true));
         M_TRY(att_post_backward(c16, m->dq, m->dk, m->dv, true, ly.q, ly.v, ly.qscale, ly.vscale, m->rope, m->mats[ly.mat0 + 1].sko, T, H,
                                 m->dcat16));
     } else {
@@ -1573,7 +1593,7 @@ int backward(ts2_model *m)
             TRACE("dout", l, m->dout, (size_t)T * W * 2, TR_F16);
             TRACE("dscale", l, m->dscale, (size_t)T * H * 4, TR_F32);
             M_TRY(attention_backward(c, ly.q, ly.k, ly.v, m->dout, ly.lse, m->dscale, b.span_start[ly.att_type], b.span_finish[ly.att_type],
-                                     b.rev_first[ly.att_type], b.rev_last[ly.att_type], T, H, ly.slope, m->dq, m->dk, m->dv, true));
+                                 att_plan(m, ly), T, H, ly.slope, m->dq, m->dk, m->dv, true));
             TRACE("dq", l, m->dq, (size_t)T * W * 2, TR_F16);
             TRACE("dk", l, m->dk, (size_t)T * W * 2, TR_F16);
             TRACE("dv", l, m->dv, (size_t)T * W * 2, TR_F16);
@@ -1762,6 +1782,12 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
         spans[a] = {raw + o_ptr[a], raw + o_start[a], raw + o_finish[a], n_spans[a], b.span_start[a], b.span_finish[a], b.rev_first[a], b.rev_last[a]};
     }
     M_TRY(batch_prepare(c, bt, spans.data(), na, b.ix, &b.ix_sorted));
+    for (int a = 0; a < na; ++a) {
+        M_TRY(att_layout(c, b.span_start[a], b.span_finish[a], b.rev_first[a], b.rev_last[a], T, b.att_layout[a]));
+        // a big batch: count what its own spans need (a pass over them on the host, beside the step that is running)
+        b.ds_fits[a] = att_ds_bytes(T, nullptr, nullptr, nullptr) * m->H <= m->att_bwd.ds_bytes ||
+                       att_ds_bytes(T, nd->att[a].span_ptr, nd->att[a].span_start, nd->att[a].span_finish) * m->H <= m->att_bwd.ds_bytes;
+    }
     b.node_count = T;
     b.target_count = n_targets;
     return TS2_OK;
