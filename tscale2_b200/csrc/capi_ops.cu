@@ -305,6 +305,25 @@ int ts2_op_ffn_act_backward(int device, void *stream, int prec, const void *drg,
                             2 * F, wscale, T, F, d_wide_gate);
 }
 
+int ts2_op_ffn_backward_fused(int device, void *stream, const void *g, const void *Wt, float alpha, const void *wide_gate,
+                              const float *wscale, int T, int D, int F, void *d_wide_gate)
+{
+    if (!g || !Wt || !wide_gate || !wscale || !d_wide_gate || T <= 0 || D <= 0 || D % 16 || F <= 0 || F % 128)
+        return fail(TS2_ERR_INVALID_ARG, "ts2_op_ffn_backward_fused: bad arguments");
+    if (!gemm_takes_act_backward(device, KIND_E4M3, T, F))
+        return fail(TS2_ERR_UNSUPPORTED, "ts2_op_ffn_backward_fused: this shape runs as two steps");
+    GemmArgs a;
+    a.device = device;
+    a.stream = (cudaStream_t)stream;
+    a.M = T, a.N = F, a.K = D;
+    a.A = g, a.lda = D, a.B = Wt, a.ldb = D, a.C = d_wide_gate, a.ldc = 2 * (int64_t)F;
+    a.epi.alpha = alpha;
+    a.epi.out_kind = TS2_OUT_F16;
+    a.epi.bwd_wg = wide_gate;
+    a.epi.act_scale = const_cast<float *>(wscale);
+    return gemm(a);
+}
+
 int ts2_op_att_gate_backward(int device, void *stream, int prec, const void *drg, const void *qkvg, const void *o, int T, int Q,
                              void *d4, void *dout, float *dscale)
 {

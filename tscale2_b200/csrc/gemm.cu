@@ -862,10 +862,10 @@ static Plan fixed_plan(int device, int kind, int64_t M, int64_t N, int64_t K)
     return pl;
 }
 
-enum { FORM_F32, FORM_ADD, FORM_16, FORM_GATED };
+enum { FORM_F32, FORM_ADD, FORM_16, FORM_GATED, FORM_ACT_BWD };
 static int form_of(const Epilogue &e)
 {
-    return e.pair_stride ? FORM_GATED : e.out_kind == TS2_OUT_F32_ADD ? FORM_ADD : e.out_kind == TS2_OUT_F32 ? FORM_F32 : FORM_16;
+    return e.bwd_wg ? FORM_ACT_BWD : e.pair_stride ? FORM_GATED : e.out_kind == TS2_OUT_F32_ADD ? FORM_ADD : e.out_kind == TS2_OUT_F32 ? FORM_F32 : FORM_16;
 }
 
 // Tile and K split with the smallest estimated time.  The estimate follows measurements of single launches (us):
@@ -895,7 +895,8 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
         if (group_mode && (pl.pair() || pl.bn != ((N % 256 == 0 || N > 1024) ? 256 : 128)))
             continue;
         // a token-major one-byte operand comes in boxes of 128 columns; the gated form takes 128 wide and 128 gate columns
-        if ((pl.bn == 64 && mn && es == 1) || (form == FORM_GATED && pl.bn != 256))
+        if ((pl.bn == 64 && mn && es == 1) || (form == FORM_GATED && pl.bn != 256) ||
+            (form == FORM_ACT_BWD && !pl.pair()))
             continue;
         pl.m_tiles = (int)ceil_div(M, pl.bm);
         pl.n_tiles = (int)ceil_div(N, pl.bn);
@@ -903,7 +904,7 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
         const int workers = pl.pair() ? sms / 2 : sms;
         const long long tiles = std::max(1, pl.m_tiles * pl.n_tiles); // an empty problem is rejected by gemm(); keep the arithmetic defined
         const double te = shape.epilogue * (form == FORM_ADD && !pl.pair() ? 2.5 : 1.0);
-        const int most = group_mode || form == FORM_GATED ? 1 : (int)std::min<long long>(2 * workers / tiles, pl.k_blocks / 4);
+        const int most = group_mode || form >= FORM_GATED ? 1 : (int)std::min<long long>(2 * workers / tiles, pl.k_blocks / 4);
         for (int splits = 1; splits <= std::max(1, most); ++splits) {
             finish_plan(pl, sms, splits, group_mode, groups);
             if (pl.splits != splits)
@@ -919,6 +920,14 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
         }
     }
     return best;
+}
+
+// From one wave of pairs on the epilogue form wins over contraction + ffn_act_backward (us, M x N x K): 1600 x 3072 x 768 25.1 ->
+// 23.6, 5000 x 1024 x 256 21.9 -> 20.8, 4000 x 3072 x 768 43.9 -> 32.7, 65536 x 3072 x 768 464 -> 329, 32768 x 8192 x 2048
+// 865 -> 613; below, pairs leave SMs without a tile that smaller tiles of single CTAs would use.
+bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N)
+{
+    return kind == KIND_E4M3 && N % 128 == 0 && ceil_div(M, 2 * BM) * ceil_div(N, 256) >= sm_count(device) / 2;
 }
 
 size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int out_kind)
@@ -1107,6 +1116,10 @@ int gemm(const GemmArgs &a)
         pl.n_tiles = (int)(a.epi.pair_stride / 128);
         finish_plan(pl, sm_count(a.device), 1, 0, 1);
     }
+    const bool act_bwd = a.epi.bwd_wg != nullptr;
+    if (act_bwd && (paired || a.mn_major || a.group_mode || a.kind != KIND_E4M3 || a.epi.out_kind != TS2_OUT_F16 || a.N % 128 ||
+                    a.ldc != 2 * a.N || !a.epi.act_scale || ((uintptr_t)a.epi.bwd_wg & 15) || !pl.pair() || pl.splits != 1))
+        return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of the activation's backward form");
     if (pl.splits > 1) {
         const size_t need = pl.workspace();
         if (!a.workspace || a.workspace_bytes < need)
@@ -1175,7 +1188,10 @@ int gemm(const GemmArgs &a)
     CUtensorMap tmC = tmA, tmCin = tmA;
     p.tma_store = 0;
     if (pl.pair()) { // every output leaves by TMA, partial tiles as rows of 256 in the workspace
-        if (pl.splits > 1)
+        if (act_bwd) {
+            if ((rc = make_tmap(&tmC, a.C, 1, 2 * a.N, a.M, 2 * a.N, 32, 64)) == TS2_OK)
+                rc = make_tmap(&tmCin, a.epi.bwd_wg, 2, 2 * a.N, a.M, 2 * a.N, 32);
+        } else if (pl.splits > 1)
             rc = make_tmap(&tmC, a.workspace, 4, pl.bn, (int64_t)pl.m_tiles * pl.n_tiles * pl.splits * pl.bm, pl.bn, 32);
         else
             rc = make_tmap(&tmC, a.C, out_es, a.N, a.M, a.ldc, 32, paired ? 64 : STAGE_ROW_BYTES);
@@ -1209,7 +1225,7 @@ int gemm(const GemmArgs &a)
     rc = TS2_ERR_UNSUPPORTED;
     if (pl.pair()) {
         const int sms = std::max(2, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)) & ~1;
-        rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, paired, std::min(pl.grid, sms), tmA, tmB, tmC, tmCin, p);
+        rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, act_bwd ? 2 : paired ? 1 : 0, std::min(pl.grid, sms), tmA, tmB, tmC, tmCin, p);
         if (rc == TS2_OK && pl.splits > 1)
             rc = reduce_splits<2 * BM, 256>(a, pl, p);
     } else if (paired) {
@@ -1245,7 +1261,8 @@ int gemm(const GemmArgs &a)
         std::lock_guard<std::mutex> lk(g_time_mu);
         // algorithmic bytes: both operands once, the output once, the residual input of the accumulate form once
         const double mn = (double)a.M * (double)a.N;
-        const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + mn * out_es + (a.epi.out_kind == TS2_OUT_F32_ADD ? mn * 4 : 0);
+        const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + (act_bwd ? mn * 6 : mn * out_es) +
+                             (a.epi.out_kind == TS2_OUT_F32_ADD ? mn * 4 : 0);
         g_timed.push_back({ea, eb, 2.0 * mn * (double)a.K, bytes, a.tag});
     }
     return rc;

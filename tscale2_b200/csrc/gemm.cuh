@@ -28,6 +28,11 @@ struct Epilogue {
     float *act_scale = nullptr;
     float act_mult = 1.f;
     int act_kind = 0;
+    // Backward of that activation on the product (e4m3 operands, where gemm_takes_act_backward() says so): the product, the
+    // gradient of the gated activation, is rounded to fp16 and goes through the gate and the tile normalisation on the
+    // spot.  bwd_wg: [M][2N] fp16 = [normalised wide | gate], rows of 2N; act_scale: [M][N / 128], read;
+    // C: e4m3 [M][2N] = [gradient of wide | gradient of gate], ldc = 2N.
+    const void *bwd_wg = nullptr;
 };
 
 struct GemmArgs {
@@ -60,6 +65,8 @@ struct GemmArgs {
 // bytes of scratch this shape needs for its K splits (0: none); out_kind < 0: whatever the output
 size_t gemm_workspace_bytes(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_t K, int out_kind = -1);
 int gemm(const GemmArgs &a);
+// whether the epilogue can apply the backward of the gated activation (Epilogue::bwd_wg) to a product of this shape
+bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N);
 
 // 2-D TMA descriptor over a row-major [rows][ld] array of es-byte elements: box = row_bytes (128 or 64, swizzled alike) x
 // box_rows, out-of-range elements read as zero

@@ -26,14 +26,17 @@ namespace {
 constexpr int PM = 256, PN = 256; // the pair's tile
 constexpr int P_HALF_BYTES = 128 * STAGE_ROW_BYTES; // a CTA's half of either operand, one K block
 constexpr int P_STAGE_BYTES = 2 * P_HALF_BYTES;
-constexpr int P_STAGES = 4;
-constexpr int P_STG_OFF = P_STAGES * P_STAGE_BYTES;
-constexpr int P_STG_BYTES = 8 * 3 * 4096;
-constexpr int P_BAR_OFF = P_STG_OFF + P_STG_BYTES;
-constexpr int P_SMEM = P_BAR_OFF + 1024 + 1024; // + alignment slack
-static_assert(P_SMEM <= 232448, "shared memory budget");
 constexpr int P_THREADS = 320, P_THREADS_16 = 576;
-enum { P_F32 = 0, P_16 = 1, P_GATED = 2 };
+enum { P_F32 = 0, P_16 = 1, P_GATED = 2, P_ACT_BWD = 3 };
+// shared memory of a form: ring, epilogue staging, barriers, alignment slack
+template <int FORM>
+struct PairSmem {
+    static constexpr int STAGES = FORM == P_ACT_BWD ? 3 : 4;
+    static constexpr int STG_OFF = STAGES * P_STAGE_BYTES;
+    static constexpr int BAR_OFF = STG_OFF + (FORM == P_ACT_BWD ? 16 * 2 * 4096 : 8 * 3 * 4096);
+    static constexpr int TOTAL = BAR_OFF + 1024 + 1024;
+    static_assert(TOTAL <= 232448, "shared memory budget");
+};
 
 __device__ __forceinline__ uint32_t cluster_rank()
 {
@@ -120,7 +123,7 @@ __device__ __forceinline__ PairUnit pair_unit(const GemmParams &p, int u)
 __device__ __forceinline__ uint32_t piece(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
 // FORM of the epilogue: P_F32 (fp32 output, accumulate form, partial tiles; 8 warps), P_16 (fp16 / bf16 output; 16 warps),
-// P_GATED (gated activation; 16 warps)
+// P_GATED (gated activation; 16 warps), P_ACT_BWD (its backward; 16 warps)
 template <int ES, int MMA, bool MN, int FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_THREADS : P_THREADS_16, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -130,13 +133,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
     constexpr int UMMA_K = 32 / ES, K_STEPS = 4, BK = ELEMS_PER_ROW;
     constexpr bool GATED = FORM == P_GATED;
     constexpr int EPI_WARPS = FORM == P_F32 ? 8 : 16;
+    constexpr int P_STAGES = PairSmem<FORM>::STAGES, P_STG_OFF = PairSmem<FORM>::STG_OFF, P_BAR_OFF = PairSmem<FORM>::BAR_OFF;
 
     extern __shared__ uint8_t pair_smem[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)pair_smem + 1023) & ~(uintptr_t)1023); // the same offset in both CTAs
     uint64_t *bars = (uint64_t *)(smem + P_BAR_OFF);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + P_STAGES), tfull0 = smem_u32(bars + 2 * P_STAGES),
                    tempty0 = smem_u32(bars + 2 * P_STAGES + 2), drain = smem_u32(bars + 2 * P_STAGES + 4),
-                   cin0 = smem_u32(bars + 2 * P_STAGES + 5); // [warp][3]: residual block landed
+                   cin0 = smem_u32(bars + 2 * P_STAGES + 5); // [warp][3]: residual block landed; P_ACT_BWD: see there
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * P_STAGES + 5 + 24);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
@@ -152,7 +156,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
             mbar_init(tempty0 + 8 * a, 2 * EPI_WARPS); // the leader's counts the epilogue warps of both CTAs
         }
         for (int i = 0; i < 24; ++i)
-            mbar_init(cin0 + 8 * i, 1);
+            mbar_init(cin0 + 8 * i, FORM == P_ACT_BWD && i >= 16 ? 2 : 1);
         mbar_init(drain, 1);
         *abort_flag = 0;
         fence_barrier_init();
@@ -409,6 +413,143 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                     }
                 }
             }
+        } else if constexpr (FORM == P_ACT_BWD) {
+            // Backward of the gated activation (ffn_act_backward in kernels_elem.cu, same arithmetic) on the accumulator: a warp
+            // takes 32 rows x 64 columns; the two warps of a 128-wide normalisation tile add their halves of its projection.
+            // [wide | gate] values arrive by TMA in two 4 KB blocks per warp, a tile ahead; both gradients leave through the gate's
+            // block.  As a kernel of its own this read the product back: 65536 x 3072 x 768 took 155 + 309 us, both bound by
+            // their bytes; the product (2 x 403 MB of 2 GB) no longer goes through memory, 329 us.
+            const int part = ew >> 2;
+            uint8_t *const wblk = smem + P_STG_OFF + ew * 8192, *const gblk = wblk + 4096;
+            const uint32_t in_bar = cin0 + 8 * ew, mate = cin0 + 8 * (16 + (ew & 3) + 4 * (part >> 1)); // mate: both warps of a tile
+            const volatile float *const theirs = (const volatile float *)(smem + P_STG_OFF + (ew ^ 4) * 8192 + 4096 + 2048) + lane;
+            float *const mine = (float *)(gblk + 2048) + lane;
+            auto fetch = [&](int u, bool gate) { // lane 0
+                const PairUnit un = pair_unit(p, u);
+                const int col = un.n0 + part * 64, r0 = un.m0 + (int)rank * 128 + quarter * 32;
+                if (!gate)
+                    mbar_arrive_expect_tx(in_bar, 8192);
+                tma_load_2d(smem_u32(gate ? gblk : wblk), &tmCin, in_bar, gate ? p.N + col : col, r0);
+            };
+            if (lane == 0 && first < units) {
+                fetch(first, false);
+                fetch(first, true);
+            }
+            uint32_t in_phase = 0;
+            bool ok = true, coming = true; // coming: blocks of the next tile are on their way
+            for (int u = first; u < units; u += step) {
+                const PairUnit un = pair_unit(p, u);
+                const int m0 = un.m0 + (int)rank * 128, col = un.n0 + part * 64;
+                const long long row = m0 + row_in_cta;
+                const float scale = row < p.M && col < p.N ? p.act_scale[row * (p.N >> 7) + (col >> 7)] : 0.f;
+                ok = __all_sync(0xffffffffu, mbar_wait(in_bar, in_phase, abort_flag));
+                if (!ok)
+                    break;
+                in_phase ^= 1;
+                coming = false;
+                ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag));
+                if (!ok)
+                    break;
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * PN + part * 64;
+                const __half2 one = __float2half2_rn(1.f), two = __float2half2_rn(2.f);
+                __half2 dw[32]; // gradient of the normalised wide values
+                uint32_t dg[16];
+                float proj = 0.f;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + h * 32, r);
+                    tmem_ld_wait();
+                    if (h == 1) { // the accumulator is read: the next tile may have it
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0)
+                            mbar_arrive_cluster(map_to_leader(tempty0 + 8 * acc));
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint4 w4 = *(const uint4 *)(wblk + piece(lane, 4 * h + i)), g4 = *(const uint4 *)(gblk + piece(lane, 4 * h + i));
+                        const uint32_t wv[4] = {w4.x, w4.y, w4.z, w4.w}, gv[4] = {g4.x, g4.y, g4.z, g4.w};
+                        __half2 dgate[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int e = 8 * i + 2 * j;
+                            const __half2 g = sat_half2(__uint_as_float(r[e]) * alpha, __uint_as_float(r[e + 1]) * alpha);
+                            const __half2 w = h2_from_bits(wv[j]), m = lolu_mult_h2(h2_from_bits(gv[j]));
+                            dgate[j] = __hmul2(g, __hmul2(w, __hmul2(__hmul2(m, two), __hsub2(one, m))));
+                            const __half2 d = __hmul2(g, m);
+                            dw[16 * h + 4 * i + j] = d;
+                            const float2 pr = __half22float2(__hmul2(w, d));
+                            proj += pr.x + pr.y;
+                        }
+                        dg[8 * h + 2 * i] = e4m3x4_from_h2(dgate[0], dgate[1]);
+                        dg[8 * h + 2 * i + 1] = e4m3x4_from_h2(dgate[2], dgate[3]);
+                    }
+                }
+                __syncwarp(); // every lane has read its row of the gate's block
+                uint8_t *const srow = gblk + lane * 64; // blocks of 32 rows x 64 bytes (64-byte swizzle)
+                const int sw = (lane >> 1) & 3;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    *(uint4 *)(srow + ((i ^ sw) << 4)) = make_uint4(dg[4 * i], dg[4 * i + 1], dg[4 * i + 2], dg[4 * i + 3]);
+                *mine = proj;
+                // first phase: both halves are written; second: both are read.  Two phases per tile: the parities are fixed
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(mate);
+                ok = __all_sync(0xffffffffu, mbar_wait(mate, 0, abort_flag));
+                if (!ok)
+                    break;
+                proj = (proj + *theirs) * (1.f / 128);
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(mate);
+                ok = __all_sync(0xffffffffu, mbar_wait(mate, 1, abort_flag));
+                if (!ok)
+                    break;
+                const __half2 nproj = __float2half2_rn(-proj), sc = __float2half2_rn(scale);
+                uint32_t dx[16];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint4 w4 = *(const uint4 *)(wblk + piece(lane, i));
+                    const uint32_t wv[4] = {w4.x, w4.y, w4.z, w4.w};
+                    __half2 d[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        d[j] = __hmul2(sc, __hfma2(h2_from_bits(wv[j]), nproj, dw[4 * i + j]));
+                    dx[2 * i] = e4m3x4_from_h2(d[0], d[1]);
+                    dx[2 * i + 1] = e4m3x4_from_h2(d[2], d[3]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    *(uint4 *)(srow + 2048 + ((i ^ sw) << 4)) = make_uint4(dx[4 * i], dx[4 * i + 1], dx[4 * i + 2], dx[4 * i + 3]);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    if (col < p.N) {
+                        tma_store_2d(&tmC, smem_u32(gblk), p.N + col, m0 + quarter * 32);
+                        tma_store_2d(&tmC, smem_u32(gblk) + 2048, col, m0 + quarter * 32);
+                    }
+                    bulk_commit();
+                    if (u + step < units) {
+                        fetch(u + step, false);
+                        bulk_wait_read<0>(); // the stores have read the gate's block
+                        fetch(u + step, true);
+                    }
+                }
+                coming = u + step < units;
+                __syncwarp();
+                acc ^= 1;
+                if (acc == 0)
+                    acc_phase ^= 1;
+            }
+            // abort path: blocks may still be on their way into this CTA's shared memory
+            if (!ok && lane == 0 && coming) {
+                long long t0 = clock64();
+                while (!mbar_try_wait(in_bar, in_phase) && clock64() - t0 < 200000000ll) {
+                }
+            }
         } else if constexpr (FORM == P_16) {
             // Sixteen warps, four per lane quarter, 64 columns of the tile each: one block of 32 rows x 128 bytes in the 128-byte
             // swizzle and one store per tile.  With eight warps a tile of K = 768 took 3.6 us, 2.6 of them its main loop and
@@ -619,19 +760,19 @@ int launch_pair(int device, cudaStream_t stream, int grid, const CUtensorMap &tm
     auto kern = gemm_pair_kernel<ES, MMA, MN, FORM>;
     static bool configured[16] = {};
     if (!configured[device & 15]) {
-        TS2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
+        TS2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<FORM>::TOTAL));
         configured[device & 15] = true;
     }
-    TS2_LAUNCH((kern), grid, FORM == P_F32 ? P_THREADS : P_THREADS_16, P_SMEM, stream, tmA, tmB, tmC, tmCin, p);
+    TS2_LAUNCH((kern), grid, FORM == P_F32 ? P_THREADS : P_THREADS_16, PairSmem<FORM>::TOTAL, stream, tmA, tmB, tmC, tmCin, p);
     return TS2_OK;
 }
 
 } // namespace
 
-int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, bool gated, int grid, const CUtensorMap &tmA,
+int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, int form_arg, int grid, const CUtensorMap &tmA,
                      const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const GemmParams &p)
 {
-    const int form = gated ? P_GATED : p.splits == 1 && (p.out_kind == TS2_OUT_F16 || p.out_kind == TS2_OUT_BF16) ? P_16 : P_F32;
+    const int form = form_arg == 2 ? P_ACT_BWD : form_arg == 1 ? P_GATED : p.splits == 1 && (p.out_kind == TS2_OUT_F16 || p.out_kind == TS2_OUT_BF16) ? P_16 : P_F32;
 #define TS2_PAIR_CASE(ES_, MMA_, MN_, FORM_)                          \
     if (es == ES_ && mma == MMA_ && mn == MN_ && form == FORM_)       \
         return launch_pair<ES_, MMA_, MN_, FORM_>(device, stream, grid, tmA, tmB, tmC, tmCin, p);
@@ -642,6 +783,7 @@ int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, 
     TS2_PAIR_CASE(ES_, MMA_, true, P_F32)      \
     TS2_PAIR_CASE(ES_, MMA_, true, P_16)
     TS2_PAIR_CASES(1, 0)
+    TS2_PAIR_CASE(1, 0, false, P_ACT_BWD)
     TS2_PAIR_CASES(2, 1)
     TS2_PAIR_CASES(1, 2)
 #undef TS2_PAIR_CASES

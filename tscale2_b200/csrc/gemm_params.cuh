@@ -47,7 +47,8 @@ struct GemmParams {
 
 // gemm_pair.cu: the contraction on pairs of CTAs (tiles of 256 x 256).  tmB's box is 128 rows (K-major) or one K block
 // (token-major); tmC's and tmCin's are 32 rows x 128 bytes.  grid: CTAs, an even number.
-int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, bool gated, int grid, const CUtensorMap &tmA,
+// form: 0 by output kind, 1 gated activation, 2 its backward (tmC: 32 rows x 64 bytes, tmCin: [wide | gate] in 32 rows x 128)
+int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, int form, int grid, const CUtensorMap &tmA,
                      const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const GemmParams &p);
 
 } // namespace ts2

@@ -1577,8 +1577,16 @@ int backward(ts2_model *m)
         e3.alpha = 1.f / (32.f * sqrtf((float)D));
         e3.out_kind = TS2_OUT_F16;
         TRACE("g_fast", l, m->g_fast, (size_t)T * D * fsz, fsz == 2 ? TR_F16 : TR_RAW);
-        M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->drg, W, e3));
-        TRACE("drg", l, m->drg, (size_t)T * W * 2, TR_F16);
+        // FFN, many tiles: the contraction's epilogue goes on through the activation; drg never reaches memory
+        const bool act_fused = ly.type != TS2_LAYER_ATT && gemm_takes_act_backward(m->device, m->kind, T, W);
+        if (act_fused) {
+            e3.bwd_wg = ly.cat16;
+            e3.act_scale = ly.wscale;
+            M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->dcat, C, e3));
+        } else {
+            M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->drg, W, e3));
+            TRACE("drg", l, m->drg, (size_t)T * W * 2, TR_F16);
+        }
         if (tune_layers) {
             // dWc = g^T . rg   (SumRankOne)
             Epilogue e6;
@@ -1599,7 +1607,7 @@ int backward(ts2_model *m)
             TRACE("dv", l, m->dv, (size_t)T * W * 2, TR_F16);
             M_TRY(att_post_backward(c, m->dq, m->dk, m->dv, true, ly.q, ly.v, ly.qscale, ly.vscale, m->rope, m->mats[ly.mat0 + 1].sko, T, H,
                                     m->dcat));
-        } else {
+        } else if (!act_fused) {
             M_TRY(ffn_act_backward(c, m->drg, ly.cat16, ly.cat16, 2 * W, ly.wscale, T, W, m->dcat));
         }
         TRACE("dcat", l, m->dcat, (size_t)T * C * fsz, fsz == 2 ? TR_F16 : TR_RAW);
