@@ -431,11 +431,13 @@ int ts2_op_cast_grad(int device, void *stream, int prec, const float *g, int64_t
                      float *ginv);
 int ts2_op_ffn_act_backward(int device, void *stream, int prec, const void *drg, const void *wide_gate, const float *wscale, int T,
                             int F, void *d_wide_gate);
-/* Both steps of the FFN branch in one kernel, e4m3 operands: drg = g . Wt^T * alpha (g [T][D], Wt [F][D]; rounded to fp16),
- * then ts2_op_ffn_act_backward on it.  TS2_ERR_UNSUPPORTED where the contraction's tiles do not carry that epilogue (few
+/* Both steps of a branch in one kernel, e4m3 operands: drg = g . Wt^T * alpha (g [T][D], Wt [F][D] or [Q][D]; rounded to
+ * fp16), then ts2_op_ffn_act_backward or ts2_op_att_gate_backward on it.  TS2_ERR_UNSUPPORTED where the contraction's tiles do not carry that epilogue (few
  * tiles); the engine then takes the two steps one after the other. */
 int ts2_op_ffn_backward_fused(int device, void *stream, const void *g, const void *Wt, float alpha, const void *wide_gate,
                               const float *wscale, int T, int D, int F, void *d_wide_gate);
+int ts2_op_att_gate_backward_fused(int device, void *stream, const void *g, const void *Wt, float alpha, const void *qkvg, const void *o,
+                                   int T, int D, int Q, void *d4, void *dout, float *dscale);
 int ts2_op_att_gate_backward(int device, void *stream, int prec, const void *drg, const void *qkvg, const void *o, int T, int Q,
                              void *d4, void *dout, float *dscale);
 /* Row quantization of the int8 pipeline's gradient operands (NormalizeVecsRowMaxKernel with TCudaRngLCG,

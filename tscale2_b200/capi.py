@@ -147,6 +147,7 @@ def _declare(lib):
         "ts2_op_cast_grad": (i32, [i32, vp, i32, vp, i64, vp, vp, vp]),
         "ts2_op_ffn_act_backward": (i32, [i32, vp, i32, vp, vp, vp, i32, i32, vp]),
         "ts2_op_ffn_backward_fused": (i32, [i32, vp, vp, vp, f32, vp, vp, i32, i32, i32, vp]),
+        "ts2_op_att_gate_backward_fused": (i32, [i32, vp, vp, vp, f32, vp, vp, i32, i32, i32, vp, vp, vp]),
         "ts2_op_att_gate_backward": (i32, [i32, vp, i32, vp, vp, vp, i32, i32, vp, vp, vp]),
         "ts2_op_rowquant_i8": (i32, [i32, vp, vp, i32, i32, vp, vp]),
         "ts2_op_attention_reverse_ranges": (i32, [i32, vp, vp, vp, i32, vp, vp]),

@@ -324,6 +324,24 @@ int ts2_op_ffn_backward_fused(int device, void *stream, const void *g, const voi
     return gemm(a);
 }
 
+int ts2_op_att_gate_backward_fused(int device, void *stream, const void *g, const void *Wt, float alpha, const void *qkvg, const void *o,
+                                   int T, int D, int Q, void *d4, void *dout, float *dscale)
+{
+    if (!g || !Wt || !qkvg || !o || !d4 || !dout || !dscale || T <= 0 || D <= 0 || D % 16 || Q <= 0 || Q % 128)
+        return fail(TS2_ERR_INVALID_ARG, "ts2_op_att_gate_backward_fused: bad arguments");
+    if (!gemm_takes_act_backward(device, KIND_E4M3, T, Q))
+        return fail(TS2_ERR_UNSUPPORTED, "ts2_op_att_gate_backward_fused: this shape runs as two steps");
+    GemmArgs a;
+    a.device = device;
+    a.stream = (cudaStream_t)stream;
+    a.M = T, a.N = Q, a.K = D;
+    a.A = g, a.lda = D, a.B = Wt, a.ldb = D, a.C = d4, a.ldc = 4 * (int64_t)Q;
+    a.epi.alpha = alpha;
+    a.epi.out_kind = TS2_OUT_F16;
+    a.epi.bwd_wg = qkvg, a.epi.bwd_o = o, a.epi.bwd_dout = dout, a.epi.bwd_dscale = dscale;
+    return gemm(a);
+}
+
 int ts2_op_att_gate_backward(int device, void *stream, int prec, const void *drg, const void *qkvg, const void *o, int T, int Q,
                              void *d4, void *dout, float *dscale)
 {

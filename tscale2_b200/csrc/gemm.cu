@@ -924,10 +924,12 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
 
 // From one wave of pairs on the epilogue form wins over contraction + ffn_act_backward (us, M x N x K): 1600 x 3072 x 768 25.1 ->
 // 23.6, 5000 x 1024 x 256 21.9 -> 20.8, 4000 x 3072 x 768 43.9 -> 32.7, 65536 x 3072 x 768 464 -> 329, 32768 x 8192 x 2048
-// 865 -> 613; below, pairs leave SMs without a tile that smaller tiles of single CTAs would use.
+// 865 -> 613, and over contraction + att_gate_backward: 4000 x 1536 x 768 23.4 -> 19.7, 16384 x 512 x 512 26.0 -> 19.0,
+// 65536 x 1536 x 768 240 -> 184; below, pairs leave SMs without a tile that smaller tiles of single CTAs would use.  A narrow
+// matrix whose last tile is half empty loses: 12800 x 384 x 256 17.3 -> 17.8, 20000 x 128 x 256 13.5 -> 16.2.
 bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N)
 {
-    return kind == KIND_E4M3 && N % 128 == 0 && ceil_div(M, 2 * BM) * ceil_div(N, 256) >= sm_count(device) / 2;
+    return kind == KIND_E4M3 && N % 128 == 0 && (N % 256 == 0 || N > 512) && ceil_div(M, 2 * BM) * ceil_div(N, 256) >= sm_count(device) / 2;
 }
 
 size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int out_kind)
@@ -1116,9 +1118,11 @@ int gemm(const GemmArgs &a)
         pl.n_tiles = (int)(a.epi.pair_stride / 128);
         finish_plan(pl, sm_count(a.device), 1, 0, 1);
     }
-    const bool act_bwd = a.epi.bwd_wg != nullptr;
+    const bool act_bwd = a.epi.bwd_wg != nullptr, gate_bwd = act_bwd && a.epi.bwd_o;
+    const int64_t bwd_ld = (gate_bwd ? 4 : 2) * a.N;
     if (act_bwd && (paired || a.mn_major || a.group_mode || a.kind != KIND_E4M3 || a.epi.out_kind != TS2_OUT_F16 || a.N % 128 ||
-                    a.ldc != 2 * a.N || !a.epi.act_scale || ((uintptr_t)a.epi.bwd_wg & 15) || !pl.pair() || pl.splits != 1))
+                    a.ldc != bwd_ld || !(gate_bwd ? a.epi.bwd_dscale && a.epi.bwd_dout : a.epi.act_scale != nullptr) ||
+                    (((uintptr_t)a.epi.bwd_wg | (uintptr_t)a.epi.bwd_o | (uintptr_t)a.epi.bwd_dout) & 15) || !pl.pair() || pl.splits != 1))
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of the activation's backward form");
     if (pl.splits > 1) {
         const size_t need = pl.workspace();
@@ -1183,14 +1187,17 @@ int gemm(const GemmArgs &a)
     p.act_scale = a.epi.act_scale;
     p.act_mult = a.epi.act_mult;
     p.act_kind = a.epi.act_kind;
+    p.bwd_dscale = a.epi.bwd_dscale;
     // coalesced TMA-store epilogue (the accumulate form adds its residual input first; split units go to the workspace;
     // per-group C offsets of mode 2 are not expressible as one 2-D map)
-    CUtensorMap tmC = tmA, tmCin = tmA;
+    CUtensorMap tmC = tmA, tmCin = tmA, tmX = tmA, tmY = tmA;
     p.tma_store = 0;
     if (pl.pair()) { // every output leaves by TMA, partial tiles as rows of 256 in the workspace
         if (act_bwd) {
-            if ((rc = make_tmap(&tmC, a.C, 1, 2 * a.N, a.M, 2 * a.N, 32, 64)) == TS2_OK)
-                rc = make_tmap(&tmCin, a.epi.bwd_wg, 2, 2 * a.N, a.M, 2 * a.N, 32);
+            if ((rc = make_tmap(&tmC, a.C, 1, bwd_ld, a.M, bwd_ld, 32, 64)) == TS2_OK)
+                rc = make_tmap(&tmCin, a.epi.bwd_wg, 2, bwd_ld, a.M, bwd_ld, 32);
+            if (gate_bwd && rc == TS2_OK && (rc = make_tmap(&tmX, a.epi.bwd_o, 2, a.N, a.M, a.N, 32)) == TS2_OK)
+                rc = make_tmap(&tmY, a.epi.bwd_dout, 2, a.N, a.M, a.N, 32);
         } else if (pl.splits > 1)
             rc = make_tmap(&tmC, a.workspace, 4, pl.bn, (int64_t)pl.m_tiles * pl.n_tiles * pl.splits * pl.bm, pl.bn, 32);
         else
@@ -1225,7 +1232,8 @@ int gemm(const GemmArgs &a)
     rc = TS2_ERR_UNSUPPORTED;
     if (pl.pair()) {
         const int sms = std::max(2, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)) & ~1;
-        rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, act_bwd ? 2 : paired ? 1 : 0, std::min(pl.grid, sms), tmA, tmB, tmC, tmCin, p);
+        rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, gate_bwd ? 3 : act_bwd ? 2 : paired ? 1 : 0, std::min(pl.grid, sms), tmA, tmB,
+                              tmC, tmCin, tmX, tmY, p);
         if (rc == TS2_OK && pl.splits > 1)
             rc = reduce_splits<2 * BM, 256>(a, pl, p);
     } else if (paired) {
@@ -1261,7 +1269,7 @@ int gemm(const GemmArgs &a)
         std::lock_guard<std::mutex> lk(g_time_mu);
         // algorithmic bytes: both operands once, the output once, the residual input of the accumulate form once
         const double mn = (double)a.M * (double)a.N;
-        const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + (act_bwd ? mn * 6 : mn * out_es) +
+        const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + (gate_bwd ? mn * 7 : act_bwd ? mn * 6 : mn * out_es) +
                              (a.epi.out_kind == TS2_OUT_F32_ADD ? mn * 4 : 0);
         g_timed.push_back({ea, eb, 2.0 * mn * (double)a.K, bytes, a.tag});
     }

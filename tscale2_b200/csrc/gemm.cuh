@@ -32,7 +32,12 @@ struct Epilogue {
     // gradient of the gated activation, is rounded to fp16 and goes through the gate and the tile normalisation on the
     // spot.  bwd_wg: [M][2N] fp16 = [normalised wide | gate], rows of 2N; act_scale: [M][N / 128], read;
     // C: e4m3 [M][2N] = [gradient of wide | gradient of gate], ldc = 2N.
-    const void *bwd_wg = nullptr;
+    // With bwd_o, backward of the attention gate instead: bwd_wg: [M][4N] fp16 with the gate in columns [3N, 4N),
+    // bwd_o, bwd_dout: [M][N] fp16 (attention output, its gradient), bwd_dscale: [M][N / 128] = sum of both's products per
+    // head, C: e4m3 [M][4N], of which columns [3N, 4N) are written, ldc = 4N.
+    const void *bwd_wg = nullptr, *bwd_o = nullptr;
+    void *bwd_dout = nullptr;
+    float *bwd_dscale = nullptr;
 };
 
 struct GemmArgs {

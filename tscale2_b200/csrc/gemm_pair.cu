@@ -27,13 +27,14 @@ constexpr int PM = 256, PN = 256; // the pair's tile
 constexpr int P_HALF_BYTES = 128 * STAGE_ROW_BYTES; // a CTA's half of either operand, one K block
 constexpr int P_STAGE_BYTES = 2 * P_HALF_BYTES;
 constexpr int P_THREADS = 320, P_THREADS_16 = 576;
-enum { P_F32 = 0, P_16 = 1, P_GATED = 2, P_ACT_BWD = 3 };
+enum { P_F32 = 0, P_16 = 1, P_GATED = 2, P_ACT_BWD = 3, P_GATE_BWD = 4 };
+constexpr bool is_bwd(int form) { return form == P_ACT_BWD || form == P_GATE_BWD; }
 // shared memory of a form: ring, epilogue staging, barriers, alignment slack
 template <int FORM>
 struct PairSmem {
-    static constexpr int STAGES = FORM == P_ACT_BWD ? 3 : 4;
+    static constexpr int STAGES = is_bwd(FORM) ? 3 : 4;
     static constexpr int STG_OFF = STAGES * P_STAGE_BYTES;
-    static constexpr int BAR_OFF = STG_OFF + (FORM == P_ACT_BWD ? 16 * 2 * 4096 : 8 * 3 * 4096);
+    static constexpr int BAR_OFF = STG_OFF + (is_bwd(FORM) ? 16 * 2 * 4096 : 8 * 3 * 4096);
     static constexpr int TOTAL = BAR_OFF + 1024 + 1024;
     static_assert(TOTAL <= 232448, "shared memory budget");
 };
@@ -123,11 +124,13 @@ __device__ __forceinline__ PairUnit pair_unit(const GemmParams &p, int u)
 __device__ __forceinline__ uint32_t piece(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
 // FORM of the epilogue: P_F32 (fp32 output, accumulate form, partial tiles; 8 warps), P_16 (fp16 / bf16 output; 16 warps),
-// P_GATED (gated activation; 16 warps), P_ACT_BWD (its backward; 16 warps)
+// P_GATED (gated activation; 16 warps), P_ACT_BWD (its backward; 16 warps), P_GATE_BWD (backward of the attention gate;
+// 16 warps)
 template <int ES, int MMA, bool MN, int FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_THREADS : P_THREADS_16, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmCin, const GemmParams p)
+                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmCin,
+                     const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmParams p)
 {
     constexpr int ELEMS_PER_ROW = STAGE_ROW_BYTES / ES;
     constexpr int UMMA_K = 32 / ES, K_STEPS = 4, BK = ELEMS_PER_ROW;
@@ -140,7 +143,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
     uint64_t *bars = (uint64_t *)(smem + P_BAR_OFF);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + P_STAGES), tfull0 = smem_u32(bars + 2 * P_STAGES),
                    tempty0 = smem_u32(bars + 2 * P_STAGES + 2), drain = smem_u32(bars + 2 * P_STAGES + 4),
-                   cin0 = smem_u32(bars + 2 * P_STAGES + 5); // [warp][3]: residual block landed; P_ACT_BWD: see there
+                   cin0 = smem_u32(bars + 2 * P_STAGES + 5); // [warp][3]: residual block landed; the backward forms: see there
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * P_STAGES + 5 + 24);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
@@ -156,7 +159,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
             mbar_init(tempty0 + 8 * a, 2 * EPI_WARPS); // the leader's counts the epilogue warps of both CTAs
         }
         for (int i = 0; i < 24; ++i)
-            mbar_init(cin0 + 8 * i, FORM == P_ACT_BWD && i >= 16 ? 2 : 1);
+            mbar_init(cin0 + 8 * i, is_bwd(FORM) && i >= 16 ? 2 : 1);
         mbar_init(drain, 1);
         *abort_flag = 0;
         fence_barrier_init();
@@ -413,13 +416,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                     }
                 }
             }
-        } else if constexpr (FORM == P_ACT_BWD) {
+        } else if constexpr (is_bwd(FORM)) {
             // Backward of the gated activation (ffn_act_backward in kernels_elem.cu, same arithmetic) on the accumulator: a warp
             // takes 32 rows x 64 columns; the two warps of a 128-wide normalisation tile add their halves of its projection.
             // [wide | gate] values arrive by TMA in two 4 KB blocks per warp, a tile ahead; both gradients leave through the gate's
             // block.  As a kernel of its own this read the product back: 65536 x 3072 x 768 took 155 + 309 us, both bound by
             // their bytes; the product (2 x 403 MB of 2 GB) no longer goes through memory, 329 us.
-            const int part = ew >> 2;
+            // P_GATE_BWD, the attention gate (att_gate_backward): o in place of the wide values, the gradient of o in place of
+            // theirs, which leaves through o's block, and the sum of the products of both over the 128 columns of a head.
+            // 65536 x 1536 x 768 as two kernels 82 + 158 us, in one 184.
+            constexpr bool ATT = FORM == P_GATE_BWD;
+            const int part = ew >> 2, gate0 = ATT ? 3 * p.N : p.N; // first gate column
             uint8_t *const wblk = smem + P_STG_OFF + ew * 8192, *const gblk = wblk + 4096;
             const uint32_t in_bar = cin0 + 8 * ew, mate = cin0 + 8 * (16 + (ew & 3) + 4 * (part >> 1)); // mate: both warps of a tile
             const volatile float *const theirs = (const volatile float *)(smem + P_STG_OFF + (ew ^ 4) * 8192 + 4096 + 2048) + lane;
@@ -429,7 +436,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                 const int col = un.n0 + part * 64, r0 = un.m0 + (int)rank * 128 + quarter * 32;
                 if (!gate)
                     mbar_arrive_expect_tx(in_bar, 8192);
-                tma_load_2d(smem_u32(gate ? gblk : wblk), &tmCin, in_bar, gate ? p.N + col : col, r0);
+                if (gate)
+                    tma_load_2d(smem_u32(gblk), &tmCin, in_bar, gate0 + col, r0);
+                else
+                    tma_load_2d(smem_u32(wblk), ATT ? &tmX : &tmCin, in_bar, col, r0);
             };
             if (lane == 0 && first < units) {
                 fetch(first, false);
@@ -441,7 +451,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                 const PairUnit un = pair_unit(p, u);
                 const int m0 = un.m0 + (int)rank * 128, col = un.n0 + part * 64;
                 const long long row = m0 + row_in_cta;
-                const float scale = row < p.M && col < p.N ? p.act_scale[row * (p.N >> 7) + (col >> 7)] : 0.f;
+                const float scale = !ATT && row < p.M && col < p.N ? p.act_scale[row * (p.N >> 7) + (col >> 7)] : 0.f;
                 ok = __all_sync(0xffffffffu, mbar_wait(in_bar, in_phase, abort_flag));
                 if (!ok)
                     break;
@@ -453,7 +463,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * PN + part * 64;
                 const __half2 one = __float2half2_rn(1.f), two = __float2half2_rn(2.f);
-                __half2 dw[32]; // gradient of the normalised wide values
+                __half2 dw[32]; // gradient of the normalised wide values (of o)
                 uint32_t dg[16];
                 float proj = 0.f;
 #pragma unroll
@@ -480,9 +490,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                             dgate[j] = __hmul2(g, __hmul2(w, __hmul2(__hmul2(m, two), __hsub2(one, m))));
                             const __half2 d = __hmul2(g, m);
                             dw[16 * h + 4 * i + j] = d;
-                            const float2 pr = __half22float2(__hmul2(w, d));
-                            proj += pr.x + pr.y;
+                            if constexpr (ATT) { // from the fp16 values the attention kernels will read
+                                const float2 a = __half22float2(d), b = __half22float2(w);
+                                proj = fmaf(a.x, b.x, fmaf(a.y, b.y, proj));
+                            } else {
+                                const float2 pr = __half22float2(__hmul2(w, d));
+                                proj += pr.x + pr.y;
+                            }
                         }
+                        if constexpr (ATT) // over the values it came from, which only this thread reads
+                            *(uint4 *)(wblk + piece(lane, 4 * h + i)) =
+                                make_uint4(bits_from_h2(dw[16 * h + 4 * i]), bits_from_h2(dw[16 * h + 4 * i + 1]),
+                                           bits_from_h2(dw[16 * h + 4 * i + 2]), bits_from_h2(dw[16 * h + 4 * i + 3]));
                         dg[8 * h + 2 * i] = e4m3x4_from_h2(dgate[0], dgate[1]);
                         dg[8 * h + 2 * i + 1] = e4m3x4_from_h2(dgate[2], dgate[3]);
                     }
@@ -501,40 +520,50 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                 ok = __all_sync(0xffffffffu, mbar_wait(mate, 0, abort_flag));
                 if (!ok)
                     break;
-                proj = (proj + *theirs) * (1.f / 128);
+                proj += *theirs;
+                if (ATT && (part & 1) == 0 && row < p.M && col < p.N)
+                    p.bwd_dscale[row * (p.N >> 7) + (col >> 7)] = proj;
                 __syncwarp();
                 if (lane == 0)
                     mbar_arrive(mate);
                 ok = __all_sync(0xffffffffu, mbar_wait(mate, 1, abort_flag));
                 if (!ok)
                     break;
-                const __half2 nproj = __float2half2_rn(-proj), sc = __float2half2_rn(scale);
-                uint32_t dx[16];
+                if constexpr (!ATT) {
+                    const __half2 nproj = __float2half2_rn(proj * (-1.f / 128)), sc = __float2half2_rn(scale);
+                    uint32_t dx[16];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint4 w4 = *(const uint4 *)(wblk + piece(lane, i));
-                    const uint32_t wv[4] = {w4.x, w4.y, w4.z, w4.w};
-                    __half2 d[4];
+                    for (int i = 0; i < 8; ++i) {
+                        const uint4 w4 = *(const uint4 *)(wblk + piece(lane, i));
+                        const uint32_t wv[4] = {w4.x, w4.y, w4.z, w4.w};
+                        __half2 d[4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        d[j] = __hmul2(sc, __hfma2(h2_from_bits(wv[j]), nproj, dw[4 * i + j]));
-                    dx[2 * i] = e4m3x4_from_h2(d[0], d[1]);
-                    dx[2 * i + 1] = e4m3x4_from_h2(d[2], d[3]);
+                        for (int j = 0; j < 4; ++j)
+                            d[j] = __hmul2(sc, __hfma2(h2_from_bits(wv[j]), nproj, dw[4 * i + j]));
+                        dx[2 * i] = e4m3x4_from_h2(d[0], d[1]);
+                        dx[2 * i + 1] = e4m3x4_from_h2(d[2], d[3]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        *(uint4 *)(srow + 2048 + ((i ^ sw) << 4)) = make_uint4(dx[4 * i], dx[4 * i + 1], dx[4 * i + 2], dx[4 * i + 3]);
                 }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    *(uint4 *)(srow + 2048 + ((i ^ sw) << 4)) = make_uint4(dx[4 * i], dx[4 * i + 1], dx[4 * i + 2], dx[4 * i + 3]);
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
                     if (col < p.N) {
-                        tma_store_2d(&tmC, smem_u32(gblk), p.N + col, m0 + quarter * 32);
-                        tma_store_2d(&tmC, smem_u32(gblk) + 2048, col, m0 + quarter * 32);
+                        tma_store_2d(&tmC, smem_u32(gblk), gate0 + col, m0 + quarter * 32);
+                        if constexpr (ATT)
+                            tma_store_2d(&tmY, smem_u32(wblk), col, m0 + quarter * 32);
+                        else
+                            tma_store_2d(&tmC, smem_u32(gblk) + 2048, col, m0 + quarter * 32);
                     }
                     bulk_commit();
                     if (u + step < units) {
-                        fetch(u + step, false);
-                        bulk_wait_read<0>(); // the stores have read the gate's block
+                        if constexpr (!ATT)
+                            fetch(u + step, false);
+                        bulk_wait_read<0>(); // the stores have read their blocks
+                        if constexpr (ATT)
+                            fetch(u + step, false);
                         fetch(u + step, true);
                     }
                 }
@@ -755,7 +784,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
 
 template <int ES, int MMA, bool MN, int FORM>
 int launch_pair(int device, cudaStream_t stream, int grid, const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmC,
-                const CUtensorMap &tmCin, const GemmParams &p)
+                const CUtensorMap &tmCin, const CUtensorMap &tmX, const CUtensorMap &tmY, const GemmParams &p)
 {
     auto kern = gemm_pair_kernel<ES, MMA, MN, FORM>;
     static bool configured[16] = {};
@@ -763,19 +792,20 @@ int launch_pair(int device, cudaStream_t stream, int grid, const CUtensorMap &tm
         TS2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<FORM>::TOTAL));
         configured[device & 15] = true;
     }
-    TS2_LAUNCH((kern), grid, FORM == P_F32 ? P_THREADS : P_THREADS_16, PairSmem<FORM>::TOTAL, stream, tmA, tmB, tmC, tmCin, p);
+    TS2_LAUNCH((kern), grid, FORM == P_F32 ? P_THREADS : P_THREADS_16, PairSmem<FORM>::TOTAL, stream, tmA, tmB, tmC, tmCin, tmX, tmY, p);
     return TS2_OK;
 }
 
 } // namespace
 
 int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, int form_arg, int grid, const CUtensorMap &tmA,
-                     const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const GemmParams &p)
+                     const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const CUtensorMap &tmX, const CUtensorMap &tmY,
+                     const GemmParams &p)
 {
-    const int form = form_arg == 2 ? P_ACT_BWD : form_arg == 1 ? P_GATED : p.splits == 1 && (p.out_kind == TS2_OUT_F16 || p.out_kind == TS2_OUT_BF16) ? P_16 : P_F32;
+    const int form = form_arg == 3 ? P_GATE_BWD : form_arg == 2 ? P_ACT_BWD : form_arg == 1 ? P_GATED : p.splits == 1 && (p.out_kind == TS2_OUT_F16 || p.out_kind == TS2_OUT_BF16) ? P_16 : P_F32;
 #define TS2_PAIR_CASE(ES_, MMA_, MN_, FORM_)                          \
     if (es == ES_ && mma == MMA_ && mn == MN_ && form == FORM_)       \
-        return launch_pair<ES_, MMA_, MN_, FORM_>(device, stream, grid, tmA, tmB, tmC, tmCin, p);
+        return launch_pair<ES_, MMA_, MN_, FORM_>(device, stream, grid, tmA, tmB, tmC, tmCin, tmX, tmY, p);
 #define TS2_PAIR_CASES(ES_, MMA_)              \
     TS2_PAIR_CASE(ES_, MMA_, false, P_F32)     \
     TS2_PAIR_CASE(ES_, MMA_, false, P_16)      \
@@ -784,6 +814,7 @@ int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, 
     TS2_PAIR_CASE(ES_, MMA_, true, P_16)
     TS2_PAIR_CASES(1, 0)
     TS2_PAIR_CASE(1, 0, false, P_ACT_BWD)
+    TS2_PAIR_CASE(1, 0, false, P_GATE_BWD)
     TS2_PAIR_CASES(2, 1)
     TS2_PAIR_CASES(1, 2)
 #undef TS2_PAIR_CASES

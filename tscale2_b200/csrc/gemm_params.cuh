@@ -43,12 +43,15 @@ struct GemmParams {
     float *act_scale = nullptr;
     float act_mult = 1.f;
     int act_kind = 0; // format of act_out: 0 e4m3, 1 fp16, 2 int8
+    float *bwd_dscale = nullptr; // backward of the attention gate (see Epilogue)
 };
 
 // gemm_pair.cu: the contraction on pairs of CTAs (tiles of 256 x 256).  tmB's box is 128 rows (K-major) or one K block
 // (token-major); tmC's and tmCin's are 32 rows x 128 bytes.  grid: CTAs, an even number.
-// form: 0 by output kind, 1 gated activation, 2 its backward (tmC: 32 rows x 64 bytes, tmCin: [wide | gate] in 32 rows x 128)
+// form: 0 by output kind, 1 gated activation, 2 its backward (tmC: 32 rows x 64 bytes, tmCin: [wide | gate] in 32 rows x 128),
+// 3 backward of the attention gate (the same, and tmX: o, tmY: dout, both 32 rows x 128); tmX, tmY otherwise unused
 int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, int form, int grid, const CUtensorMap &tmA,
-                     const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const GemmParams &p);
+                     const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const CUtensorMap &tmX, const CUtensorMap &tmY,
+                     const GemmParams &p);
 
 } // namespace ts2

@@ -1577,11 +1577,17 @@ int backward(ts2_model *m)
         e3.alpha = 1.f / (32.f * sqrtf((float)D));
         e3.out_kind = TS2_OUT_F16;
         TRACE("g_fast", l, m->g_fast, (size_t)T * D * fsz, fsz == 2 ? TR_F16 : TR_RAW);
-        // FFN, many tiles: the contraction's epilogue goes on through the activation; drg never reaches memory
-        const bool act_fused = ly.type != TS2_LAYER_ATT && gemm_takes_act_backward(m->device, m->kind, T, W);
+        // many tiles: the contraction's epilogue goes on through the activation or the gate; drg never reaches memory
+        const bool act_fused = gemm_takes_act_backward(m->device, m->kind, T, W);
         if (act_fused) {
             e3.bwd_wg = ly.cat16;
-            e3.act_scale = ly.wscale;
+            if (ly.type == TS2_LAYER_ATT) {
+                e3.bwd_o = ly.o;
+                e3.bwd_dout = m->dout;
+                e3.bwd_dscale = m->dscale;
+            } else {
+                e3.act_scale = ly.wscale;
+            }
             M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->dcat, C, e3));
         } else {
             M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->drg, W, e3));
@@ -1597,7 +1603,8 @@ int backward(ts2_model *m)
             TRACE("dW_c", l, mc.grad, (size_t)D * W * 4, TR_F32);
         }
         if (ly.type == TS2_LAYER_ATT) {
-            M_TRY(att_gate_backward(c, m->drg, ly.cat16, ly.o, T, W, m->dcat, m->dout, m->dscale));
+            if (!act_fused)
+                M_TRY(att_gate_backward(c, m->drg, ly.cat16, ly.o, T, W, m->dcat, m->dout, m->dscale));
             TRACE("dout", l, m->dout, (size_t)T * W * 2, TR_F16);
             TRACE("dscale", l, m->dscale, (size_t)T * H * 4, TR_F32);
             M_TRY(attention_backward(c, ly.q, ly.k, ly.v, m->dout, ly.lse, m->dscale, b.span_start[ly.att_type], b.span_finish[ly.att_type],
