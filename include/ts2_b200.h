@@ -471,6 +471,11 @@ int ts2_moe_route(int device, const float *logits, int T, int expert_count, int 
 int ts2_attention_forward(int device, void *stream, int variant, const void *q, const void *k, const void *v,
                           const int32_t *span_start, const int32_t *span_finish, int T, int head_count, float alibi_slope,
                           void *o, float *lse);
+/* The engine's form of variant 2: also rg [T][Q] = s * sigmoid(2 gate) * o in the operand format of prec (s: 16 e4m3, 1 fp16, 24
+ * int8); gate fp16, rows of gate_ld elements, 16-byte aligned base and pitch. */
+int ts2_op_attention_gated_forward(int device, void *stream, int prec, const void *q, const void *k, const void *v,
+                                   const int32_t *span_start, const int32_t *span_finish, int T, int head_count, float alibi_slope,
+                                   const void *gate, int64_t gate_ld, void *o, float *lse, void *rg);
 int ts2_attention_backward(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
                            const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
                            int head_count, float alibi_slope, void *dq, void *dk, void *dv);

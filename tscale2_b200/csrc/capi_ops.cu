@@ -410,6 +410,24 @@ int ts2_attention_forward(int device, void *stream, int variant, const void *q, 
     return rc;
 }
 
+int ts2_op_attention_gated_forward(int device, void *stream, int prec, const void *q, const void *k, const void *v,
+                                   const int32_t *span_start, const int32_t *span_finish, int T, int head_count, float alibi_slope,
+                                   const void *gate, int64_t gate_ld, void *o, float *lse, void *rg)
+{
+    if (T <= 0 || head_count <= 0 || !q || !k || !v || !o || !lse || !span_start || !span_finish || !gate || !rg || kind_of(prec) < 0 ||
+        gate_ld < 128ll * head_count || gate_ld % 8 || (((uintptr_t)gate | (uintptr_t)rg) & 15))
+        return fail(TS2_ERR_INVALID_ARG, "ts2_op_attention_gated_forward: bad arguments");
+    TS2_CUDA(cudaSetDevice(device));
+    const Ctx c = op_ctx(device, stream, prec);
+    SpanScratch spans(c, span_start, span_finish, T, 2 * (size_t)T);
+    if (spans.rc != TS2_OK)
+        return spans.rc;
+    const int rc = attention_forward(c, (const __half *)q, (const __half *)k, (const __half *)v, spans.d, spans.d + T, T, head_count,
+                                     alibi_slope, (__half *)o, lse, AttGate{(const __half *)gate, gate_ld, rg});
+    cudaStreamSynchronize(c.stream);
+    return rc;
+}
+
 int ts2_attention_backward(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
                            const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
                            int head_count, float alibi_slope, void *dq, void *dk, void *dv)

@@ -115,8 +115,6 @@ int i8_to_half(const Ctx &c, const void *src, size_t n, __half *dst);
 int ffn_act_backward(const Ctx &c, const __half *drg, const __half *wg, const __half *what, int what_ld, const float *wscale, int T, int F,
                      void *d2);
 
-// attention gate: rg = sigmoid(2 gate) * o  (LoLU, cpu_util.cpp:139-168); gate inside qkvg [T][4Q] at column 3Q
-int att_gate_forward(const Ctx &c, const __half *qkvg, const __half *o, int T, int Q, void *rg);
 // dgate -> d4[:, 3Q:4Q] (fast), do (fp16) and dScale[t][h] = sum do*o  (BackpropLoLU + ComputeDScale)
 int att_gate_backward(const Ctx &c, const __half *drg, const __half *qkvg, const __half *o, int T, int Q, void *d4, __half *dout,
                       float *dscale);
@@ -143,8 +141,14 @@ int fill_rope(const Ctx &c, float *rope, int T);
 
 // attention over one span per node (ComputeValLookup / GradQ / GradK, layer_att_reference.h:41-212)
 // o [T][Q] fp16, lse [T][H] = maxDP + log2(sumWeight); dq, dk, dv fp32, or fp16 with grads16
+// gate: also rg = s_act * sigmoid(2 gate) * o in the operand format (LoLU, cpu_util.cpp:139-168)
+struct AttGate {
+    const __half *gate = nullptr; // [T][Q], rows of ld elements, 16-byte aligned
+    int64_t ld = 0;
+    void *rg = nullptr;           // [T][Q]
+};
 int attention_forward(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
-                      int T, int H, float slope, __half *o, float *lse);
+                      int T, int H, float slope, __half *o, float *lse, const AttGate &gate);
 // What the backward kernels need besides the layer's tensors.
 //  layout (att_layout_bytes): the batch's spans in the form they read, made once per batch by att_layout
 //  scratch (att_bwd_scratch_bytes): per-node records of the call
@@ -172,7 +176,7 @@ int attention_backward_mma(const Ctx &c, const __half *q, const __half *k, const
                            const float *dscale, const int *span_start, const int *span_finish, const int *rev_first,
                            const int *rev_last, int T, int H, float slope, float *dq, float *dk, float *dv);
 int attention_forward_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
-                         int T, int H, float slope, __half *o, float *lse);
+                         int T, int H, float slope, __half *o, float *lse, const AttGate *gate = nullptr);
 int attention_forward_rowwise(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start,
                               const int *span_finish, int T, int H, float slope, __half *o, float *lse);
 int attention_backward_rowwise(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,

@@ -321,9 +321,9 @@ int attention_backward_rowwise(const Ctx &c, const __half *q, const __half *k, c
 }
 
 int attention_forward(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
-                      int T, int H, float slope, __half *o, float *lse)
+                      int T, int H, float slope, __half *o, float *lse, const AttGate &gate)
 {
-    return attention_forward_tc(c, q, k, v, span_start, span_finish, T, H, slope, o, lse);
+    return attention_forward_tc(c, q, k, v, span_start, span_finish, T, H, slope, o, lse, &gate);
 }
 
 } // namespace ts2

@@ -16,6 +16,10 @@
 //              than 8 (2^8 headroom in fp16 P and fp32 sums), which keeps tcgen05.ld/st of O off
 //              the common path
 // The zero "sink" vector of the reference is the initial state m = 0, l = 1.
+// The engine's form (GATE >= 0) also applies the output gate and writes the next contraction's operand (0 e4m3, 1 fp16,
+// 2 int8).  As a kernel of its own that was bound by its bytes (o read back, the gate read, the operand written); here the
+// gate's tile comes into the K ring behind the last product of the block, prefetched into L2 when the block starts.
+// 65536 nodes x 12 heads, e4m3: 394 + 112 us as two kernels, 450 in one.
 // Two CTAs fit an SM (112 KB shared memory, 256 TMEM columns each), so one CTA's softmax overlaps
 // the other's MMAs.  Every wait is bounded (see mbar_wait); a give-up raises the status word.
 #include "att_tc.cuh"
@@ -33,12 +37,48 @@ struct AttTcParams {
     const int *span_start, *span_finish;
     __half *o;
     float *lse;
+    void *rg;
+    float s_act;
     int32_t *status;
 };
 
+// s_act * sigmoid(2 gate) * o of eight elements in operand format FT, as two (one-byte formats) or four words
+template <int FT>
+__device__ __forceinline__ void gate_pack8(uint4 gate, uint4 o, float s_act, uint32_t *w)
+{
+    const uint32_t g[4] = {gate.x, gate.y, gate.z, gate.w}, x[4] = {o.x, o.y, o.z, o.w};
+    if constexpr (FT == 0) { // packed fp16 (see fast_types.cuh): e4m3 keeps 4 of its 11 bits
+        const __half2 sa = __float2half2_rn(s_act);
+        __half2 r[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            r[i] = __hmul2(__hmul2(lolu_mult_h2(h2_from_bits(g[i])), h2_from_bits(x[i])), sa);
+        w[0] = e4m3x4_from_h2(r[0], r[1]);
+        w[1] = e4m3x4_from_h2(r[2], r[3]);
+    } else {
+        float r[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 a = __half22float2(h2_from_bits(g[i])), b = __half22float2(h2_from_bits(x[i]));
+            r[2 * i] = lolu_mult(a.x) * b.x * s_act;
+            r[2 * i + 1] = lolu_mult(a.y) * b.y * s_act;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if constexpr (FT == 1) {
+                w[2 * i] = bits_from_h2(sat_half2(r[4 * i], r[4 * i + 1]));
+                w[2 * i + 1] = bits_from_h2(sat_half2(r[4 * i + 2], r[4 * i + 3]));
+            } else {
+                w[i] = sat_i8(r[4 * i]) | (sat_i8(r[4 * i + 1]) << 8) | (sat_i8(r[4 * i + 2]) << 16) | (sat_i8(r[4 * i + 3]) << 24);
+            }
+    }
+}
+
+template <int GATE>
 __global__ void __launch_bounds__(TC_THREADS, 2)
     att_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const AttTcParams p)
+                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
+                      const __grid_constant__ CUtensorMap tmG, const AttTcParams p)
 {
     extern __shared__ __align__(1024) uint8_t att_tc_smem[];
     uint8_t *smem = att_tc_smem;
@@ -54,6 +94,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
     uint32_t *tmem_slot = (uint32_t *)(bars + 13);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
     int &s_lo = *(int *)(tmem_slot + 2), &s_hi = *(int *)(tmem_slot + 3);
+    const uint32_t gate_full = smem_u32(bars + 15);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int T = p.T, H = p.H, h = blockIdx.y, t0 = blockIdx.x * TC_BM;
@@ -89,6 +130,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
         }
         mbar_init(p_full, 256);
         mbar_init(o_ready, 1);
+        mbar_init(gate_full, 1);
         *abort_flag = 0;
         fence_barrier_init();
         prefetch_tmap(&tmQ);
@@ -106,12 +148,16 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
 
     const int n_tiles = tile1 - tile0 + 1;
     if (warp == 0) {
+        bool ok = true;
         if (lane == 0 && n_tiles > 0) {
+            if (GATE >= 0) { // into L2 by the time the K ring is free for them
+                tma_prefetch_2d(&tmG, col0, t0);
+                tma_prefetch_2d(&tmG, col0 + 64, t0);
+            }
             mbar_arrive_expect_tx(q_full, Q_BYTES);
             tma_load_2d(sQ, &tmQ, q_full, col0, t0);
             tma_load_2d(sQ + Q_BYTES / 2, &tmQ, q_full, col0 + 64, t0);
             // order of need: K(0), then for every tile K(j+1) before V(j)
-            bool ok = true;
             for (int j = -1; j < n_tiles && ok; ++j) {
                 if (j + 1 < n_tiles) {
                     const int jj = j + 1, st = jj & 1;
@@ -131,6 +177,16 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
                     tma_load_2d(dv, &tmV, fb, col0, (tile0 + j) * TC_BN);
                     tma_load_2d(dv + KV_BYTES / 2, &tmV, fb, col0 + 64, (tile0 + j) * TC_BN);
                 }
+            }
+        }
+        if (GATE >= 0 && lane == 0 && ok) {
+            // the block's gates, 64 columns into each K stage once its last product is done
+            mbar_arrive_expect_tx(gate_full, 2 * KV_BYTES);
+            for (int jj = n_tiles; jj < n_tiles + 2; ++jj) {
+                const int st = jj & 1;
+                if (!mbar_wait(k_empty0 + 8 * st, ((jj >> 1) & 1) ^ 1, abort_flag))
+                    break;
+                tma_load_2d(sK + st * KV_BYTES, &tmG, gate_full, col0 + 64 * st, t0);
             }
         }
     } else if (warp == 1) {
@@ -311,6 +367,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
         pair_barrier(quarter);
         l += lx[(half ^ 1) * TC_BM + row];
         const float inv = 1.f / l;
+        if constexpr (GATE >= 0)
+            ok = __all_sync(0xffffffffu, mbar_wait(gate_full, 0, abort_flag)) && ok;
         // A warp's 32 rows x 64 fp16 columns go through a 4 KB block of the Q tile (idle now: every MMA is complete),
         // rows of 128 bytes with the 128-byte swizzle (16-byte chunk c of row r at c ^ (r & 7)), and one TMA store:
         // direct stores would write 16 bytes into each of 32 different lines per instruction.  Rows past T are clipped.
@@ -327,14 +385,27 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
                 for (int i = 0; i < 32; ++i)
                     r[i] = 0u;
             }
+            constexpr int WORDS = GATE == 1 ? 4 : 2; // per 8 elements
+            uint32_t w[4 * WORDS];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 __half2 h0 = sat_half2(__uint_as_float(r[8 * i]) * inv, __uint_as_float(r[8 * i + 1]) * inv),
                         h1 = sat_half2(__uint_as_float(r[8 * i + 2]) * inv, __uint_as_float(r[8 * i + 3]) * inv),
                         h2 = sat_half2(__uint_as_float(r[8 * i + 4]) * inv, __uint_as_float(r[8 * i + 5]) * inv),
                         h3 = sat_half2(__uint_as_float(r[8 * i + 6]) * inv, __uint_as_float(r[8 * i + 7]) * inv);
-                *(uint4 *)(srow + (((cc * 4 + i) ^ (lane & 7)) << 4)) = make_uint4(*(uint32_t *)&h0, *(uint32_t *)&h1, *(uint32_t *)&h2, *(uint32_t *)&h3);
+                const uint4 o8 = make_uint4(*(uint32_t *)&h0, *(uint32_t *)&h1, *(uint32_t *)&h2, *(uint32_t *)&h3);
+                *(uint4 *)(srow + (((cc * 4 + i) ^ (lane & 7)) << 4)) = o8;
+                if constexpr (GATE >= 0)
+                    gate_pack8<GATE>(*(const uint4 *)(smem + Q_BYTES + half * KV_BYTES + row * 128 + (((cc * 4 + i) ^ (row & 7)) << 4)), o8,
+                                     p.s_act, w + i * WORDS);
             }
+            if constexpr (GATE >= 0)
+                if (t < T) {
+                    uint4 *out = (uint4 *)((uint8_t *)p.rg + ((size_t)t * (H * TC_HD) + h * TC_HD + c * 32) * (GATE == 1 ? 2 : 1));
+#pragma unroll
+                    for (int i = 0; i < WORDS; ++i)
+                        out[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+                }
         }
         fence_proxy_async();
         __syncwarp();
@@ -355,11 +426,13 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
 }
 
 int attention_forward_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
-                         int T, int H, float slope, __half *o, float *lse)
+                         int T, int H, float slope, __half *o, float *lse, const AttGate *gate)
 {
     static bool configured[16] = {};
     if (!configured[c.device & 15]) {
-        TS2_CUDA(cudaFuncSetAttribute(att_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM));
+        for (const void *kern : {(const void *)att_fwd_tc_kernel<-1>, (const void *)att_fwd_tc_kernel<0>,
+                                 (const void *)att_fwd_tc_kernel<1>, (const void *)att_fwd_tc_kernel<2>})
+            TS2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM));
         configured[c.device & 15] = true;
     }
     const int Q = H * TC_HD;
@@ -373,6 +446,9 @@ int attention_forward_tc(const Ctx &c, const __half *q, const __half *k, const _
         return rc;
     if ((rc = make_tensor_map(&tmO, o, 2, Q, T, Q, 32)) != TS2_OK) // output: boxes of 64 fp16 columns x 32 rows
         return rc;
+    CUtensorMap tmG = tmO;
+    if (gate && (rc = make_tensor_map(&tmG, gate->gate, 2, Q, T, gate->ld, TC_BM)) != TS2_OK)
+        return rc;
     AttTcParams p;
     p.T = T;
     p.H = H;
@@ -381,11 +457,18 @@ int attention_forward_tc(const Ctx &c, const __half *q, const __half *k, const _
     p.span_finish = span_finish;
     p.o = o;
     p.lse = lse;
+    p.rg = gate ? gate->rg : nullptr;
+    p.s_act = c.s_act;
     p.status = device_status_word(c.device);
     if (!p.status)
         return fail(TS2_ERR_CUDA, "attention: no device status word");
     dim3 grid((unsigned)ceil_div(T, TC_BM), (unsigned)H);
-    TS2_LAUNCH((att_fwd_tc_kernel), grid, TC_THREADS, FWD_SMEM, c.stream, tmQ, tmK, tmV, tmO, p);
+    switch (gate ? c.ft : -1) {
+    case 0: TS2_LAUNCH((att_fwd_tc_kernel<0>), grid, TC_THREADS, FWD_SMEM, c.stream, tmQ, tmK, tmV, tmO, tmG, p); break;
+    case 1: TS2_LAUNCH((att_fwd_tc_kernel<1>), grid, TC_THREADS, FWD_SMEM, c.stream, tmQ, tmK, tmV, tmO, tmG, p); break;
+    case 2: TS2_LAUNCH((att_fwd_tc_kernel<2>), grid, TC_THREADS, FWD_SMEM, c.stream, tmQ, tmK, tmV, tmO, tmG, p); break;
+    default: TS2_LAUNCH((att_fwd_tc_kernel<-1>), grid, TC_THREADS, FWD_SMEM, c.stream, tmQ, tmK, tmV, tmO, tmG, p);
+    }
     return TS2_OK;
 }
 

@@ -492,92 +492,6 @@ int ffn_act_backward(const Ctx &c, const __half *drg, const __half *wg, const __
 
 // ---------------------------------------------------------------------------------
 template <int FT>
-__global__ void att_gate_forward_kernel(const __half *__restrict__ qkvg, const __half *__restrict__ o, int T, int Q, float s_act,
-                                        void *__restrict__ rg)
-{
-    grid_dep_wait();
-    const int tiles = Q / TILE;
-    constexpr int R = 2;
-    WARP_BATCH_LOOP((long long)T * tiles, R)
-    {
-        float4 gate[R], ov[R];
-        size_t t[R];
-        int off[R];
-        bool ok[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const unsigned item = base + r * wstride;
-            ok[r] = item < total_items;
-            t[r] = ok[r] ? item / tiles : 0;
-            off[r] = (ok[r] ? (int)(item % tiles) : 0) * TILE + lane * 4;
-            gate[r] = ok[r] ? load_half4(qkvg + t[r] * 4 * Q + 3 * Q + off[r]) : make_float4(0, 0, 0, 0);
-            ov[r] = ok[r] ? load_half4(o + t[r] * Q + off[r]) : make_float4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if (!ok[r])
-                continue;
-            const float4 res = make_float4(lolu_mult_ft<FT>(gate[r].x) * ov[r].x, lolu_mult_ft<FT>(gate[r].y) * ov[r].y,
-                                           lolu_mult_ft<FT>(gate[r].z) * ov[r].z, lolu_mult_ft<FT>(gate[r].w) * ov[r].w);
-            Fast<FT>::store4(rg, t[r] * Q + off[r], scale4(res, s_act));
-        }
-    }
-}
-
-__global__ void att_gate_forward_e4m3_kernel(const __half *__restrict__ qkvg, const __half *__restrict__ o, int T, int Q, float s_act,
-                                             uint8_t *__restrict__ rg)
-{
-    grid_dep_wait();
-    const int tiles = Q / TILE;
-    constexpr int R = 4;
-    const __half2 sa = __float2half2_rn(s_act);
-    WARP_BATCH_LOOP((long long)T * tiles, R)
-    {
-        uint2 gate[R], ov[R];
-        size_t t[R];
-        int off[R];
-        bool ok[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const unsigned item = base + r * wstride;
-            ok[r] = item < total_items;
-            t[r] = ok[r] ? item / tiles : 0;
-            off[r] = (ok[r] ? (int)(item % tiles) : 0) * TILE + lane * 4;
-            const uint2 z = make_uint2(0u, 0u);
-            gate[r] = ok[r] ? *(const uint2 *)(qkvg + t[r] * 4 * Q + 3 * Q + off[r]) : z;
-            ov[r] = ok[r] ? *(const uint2 *)(o + t[r] * Q + off[r]) : z;
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if (!ok[r])
-                continue;
-            const __half2 r0 = __hmul2(__hmul2(lolu_mult_h2(h2_from_bits(gate[r].x)), h2_from_bits(ov[r].x)), sa);
-            const __half2 r1 = __hmul2(__hmul2(lolu_mult_h2(h2_from_bits(gate[r].y)), h2_from_bits(ov[r].y)), sa);
-            *(uint32_t *)(rg + t[r] * Q + off[r]) = e4m3x4_from_h2(r0, r1);
-        }
-    }
-}
-
-int att_gate_forward(const Ctx &c, const __half *qkvg, const __half *o, int T, int Q, void *rg)
-{
-    if (c.ft == 0) {
-        TS2_LAUNCH((att_gate_forward_e4m3_kernel), grid_for(c, att_gate_forward_e4m3_kernel, (long long)T * (Q / TILE)), THREADS, 0,
-                   c.stream, qkvg, o, T, Q, c.s_act, (uint8_t *)rg);
-        return TS2_OK;
-    }
-    const int grid = c.ft == 0   ? grid_for(c, att_gate_forward_kernel<0>, (long long)T * (Q / TILE))
-                     : c.ft == 1 ? grid_for(c, att_gate_forward_kernel<1>, (long long)T * (Q / TILE))
-                                 : grid_for(c, att_gate_forward_kernel<2>, (long long)T * (Q / TILE));
-    if (c.ft == 0)
-        TS2_LAUNCH((att_gate_forward_kernel<0>), grid, THREADS, 0, c.stream, qkvg, o, T, Q, c.s_act, rg);
-    else if (c.ft == 1)
-        TS2_LAUNCH((att_gate_forward_kernel<1>), grid, THREADS, 0, c.stream, qkvg, o, T, Q, c.s_act, rg);
-    else
-        TS2_LAUNCH((att_gate_forward_kernel<2>), grid, THREADS, 0, c.stream, qkvg, o, T, Q, c.s_act, rg);
-    return TS2_OK;
-}
-
-template <int FT>
 __global__ void att_gate_backward_kernel(const __half *__restrict__ drg, const __half *__restrict__ qkvg, const __half *__restrict__ o,
                                          int T, int Q, void *__restrict__ d4, __half *__restrict__ dout, float *__restrict__ dscale)
 {

@@ -1263,10 +1263,10 @@ int forward(ts2_model *m)
             TRACE("q", l, ly.q, (size_t)T * W * 2, TR_F16);
             TRACE("k", l, ly.k, (size_t)T * W * 2, TR_F16);
             TRACE("v", l, ly.v, (size_t)T * W * 2, TR_F16);
-            M_TRY(attention_forward(c, ly.q, ly.k, ly.v, b.span_start[ly.att_type], b.span_finish[ly.att_type], T, H, ly.slope, ly.o, ly.lse));
+            M_TRY(attention_forward(c, ly.q, ly.k, ly.v, b.span_start[ly.att_type], b.span_finish[ly.att_type], T, H, ly.slope, ly.o, ly.lse,
+                                    AttGate{ly.cat16 + 3 * (size_t)W, C, ly.rg}));
             TRACE("att_o", l, ly.o, (size_t)T * W * 2, TR_F16);
             TRACE("att_lse", l, ly.lse, (size_t)T * H * 4, TR_F32);
-            M_TRY(att_gate_forward(c, ly.cat16, ly.o, T, W, ly.rg));
         } else {
             TRACE("wscale", l, ly.wscale, (size_t)T * (W / 128) * 4, TR_F32);
         }
