@@ -1120,7 +1120,8 @@ int gemm(const GemmArgs &a)
     }
     const bool act_bwd = a.epi.bwd_wg != nullptr, gate_bwd = act_bwd && a.epi.bwd_o;
     const int64_t bwd_ld = (gate_bwd ? 4 : 2) * a.N;
-    if (act_bwd && (paired || a.mn_major || a.group_mode || a.kind != KIND_E4M3 || a.epi.out_kind != TS2_OUT_F16 || a.N % 128 ||
+    if (act_bwd && (paired || a.mn_major || a.group_mode || a.epi.row_scale || a.epi.col_scale || a.kind != KIND_E4M3 ||
+                    a.epi.out_kind != TS2_OUT_F16 || a.N % 128 ||
                     a.ldc != bwd_ld || !(gate_bwd ? a.epi.bwd_dscale && a.epi.bwd_dout : a.epi.act_scale != nullptr) ||
                     (((uintptr_t)a.epi.bwd_wg | (uintptr_t)a.epi.bwd_o | (uintptr_t)a.epi.bwd_dout) & 15) || !pl.pair() || pl.splits != 1))
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of the activation's backward form");
