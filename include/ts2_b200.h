@@ -179,6 +179,10 @@ int ts2_get_label_index(ts2_model *m, uint32_t *labels, uint32_t *nodes, int64_t
 int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model);
 /* IModel::WaitAllCompute, src/gpt/compute/model.h:54 — bounded wait */
 int ts2_wait(ts2_model *m);
+/* Wall time after which a call that waits for the device (ts2_wait and everything that reads results, and ts2_set_batch
+ * once two earlier batches are still queued) gives up with TS2_ERR_TIMEOUT; 120 s unless set.  What was queued stays queued:
+ * the call can be repeated. */
+int ts2_set_wait_limit(ts2_model *m, double seconds);
 /* IModelInstance::ComputeScore, src/gpt/compute/model.h:39: mean log p(target) (natural log) */
 int ts2_forward_score(ts2_model *m, float *out_score);
 /* IModel::GetAvrgTrainErr, src/gpt/compute/model.h:55: mean -log p(target) of the last backprop */

@@ -222,6 +222,7 @@ struct ts2_model {
     size_t pinned_bytes = 0;
     HostReport *report = nullptr;  // pinned; written by the kernel that every wait queues (queue_report)
     bool unreported = false;       // work was queued since the last wait
+    double wait_limit_s = 120;     // wall time after which a wait gives up (poll_until)
     bool grads_dirty = false; // the flat gradient holds an accumulated, not yet applied gradient
     // dense dW contractions write their whole matrix: the first of an accumulation overwrites what is there
     int dense_dw_out() const { return grads_dirty ? TS2_OUT_F32_ADD : TS2_OUT_F32; }
@@ -267,6 +268,30 @@ int mfail(ts2_model *m, int code)
         if (_rc != TS2_OK)          \
             return mfail(m, _rc);   \
     } while (0)
+
+// Bounded wait: polls until `query` (of an event or a stream) no longer answers "not ready", for up to wait_limit_s of
+// wall time.  Every wait of the training path comes here: a device that will not finish (a collective whose peer is
+// gone) becomes an error code.
+template <class Q>
+int poll_until(const ts2_model *m, Q query)
+{
+    cudaError_t e;
+    const auto t0 = std::chrono::steady_clock::now();
+    while ((e = query()) == cudaErrorNotReady) {
+        const double waited = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        if (waited > m->wait_limit_s)
+            return fail(TS2_ERR_TIMEOUT, "the device did not finish within %g s", m->wait_limit_s);
+        if (waited > 0.02) // a sleep takes 100 us with the kernel's timer slack: not worth it in steps of a few ms
+            std::this_thread::sleep_for(std::chrono::microseconds(50));
+    }
+    if (e != cudaSuccess)
+        return fail(TS2_ERR_CUDA, "stream failed: %s", cudaGetErrorString(e));
+    return TS2_OK;
+}
+int poll_stream(const ts2_model *m)
+{
+    return poll_until(m, [&] { return cudaStreamQuery(m->stream); });
+}
 
 template <class T>
 int dalloc(ts2_model *m, T **p, size_t count)
@@ -627,7 +652,7 @@ int ep_prepare(ts2_model *m, Layer &ly)
     const int E = m->E, N = m->world;
     M_NCCL(ncclAllGather(m->cnt_own, m->cnt_all, E, ncclInt32, m->comm_x, m->stream));
     TS2_CUDA(cudaMemcpyAsync(m->h_cnt, m->cnt_all, (size_t)N * E * 4, cudaMemcpyDeviceToHost, m->stream));
-    TS2_CUDA(cudaStreamSynchronize(m->stream));
+    M_TRY(poll_stream(m));
     int max_x = 0;
     ep_plan(N, m->rank, E, m->h_cnt, &ly.plan, &max_x);
     if (max_x > m->x_cap) // every rank sees the same counts and takes the same decision
@@ -1754,9 +1779,9 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
                         n_spans, T);
     }
     const int slot = b.next_slot;
+    if (b.slot_used[slot]) // the copy that last read this slot sits behind the step before: this is what holds a fast host back
+        M_TRY(poll_until(m, [&] { return cudaEventQuery(b.slot_ev[slot]); }));
     b.next_slot ^= 1;
-    if (b.slot_used[slot])
-        TS2_CUDA(cudaEventSynchronize(b.slot_ev[slot])); // the copy that last read this slot
     uint32_t *h = (uint32_t *)m->pinned + (size_t)slot * b.raw_cap;
     size_t used = 0;
     auto put = [&](const void *src, size_t n) {
@@ -1834,23 +1859,6 @@ int report_batch_status(ts2_model *m)
         return fail(TS2_ERR_INVALID_ARG, "batch: label %d (entry %d, node %d) out of range", d0, where, d1);
     }
     return fail(TS2_ERR_INVALID_ARG, "batch: malformed (code %d)", code);
-}
-
-// bounded wait: poll the stream for up to 120 s of wall time, then report a timeout
-int poll_stream(ts2_model *m)
-{
-    cudaError_t e;
-    const auto t0 = std::chrono::steady_clock::now();
-    while ((e = cudaStreamQuery(m->stream)) == cudaErrorNotReady) {
-        const double waited = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-        if (waited > 120.0)
-            return fail(TS2_ERR_TIMEOUT, "the device did not finish within 120 s");
-        if (waited > 0.02) // a sleep takes 100 us with the kernel's timer slack: not worth it in steps of a few ms
-            std::this_thread::sleep_for(std::chrono::microseconds(50));
-    }
-    if (e != cudaSuccess)
-        return fail(TS2_ERR_CUDA, "stream failed: %s", cudaGetErrorString(e));
-    return TS2_OK;
 }
 
 // Waits for everything queued and reports what the device recorded.  One small kernel at the end of the queue writes the
@@ -2063,6 +2071,14 @@ int ts2_wait(ts2_model *m)
         return fail(TS2_ERR_INVALID_ARG, "null model");
     TS2_CUDA(cudaSetDevice(m->device));
     M_TRY(wait_stream(m));
+    return TS2_OK;
+}
+
+int ts2_set_wait_limit(ts2_model *m, double seconds)
+{
+    if (!m || !(seconds > 0))
+        return fail(TS2_ERR_INVALID_ARG, "ts2_set_wait_limit: pass a model and a positive time");
+    m->wait_limit_s = seconds;
     return TS2_OK;
 }
 
