@@ -1665,12 +1665,13 @@ int backward(ts2_model *m)
         TRACE("g", l, m->g, (size_t)T * D * 4, TR_F32);
         M_TRY(tap_gradient(m, l));
     }
-    if (!(m->descr.flags & TS2_MPF_DISABLE_TUNE_EMBED))
+    if (!(m->descr.flags & TS2_MPF_DISABLE_TUNE_EMBED)) {
         if (!m->batch.ix_sorted) {
             M_TRY(label_index_sort(c, (uint32_t)m->descr.label_count, m->batch.ix));
             m->batch.ix_sorted = true;
         }
         M_TRY(embed_backward_indexed(c, m->g, b.ix, D, m->mats[0].grad));
+    }
     M_TRY(reduce_matrices(m, 0, 1));
     return TS2_OK;
 }
