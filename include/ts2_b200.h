@@ -369,7 +369,8 @@ int ts2_gemm_dx(int device, void *stream, int prec, int out_kind, int64_t T, int
  * src/gpt/compute/cpu_util.cpp:50-67; TMatMulBuffers::BackpropDelta,
  * src/gpt/compute/matmul_fwdbwd.cuh:149-162).  Both operands are token-major;
  * the contraction dimension T is split over the SMs and the partial tiles are
- * reduced through `workspace` (ts2_gemm_dw_workspace_bytes). */
+ * reduced through `workspace` (ts2_gemm_dw_workspace_bytes; with less than that, or none, an output with
+ * tiles for more than half the SMs, or a T too short to split, is computed without a split; any other is refused). */
 size_t ts2_gemm_dw_workspace_bytes(int64_t T, int64_t in_dim, int64_t out_dim);
 int ts2_gemm_dw(int device, void *stream, int prec, int out_kind, int64_t T, int64_t in_dim, int64_t out_dim,
                 const void *dY, const void *X, void *dW, float alpha, void *workspace, size_t workspace_bytes);

@@ -129,12 +129,13 @@ int ts2_gemm_tn(int device, void *stream, int prec, int out_kind, int64_t M, int
         // tiles; this entry point takes it from the library's stream-ordered scratch pool for the call.
         void *ws = nullptr;
         TS2_CUDA(cudaSetDevice(device));
-        if (int rc = scratch_alloc(device, need, a.stream, &ws))
-            return rc;
-        a.workspace = ws;
-        a.workspace_bytes = need;
-        int rc = gemm(a);
-        scratch_free(a.stream, ws);
+        if (scratch_alloc(device, need, a.stream, &ws) == TS2_OK) {
+            a.workspace = ws;
+            a.workspace_bytes = need;
+        }
+        int rc = gemm(a); // without scratch: a plan that needs none, if there is one
+        if (ws)
+            scratch_free(a.stream, ws);
         return rc;
     }
     return gemm(a);

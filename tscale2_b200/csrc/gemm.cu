@@ -846,7 +846,8 @@ static void finish_plan(Plan &pl, int sms, int splits, int group_mode, int group
 }
 
 // 256-column tiles (128 for a narrow output), K split when fewer than half the SMs would have a tile: what
-// ts2_gemm_dw_noalloc promises its callers to fit into its fixed scratch depends on this rule
+// ts2_gemm_dw_noalloc promises its callers to fit into its fixed scratch depends on this rule, and what a caller of the
+// other entry points may leave out (see gemm())
 static Plan fixed_plan(int device, int kind, int64_t M, int64_t N, int64_t K)
 {
     Plan pl;
@@ -1125,9 +1126,13 @@ int gemm(const GemmArgs &a)
                     a.ldc != bwd_ld || !(gate_bwd ? a.epi.bwd_dscale && a.epi.bwd_dout : a.epi.act_scale != nullptr) ||
                     (((uintptr_t)a.epi.bwd_wg | (uintptr_t)a.epi.bwd_o | (uintptr_t)a.epi.bwd_dout) & 15) || !pl.pair() || pl.splits != 1))
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of the activation's backward form");
-    if (pl.splits > 1) {
+    const size_t room = a.workspace ? a.workspace_bytes : 0;
+    if (pl.workspace() > room) {
+        // The fastest plan splits outputs that others leave whole (2048 x 1280 from 16384 tokens): without scratch for it the
+        // fixed plan serves, which asks for some only where few SMs would have a tile.
         const size_t need = pl.workspace();
-        if (!a.workspace || a.workspace_bytes < need)
+        pl = fixed_plan(a.device, a.kind, a.M, a.N, a.K);
+        if (pl.workspace() > room)
             return fail(TS2_ERR_INVALID_ARG, "gemm: split-K needs %zu workspace bytes, got %zu", need, a.workspace_bytes);
     }
     CUtensorMap tmA, tmB;
