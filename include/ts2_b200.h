@@ -173,6 +173,14 @@ int ts2_get_batch_tables(ts2_model *m, int attention_type, int32_t *span_start, 
  * embedding gradient sums a label's nodes in this order, so it does not depend on the schedule. */
 int ts2_get_label_index(ts2_model *m, uint32_t *labels, uint32_t *nodes, int64_t capacity, int64_t *count);
 
+/* Device memory for the attention backward pass's score gradients (fp16, 32 KB per head and pair of 128-node blocks that
+ * meet).  ts2_create takes what any batch of max_nodes nodes may need, at most 4 GB and at most a quarter of what the
+ * device has left; for a batch that needs more than there is, dQ recomputes the scores (slower, the same result within
+ * rounding).  The first call waits for the device and changes the limit, 0 gives the memory back; the second tells the
+ * buffer's size and whether the current batch uses it (either pointer may be NULL). */
+int ts2_set_score_gradient_limit(ts2_model *m, int64_t bytes);
+int ts2_get_score_gradients(ts2_model *m, int attention_type, int64_t *buffer_bytes, int *batch_fits);
+
 /* IModel::Backprop, src/gpt/compute/model.h:53 — asynchronous: enqueues the
  * forward pass, the backward pass and (TS2_GRADIENT_APPLY) the gradient
  * reduction + optimizer + requantization. */

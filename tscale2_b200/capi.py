@@ -91,6 +91,8 @@ def _declare(lib):
         "ts2_destroy": (None, [vp]),
         "ts2_last_error": (C.c_char_p, [vp]),
         "ts2_set_batch": (i32, [vp, P(BatchNodes)]),
+        "ts2_set_score_gradient_limit": (i32, [vp, i64]),
+        "ts2_get_score_gradients": (i32, [vp, i32, P(i64), P(i32)]),
         "ts2_backprop": (i32, [vp, P(TrainingStep), i32]),
         "ts2_wait": (i32, [vp]),
         "ts2_set_wait_limit": (i32, [vp, C.c_double]),

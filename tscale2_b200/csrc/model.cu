@@ -293,6 +293,31 @@ int poll_stream(const ts2_model *m)
     return poll_until(m, [&] { return cudaStreamQuery(m->stream); });
 }
 
+void free_score_gradients(ts2_model *m)
+{
+    if (m->att_bwd.ds)
+        cudaFree(m->att_bwd.ds);
+    m->att_bwd.ds = nullptr;
+    m->att_bwd.ds_bytes = 0;
+}
+
+// The buffer for the attention's score gradients is an optional one (without it, or for a batch that needs more, dQ
+// recomputes the scores): at most `limit` bytes, no more than any batch of this model needs, and at most a quarter of what
+// the device has left, so that a model and its neighbours that fill a card without it still do.
+void size_score_gradients(ts2_model *m, size_t limit)
+{
+    free_score_gradients(m);
+    size_t left = 0, total = 0;
+    if (cudaMemGetInfo(&left, &total) != cudaSuccess)
+        left = 0;
+    const size_t bytes = std::min(std::min(limit, left / 4), att_ds_bytes(m->max_nodes, nullptr, nullptr, nullptr) * m->H);
+    if (bytes && cudaMalloc(&m->att_bwd.ds, bytes) == cudaSuccess)
+        m->att_bwd.ds_bytes = bytes;
+    else
+        m->att_bwd.ds = nullptr;
+    cudaGetLastError();
+}
+
 template <class T>
 int dalloc(ts2_model *m, T **p, size_t count)
 {
@@ -302,7 +327,9 @@ int dalloc(ts2_model *m, T **p, size_t count)
     if (e != cudaSuccess) {
         cudaGetLastError();
         scratch_trim(m->device);
+        free_score_gradients(m);
         e = cudaMalloc(&q, bytes);
+        cudaGetLastError();
     }
     if (e != cudaSuccess)
         return fail(TS2_ERR_CUDA, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
@@ -1067,11 +1094,8 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
     M_TRY(dalloc(m, &m->dq, (size_t)T * m->Q));
     M_TRY(dalloc(m, &m->dk, (size_t)T * m->Q));
     M_TRY(dalloc(m, &m->dv, (size_t)T * m->Q));
-    if (m->Q) {
+    if (m->Q)
         M_TRY(dalloc(m, (uint8_t **)&m->att_bwd.scratch, att_bwd_scratch_bytes(T, m->H)));
-        m->att_bwd.ds_bytes = std::min(ATT_DS_MAX_BYTES, att_ds_bytes(T, nullptr, nullptr, nullptr) * m->H);
-        M_TRY(dalloc(m, (uint8_t **)&m->att_bwd.ds, m->att_bwd.ds_bytes));
-    }
     M_TRY(dalloc(m, &m->rope, (size_t)T * 128));
     M_TRY(dalloc(m, &m->absmax, L + 2));
     M_TRY(dalloc(m, &m->ginv, 4));
@@ -1165,6 +1189,8 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
     M_TRY(build_post_quantize(m));
     M_TRY(requantize_all(m));
     TS2_CUDA(cudaStreamSynchronize(m->stream));
+    if (m->Q)
+        size_score_gradients(m, ATT_DS_MAX_BYTES); // last: whatever a step cannot do without comes first
     return TS2_OK;
 }
 
@@ -1826,8 +1852,9 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
     for (int a = 0; a < na; ++a) {
         M_TRY(att_layout(c, b.span_start[a], b.span_finish[a], b.rev_first[a], b.rev_last[a], T, b.att_layout[a]));
         // a big batch: count what its own spans need (a pass over them on the host, beside the step that is running)
-        b.ds_fits[a] = att_ds_bytes(T, nullptr, nullptr, nullptr) * m->H <= m->att_bwd.ds_bytes ||
-                       att_ds_bytes(T, nd->att[a].span_ptr, nd->att[a].span_start, nd->att[a].span_finish) * m->H <= m->att_bwd.ds_bytes;
+        b.ds_fits[a] = m->att_bwd.ds && (att_ds_bytes(T, nullptr, nullptr, nullptr) * m->H <= m->att_bwd.ds_bytes ||
+                                         att_ds_bytes(T, nd->att[a].span_ptr, nd->att[a].span_start, nd->att[a].span_finish) * m->H <=
+                                             m->att_bwd.ds_bytes);
     }
     b.node_count = T;
     b.target_count = n_targets;
@@ -1981,6 +2008,7 @@ void ts2_destroy(ts2_model *m)
     }
     for (void *p : m->allocs)
         cudaFree(p);
+    free_score_gradients(m);
     if (m->pinned)
         cudaFreeHost(m->pinned);
     for (cudaEvent_t e : m->batch.slot_ev)
@@ -2023,6 +2051,31 @@ int ts2_set_batch(ts2_model *m, const ts2_batch_nodes *nodes)
         M_TRY(wait_stream(m));
     m->unreported = true;
     M_TRY(stage_batch(m, nodes));
+    return TS2_OK;
+}
+
+int ts2_set_score_gradient_limit(ts2_model *m, int64_t bytes)
+{
+    if (!m || bytes < 0)
+        return fail(TS2_ERR_INVALID_ARG, "ts2_set_score_gradient_limit: pass a model and a number of bytes");
+    TS2_CUDA(cudaSetDevice(m->device));
+    M_TRY(wait_stream(m));
+    if (m->Q)
+        size_score_gradients(m, (size_t)bytes);
+    // the spans of the current batch are no longer at hand: it keeps the buffer if any batch of its size would fit
+    for (size_t a = 0; a < m->batch.ds_fits.size(); ++a)
+        m->batch.ds_fits[a] = m->att_bwd.ds && att_ds_bytes(m->batch.node_count, nullptr, nullptr, nullptr) * m->H <= m->att_bwd.ds_bytes;
+    return TS2_OK;
+}
+
+int ts2_get_score_gradients(ts2_model *m, int attention_type, int64_t *buffer_bytes, int *batch_fits)
+{
+    if (!m || attention_type < 0 || attention_type >= (int)m->batch.ds_fits.size())
+        return fail(TS2_ERR_INVALID_ARG, "ts2_get_score_gradients: bad arguments");
+    if (buffer_bytes)
+        *buffer_bytes = (int64_t)m->att_bwd.ds_bytes;
+    if (batch_fits)
+        *batch_fits = m->att_bwd.ds && m->batch.node_count > 0 && m->batch.ds_fits[attention_type];
     return TS2_OK;
 }
 
