@@ -341,6 +341,9 @@ int ts2_get_kernel_bytes(ts2_model *m, double *gemm_bytes_total);
 int ts2_device_count(void);
 int ts2_dev_alloc(int device, size_t bytes, void **ptr);
 int ts2_dev_free(int device, void *ptr);
+/* Gives the scratch that the operator-level calls keep between calls (up to 2 GB per device) back to the driver, as far as
+ * no queued work uses it; the next call that needs scratch takes it anew. */
+int ts2_dev_trim(int device);
 int ts2_dev_upload(int device, void *dst, const void *host_src, size_t bytes);
 int ts2_dev_download(int device, void *host_dst, const void *src, size_t bytes);
 int ts2_dev_memset(int device, void *dst, int value, size_t bytes);

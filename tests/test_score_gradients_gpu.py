@@ -1,8 +1,8 @@
 """The buffer for the attention's score gradients is optional: a card without room for it still takes the model, a batch
 that needs more than there is recomputes the scores, and the memory can be given back.
 
-Both ways round the same fp32 values to fp16 (2^-11) before the dQ product and dQ itself to fp16 after it, in another
-order of summation, so that single roundings differ: gradients agree to well under 2^-11 = 5e-4 of their norm."""
+Both ways round the same fp32 values to fp16 (2^-11) before the dQ product and dQ itself to fp16 after it; where an order of
+summation differs single roundings do, so gradients agree to well under 2^-11 = 5e-4 of their norm."""
 import ctypes as C
 
 import numpy as np

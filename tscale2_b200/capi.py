@@ -135,6 +135,7 @@ def _declare(lib):
         "ts2_selftest_wait_limit_noalloc": (i32, [i32]),
         "ts2_dev_alloc": (i32, [i32, C.c_size_t, P(vp)]),
         "ts2_dev_free": (i32, [i32, vp]),
+        "ts2_dev_trim": (i32, [i32]),
         "ts2_dev_upload": (i32, [i32, vp, vp, C.c_size_t]),
         "ts2_dev_download": (i32, [i32, vp, vp, C.c_size_t]),
         "ts2_dev_memset": (i32, [i32, vp, i32, C.c_size_t]),

@@ -43,6 +43,13 @@ int ts2_dev_alloc(int device, size_t bytes, void **ptr)
     return TS2_OK;
 }
 
+int ts2_dev_trim(int device)
+{
+    TS2_CUDA(cudaSetDevice(device));
+    scratch_trim(device);
+    return TS2_OK;
+}
+
 int ts2_dev_free(int device, void *ptr)
 {
     TS2_CUDA(cudaSetDevice(device));
@@ -129,7 +136,7 @@ int ts2_gemm_tn(int device, void *stream, int prec, int out_kind, int64_t M, int
         // tiles; this entry point takes it from the library's stream-ordered scratch pool for the call.
         void *ws = nullptr;
         TS2_CUDA(cudaSetDevice(device));
-        if (scratch_alloc(device, need, a.stream, &ws) == TS2_OK) {
+        if (scratch_try_alloc(device, need, a.stream, &ws)) {
             a.workspace = ws;
             a.workspace_bytes = need;
         }
@@ -456,7 +463,7 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
         plan.layout = (uint8_t *)d + tables;
         plan.scratch = (uint8_t *)d + tables + layout;
         plan.ds_bytes = att_ds_bytes(T, nullptr, span_start, span_finish) * head_count;
-        if (plan.ds_bytes == 0 || plan.ds_bytes > ATT_DS_MAX_BYTES || scratch_alloc(device, plan.ds_bytes, c.stream, &plan.ds) != TS2_OK)
+        if (plan.ds_bytes == 0 || plan.ds_bytes > ATT_DS_MAX_BYTES || !scratch_try_alloc(device, plan.ds_bytes, c.stream, &plan.ds))
             plan.ds = nullptr, plan.ds_bytes = 0;
         if ((rc = att_layout(c, d, d + T, d + 2 * (size_t)T, d + 3 * (size_t)T, T, plan.layout)) == TS2_OK)
             rc = attention_backward(c, Q, K, V, DO, lse, dscale, d, d + T, plan, T, head_count, alibi_slope, dq, dk, dv, variant == 3);

@@ -116,19 +116,31 @@ static cudaMemPool_t scratch_pool(int device, bool create)
             p = nullptr;
             return nullptr;
         }
-        uint64_t keep = 2ull << 30;
+        uint64_t keep = SCRATCH_KEEP_BYTES;
         cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     return p;
 }
 
-int scratch_alloc(int device, size_t bytes, cudaStream_t stream, void **ptr)
+bool scratch_try_alloc(int device, size_t bytes, cudaStream_t stream, void **ptr)
 {
     cudaMemPool_t p = scratch_pool(device, true);
-    if (!p)
-        return fail(TS2_ERR_CUDA, "no scratch pool");
-    TS2_CUDA(cudaMallocFromPoolAsync(ptr, bytes, p, stream));
-    return TS2_OK;
+    cudaError_t e = p ? cudaMallocFromPoolAsync(ptr, bytes, p, stream) : cudaErrorMemoryAllocation;
+    if (p && e != cudaSuccess) {
+        cudaGetLastError();
+        cudaMemPoolTrimTo(p, 0); // what it keeps may be in the way of a block of another size
+        e = cudaMallocFromPoolAsync(ptr, bytes, p, stream);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *ptr = nullptr;
+    }
+    return e == cudaSuccess;
+}
+
+int scratch_alloc(int device, size_t bytes, cudaStream_t stream, void **ptr)
+{
+    return scratch_try_alloc(device, bytes, stream, ptr) ? TS2_OK : fail(TS2_ERR_CUDA, "no room for %zu bytes of scratch", bytes);
 }
 
 void scratch_free(cudaStream_t stream, void *ptr) { cudaFreeAsync(ptr, stream); }

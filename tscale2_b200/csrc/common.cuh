@@ -92,10 +92,15 @@ int32_t *static_status_word_if_ready(int device);
 // returns TS2_OK or TS2_ERR_DEVICE_STATUS (with the message set).  Allocates nothing.
 int collect_device_status(int device);
 
-// Scratch of the operator-level calls, stream-ordered, from a pool of the library's own on each device that keeps up to
-// 2 GB between calls (what the largest attention call of a few tens of thousand nodes takes) (a default pool keeps nothing: after every synchronisation the next call mapped its scratch anew,
-// 0.3 - 0.5 ms).  Any thread and stream; scratch_trim gives what is unused back (called when an allocation fails).
+// Scratch of the operator-level calls, stream-ordered, from a pool of the library's own on each device.  A default pool
+// keeps nothing: after every synchronisation the next call mapped its scratch anew, 0.3 - 0.5 ms.  This one keeps up to
+// SCRATCH_KEEP_BYTES between calls; a call that needs more (an attention call's score gradients may take 4 GB) maps what
+// is above that each time.  Any thread and stream; scratch_trim (ts2_dev_trim) gives back what no queued work uses.
+// An allocation that fails is tried once more on a trimmed pool and leaves no CUDA error behind; scratch_try_alloc is for
+// callers that can do without and leaves no message either.
+constexpr size_t SCRATCH_KEEP_BYTES = (size_t)2 << 30;
 int scratch_alloc(int device, size_t bytes, cudaStream_t stream, void **ptr);
+bool scratch_try_alloc(int device, size_t bytes, cudaStream_t stream, void **ptr);
 void scratch_free(cudaStream_t stream, void *ptr);
 void scratch_trim(int device);
 
