@@ -1,5 +1,6 @@
 // Library-wide state: last error, launch counter, per-device status word.
 #include "common.cuh"
+#include <cuda.h>
 #include <cstdarg>
 #include <map>
 #include <mutex>
@@ -99,6 +100,23 @@ int collect_device_status(int device)
                     "device status word = 0x%x%s (bit0: a bounded wait in a kernel timed out, bit1: a kernel refused its arguments)",
                     seen[0] | seen[1], seen[1] ? " (raised by ts2_gemm_dw_noalloc)" : "");
     return TS2_OK;
+}
+
+bool one_pinned_range(const void *p, size_t bytes)
+{
+    using Query = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (Query)f;
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
+    return query && query(&base, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) == CUDA_SUCCESS &&
+           query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) == CUDA_SUCCESS && at >= base && at + bytes <= base + size;
 }
 
 static cudaMemPool_t scratch_pool(int device, bool create)

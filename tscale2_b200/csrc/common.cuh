@@ -92,6 +92,9 @@ int32_t *static_status_word_if_ready(int device);
 // returns TS2_OK or TS2_ERR_DEVICE_STATUS (with the message set).  Allocates nothing.
 int collect_device_status(int device);
 
+// whether the host memory [p, p + bytes) lies inside one page-locked allocation or registration; false for pageable memory
+bool one_pinned_range(const void *p, size_t bytes);
+
 // Scratch of the operator-level calls, stream-ordered, from a pool of the library's own on each device.  A default pool
 // keeps nothing: after every synchronisation the next call mapped its scratch anew, 0.3 - 0.5 ms.  This one keeps up to
 // SCRATCH_KEEP_BYTES between calls; a call that needs more (an attention call's score gradients may take 4 GB) maps what

@@ -2180,35 +2180,40 @@ int ts2_get_params(ts2_model *m, int what, ts2_matrix_view *mats_out, int n_mats
     if (what != TS2_PARAM_GRADIENT)
         M_TRY(sync_master(m));
     M_TRY(wait_stream(m));
-    // matrices that follow one another on both sides leave in one copy, all copies are queued before any is waited for
+    for (int i = 0; i < n_mats; ++i)
+        if (mats_out[i].data && (mats_out[i].x_size != m->mats[i].x || mats_out[i].y_size != m->mats[i].y))
+            return mfail(m, fail(TS2_ERR_INVALID_ARG, "matrix %d: shape mismatch", i));
+    // Matrices that follow one another on both sides leave in one copy, all copies are queued before any is waited for.
+    // A copy stays inside one page-locked range: neighbours in address may be allocations (or registrations) of their own,
+    // or pageable, and a copy across such a border is not a valid one.
     const float *src0 = nullptr;
     float *dst0 = nullptr;
     size_t run = 0;
+    cudaError_t err = cudaSuccess;
     auto flush = [&]() {
-        const cudaError_t e = run ? cudaMemcpyAsync(dst0, src0, run * 4, cudaMemcpyDeviceToHost, m->stream) : cudaSuccess;
+        if (run && err == cudaSuccess)
+            err = cudaMemcpyAsync(dst0, src0, run * 4, cudaMemcpyDeviceToHost, m->stream);
         run = 0;
-        return e;
     };
     for (int i = 0; i < n_mats; ++i) {
         Matrix &mt = m->mats[i];
         if (!mats_out[i].data)
             continue;
-        if (mats_out[i].x_size != mt.x || mats_out[i].y_size != mt.y) {
-            cudaStreamSynchronize(m->stream); // earlier matrices may be on their way
-            return mfail(m, fail(TS2_ERR_INVALID_ARG, "matrix %d: shape mismatch", i));
-        }
         const float *src = what == TS2_PARAM_WEIGHTS ? mt.w : what == TS2_PARAM_MOMENTUM ? mt.avg : mt.grad;
         const size_t n = (size_t)mt.x * mt.y;
-        if (run && (src != src0 + run || mats_out[i].data != dst0 + run))
-            TS2_CUDA(flush());
+        if (run && (src != src0 + run || mats_out[i].data != dst0 + run || !one_pinned_range(dst0, (run + n) * 4)))
+            flush();
         if (!run) {
             src0 = src;
             dst0 = mats_out[i].data;
         }
         run += n;
     }
-    TS2_CUDA(flush());
-    M_TRY(poll_stream(m));
+    flush();
+    // the steps are over (wait_stream): only these copies remain, and none may still be on its way when the call returns
+    const cudaError_t done = cudaStreamSynchronize(m->stream);
+    TS2_CUDA(err);
+    TS2_CUDA(done);
     return TS2_OK;
 }
 
