@@ -368,7 +368,8 @@ int ts2_op_rowquant_i8(int device, void *stream, const float *x, int T, int D, i
     return rowquant_grad(op_ctx(device, stream, TS2_PREC_INT8), x, T, D, nullptr, q, row_scale, nullptr, nullptr, 1.f, nullptr, nullptr);
 }
 
-// device copies of a call's host span arrays (start at d, finish at d + T) and whatever scratch follows them
+// device copies of a call's host span arrays (start at d, finish at d + T) and whatever scratch follows them; the call does
+// not return, on whichever path, before its work and the copies from the caller's arrays are done
 struct SpanScratch {
     int *d = nullptr;
     int rc = TS2_OK;
@@ -387,8 +388,10 @@ struct SpanScratch {
     }
     ~SpanScratch()
     {
-        if (d)
-            scratch_free(stream, d);
+        if (!d)
+            return;
+        cudaStreamSynchronize(stream);
+        scratch_free(stream, d);
     }
     SpanScratch(const SpanScratch &) = delete;
     SpanScratch &operator=(const SpanScratch &) = delete;
@@ -414,7 +417,6 @@ int ts2_attention_forward(int device, void *stream, int variant, const void *q, 
                                                     alibi_slope, (__half *)o, lse)
                             : attention_forward_rowwise(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,
                                                       alibi_slope, (__half *)o, lse);
-    cudaStreamSynchronize(c.stream);
     return rc;
 }
 
@@ -432,7 +434,6 @@ int ts2_op_attention_gated_forward(int device, void *stream, int prec, const voi
         return spans.rc;
     const int rc = attention_forward(c, (const __half *)q, (const __half *)k, (const __half *)v, spans.d, spans.d + T, T, head_count,
                                      alibi_slope, (__half *)o, lse, AttGate{(const __half *)gate, gate_ld, rg});
-    cudaStreamSynchronize(c.stream);
     return rc;
 }
 
@@ -474,7 +475,6 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
                           : attention_backward_rowwise(c, Q, K, V, DO, lse, dscale, d, d + T, d + 2 * T, d + 3 * T, T, head_count, alibi_slope,
                                                        fq, fk, fv);
     }
-    cudaStreamSynchronize(c.stream);
     return rc;
 }
 
