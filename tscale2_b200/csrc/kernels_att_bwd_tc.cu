@@ -382,7 +382,8 @@ size_t att_ds_bytes(int T, const int *span_ptr, const int *span_start, const int
             has = span_ptr[t + 1] == at + 1 && at >= 0 && at < span_ptr[T];
         }
         const int s = has ? span_start[at] : 0, f = has ? span_finish[at] : -1;
-        has = has && s >= 0 && f < T && f >= s;
+        // ts2_set_batch drops a span outside the batch; the operator-level calls take theirs as they come
+        has = has && f >= s && (!span_ptr || (s >= 0 && f < T));
         mx = std::max(mx, has ? f : -1);
         run_max[t] = mx;
         suf_min[t] = has ? s : T;
