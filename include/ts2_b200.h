@@ -220,7 +220,8 @@ int ts2_get_fast_weights(ts2_model *m, int index, void *dst, int64_t dst_bytes, 
  * ts2_set_debug_taps before the call; costs one copy per layer). */
 int ts2_set_debug_taps(ts2_model *m, int enable);
 /* raw copy of an internal per-layer buffer after the last step, for tests: "rg", "dcat", "cat16", "n_fast",
- * "n_rows", "logits", "ids", "weights", "slot_of", "token_of", "seg_ptr", "moe_g", "drg", "capture" (the caller knows the layout) */
+ * "n_rows", "logits", "ids", "weights", "slot_of", "token_of", "seg_ptr", "moe_g", "drg", "capture" (the caller knows the layout).
+ * "drg" is TS2_ERR_UNSUPPORTED after a step that did not write it (e4m3 layers of many tiles, unless the debug trace is on) */
 int ts2_debug_read(ts2_model *m, const char *name, int layer, void *dst, int64_t bytes);
 int ts2_get_state_tap(ts2_model *m, int layer, int gradient, float *dst, int64_t n_floats);
 

@@ -176,6 +176,7 @@ struct ts2_model {
     __half *logits = nullptr;
     int chunk = 0;
     __half *drg = nullptr, *dout = nullptr;
+    bool drg_written = true; // drg holds what the last layer of the last backward pass put there, not something older
     void *dcat = nullptr;
     float *dscale = nullptr;
     AttBwdPlan att_bwd; // of the model: records, score gradients
@@ -1550,6 +1551,7 @@ int backward(ts2_model *m)
             e3.out_kind = TS2_OUT_F16;
             if (xrows) {
                 M_TRY(gemm_rows_grouped(m, ly, xrows, X, D, m->moe_g, D, ly.WcT, D, m->drg, X, e3));
+                m->drg_written = true;
                 if (tune_layers) {
                     Epilogue e6;
                     e6.alpha = 1.f / m->s_act;
@@ -1630,6 +1632,11 @@ int backward(ts2_model *m)
         TRACE("g_fast", l, m->g_fast, (size_t)T * D * fsz, fsz == 2 ? TR_F16 : TR_RAW);
         // many tiles: the contraction's epilogue goes on through the activation or the gate; drg never reaches memory
         const bool act_fused = gemm_takes_act_backward(m->device, m->kind, T, W);
+        m->drg_written = !act_fused || m->trace_on;
+        if (m->drg_written) { // the fused form does without; a traced step has it all the same, and is otherwise the same step
+            M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->drg, W, e3));
+            TRACE("drg", l, m->drg, (size_t)T * W * 2, TR_F16);
+        }
         if (act_fused) {
             e3.bwd_wg = ly.cat16;
             if (ly.type == TS2_LAYER_ATT) {
@@ -1640,9 +1647,6 @@ int backward(ts2_model *m)
                 e3.act_scale = ly.wscale;
             }
             M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->dcat, C, e3));
-        } else {
-            M_TRY(gemm_tn(m, m->kind, T, W, D, m->g_fast, D, ly.WcT, D, m->drg, W, e3));
-            TRACE("drg", l, m->drg, (size_t)T * W * 2, TR_F16);
         }
         if (tune_layers) {
             // dWc = g^T . rg   (SumRankOne)
@@ -2395,6 +2399,8 @@ int ts2_debug_read(ts2_model *m, const char *name, int layer, void *dst, int64_t
                       : n == "capture" && (size_t)bytes <= m->capture_bytes ? m->capture_buf : nullptr;
     if (!src)
         return fail(TS2_ERR_INVALID_ARG, "ts2_debug_read: unknown or absent buffer '%s'", name);
+    if (src == m->drg && !m->drg_written)
+        return fail(TS2_ERR_UNSUPPORTED, "ts2_debug_read: the last step kept drg on the chip; with ts2_set_debug_trace it also writes it");
     TS2_CUDA(cudaMemcpy(dst, src, (size_t)bytes, cudaMemcpyDeviceToHost));
     return TS2_OK;
 }
