@@ -393,6 +393,11 @@ int ts2_gemm_dw_scaled(int device, void *stream, int prec, int out_kind, int64_t
                        const void *dY, const void *X, void *dW, float alpha, const float *row_scale, const float *col_scale,
                        void *workspace, size_t workspace_bytes);
 
+/* Which kernel a contraction takes, for tests that mean one of them: plan = {tile rows (256: a pair of CTAs), tile columns,
+ * K splits} for C[M][N] over K, operands K-contiguous or (token_major) as ts2_gemm_dw reads them, gated: the FFN's
+ * gated-activation form with N = 2 x its width.  No device work. */
+int ts2_op_gemm_plan(int device, int prec, int out_kind, int token_major, int gated, int64_t M, int64_t N, int64_t K, int32_t plan[3]);
+
 /* The same contraction as ts2_gemm_dw for callers that must not allocate device memory — a host
  * whose own pools took all of it at start-up, or a loop that cannot afford cudaMalloc's device-wide
  * synchronisation.  (No counterpart in the reference: its kernels get scratch from the trainer's

@@ -143,6 +143,7 @@ def _declare(lib):
         "ts2_gemm_tn": (i32, [i32, vp, i32, i32, i64, i64, i64, vp, i64, vp, i64, vp, i64, f32, vp, vp]),
         "ts2_gemm_dx": (i32, [i32, vp, i32, i32, i64, i64, i64, vp, vp, vp, f32, vp, vp]),
         "ts2_gemm_dw_workspace_bytes": (C.c_size_t, [i64, i64, i64]),
+        "ts2_op_gemm_plan": (i32, [i32, i32, i32, i32, i32, i64, i64, i64, P(C.c_int32)]),
         "ts2_gemm_dw_noalloc": (i32, [i32, vp, i32, i32, i64, i64, i64, vp, vp, vp, f32]),
         "ts2_gemm_tn_grouped": (i32, [i32, vp, i32, i32, i64, i64, i64, vp, vp, vp, f32, i32, vp]),
         "ts2_gemm_dw_grouped": (i32, [i32, vp, i32, i32, i64, i64, i64, vp, vp, vp, f32, i32, vp]),

@@ -207,6 +207,18 @@ int ts2_gemm_dw_scaled(int device, void *stream, int prec, int out_kind, int64_t
     return gemm(a);
 }
 
+int ts2_op_gemm_plan(int device, int prec, int out_kind, int token_major, int gated, int64_t M, int64_t N, int64_t K, int32_t plan[3])
+{
+    const int kind = kind_of(prec);
+    if (kind < 0 || M <= 0 || N <= 0 || K <= 0 || !plan || (gated && (N % 256 || token_major)))
+        return fail(TS2_ERR_INVALID_ARG, "ts2_op_gemm_plan: bad arguments");
+    Epilogue e;
+    e.out_kind = out_kind;
+    e.pair_stride = gated ? N / 2 : 0;
+    gemm_plan(device, kind, token_major != 0, M, N, K, e, plan, plan + 1, plan + 2);
+    return TS2_OK;
+}
+
 // grouped contractions of the mixture-of-experts layers (device pointers; tables on the device)
 int ts2_gemm_tn_grouped(int device, void *stream, int prec, int out_kind, int64_t rows, int64_t N, int64_t K, const void *A,
                         const void *B, void *C, float alpha, int groups, const int32_t *tile_group)

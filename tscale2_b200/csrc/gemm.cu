@@ -831,8 +831,8 @@ static uint32_t instr_desc(int kind, bool mn, int bm, int bn)
 }
 
 struct Plan {
-    int bm = BM, bn; // 256 x 256: on pairs of CTAs (gemm_pair.cu)
-    int m_tiles, n_tiles, k_blocks, splits, kb_per_split, grid;
+    int bm = BM, bn = 256; // 256 x 256: on pairs of CTAs (gemm_pair.cu)
+    int m_tiles = 0, n_tiles = 0, k_blocks = 0, splits = 1, kb_per_split = 0, grid = 0;
     bool pair() const { return bm == 2 * BM; }
     size_t workspace() const { return splits > 1 ? (size_t)m_tiles * n_tiles * splits * bm * bn * sizeof(float) : 0; }
 };
@@ -943,6 +943,14 @@ size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N,
             need = std::max(need, make_plan(device, kind, mn, M, N, K, form_of(e)).workspace());
     }
     return need;
+}
+
+void gemm_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, const Epilogue &epi, int *tile_rows, int *tile_cols, int *splits)
+{
+    const Plan pl = make_plan(device, kind, mn, M, N, K, form_of(epi));
+    *tile_rows = pl.bm;
+    *tile_cols = pl.bn;
+    *splits = pl.splits;
 }
 
 // Counters of the dynamic unit scheduler: SCHED_SLOTS pairs {next unit, finished CTAs} per device, zero between

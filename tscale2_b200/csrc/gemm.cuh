@@ -70,6 +70,9 @@ struct GemmArgs {
 // bytes of scratch this shape needs for its K splits (0: none); out_kind < 0: whatever the output
 size_t gemm_workspace_bytes(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_t K, int out_kind = -1);
 int gemm(const GemmArgs &a);
+// the tile and the K split that gemm() takes for this shape when it has the scratch for it (256 rows: a pair of CTAs)
+void gemm_plan(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_t K, const Epilogue &epi, int *tile_rows, int *tile_cols,
+               int *splits);
 // whether the epilogue can apply the backward of the gated activation (Epilogue::bwd_wg) to a product of this shape
 bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N);
 
