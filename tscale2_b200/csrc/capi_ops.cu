@@ -449,9 +449,10 @@ int ts2_op_attention_gated_forward(int device, void *stream, int prec, const voi
     return rc;
 }
 
-int ts2_attention_backward(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
-                           const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
-                           int head_count, float alibi_slope, void *dq, void *dk, void *dv)
+// score_gradients: most bytes the tcgen05 kernels may set aside for them
+static int run_attention_backward(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
+                                  const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
+                                  int head_count, float alibi_slope, void *dq, void *dk, void *dv, size_t score_gradients)
 {
     if (T <= 0 || head_count <= 0 || !q || !k || !v || !dout || !lse || !dscale || !span_start || !span_finish || !dq || !dk || !dv)
         return fail(TS2_ERR_INVALID_ARG, "ts2_attention_backward: bad arguments");
@@ -476,7 +477,7 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
         plan.layout = (uint8_t *)d + tables;
         plan.scratch = (uint8_t *)d + tables + layout;
         plan.ds_bytes = att_ds_bytes(T, nullptr, span_start, span_finish) * head_count;
-        if (plan.ds_bytes == 0 || plan.ds_bytes > ATT_DS_MAX_BYTES || !scratch_try_alloc(device, plan.ds_bytes, c.stream, &plan.ds))
+        if (plan.ds_bytes == 0 || plan.ds_bytes > score_gradients || !scratch_try_alloc(device, plan.ds_bytes, c.stream, &plan.ds))
             plan.ds = nullptr, plan.ds_bytes = 0;
         if ((rc = att_layout(c, d, d + T, d + 2 * (size_t)T, d + 3 * (size_t)T, T, plan.layout)) == TS2_OK)
             rc = attention_backward(c, Q, K, V, DO, lse, dscale, d, d + T, plan, T, head_count, alibi_slope, dq, dk, dv, variant == 3);
@@ -488,6 +489,24 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
                                                        fq, fk, fv);
     }
     return rc;
+}
+
+int ts2_attention_backward(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
+                           const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
+                           int head_count, float alibi_slope, void *dq, void *dk, void *dv)
+{
+    return run_attention_backward(device, stream, variant, q, k, v, dout, lse, dscale, span_start, span_finish, T, head_count, alibi_slope, dq,
+                                  dk, dv, ATT_DS_MAX_BYTES);
+}
+
+int ts2_op_attention_backward_limited(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
+                                      const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
+                                      int head_count, float alibi_slope, void *dq, void *dk, void *dv, int64_t score_gradient_bytes)
+{
+    if ((variant != 2 && variant != 3) || score_gradient_bytes < 0)
+        return fail(TS2_ERR_INVALID_ARG, "ts2_op_attention_backward_limited: bad arguments");
+    return run_attention_backward(device, stream, variant, q, k, v, dout, lse, dscale, span_start, span_finish, T, head_count, alibi_slope, dq,
+                                  dk, dv, (size_t)score_gradient_bytes);
 }
 
 int ts2_op_attention_reverse_ranges(int device, void *stream, const int32_t *span_start, const int32_t *span_finish, int T,
