@@ -869,6 +869,16 @@ static int form_of(const Epilogue &e)
     return e.bwd_wg ? FORM_ACT_BWD : e.pair_stride ? FORM_GATED : e.out_kind == TS2_OUT_F32_ADD ? FORM_ADD : e.out_kind == TS2_OUT_F32 ? FORM_F32 : FORM_16;
 }
 
+// Units are assigned statically by default (CTA b takes units b, b + grid, ...).  Drawing them from a global counter
+// (TS2_GEMM_DYNAMIC_UNITS=1) keeps a CTA that starts late, because a communication kernel holds its SM, from
+// stretching the launch, but measured 6 - 10 % slower on the contractions of a whole step, more than it saves.  Pairs of
+// CTAs have no such form: with the switch set the plan does without them.
+static bool dynamic_units()
+{
+    static const bool on = getenv("TS2_GEMM_DYNAMIC_UNITS") != nullptr;
+    return on;
+}
+
 // Tile and K split with the smallest estimated time.  The estimate follows measurements of single launches (us):
 //  * a K block of 128 bytes takes about the same at every width, 0.28 (0.30 at 256 columns, where the tensor pipe is
 //    busy): few tiles in flight are bound by the latency of the copies in the ring, many by the pipe;
@@ -893,6 +903,8 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
         Plan pl;
         pl.bm = shape.bm;
         pl.bn = shape.bn;
+        if (pl.pair() && dynamic_units())
+            continue;
         if (group_mode && (pl.pair() || pl.bn != ((N % 256 == 0 || N > 1024) ? 256 : 128)))
             continue;
         // a token-major one-byte operand comes in boxes of 128 columns; the gated form takes 128 wide and 128 gate columns
@@ -930,7 +942,7 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
 // matrix whose last tile is half empty loses: 12800 x 384 x 256 17.3 -> 17.8, 20000 x 128 x 256 13.5 -> 16.2.
 bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N)
 {
-    return kind == KIND_E4M3 && N % 128 == 0 && (N % 256 == 0 || N > 512) && ceil_div(M, 2 * BM) * ceil_div(N, 256) >= sm_count(device) / 2;
+    return kind == KIND_E4M3 && !dynamic_units() && N % 128 == 0 && (N % 256 == 0 || N > 512) && ceil_div(M, 2 * BM) * ceil_div(N, 256) >= sm_count(device) / 2;
 }
 
 size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int out_kind)
@@ -1181,12 +1193,8 @@ int gemm(const GemmArgs &a)
     p.status = device_status_word(a.device);
     if (!p.status)
         return fail(TS2_ERR_CUDA, "gemm: no device status word");
-    // Units are assigned statically by default (CTA b takes units b, b + grid, ...).  Drawing them from a global counter
-    // (TS2_GEMM_DYNAMIC_UNITS=1) keeps a CTA that starts late, because a communication kernel holds its SM, from
-    // stretching the launch, but measured 6 - 10 % slower on the contractions of a whole step, more than it saves.
-    static const bool dynamic_units = getenv("TS2_GEMM_DYNAMIC_UNITS") != nullptr;
-    p.sched = dynamic_units ? sched_counters(a.device) : nullptr;
-    if (dynamic_units && !p.sched)
+    p.sched = dynamic_units() ? sched_counters(a.device) : nullptr;
+    if (dynamic_units() && !p.sched)
         return fail(TS2_ERR_CUDA, "gemm: no scheduler counters");
     p.group_mode = a.group_mode;
     p.groups = a.groups;
