@@ -127,7 +127,8 @@ __global__ void __launch_bounds__(BW_THREADS, 1)
                 tma_load_2d(sA2 + b * Q_BYTES, &tmA2, res_full, col0, r0 + b * TC_BM);
                 tma_load_2d(sA2 + b * Q_BYTES + Q_BYTES / 2, &tmA2, res_full, col0 + 64, r0 + b * TC_BM);
             }
-            for (int j = 0; j < n; ++j) {
+            int j = 0;
+            for (; j < n; ++j) {
                 const int st = j % STAGES, row = (u0 + j) * TC_BN;
                 if (!mbar_wait(st_empty0 + 8 * st, ((j / STAGES) & 1) ^ 1, abort_flag))
                     break;
@@ -138,6 +139,14 @@ __global__ void __launch_bounds__(BW_THREADS, 1)
                 tma_load_2d(d1 + KV_BYTES / 2, &tmB1, fb, col0 + 64, row);
                 tma_load_2d(d2, &tmB2, fb, col0, row);
                 tma_load_2d(d2 + KV_BYTES / 2, &tmB2, fb, col0 + 64, row);
+            }
+            if (*abort_flag) { // copies in flight must land before the CTA gives its shared memory back (bounded)
+                const long long c0 = clock64();
+                while (!mbar_try_wait(res_full, 0) && clock64() - c0 < 200000000ll) {
+                }
+                for (int i = max(0, j - STAGES); i < j; ++i)
+                    while (!mbar_try_wait(st_full0 + 8 * (i % STAGES), (i / STAGES) & 1) && clock64() - c0 < 200000000ll) {
+                    }
             }
         }
     } else if (warp == 1 || warp == 2) {

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
     const int n_tiles = tile1 - tile0 + 1;
     if (warp == 0) {
         bool ok = true;
+        int k_tiles = 0, v_tiles = 0; // issued so far
         if (lane == 0 && n_tiles > 0) {
             if (GATE >= 0) { // into L2 by the time the K ring is free for them
                 tma_prefetch_2d(&tmG, col0, t0);
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
                     mbar_arrive_expect_tx(fb, KV_BYTES);
                     tma_load_2d(dk, &tmK, fb, col0, (tile0 + jj) * TC_BN);
                     tma_load_2d(dk + KV_BYTES / 2, &tmK, fb, col0 + 64, (tile0 + jj) * TC_BN);
+                    ++k_tiles;
                 }
                 if (j >= 0) {
                     const int st = j & 1;
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
                     mbar_arrive_expect_tx(fb, KV_BYTES);
                     tma_load_2d(dv, &tmV, fb, col0, (tile0 + j) * TC_BN);
                     tma_load_2d(dv + KV_BYTES / 2, &tmV, fb, col0 + 64, (tile0 + j) * TC_BN);
+                    ++v_tiles;
                 }
             }
         }
@@ -188,6 +191,21 @@ __global__ void __launch_bounds__(TC_THREADS, 2)
                     break;
                 tma_load_2d(sK + st * KV_BYTES, &tmG, gate_full, col0 + 64 * st, t0);
             }
+        }
+        if (lane == 0 && *abort_flag) { // copies in flight must land before the CTA gives its shared memory back (bounded)
+            const long long c0 = clock64();
+            auto landed = [&](uint32_t bar, uint32_t parity) {
+                while (!mbar_try_wait(bar, parity) && clock64() - c0 < 200000000ll) {
+                }
+            };
+            if (n_tiles > 0)
+                landed(q_full, 0);
+            for (int i = max(0, k_tiles - 2); i < k_tiles; ++i)
+                landed(k_full0 + 8 * (i & 1), (i >> 1) & 1);
+            for (int i = max(0, v_tiles - 2); i < v_tiles; ++i)
+                landed(v_full0 + 8 * (i & 1), (i >> 1) & 1);
+            if (GATE >= 0 && ok)
+                landed(gate_full, 0);
         }
     } else if (warp == 1) {
         if (lane == 0 && n_tiles > 0) {
