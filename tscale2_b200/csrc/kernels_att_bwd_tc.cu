@@ -163,8 +163,9 @@ __global__ void __launch_bounds__(BW_THREADS, 1)
             // in step, the tensor pipe idle while both compute and the compute warps idle while both multiply.  Block 1
             // therefore starts when block 0's first products are done (block 0 then computes), after which the shared
             // tensor pipe keeps the two out of phase.
-            if (ok && b == 1 && any0)
-                ok = mbar_wait(s_full0, 0, abort_flag);
+            if (ok && b == 1 && any0) // a head start, no dependency: past its limit block 1 goes on all the same
+                for (const long long c0 = clock64(); !mbar_try_wait(s_full0, 0) && clock64() - c0 < 50000;) {
+                }
             int k = 0; // tiles of this block so far
             for (int j = 0; j < n && ok; ++j) {
                 const int st = j % STAGES, tile = u0 + j;
