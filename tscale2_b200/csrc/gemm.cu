@@ -1254,8 +1254,9 @@ int gemm(const GemmArgs &a)
     rc = TS2_ERR_UNSUPPORTED;
     if (pl.pair()) {
         const int sms = std::max(2, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)) & ~1;
-        rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, gate_bwd ? 3 : act_bwd ? 2 : paired ? 1 : 0, std::min(pl.grid, sms), tmA, tmB,
-                              tmC, tmCin, tmX, tmY, p);
+        const bool out16 = pl.splits == 1 && (a.epi.out_kind == TS2_OUT_F16 || a.epi.out_kind == TS2_OUT_BF16);
+        const PairForm form = gate_bwd ? P_GATE_BWD : act_bwd ? P_ACT_BWD : paired ? P_GATED : out16 ? P_16 : P_F32;
+        rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, form, std::min(pl.grid, sms), tmA, tmB, tmC, tmCin, tmX, tmY, p);
         if (rc == TS2_OK && pl.splits > 1)
             rc = reduce_splits<2 * BM, 256>(a, pl, p);
     } else if (paired) {

@@ -27,7 +27,6 @@ constexpr int PM = 256, PN = 256; // the pair's tile
 constexpr int P_HALF_BYTES = 128 * STAGE_ROW_BYTES; // a CTA's half of either operand, one K block
 constexpr int P_STAGE_BYTES = 2 * P_HALF_BYTES;
 constexpr int P_THREADS = 320, P_THREADS_16 = 576;
-enum { P_F32 = 0, P_16 = 1, P_GATED = 2, P_ACT_BWD = 3, P_GATE_BWD = 4 };
 constexpr bool is_bwd(int form) { return form == P_ACT_BWD || form == P_GATE_BWD; }
 // shared memory of a form: ring, epilogue staging, barriers, alignment slack
 template <int FORM>
@@ -123,9 +122,7 @@ __device__ __forceinline__ PairUnit pair_unit(const GemmParams &p, int u)
 // 16-byte piece c of row r of a 32 x 128 byte block in the 128-byte swizzle
 __device__ __forceinline__ uint32_t piece(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
-// FORM of the epilogue: P_F32 (fp32 output, accumulate form, partial tiles; 8 warps), P_16 (fp16 / bf16 output; 16 warps),
-// P_GATED (gated activation; 16 warps), P_ACT_BWD (its backward; 16 warps), P_GATE_BWD (backward of the attention gate;
-// 16 warps)
+// FORM of the epilogue (PairForm): 8 epilogue warps in P_F32, 16 in the others
 template <int ES, int MMA, bool MN, int FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_THREADS : P_THREADS_16, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -798,11 +795,10 @@ int launch_pair(int device, cudaStream_t stream, int grid, const CUtensorMap &tm
 
 } // namespace
 
-int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, int form_arg, int grid, const CUtensorMap &tmA,
+int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, PairForm form, int grid, const CUtensorMap &tmA,
                      const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const CUtensorMap &tmX, const CUtensorMap &tmY,
                      const GemmParams &p)
 {
-    const int form = form_arg == 3 ? P_GATE_BWD : form_arg == 2 ? P_ACT_BWD : form_arg == 1 ? P_GATED : p.splits == 1 && (p.out_kind == TS2_OUT_F16 || p.out_kind == TS2_OUT_BF16) ? P_16 : P_F32;
 #define TS2_PAIR_CASE(ES_, MMA_, MN_, FORM_)                          \
     if (es == ES_ && mma == MMA_ && mn == MN_ && form == FORM_)       \
         return launch_pair<ES_, MMA_, MN_, FORM_>(device, stream, grid, tmA, tmB, tmC, tmCin, tmX, tmY, p);

@@ -46,11 +46,14 @@ struct GemmParams {
     float *bwd_dscale = nullptr; // backward of the attention gate (see Epilogue)
 };
 
+// Forms of the epilogue of gemm_pair.cu: fp32 output, accumulate form and partial tiles; fp16 / bf16 output; gated
+// activation; its backward; backward of the attention gate (see Epilogue)
+enum PairForm { P_F32, P_16, P_GATED, P_ACT_BWD, P_GATE_BWD };
 // gemm_pair.cu: the contraction on pairs of CTAs (tiles of 256 x 256).  tmB's box is 128 rows (K-major) or one K block
-// (token-major); tmC's and tmCin's are 32 rows x 128 bytes.  grid: CTAs, an even number.
-// form: 0 by output kind, 1 gated activation, 2 its backward (tmC: 32 rows x 64 bytes, tmCin: [wide | gate] in 32 rows x 128),
-// 3 backward of the attention gate (the same, and tmX: o, tmY: dout, both 32 rows x 128); tmX, tmY otherwise unused
-int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, int form, int grid, const CUtensorMap &tmA,
+// (token-major); tmC's and tmCin's are 32 rows x 128 bytes (P_GATED: tmC 32 x 64).  grid: CTAs, an even number.
+// P_ACT_BWD: tmC 32 rows x 64 bytes, tmCin [wide | gate] in 32 rows x 128; P_GATE_BWD: the same, and tmX: o, tmY: dout, both
+// 32 rows x 128; tmX, tmY otherwise unused
+int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, PairForm form, int grid, const CUtensorMap &tmA,
                      const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const CUtensorMap &tmX, const CUtensorMap &tmY,
                      const GemmParams &p);
 

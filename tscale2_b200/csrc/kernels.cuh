@@ -74,7 +74,7 @@ struct BatchSpans {
 };
 int batch_prepare(const Ctx &c, const BatchTables &b, const BatchSpans *att, int n_types, LabelIndex &ix, bool *sorted);
 size_t label_index_hist_elems(size_t label_cap);
-size_t label_index_partial_elems(size_t label_cap, int D);
+size_t label_index_partial_elems(int device, size_t label_cap, int D);
 // validates label_arr / label_ptr in place (bad labels become label 0, label_ptr is clamped to n_labels) and writes the
 // unsorted entries of ix; label_index_sort orders them (a stable radix sort, 8 bits per pass)
 int label_index_entries(const Ctx &c, uint32_t *label_arr, uint32_t *label_ptr, int T, uint32_t n_labels, uint32_t label_count,

@@ -513,18 +513,18 @@ __global__ void __launch_bounds__(SB_THREADS) small_batch_kernel(const SmallBatc
 }
 
 // ---- embedding gradient through the inverse index ----------------------------------------
-// The sorted entries are cut into chunks (of 64; fewer where that leaves SMs idle); one warp walks one chunk for one 128-wide tile of the state and
-// sums the runs of equal labels in entry order.  A run that lies inside its chunk is added to its row of dE by that
+// The sorted entries are cut into chunks (of 64; fewer where that leaves SMs idle); one warp walks one chunk for one
+// 128-wide tile of the state and sums the runs of equal labels in entry order.  A run that lies inside its chunk is added to its row of dE by that
 // warp alone.  A run that crosses a chunk border leaves partial sums (slot 1: the run leaves the chunk at its end and
 // did not enter it at the start; slot 0: the run entered at the start), which embed_chain_kernel adds up chunk by chunk.
 // What bounds it: a big batch, the bytes of g (read once); a small one, the latency of a warp's walk.  With chunks of 64
 // a batch of 512 tokens x 2 tiles gave work to 16 warps, each of which waited for 64 rows of dE in turn (29 us).
 constexpr int EMB_CHUNK = 64, EMB_CHUNK_MIN = 8;
-constexpr unsigned EMB_ITEMS = 148 * 16; // warps that fill the device
-static unsigned emb_chunk(size_t n, int tiles)
+static unsigned emb_items(int device) { return 16 * sm_count(device); } // warps that fill the device
+static unsigned emb_chunk(int device, size_t n, int tiles)
 {
     unsigned chunk = EMB_CHUNK;
-    while (chunk > EMB_CHUNK_MIN && (n + chunk - 1) / chunk * tiles < EMB_ITEMS)
+    while (chunk > EMB_CHUNK_MIN && (n + chunk - 1) / chunk * tiles < emb_items(device))
         chunk /= 2;
     return chunk;
 }
@@ -537,7 +537,8 @@ __device__ __forceinline__ void add4(float4 &a, const float4 &g, float w)
     a.w += g.w * w;
 }
 
-// row += a without waiting for the row: each kernel has one writer per row, so the order of the additions is fixed
+// row += a without waiting for the row: each kernel has one writer per row, so the order of the additions is fixed.
+// (A reduction in global memory takes subnormals, fp32 below 1.2e-38, as zero; the loaded and added form did not.)
 __device__ __forceinline__ void accumulate_row(float *row, const float4 &a)
 {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w) : "memory");
@@ -735,10 +736,10 @@ size_t label_index_hist_elems(size_t label_cap)
     return counters + (counters + 1023) / 1024; // and the block sums of their scan
 }
 
-size_t label_index_partial_elems(size_t label_cap, int D)
+size_t label_index_partial_elems(int device, size_t label_cap, int D)
 {
-    // smaller chunks are only taken while twice their size gives fewer than EMB_ITEMS items
-    const size_t tiles = D / TILE, small = std::min((label_cap + EMB_CHUNK_MIN - 1) / EMB_CHUNK_MIN, 2 * (size_t)EMB_ITEMS / tiles + 2);
+    // smaller chunks are only taken while twice their size gives fewer than emb_items() items
+    const size_t tiles = D / TILE, small = std::min((label_cap + EMB_CHUNK_MIN - 1) / EMB_CHUNK_MIN, 2 * (size_t)emb_items(device) / tiles + 2);
     return std::max((label_cap + EMB_CHUNK - 1) / EMB_CHUNK, small) * 2 * (size_t)D;
 }
 
@@ -786,7 +787,7 @@ int embed_backward_indexed(const Ctx &c, const float *g, const LabelIndex &ix, i
 {
     if (ix.n == 0)
         return TS2_OK;
-    const uint32_t chunk = emb_chunk(ix.n, D / TILE), nchunks = (ix.n + chunk - 1) / chunk;
+    const uint32_t chunk = emb_chunk(c.device, ix.n, D / TILE), nchunks = (ix.n + chunk - 1) / chunk;
     const long long items = (long long)nchunks * (D / TILE);
     const int grid = (int)std::max<long long>(1, std::min<long long>((items + BP_WARPS - 1) / BP_WARPS, (long long)sm_count(c.device) * 8));
     TS2_LAUNCH((embed_runs_kernel), grid, BP_THREADS, 0, c.stream, g, ix.key[ix.sorted], ix.val[ix.sorted], ix.n, chunk, D, dE, ix.partial);

@@ -1137,7 +1137,7 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
         M_TRY(dalloc(m, &b.ix.val[i], b.label_cap));
     }
     M_TRY(dalloc(m, &b.ix.hist, label_index_hist_elems(b.label_cap)));
-    M_TRY(dalloc(m, &b.ix.partial, label_index_partial_elems(b.label_cap, D)));
+    M_TRY(dalloc(m, &b.ix.partial, label_index_partial_elems(m->device, b.label_cap, D)));
     m->pinned_bytes = 2 * b.raw_cap * 4 + sizeof(HostReport);
     TS2_CUDA(cudaMallocHost(&m->pinned, m->pinned_bytes));
     m->report = (HostReport *)((uint32_t *)m->pinned + 2 * b.raw_cap);
