@@ -99,14 +99,17 @@ def time_attention(lib, T, heads, variant, iters, warmup=2, doc=1024):
     return out
 
 
-def time_steps(blocks, T, seq, iters, prec_name, dim=768, heads=12, ffn_tiles=24, vocab=50304):
+def time_steps(blocks, T, seq, iters, prec_name, score_gradients, dim=768, heads=12, ffn_tiles=24, vocab=50304):
     """Applied training steps of a model with the headline benchmark's layer shapes but only `blocks` blocks: every
-    kernel of the step runs at full width on a few GB of device memory, which is what a profiler capture wants."""
+    kernel of the step runs at full width on a few GB of device memory, which is what a profiler capture wants (with
+    score_gradients, bytes for the attention's score gradients, no more than the batch needs)."""
     from . import host
     from .model import Model
     spec = host.ModelSpec(dim=dim, head_count=heads, ffn_tiles=ffn_tiles, vocab=vocab, attention_widths=[seq],
                           precision=PREC[prec_name][0]).add_blocks(blocks)
     model = Model(spec, host.init_weights(spec, 1000), T)
+    if score_gradients is not None:
+        check(model.lib.ts2_set_score_gradient_limit(model.h, score_gradients))
     model.set_batch(host.synthetic_batch(spec, T // seq, seq, 1000))
     step = host.training_step(rate=0.01, iteration=10)
     model.backprop(step, apply=True)
@@ -128,6 +131,7 @@ def main():
     ap.add_argument("--heads", type=int, default=12)
     ap.add_argument("--variant", type=int, default=3, choices=[0, 1, 2, 3])
     ap.add_argument("--prec", default="fp8", choices=sorted(PREC))
+    ap.add_argument("--score-gradients", type=int, default=None)
     ap.add_argument("--M", type=int, default=16384)
     ap.add_argument("--N", type=int, default=4096)
     ap.add_argument("--K", type=int, default=4096)
@@ -136,7 +140,8 @@ def main():
     args = ap.parse_args()
     lib = capi.load_library()
     if args.op == "step":
-        print(json.dumps(time_steps(args.blocks, args.T, args.seq, args.iters, args.prec if args.prec != "int8" else "fp8")))
+        print(json.dumps(time_steps(args.blocks, args.T, args.seq, args.iters, args.prec if args.prec != "int8" else "fp8",
+                                    args.score_gradients)))
     elif args.op == "att":
         print(json.dumps(time_attention(lib, args.T, args.heads, args.variant, args.iters, args.warmup)))
     elif args.op == "config2":
