@@ -501,7 +501,7 @@ int ts2_op_attention_gated_forward(int device, void *stream, int prec, const voi
 int ts2_attention_backward(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
                            const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
                            int head_count, float alibi_slope, void *dq, void *dk, void *dv);
-/* variants 2 and 3 with a bound of the caller's on the device memory for score gradients (ts2_attention_backward: 4 GB):
+/* variants 2 and 3 with a bound of the caller's on the device memory for score gradients (ts2_attention_backward: 1.9 GB):
  * a call whose spans need more recomputes the scores for dq, as the engine does with a batch beyond its buffer */
 int ts2_op_attention_backward_limited(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
                                       const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,

@@ -17,7 +17,8 @@ SCORE_GRADIENTS = 64 * 65 // 2 * 2 * 16384 * H  # one causal document
 
 
 class Call:
-    def __init__(self):
+    def __init__(self, T=T, H=H):
+        self.T, self.H = T, H
         self.lib = capi.load_library()
         rng = np.random.default_rng(5)
         self.q, self.k, self.v, self.dout = (DeviceBuffer.from_numpy(rng.standard_normal((T, 128 * H)).astype(np.float16)) for _ in range(4))
@@ -32,8 +33,8 @@ class Call:
 
     def backward(self):
         check(self.lib.ts2_attention_backward(0, None, 2, self.q.ptr, self.k.ptr, self.v.ptr, self.dout.ptr, self.lse.ptr, self.dscale.ptr,
-                                              *self.spans, T, H, 0.0, *[g.ptr for g in self.grads]))
-        return [g.download((T, 128 * H), np.float32) for g in self.grads]
+                                              *self.spans, self.T, self.H, 0.0, *[g.ptr for g in self.grads]))
+        return [g.download((self.T, 128 * self.H), np.float32) for g in self.grads]
 
 
 def free_bytes():
@@ -70,3 +71,14 @@ def test_kept_scratch_is_given_back():
     assert free_bytes() < before - SCORE_GRADIENTS // 2
     check(call.lib.ts2_dev_trim(0))
     assert free_bytes() > before - (64 << 20)
+
+
+@pytest.mark.parametrize("heads,stored", [(6, True), (8, False)])  # 1.6 GB and 2.2 GB of score gradients
+def test_a_call_takes_no_more_than_the_pool_keeps(heads, stored):
+    """More would be mapped anew by every call, which takes longer than recomputing the scores."""
+    call = Call(16384, heads)
+    check(call.lib.ts2_dev_trim(0))
+    before = free_bytes()
+    call.backward()
+    assert (free_bytes() < before - (1 << 30)) == stored
+    check(call.lib.ts2_dev_trim(0))

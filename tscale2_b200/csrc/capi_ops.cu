@@ -495,8 +495,11 @@ int ts2_attention_backward(int device, void *stream, int variant, const void *q,
                            const float *lse, const float *dscale, const int32_t *span_start, const int32_t *span_finish, int T,
                            int head_count, float alibi_slope, void *dq, void *dk, void *dv)
 {
+    // Score gradients beyond what the pool keeps between calls would be mapped anew by each call, which costs more than
+    // recomputing the scores (64 MB are left to the call's tables).  Documents of 4096, per call, stored / recomputed, ms:
+    // 8 x 15 heads (1.9 GB) 1.68 / 2.54, 8 x 16 (2.06 GB) 4.9 / 2.5, 8 x 24 (3.1 GB) 26 / 3.6.
     return run_attention_backward(device, stream, variant, q, k, v, dout, lse, dscale, span_start, span_finish, T, head_count, alibi_slope, dq,
-                                  dk, dv, ATT_DS_MAX_BYTES);
+                                  dk, dv, SCRATCH_KEEP_BYTES / 32 * 31);
 }
 
 int ts2_op_attention_backward_limited(int device, void *stream, int variant, const void *q, const void *k, const void *v, const void *dout,
