@@ -457,11 +457,11 @@ def main():
     # DRAM traffic per launch needs ncu, so it is not measured in this run.  For the headline workload it comes from a
     # small-case capture (profiles/gemm_dram_traffic_one_block_step.md): one block of the same model at the same number
     # of nodes launches exactly the contractions of one layer pair and of the final layer; 12 x the layer launches + the
-    # final layer's moved 0.980 x the algorithmic bytes the library counted for the same launches (operands once, outputs
+    # final layer's moved 0.991 x the algorithmic bytes the library counted for the same launches (operands once, outputs
     # once; the last lines written are still in L2 when a kernel ends).  Other workloads: null.
     traffic = None
     if args.workload == "c3_dense12_d768" and args.precision == "fp8" and gemm_n:
-        traffic = 0.980 * gemm_bytes / gemm_n
+        traffic = 0.991 * gemm_bytes / gemm_n
     by_class = {}
     for name, (c_ms, c_n, c_fl) in gemm_classes.items():
         if c_n:
@@ -475,11 +475,11 @@ def main():
         backward["frac_of_cublaslt_fp8_sustained"] = backward["tflops"] / vendor_fp8["sustained"]
     roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                "traffic_source": ("small-case ncu capture scaled by the units processed: 0.980 x algorithmic bytes "
+                "traffic_source": ("small-case ncu capture scaled by the units processed: 0.991 x algorithmic bytes "
                                    "(profiles/gemm_dram_traffic_one_block_step.md)") if traffic else None,
                 "algorithmic_bytes_per_launch": gemm_bytes / gemm_n if gemm_n else None,
                 "hbm_gbs_algorithmic": gemm_bytes / (gemm_ms / 1e3) / 1e9 if gemm_ms > 0 else None,
-                "hbm_peak_gbs": peaks.get("hbm_gbs"), "kernel": "gemm_kernel (tcgen05)",
+                "hbm_peak_gbs": peaks.get("hbm_gbs"), "kernel": "gemm_pair_kernel and gemm_kernel (tcgen05)",
                 "launches_per_step": gemm_n / args.steps, "share_of_step": gemm_ms / ms_max, "peak_source": peak_note,
                 "step_flops_per_token": fpt, "step_tflops": value / world * fpt / 1e12,
                 "by_class": by_class, "backward_gemm": backward, "fp8_cublaslt_tflops": vendor_fp8}
