@@ -269,7 +269,7 @@ def run_c2_gemm(args):
                        "l2": "operands and output of one launch are 208-224 MB, larger than L2"},
             "variants": out,
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
-                         "kernel": "gemm_kernel (tcgen05), isolated launches", "fp8_cublaslt_tflops": vendor,
+                         "kernel": "gemm_pair_kernel (tcgen05), isolated launches", "fp8_cublaslt_tflops": vendor,
                          "peak_source": f"2 x bf16_tflops (burst: isolated launches) of MEASURED_PEAKS.json ({peak_src}); nominal dense fp8 is 4500"},
             "gpu_launches": int(2 * 2 * args.steps)}
     print(json.dumps(line))

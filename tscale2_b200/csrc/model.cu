@@ -328,7 +328,8 @@ int dalloc(ts2_model *m, T **p, size_t count)
     if (e != cudaSuccess) {
         cudaGetLastError();
         scratch_trim(m->device);
-        free_score_gradients(m);
+        if (m->att_bwd.ds && poll_stream(m) == TS2_OK) // a queued step may still use it
+            free_score_gradients(m);
         e = cudaMalloc(&q, bytes);
         cudaGetLastError();
     }
