@@ -97,7 +97,8 @@ bool one_pinned_range(const void *p, size_t bytes);
 
 // Scratch of the operator-level calls, stream-ordered, from a pool of the library's own on each device.  A default pool
 // keeps nothing: after every synchronisation the next call mapped its scratch anew, 0.3 - 0.5 ms.  This one keeps up to
-// SCRATCH_KEEP_BYTES between calls; a call that needs more maps it each time, tens of milliseconds for a few GB.  Any thread and stream; scratch_trim (ts2_dev_trim) gives back what no queued work uses.
+// SCRATCH_KEEP_BYTES between calls; a call that needs more maps it each time, tens of milliseconds for a few GB.  Any
+// thread and stream; scratch_trim (ts2_dev_trim) gives back what no queued work uses.
 // An allocation that fails is tried once more on a trimmed pool and leaves no CUDA error behind; scratch_try_alloc is for
 // callers that can do without and leaves no message either.
 constexpr size_t SCRATCH_KEEP_BYTES = (size_t)2 << 30;

@@ -50,7 +50,7 @@ struct GemmParams {
 // activation; its backward; backward of the attention gate (see Epilogue)
 enum PairForm { P_F32, P_16, P_GATED, P_ACT_BWD, P_GATE_BWD };
 // gemm_pair.cu: the contraction on pairs of CTAs (tiles of 256 x 256).  tmB's box is 128 rows (K-major) or one K block
-// (token-major); tmC's and tmCin's are 32 rows x 128 bytes (P_GATED: tmC 32 x 64).  grid: CTAs, an even number.
+// (token-major); tmC's and tmCin's are 32 rows x 128 bytes (P_GATED: tmC 32 x 64 bytes).  grid: CTAs, an even number.
 // P_ACT_BWD: tmC 32 rows x 64 bytes, tmCin [wide | gate] in 32 rows x 128; P_GATE_BWD: the same, and tmX: o, tmY: dout, both
 // 32 rows x 128; tmX, tmY otherwise unused
 int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, PairForm form, int grid, const CUtensorMap &tmA,

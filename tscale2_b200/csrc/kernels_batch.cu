@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(SB_THREADS) small_batch_kernel(const SmallBatc
 
 // ---- embedding gradient through the inverse index ----------------------------------------
 // The sorted entries are cut into chunks (of 64; fewer where that leaves SMs idle); one warp walks one chunk for one
-// 128-wide tile of the state and sums the runs of equal labels in entry order.  A run that lies inside its chunk is added to its row of dE by that
-// warp alone.  A run that crosses a chunk border leaves partial sums (slot 1: the run leaves the chunk at its end and
+// 128-wide tile of the state and sums the runs of equal labels in entry order.  A run that lies inside its chunk is added
+// to its row of dE by that warp alone.  A run that crosses a chunk border leaves partial sums (slot 1: the run leaves the chunk at its end and
 // did not enter it at the start; slot 0: the run entered at the start), which embed_chain_kernel adds up chunk by chunk.
 // What bounds it: a big batch, the bytes of g (read once); a small one, the latency of a warp's walk.  With chunks of 64
 // a batch of 512 tokens x 2 tiles gave work to 16 warps, each of which waited for 64 rows of dE in turn (29 us).
