@@ -15,12 +15,14 @@
 // What bounds it: before, one CTA per item with one group of 16 warps took 2850 clocks per 128 x 64 tile against about 1280
 // that its MMAs take (S and dP are bound by the shared-memory reads of N = 64, 48 clocks per K step), and some 8000 clocks
 // per item for its start and end; and dQ recomputed S, dP and the exponentials in a kernel as long.  Here dS costs its
-// bytes once out and once in.
+// bytes once out and once in.  S and dP are handed over one by one, and so are P and dS: the exponentials run while dP is still
+// being multiplied, dV's product while dS is computed (64 x 1024 nodes, 12 heads 601 -> 573 us, 8 x 2048, 4 heads 124 -> 115).
 //
 // Everything that is handed over once per tile has one barrier per S / dP pair: the next phase of a pair's barrier belongs
 // to the tile two further on, which cannot start before the waiter of this phase has acted, so a parity test can never
 // miss a phase.  Every wait is bounded; a give-up raises the status word.
 #include "att_tc.cuh"
+#include <type_traits>
 
 namespace ts2 {
 
@@ -73,8 +75,9 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
     const uint32_t kv_full = smem_u32(bars), kv_empty = smem_u32(bars + 1), st_full0 = smem_u32(bars + 2), st_empty0 = smem_u32(bars + 5),
                    s_full0 = smem_u32(bars + 8), pair_free0 = smem_u32(bars + 10), g_full0 = smem_u32(bars + 12), g_free0 = smem_u32(bars + 14),
                    acc_done = smem_u32(bars + 16), acc_free = smem_u32(bars + 17), rfull0 = smem_u32(bars + 18), rempty0 = smem_u32(bars + 22),
-                   mate0 = smem_u32(bars + 26); // [8]: the two warps that share a group's lane quarter
-    uint32_t *tmem_slot = (uint32_t *)(bars + 34);
+                   mate0 = smem_u32(bars + 26), // [8]: the two warps that share a group's lane quarter
+                   dp_full0 = smem_u32(bars + 34), p_full0 = smem_u32(bars + 36);
+    uint32_t *tmem_slot = (uint32_t *)(bars + 38);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
     volatile int *ring = (volatile int *)(tmem_slot + 2); // [KV_RING] item numbers, -1 = no more
 
@@ -93,6 +96,8 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
         for (int g = 0; g < 2; ++g) {
             mbar_init(s_full0 + 8 * g, 1);
             mbar_init(pair_free0 + 8 * g, 1);
+            mbar_init(dp_full0 + 8 * g, 1);
+            mbar_init(p_full0 + 8 * g, 8);
             mbar_init(g_full0 + 8 * g, 8);
             mbar_init(g_free0 + 8 * g, 2); // the MMAs that read the tile, and its store
         }
@@ -209,7 +214,7 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
                 ok = mbar_wait(kv_full, live & 1, abort_flag);
                 ++live;
                 for (int j = 0; j < n && ok; ++j, ++gt) { // S^T and dP^T of tile gt into pair gt & 1
-                    // the pair held P of tile gt - 2: the MMAs that read it must be complete before these write there
+                    // the pair's S block held P of tile gt - 2: the MMAs that read it must be complete before these write there
                     const int st = gt % KV_STAGES;
                     if ((gt >= 2 && !mbar_wait(pair_free0 + 8 * (gt & 1), ((gt - 2) >> 1) & 1, abort_flag)) ||
                         !mbar_wait(st_full0 + 8 * st, (gt / KV_STAGES) & 1, abort_flag)) {
@@ -223,9 +228,16 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
                     // 8 steps of 16 head dims; operands are two 64-dim atoms each
                     umma_f16_x4(tS, dK, dQ, idesc_s, 0u, 2u, 2u);
                     umma_f16_x4(tS, dK + (Q_BYTES / 2 >> 4), dQ + (KV_BYTES / 2 >> 4), idesc_s, 1u, 2u, 2u);
+                    tc_commit(s_full0 + 8 * (gt & 1));
+                    // its dP block was last read by the compute warps on their way to dS of tile gt - 2
+                    if (gt >= 2 && !mbar_wait(g_full0 + 8 * (gt & 1), ((gt - 2) >> 1) & 1, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
                     umma_f16_x4(tDP, dV, dD, idesc_s, 0u, 2u, 2u);
                     umma_f16_x4(tDP, dV + (Q_BYTES / 2 >> 4), dD + (KV_BYTES / 2 >> 4), idesc_s, 1u, 2u, 2u);
-                    tc_commit(s_full0 + 8 * (gt & 1));
+                    tc_commit(dp_full0 + 8 * (gt & 1));
                     if (j == n - 1)
                         tc_commit(kv_empty); // the next item's K and V may come in
                 }
@@ -249,7 +261,7 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
                 ++live;
                 for (int j = 0; j < n && ok; ++j, ++gt) {
                     const int st = gt % KV_STAGES, pr = gt & 1;
-                    if (!mbar_wait(g_full0 + 8 * pr, (gt >> 1) & 1, abort_flag) || !mbar_wait(st_full0 + 8 * st, (gt / KV_STAGES) & 1, abort_flag)) {
+                    if (!mbar_wait(p_full0 + 8 * pr, (gt >> 1) & 1, abort_flag) || !mbar_wait(st_full0 + 8 * st, (gt / KV_STAGES) & 1, abort_flag)) {
                         ok = false;
                         break;
                     }
@@ -265,6 +277,11 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
                     for (int kk = 0; kk < 4; ++kk)
                         umma_f16_ts(tDV, tS + 16 * kk, dDm + (uint64_t)(kk * 128), idesc_acc, (j > 0 || kk > 0) ? 1u : 0u);
                     tc_commit(pair_free0 + 8 * pr);
+                    if (!mbar_wait(g_full0 + 8 * pr, (gt >> 1) & 1, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
                     umma_f16_x4(tDK, dG, dQm, idesc_acc, j > 0 ? 1u : 0u, 2u, 128u);
                     tc_commit(st_empty0 + 8 * st);
                     tc_commit(g_free0 + 8 * pr);
@@ -306,7 +323,8 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
         const uint32_t tS = tmem_base + (grp ? 384 : 0) + lane_addr + half * 32, tDP = tS + TC_BN;
         const float ds = att_dot_scale_tc(), c2 = ds * 0.693147f, slope = p.slope;
         uint8_t *const gbuf = smem + KV_G_OFF + grp * KV_G_BYTES;
-        const uint32_t s_full = s_full0 + 8 * grp, g_full = g_full0 + 8 * grp, g_free = g_free0 + 8 * grp, mate = mate0 + 8 * (grp * 4 + quarter);
+        const uint32_t s_full = s_full0 + 8 * grp, g_full = g_full0 + 8 * grp, g_free = g_free0 + 8 * grp, dp_full = dp_full0 + 8 * grp,
+                       p_full = p_full0 + 8 * grp, mate = mate0 + 8 * (grp * 4 + quarter);
         int gt = 0, live = 0, last_gt = -1; // last_gt: this group's latest tile
         uint32_t mate_phase = 0;
         bool ok = true;
@@ -326,12 +344,11 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
                 if ((gt & 1) != grp)
                     continue;
                 const int st = gt % KV_STAGES;
-                // s_full says the products are done; the tile's per-node records came with the same stage by bulk copies, and
+                // s_full says the product is done; the tile's per-node records came with the same stage by bulk copies, and
                 // the threads that read them observe that stage's barrier themselves (it has long completed: the issuer
                 // waited for it before the products), which is what orders the copies' writes before these reads
                 ok = __all_sync(0xffffffffu, mbar_wait(s_full, (gt >> 1) & 1, abort_flag) &&
-                                                 mbar_wait(st_full0 + 8 * st, (gt / KV_STAGES) & 1, abort_flag) &&
-                                                 (gt < 2 || mbar_wait(g_free, ((gt - 2) >> 1) & 1, abort_flag)));
+                                                 mbar_wait(st_full0 + 8 * st, (gt / KV_STAGES) & 1, abort_flag));
                 if (!ok)
                     break;
                 tc_fence_after();
@@ -339,51 +356,71 @@ __global__ void __launch_bounds__(KV_THREADS, 1)
                 const float4 *node = (const float4 *)mt + half * 16; // {-lse, -dscale c2} of two nodes
                 const int2 info = *(const int2 *)(mt + ATT_NODE_BYTES + TC_BN * 8); // {latest span start, earliest span end} of the tile
                 const bool plain = slope == 0.f && info.x <= r0 && info.y >= r0 + TC_BM - 1; // every node sees every key
+                // P from the scores, in time for its product while dP is still on its way
+                uint32_t w[32]; // scores, then weights
+                tmem_ld32(tS, w);
+                tmem_ld_wait();
+                auto weights = [&](auto plain_tag) {
+                    constexpr bool PLAIN = decltype(plain_tag)::value;
 #pragma unroll
-                for (int q16 = 0; q16 < 2; ++q16) {
-                    uint32_t rs[16], rp[16], pv[8], gk[8];
-                    tmem_ld16(tS + q16 * 16, rs);
-                    tmem_ld16(tDP + q16 * 16, rp);
-                    tmem_ld_wait();
-                    if (plain) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const float4 m = node[q16 * 8 + i];
-                            float w0, w1;
-                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w0) : "f"(fmaf(__uint_as_float(rs[2 * i]), ds, m.x)));
-                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w1) : "f"(fmaf(__uint_as_float(rs[2 * i + 1]), ds, m.z)));
-                            const __half2 hv = sat_half2(w0, w1);
-                            const __half2 hk = sat_half2(w0 * fmaf(__uint_as_float(rp[2 * i]), c2, m.y), w1 * fmaf(__uint_as_float(rp[2 * i + 1]), c2, m.w));
-                            pv[i] = *(const uint32_t *)&hv;
-                            gk[i] = *(const uint32_t *)&hk;
-                        }
-                    } else {
+                    for (int q16 = 0; q16 < 2; ++q16) {
+                        uint32_t pv[8];
                         const int4 *span = (const int4 *)(mt + ATT_NODE_BYTES) + half * 16 + q16 * 8; // {start, length} of two nodes
                         const int c0 = (tb.x + j) * TC_BN + half * 32 + q16 * 16 - rr;               // node - key
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
+                            const int e = 16 * q16 + 2 * i;
                             const float4 m = node[q16 * 8 + i];
-                            const int4 sp = span[i];
-                            const float o0 = slope != 0.f ? m.x - slope * (float)(c0 + 2 * i) : m.x;
-                            const float o1 = slope != 0.f ? m.z - slope * (float)(c0 + 2 * i + 1) : m.z;
-                            float w0, w1;
-                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w0) : "f"(fmaf(__uint_as_float(rs[2 * i]), ds, o0)));
-                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w1) : "f"(fmaf(__uint_as_float(rs[2 * i + 1]), ds, o1)));
-                            w0 = (unsigned)(rr - sp.x) <= (unsigned)sp.y ? w0 : 0.f;
-                            w1 = (unsigned)(rr - sp.z) <= (unsigned)sp.w ? w1 : 0.f;
-                            const __half2 hv = sat_half2(w0, w1);
-                            const __half2 hk = sat_half2(w0 * fmaf(__uint_as_float(rp[2 * i]), c2, m.y), w1 * fmaf(__uint_as_float(rp[2 * i + 1]), c2, m.w));
-                            pv[i] = *(const uint32_t *)&hv;
-                            gk[i] = *(const uint32_t *)&hk;
+                            float o0 = m.x, o1 = m.z, w0, w1;
+                            if (!PLAIN && slope != 0.f) {
+                                o0 -= slope * (float)(c0 + 2 * i);
+                                o1 -= slope * (float)(c0 + 2 * i + 1);
+                            }
+                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w0) : "f"(fmaf(__uint_as_float(w[e]), ds, o0)));
+                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w1) : "f"(fmaf(__uint_as_float(w[e + 1]), ds, o1)));
+                            if (!PLAIN) {
+                                const int4 sp = span[i];
+                                w0 = (unsigned)(rr - sp.x) <= (unsigned)sp.y ? w0 : 0.f;
+                                w1 = (unsigned)(rr - sp.z) <= (unsigned)sp.w ? w1 : 0.f;
+                            }
+                            w[e] = __float_as_uint(w0);
+                            w[e + 1] = __float_as_uint(w1);
+                            pv[i] = bits_from_h2(sat_half2(w0, w1));
                         }
+                        tmem_st8(tS + q16 * 16, pv); // where this thread's own S values were
                     }
-                    tmem_st8(tS + q16 * 16, pv); // where this thread's own S values were
-                    const int c = half * 4 + q16 * 2;
-                    *(uint4 *)(gbuf + piece128(row, c)) = make_uint4(gk[0], gk[1], gk[2], gk[3]);
-                    *(uint4 *)(gbuf + piece128(row, c + 1)) = make_uint4(gk[4], gk[5], gk[6], gk[7]);
+                };
+                if (plain)
+                    weights(std::true_type());
+                else
+                    weights(std::false_type());
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(p_full);
+                // dS
+                ok = __all_sync(0xffffffffu, mbar_wait(dp_full, (gt >> 1) & 1, abort_flag) &&
+                                                 (gt < 2 || mbar_wait(g_free, ((gt - 2) >> 1) & 1, abort_flag)));
+                if (!ok)
+                    break;
+                tc_fence_after();
+                uint32_t rp[32];
+                tmem_ld32(tDP, rp);
+                tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t gk[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int e = 8 * c + 2 * i;
+                        const float4 m = node[4 * c + i];
+                        gk[i] = bits_from_h2(sat_half2(__uint_as_float(w[e]) * fmaf(__uint_as_float(rp[e]), c2, m.y),
+                                                       __uint_as_float(w[e + 1]) * fmaf(__uint_as_float(rp[e + 1]), c2, m.w)));
+                    }
+                    *(uint4 *)(gbuf + piece128(row, half * 4 + c)) = make_uint4(gk[0], gk[1], gk[2], gk[3]);
                 }
                 last_gt = gt;
-                tmem_st_wait();
                 fence_proxy_async(); // dS^T is read by MMAs and by its store
                 tc_fence_before();
                 __syncwarp();
