@@ -7,7 +7,7 @@
 // independent second formulation for the tests; the engine runs the tcgen05 kernels of
 // kernels_att_tc.cu (kernels_att_mma.cu holds an mma.sync formulation, also kept for the tests).
 #include "kernels.cuh"
-#include "fast_types.cuh"
+#include "row_math.cuh"
 
 namespace ts2 {
 
@@ -60,54 +60,9 @@ int fill_rope(const Ctx &c, float *rope, int T)
     return TS2_OK;
 }
 
-__device__ __forceinline__ float4 rope_apply(float4 v, float4 cs, float dir)
-{
-    // pairs (0,1) and (2,3) of the lane's four elements; cs = (cos0, sin0, cos1, sin1)
-    const float s0 = cs.y * dir, s1 = cs.w * dir;
-    return make_float4(v.x * cs.x - v.y * s0, v.x * s0 + v.y * cs.x, v.z * cs.z - v.w * s1, v.z * s1 + v.w * cs.z);
-}
-
 // The two kernels below give half a warp to a (node, head): lane = 8 consecutive elements, 16-byte accesses to the fp16
 // arrays, and one set of addresses, tests and shuffles for two items.  With a warp per item and 8-byte accesses they were
 // bound by instruction issue; 65536 nodes x 12 heads, e4m3: forward 233 -> 193 us (1.2 GB), backward 272 -> 208 us (1.3 GB).
-__device__ __forceinline__ void half8_to_float(uint4 raw, float (&f)[8])
-{
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 p = __half22float2(h2_from_bits(w[i]));
-        f[2 * i] = p.x;
-        f[2 * i + 1] = p.y;
-    }
-}
-__device__ __forceinline__ uint4 float_to_half8(const float (&f)[8])
-{
-    return make_uint4(bits_from_h2(sat_half2(f[0], f[1])), bits_from_h2(sat_half2(f[2], f[3])), bits_from_h2(sat_half2(f[4], f[5])),
-                      bits_from_h2(sat_half2(f[6], f[7])));
-}
-__device__ __forceinline__ float half_warp_sum(float v)
-{
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ float dot8(const float (&a)[8], const float (&b)[8])
-{
-    return (a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3]) + (a[4] * b[4] + a[5] * b[5] + a[6] * b[6] + a[7] * b[7]);
-}
-// rotates the lane's four pairs; c0, c1: (cos, sin) of two pairs each
-__device__ __forceinline__ void rope8(float (&v)[8], float4 c0, float4 c1, float dir)
-{
-    const float4 a = rope_apply(make_float4(v[0], v[1], v[2], v[3]), c0, dir), b = rope_apply(make_float4(v[4], v[5], v[6], v[7]), c1, dir);
-    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
-}
-__device__ __forceinline__ void scale8(float (&v)[8], float s)
-{
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        v[i] *= s;
-}
 
 __global__ void att_post_forward_kernel(const __half *__restrict__ qkvg, const float *__restrict__ rope, int T, int H,
                                         __half *__restrict__ q, __half *__restrict__ k, __half *__restrict__ v,

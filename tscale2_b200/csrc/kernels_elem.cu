@@ -4,7 +4,7 @@
 // consecutive elements: 16-byte accesses for fp32, 8 for fp16, 4 for e4m3) and
 // strides over (row, tile) pairs; reductions are warp shuffles.
 #include "kernels.cuh"
-#include "fast_types.cuh"
+#include "row_math.cuh"
 
 namespace ts2 {
 
@@ -157,21 +157,10 @@ __global__ void tilenorm_backward_kernel(const float *__restrict__ x, const floa
         for (int r = 0; r < R; ++r) {
             if (!ok[r])
                 continue;
-            const float4 d = scale4(dv[r], a);
-            const float sum2 = warp_sum(dot4(xv[r], xv[r]));
-            const float dp = warp_sum(dot4(xv[r], d));
-            float4 res = make_float4(0, 0, 0, 0);
-            if (sum2 != 0.f) {
-                const float sigma = dp / sum2, scale = sqrtf(128.f / sum2);
-                res = make_float4(scale * (d.x - xv[r].x * sigma), scale * (d.y - xv[r].y * sigma), scale * (d.z - xv[r].z * sigma),
-                                  scale * (d.w - xv[r].w * sigma));
-            }
+            float4 res = tilenorm_backward4(xv[r], scale4(dv[r], a));
             res = make_float4(o[r].x + res.x, o[r].y + res.y, o[r].z + res.z, o[r].w + res.w);
             *(float4 *)(g + idx[r]) = res;
-            local_max = fmaxf(local_max, fmaxf(fmaxf(fabsf(res.x), fabsf(res.y)), fmaxf(fabsf(res.z), fabsf(res.w))));
-            // fmaxf drops a NaN operand: a NaN anywhere in the row piece turns the running maximum into inf instead
-            if (!(res.x == res.x && res.y == res.y && res.z == res.z && res.w == res.w))
-                local_max = INFINITY;
+            local_max = absmax4(local_max, res);
         }
     }
     if (absmax) {
@@ -184,10 +173,7 @@ __global__ void tilenorm_backward_kernel(const float *__restrict__ x, const floa
             float m = 0.f;
             for (int i = 0; i < WARPS; ++i)
                 m = fmaxf(m, block_max[i]);
-            if (m == m && m < 3.0e38f) // NaN / inf never become the scale reference
-                atomicMax(absmax, __float_as_uint(m));
-            else if (health)
-                atomicCAS(health, 0u, step_no); // the first step at which this boundary's gradient was not finite
+            absmax_report(m, absmax, health, step_no);
         }
     }
 }
@@ -252,79 +238,101 @@ int cast_grad(const Ctx &c, const float *g, size_t n, const unsigned *absmax, vo
 // ---------------------------------------------------------------------------------
 // Row quantization to int8 with the reference's stochastic rounding (NormalizeVecsRowMaxKernel,
 // src/gpt/compute/row_scale.cuh:12-43, TCudaRngLCG, src/lib/cuda/cuda_util.cuh:538-559): one warp per row;
-// scale = max|x| / 127; lane h owns the elements h, h + 32, h + 64, ... and draws one uniform number per element, in
-// that order, from a linear congruential generator seeded with (bits of x[h], bits of x[0], row); q = round to
-// nearest even, saturating, of x / scale + u - 0.5.  x = src * mult, mult a power of two (so the scaling is exact).
-// The quantized row goes through a shared-memory row so that it leaves in 16-byte pieces.  Optionally also writes x as
-// fp16 (the operand of the fp16 dW contraction).  SRC: float or __half.
+// scale = max|x| / 127; there are 32 streams of uniform numbers, stream h for the elements h, h + 32, h + 64, ... in that
+// order, each a linear congruential generator seeded with (bits of x[h], bits of x[0], row); q = round to nearest even,
+// saturating, of x / scale + u - 0.5.  x = src * mult, mult a power of two (so the scaling is exact).  Optionally also writes
+// x as fp16 (the operand of the fp16 dW contraction).  SRC: float or __half.
+// A lane takes runs of eight consecutive elements (16-byte accesses): run lane + 32 m lies in the streams 8 (lane % 4) .. + 7,
+// at their steps lane / 4 + 8 m, so it carries eight generators that advance eight steps at a time.  The second pass
+// reads the row again, from L1 or L2.  A lane per stream with 4-byte accesses was bound by their number: 16384 rows of 4096 and
+// 2048 fp16 values 58 -> 40 us on average, of 512 floats 15.6 -> 13.8.
 struct RowQuantLCG {
-    uint32_t state;
-    __device__ RowQuantLCG(uint32_t a, uint32_t b, uint32_t c) { state = a * 0x398bf183u + b * 0x1affc3dfu + c * 0x9023a049u; }
-    __device__ float uniform()
-    {
-        state = state * 0x448e3079u + 0xc484ef10u;
-        return (float)state * (1.0f / 4294967296.0f);
-    }
+    static constexpr uint32_t A = 0x448e3079u, C = 0xc484ef10u;
+    // eight steps at once: state -> A8 state + C8
+    static constexpr uint32_t A2 = A * A, C2 = A * C + C, A4 = A2 * A2, C4 = A2 * C2 + C2, A8 = A4 * A4, C8 = A4 * C4 + C4;
+    static __device__ __forceinline__ uint32_t seed(uint32_t a, uint32_t b, uint32_t c) { return a * 0x398bf183u + b * 0x1affc3dfu + c * 0x9023a049u; }
+    static __device__ __forceinline__ float uniform(uint32_t state) { return (float)state * (1.0f / 4294967296.0f); }
 };
 
-template <typename SRC>
-__device__ __forceinline__ float rq_load(const SRC *p, size_t i);
-template <>
-__device__ __forceinline__ float rq_load<float>(const float *p, size_t i)
+// eight consecutive elements times mult (a power of two); VEC: the array is 16-byte aligned
+template <bool VEC>
+__device__ __forceinline__ void rq_load8(const float *p, float mult, float (&f)[8])
 {
-    return p[i];
+    if (!VEC) { // a caller's array may start at any float
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            f[i] = p[i] * mult;
+        return;
+    }
+    const float4 a = scale4(*(const float4 *)p, mult), b = scale4(*(const float4 *)(p + 4), mult);
+    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
 }
-template <>
-__device__ __forceinline__ float rq_load<__half>(const __half *p, size_t i)
+template <bool VEC>
+__device__ __forceinline__ void rq_load8(const __half *p, float mult, float (&f)[8])
 {
-    return __half2float(p[i]);
+    half8_to_float(*(const uint4 *)p, f);
+    scale8(f, mult);
 }
 
-template <typename SRC>
-__global__ void rowquant_i8_kernel(const SRC *__restrict__ src, int T, int D, const unsigned *__restrict__ absmax, float target,
+template <typename SRC, bool VEC>
+__global__ void __launch_bounds__(THREADS) rowquant_i8_kernel(const SRC *__restrict__ src, int T, int D, const unsigned *__restrict__ absmax, float target,
                                    int8_t *__restrict__ q, float *__restrict__ row_scale, __half *__restrict__ x16,
                                    float *__restrict__ ginv, float f_static, const float *__restrict__ sko, float *__restrict__ fscale)
 {
     grid_dep_wait();
-    extern __shared__ int8_t rq_rows[]; // [WARPS][D]
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, runs = D / 8;
     const float mult = absmax ? grad_mult(*absmax, target) : 1.f;
     if (blockIdx.x == 0 && threadIdx.x == 0 && ginv) {
         *ginv = 1.f / mult;
         if (fscale)
             *fscale = f_static * (sko ? *sko : 1.f) / mult;
     }
-    int8_t *row_s = rq_rows + (size_t)wid * D;
     for (int t = blockIdx.x * WARPS + wid; t < T; t += gridDim.x * WARPS) {
         const SRC *row = src + (size_t)t * D;
-        float mx = 0.f;
-        for (int d = lane; d < D; d += 32)
-            mx = fmaxf(mx, fabsf(rq_load<SRC>(row, d) * mult));
-        mx = warp_max(mx);
-        float scale = 0.f;
-        if (mx > 0.f) {
-            scale = mx / 127;
-            const float inv = 1 / scale;
-            RowQuantLCG rng(__float_as_uint(rq_load<SRC>(row, lane) * mult), __float_as_uint(rq_load<SRC>(row, 0) * mult), (uint32_t)t);
-            for (int d = lane; d < D; d += 32) {
-                const float x = rq_load<SRC>(row, d) * mult;
-                row_s[d] = (int8_t)sat_i8(__fsub_rn(__fmaf_rn(x, inv, rng.uniform()), 0.5f));
-                if (x16)
-                    x16[(size_t)t * D + d] = __float2half_rn(x);
-            }
-        } else {
-            for (int d = lane; d < D; d += 32) {
-                row_s[d] = 0;
-                if (x16)
-                    x16[(size_t)t * D + d] = __float2half_rn(0.f);
-            }
+        float first[8], mx = 0.f;
+        rq_load8<VEC>(row + (lane & 3) * 8, mult, first); // the seeds of this lane's streams
+        for (int run = lane; run < runs; run += 32) {
+            float f[8];
+            rq_load8<VEC>(row + (size_t)run * 8, mult, f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                mx = fmaxf(mx, fabsf(f[i]));
         }
-        __syncwarp();
-        for (int i = lane; i < D / 16; i += 32)
-            *(uint4 *)(q + (size_t)t * D + 16 * i) = *(const uint4 *)(row_s + 16 * i);
+        mx = warp_max(mx);
+        const float scale = mx > 0.f ? mx / 127 : 0.f, inv = mx > 0.f ? 1 / scale : 0.f;
+        const uint32_t x0 = __shfl_sync(0xffffffffu, __float_as_uint(first[0]), 0);
+        uint32_t state[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            state[i] = RowQuantLCG::seed(__float_as_uint(first[i]), x0, (uint32_t)t);
+        for (int j = 0; j <= lane >> 2; ++j) // to this lane's first step
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                state[i] = state[i] * RowQuantLCG::A + RowQuantLCG::C;
+        for (int run = lane; run < runs; run += 32) {
+            const size_t at = (size_t)t * D + (size_t)run * 8;
+            float f[8];
+            rq_load8<VEC>(row + (size_t)run * 8, mult, f);
+            uint32_t w[2] = {0u, 0u};
+            if (mx > 0.f) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    w[i >> 2] |= sat_i8(__fsub_rn(__fmaf_rn(f[i], inv, RowQuantLCG::uniform(state[i])), 0.5f)) << (8 * (i & 3));
+            }
+            *(uint2 *)(q + at) = make_uint2(w[0], w[1]);
+            if (x16) {
+                __half2 h[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    h[i] = __floats2half2_rn(mx > 0.f ? f[2 * i] : 0.f, mx > 0.f ? f[2 * i + 1] : 0.f);
+                *(uint4 *)(x16 + at) = *(const uint4 *)h;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                state[i] = state[i] * RowQuantLCG::A8 + RowQuantLCG::C8;
+        }
         if (lane == 0)
             row_scale[t] = scale;
-        __syncwarp();
     }
 }
 
@@ -334,16 +342,8 @@ static int rowquant_launch(const Ctx &c, const SRC *src, int T, int D, const uns
 {
     if (D % 128 || D > 16384)
         return fail(TS2_ERR_INVALID_ARG, "rowquant: row length %d must be a multiple of 128 up to 16384", D);
-    auto kern = rowquant_i8_kernel<SRC>;
-    const size_t smem = (size_t)WARPS * D;
-    static bool configured[16] = {};
-    if (smem > 48 * 1024 && !configured[c.device & 15]) {
-        TS2_CUDA(cudaFuncSetAttribute(rowquant_i8_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, WARPS * 16384));
-        TS2_CUDA(cudaFuncSetAttribute(rowquant_i8_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, WARPS * 16384));
-        configured[c.device & 15] = true;
-    }
-    const int grid = (int)std::max<long long>(1, std::min<long long>(ceil_div(T, WARPS), (long long)sm_count(c.device) * 4));
-    TS2_LAUNCH((kern), grid, THREADS, smem, c.stream, src, T, D, absmax, 128.f, q, row_scale, x16, ginv, f_static, sko, fscale);
+    auto kern = ((uintptr_t)src & 15) ? rowquant_i8_kernel<SRC, false> : rowquant_i8_kernel<SRC, true>;
+    TS2_LAUNCH((kern), grid_for(c, kern, T), THREADS, 0, c.stream, src, T, D, absmax, 128.f, q, row_scale, x16, ginv, f_static, sko, fscale);
     return TS2_OK;
 }
 
