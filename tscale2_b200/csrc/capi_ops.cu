@@ -419,10 +419,15 @@ int ts2_attention_forward(int device, void *stream, int variant, const void *q, 
     Ctx c;
     c.device = device;
     c.stream = (cudaStream_t)stream;
-    SpanScratch spans(c, span_start, span_finish, T, 2 * (size_t)T);
+    SpanScratch spans(c, span_start, span_finish, T, 2 * (size_t)T + 2);
     if (spans.rc != TS2_OK)
         return spans.rc;
     int *d = spans.d;
+    if (variant == 2 && attention_forward_takes_pairs(device, span_start, span_finish, T, head_count, alibi_slope)) {
+        TS2_CUDA(cudaMemsetAsync(d + 2 * (size_t)T, 0, 8, c.stream));
+        return attention_forward_pair_tc(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count, alibi_slope,
+                                         (__half *)o, lse, d + 2 * (size_t)T);
+    }
     int rc = variant == 2 ? attention_forward_tc(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,
                                                  alibi_slope, (__half *)o, lse)
              : variant == 0 ? attention_forward_mma(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,
