@@ -251,15 +251,19 @@ struct CopyJob {
     long long ld_src, ld, ldT;
     int x, y, kind;
     int tile0, tiles_x; // first tile of the job among all jobs' tiles
+    // with w (fp32 [y][x]): the block is quantized (qkind as in OptSeg) by its matrix's scale and also written to q, pitch ld_src
+    const float *w = nullptr, *sko = nullptr;
+    uint8_t *q = nullptr;
+    int qkind = 0;
 };
 int qcopy_tiles(CopyJob &job); // fills tiles_x, returns the number of tiles
-int qcopy(const Ctx &c, const CopyJob *jobs, int n_jobs, int tiles);
 enum { SCALES_ATT = 0, SCALES_FFN = 1, SCALES_MOE = 2 };
 struct ScaleJob {
     float *fwd_col, *bwd_row;
     const float *skos;
     int W, ncat, kind;
 };
-int layer_scales(const Ctx &c, const ScaleJob *jobs, int n_jobs, float a);
+// all copies and scale vectors of a model in one launch
+int qcopy(const Ctx &c, const CopyJob *jobs, int n_jobs, int tiles, const ScaleJob *scales, int n_scales, float a);
 
 } // namespace ts2

@@ -194,6 +194,21 @@ __global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__
     }
 }
 
+// four weights in operand format KIND (OptSeg::qkind), as one word, or two for fp16 (first: the lower pair)
+__device__ __forceinline__ uint2 quantize4(float4 v, int kind)
+{
+    if (kind == 2) // int8: nearest even, saturating (PackFloatToInt8, src/gpt/model_params/sse_utils.h:56-78)
+        return make_uint2(sat_i8(v.x) | (sat_i8(v.y) << 8) | (sat_i8(v.z) << 16) | (sat_i8(v.w) << 24), 0u);
+    if (kind == 0)
+        return make_uint2((uint32_t)encode_e4m3_weight(v.x) | ((uint32_t)encode_e4m3_weight(v.y) << 8) | ((uint32_t)encode_e4m3_weight(v.z) << 16) |
+                              ((uint32_t)encode_e4m3_weight(v.w) << 24),
+                          0u);
+    const __half h0 = __float2half_rn(v.x), h1 = __float2half_rn(v.y), h2 = __float2half_rn(v.z), h3 = __float2half_rn(v.w);
+    return make_uint2((uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
+                      (uint32_t)__half_as_ushort(h2) | ((uint32_t)__half_as_ushort(h3) << 16));
+}
+__device__ __forceinline__ float quant_mult(float sko) { return sko == 0.f ? 0.f : 1.f / (sko * (1.f / 32)); }
+
 // ConvertMatrixKernel on the rows of the range: q = enc(w * 32 / sko) into the matrix's row-major quantized copy
 __global__ void opt_quant_kernel(const OptSeg *__restrict__ segs, int nseg, int nitems, const float *__restrict__ w,
                                  const float *__restrict__ skos)
@@ -206,24 +221,15 @@ __global__ void opt_quant_kernel(const OptSeg *__restrict__ segs, int nseg, int 
         long long base;
         int c0, c1;
         seg_row_cols(sg, r, base, c0, c1);
-        const float sko = skos[sg.mat];
-        const float mult = (sko == 0.f) ? 0.f : (1.f / (sko * (1.f / 32)));
+        const float mult = quant_mult(skos[sg.mat]);
         const float4 *src = (const float4 *)(w + base);
         uint8_t *dst = sg.qbase + (size_t)r * sg.x * sg.qsize;
         for (int i = c0 / 4 + lane; i < c1 / 4; i += 32) {
-            const float4 v = scale4(src[i], mult);
-            if (sg.qkind == 2) { // int8: nearest even, saturating (PackFloatToInt8, src/gpt/model_params/sse_utils.h:56-78)
-                *(uint32_t *)(dst + 4 * (size_t)i) = sat_i8(v.x) | (sat_i8(v.y) << 8) | (sat_i8(v.z) << 16) | (sat_i8(v.w) << 24);
-            } else if (sg.qkind == 0) {
-                const uint32_t pk = (uint32_t)encode_e4m3_weight(v.x) | ((uint32_t)encode_e4m3_weight(v.y) << 8) |
-                                    ((uint32_t)encode_e4m3_weight(v.z) << 16) | ((uint32_t)encode_e4m3_weight(v.w) << 24);
-                *(uint32_t *)(dst + 4 * (size_t)i) = pk;
-            } else {
-                const __half h0 = __float2half_rn(v.x), h1 = __float2half_rn(v.y), h2 = __float2half_rn(v.z), h3 = __float2half_rn(v.w);
-                *(uint2 *)(dst + 8 * (size_t)i) =
-                    make_uint2((uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
-                               (uint32_t)__half_as_ushort(h2) | ((uint32_t)__half_as_ushort(h3) << 16));
-            }
+            const uint2 q = quantize4(scale4(src[i], mult), sg.qkind);
+            if (sg.qkind == 1)
+                *(uint2 *)(dst + 8 * (size_t)i) = q;
+            else
+                *(uint32_t *)(dst + 4 * (size_t)i) = q.x;
         }
     }
 }
@@ -275,8 +281,9 @@ int opt_quantize(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const f
     return TS2_OK;
 }
 
-// Copies of already quantized blocks into another row-major place and / or their transpose, all of a model's in one
-// launch.  A tile is 128 bytes of 128 rows (64 rows of 2-byte values): it comes in as 16-byte vectors, lies in shared
+// Copies of quantized blocks into another row-major place and / or their transpose, all of a model's in one launch, from
+// the quantized values, or (CopyJob::w) from the weights themselves, which are quantized on the way: one launch and one pass
+// less where this rank holds whole matrices (124 M parameters 350 + 155 -> 494 us, 437 M 642 + 350 -> 947).  A tile is 128 bytes of 128 rows (64 rows of 2-byte values): it comes in as 16-byte vectors, lies in shared
 // memory with its 16-byte pieces rotated by the row group (so that both the vector writes and the word reads of eight
 // row groups are free of bank conflicts), is transposed in registers by byte permutes and leaves in 16-byte vectors.
 // Bound by its bytes (read once, written once or twice): 4 transposes of [16384 x 2048] bytes and their like took 52 us
@@ -302,12 +309,38 @@ __device__ __forceinline__ uint2 widen4(uint32_t w, int kind)
     return make_uint2((uint32_t)a.x | (uint32_t)a.y << 16, (uint32_t)b.x | (uint32_t)b.y << 16);
 }
 
-__global__ void __launch_bounds__(256) qcopy_kernel(const CopyJob *__restrict__ jobs, int n_jobs, int tiles)
+// The scale vectors of every layer from its matrices' scales (skos, in matrix order): forward column scales a (x sko_k for
+// the K block of an attention layer), dW row scales 1 / sko for the matrices that are followed by a normalisation (Q, K,
+// V; Expand), 1 elsewhere.  An expert layer has no K block and one row vector, for Expand.
+constexpr int SCALE_BLOCKS = 8; // per layer
+__device__ __forceinline__ void layer_scales(const ScaleJob &jb, float a, int block)
+{
+    const bool att = jb.kind == SCALES_ATT;
+    for (int i = block * blockDim.x + threadIdx.x; i < jb.ncat * jb.W; i += SCALE_BLOCKS * blockDim.x) {
+        const int j = i / jb.W;
+        jb.fwd_col[i] = (att && j == 1) ? a * jb.skos[1] : a;
+        if (jb.kind == SCALES_MOE) {
+            if (j == 0)
+                jb.bwd_row[i] = 1.f / jb.skos[0];
+            continue;
+        }
+        jb.bwd_row[i] = (att ? j < 3 : j == 0) ? 1.f / jb.skos[j] : 1.f;
+    }
+}
+
+// copies, and in the blocks from `blocks` on the scale vectors
+__global__ void __launch_bounds__(256) qcopy_kernel(const CopyJob *__restrict__ jobs, int n_jobs, int tiles, int blocks,
+                                                    const ScaleJob *__restrict__ scales, float a)
 {
     grid_dep_wait();
     __shared__ uint4 tile_s[128 * 8];
     const int tid = threadIdx.x;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    if ((int)blockIdx.x >= blocks) {
+        const int i = (int)blockIdx.x - blocks;
+        layer_scales(scales[i / SCALE_BLOCKS], a, i % SCALE_BLOCKS);
+        return;
+    }
+    for (int tile = blockIdx.x; tile < tiles; tile += blocks) {
         int lo = 0, hi = n_jobs - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -320,15 +353,52 @@ __global__ void __launch_bounds__(256) qcopy_kernel(const CopyJob *__restrict__ 
         const int two = jb.kind == QCOPY_2BYTE, rows = two ? 64 : 128, shift = two ? 3 : 4;
         const int t = tile - jb.tile0, tx = t % jb.tiles_x, y0 = (t / jb.tiles_x) * rows;
         const long long xb = (long long)tx * 128; // byte offset of the tile in a source row
-        for (int v = tid; v < rows * 8; v += 256) {
-            const int r = v >> 3, c = v & 7;
-            uint4 q = make_uint4(0, 0, 0, 0);
-            if (y0 + r < jb.y) {
-                q = *(const uint4 *)(jb.src + (y0 + r) * jb.ld_src + xb + c * 16);
-                if (jb.dst)
-                    *(uint4 *)(jb.dst + (y0 + r) * jb.ld + xb + c * 16) = q;
+        if (jb.w) {
+            // straight from the weights: a warp (two-byte values: half a warp) takes the 128 (64) columns of a row, four a lane
+            const float mult = quant_mult(*jb.sko);
+            const int per = two ? 16 : 32, sub = tid % per, step = 256 / per, es = two ? 2 : 1;
+            constexpr int AHEAD = 4;
+            for (int r0 = tid / per; r0 < rows; r0 += AHEAD * step) {
+                float4 f[AHEAD];
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int r = r0 + u * step;
+                    f[u] = r < rows && y0 + r < jb.y ? *(const float4 *)(jb.w + (long long)(y0 + r) * jb.x + xb / es + sub * 4) : make_float4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int r = r0 + u * step;
+                    if (r >= rows)
+                        break;
+                    const uint2 q = quantize4(scale4(f[u], mult), jb.qkind);
+                    uint8_t *const s = (uint8_t *)tile_s + (r * 8 + ((two ? sub >> 1 : sub >> 2) ^ ((r >> shift) & 7))) * 16;
+                    const bool in = y0 + r < jb.y;
+                    if (two) {
+                        *(uint2 *)(s + (sub & 1) * 8) = q;
+                        if (in)
+                            *(uint2 *)(jb.q + (y0 + r) * jb.ld_src + xb + sub * 8) = q;
+                        if (in && jb.dst)
+                            *(uint2 *)(jb.dst + (y0 + r) * jb.ld + xb + sub * 8) = q;
+                    } else {
+                        *(uint32_t *)(s + (sub & 3) * 4) = q.x;
+                        if (in)
+                            *(uint32_t *)(jb.q + (y0 + r) * jb.ld_src + xb + sub * 4) = q.x;
+                        if (in && jb.dst)
+                            *(uint32_t *)(jb.dst + (y0 + r) * jb.ld + xb + sub * 4) = q.x;
+                    }
+                }
             }
-            tile_s[r * 8 + (c ^ ((r >> shift) & 7))] = q;
+        } else {
+            for (int v = tid; v < rows * 8; v += 256) {
+                const int r = v >> 3, c = v & 7;
+                uint4 q = make_uint4(0, 0, 0, 0);
+                if (y0 + r < jb.y) {
+                    q = *(const uint4 *)(jb.src + (y0 + r) * jb.ld_src + xb + c * 16);
+                    if (jb.dst)
+                        *(uint4 *)(jb.dst + (y0 + r) * jb.ld + xb + c * 16) = q;
+                }
+                tile_s[r * 8 + (c ^ ((r >> shift) & 7))] = q;
+            }
         }
         if (jb.dstT) { // the same for the whole block
             __syncthreads();
@@ -409,37 +479,11 @@ int qcopy_tiles(CopyJob &job)
     return job.tiles_x * (int)ceil_div(job.y, es == 2 ? 64 : 128);
 }
 
-int qcopy(const Ctx &c, const CopyJob *jobs, int n_jobs, int tiles)
+int qcopy(const Ctx &c, const CopyJob *jobs, int n_jobs, int tiles, const ScaleJob *scales, int n_scales, float a)
 {
-    if (tiles > 0)
-        TS2_LAUNCH((qcopy_kernel), std::min(tiles, sm_count(c.device) * 8), 256, 0, c.stream, jobs, n_jobs, tiles);
-    return TS2_OK;
-}
-
-// The scale vectors of every layer from its matrices' scales (skos, in matrix order): forward column scales a (x sko_k for
-// the K block of an attention layer), dW row scales 1 / sko for the matrices that are followed by a normalisation (Q, K,
-// V; Expand), 1 elsewhere.  An expert layer has no K block and one row vector, for Expand.  blockIdx.y = layer.
-__global__ void layer_scales_kernel(const ScaleJob *__restrict__ jobs, float a)
-{
-    grid_dep_wait();
-    const ScaleJob jb = jobs[blockIdx.y];
-    const bool att = jb.kind == SCALES_ATT;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < jb.ncat * jb.W; i += gridDim.x * blockDim.x) {
-        const int j = i / jb.W;
-        jb.fwd_col[i] = (att && j == 1) ? a * jb.skos[1] : a;
-        if (jb.kind == SCALES_MOE) {
-            if (j == 0)
-                jb.bwd_row[i] = 1.f / jb.skos[0];
-            continue;
-        }
-        jb.bwd_row[i] = (att ? j < 3 : j == 0) ? 1.f / jb.skos[j] : 1.f;
-    }
-}
-
-int layer_scales(const Ctx &c, const ScaleJob *jobs, int n_jobs, float a)
-{
-    if (n_jobs > 0)
-        TS2_LAUNCH((layer_scales_kernel), dim3(8, n_jobs), 256, 0, c.stream, jobs, a);
+    const int blocks = std::min(tiles, sm_count(c.device) * 8);
+    if (blocks + n_scales > 0)
+        TS2_LAUNCH((qcopy_kernel), blocks + n_scales * SCALE_BLOCKS, 256, 0, c.stream, jobs, n_jobs, tiles, blocks, scales, a);
     return TS2_OK;
 }
 

@@ -150,9 +150,9 @@ struct ts2_model {
     OptMat *d_optmats = nullptr;
     OptSeg *d_segs_full = nullptr, *d_segs_shard = nullptr;
     int nseg_full = 0, nitems_full = 0, nseg_shard = 0, nitems_shard = 0;
-    CopyJob *d_copies = nullptr; // what post_quantize does
+    CopyJob *d_copies = nullptr, *d_quants = nullptr; // what post_quantize and quantize_all do
     ScaleJob *d_scales = nullptr;
-    int n_copies = 0, copy_tiles = 0, n_scales = 0;
+    int n_copies = 0, copy_tiles = 0, n_quants = 0, quant_tiles = 0, n_scales = 0;
     bool master_stale = false; // data parallel: the fp32 weights / momentum outside this rank's parts are out of date
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr, ev_grads = nullptr, ev_reduced = nullptr, ev_t0 = nullptr, ev_t1 = nullptr;
     std::string error;
@@ -803,27 +803,49 @@ int ep_exchange(ts2_model *m, const Layer &ly, bool to_owner, void *own, void *x
     return TS2_OK;
 }
 
-// the copies and scale vectors that post_quantize makes, as tables on the device (built once: no pointer in them moves)
+// the copies and scale vectors that post_quantize makes, as tables on the device (built once: no pointer in them moves), and
+// the same for quantize_all
 int build_post_quantize(ts2_model *m)
 {
     const int D = m->D;
     const size_t fs = fast_size(m);
-    std::vector<CopyJob> copies;
+    std::vector<CopyJob> copies, quants;
     std::vector<ScaleJob> scales;
-    m->copy_tiles = 0;
-    auto add = [&](const void *src, int64_t x, int64_t y, int64_t ld_src, void *dst, int64_t ld, void *dstT, int64_t ldT, int kind) {
+    m->copy_tiles = m->quant_tiles = 0;
+    auto job = [&](const void *src, int64_t x, int64_t y, int64_t ld_src, void *dst, int64_t ld, void *dstT, int64_t ldT, int kind, size_t es) {
         const bool wide = kind == QCOPY_E4M3_HALF || kind == QCOPY_I8_HALF;
         CopyJob j;
         j.src = (const uint8_t *)src, j.dst = (uint8_t *)dst, j.dstT = (uint8_t *)dstT;
-        j.ld_src = ld_src * fs, j.ld = ld * fs, j.ldT = ldT * (wide ? 2 : fs);
+        j.ld_src = ld_src * es, j.ld = ld * es, j.ldT = ldT * (wide ? 2 : es);
         j.x = (int)x, j.y = (int)y, j.kind = kind;
+        return j;
+    };
+    auto add = [&](const void *src, int64_t x, int64_t y, int64_t ld_src, void *dst, int64_t ld, void *dstT, int64_t ldT, int kind) {
+        CopyJob j = job(src, x, y, ld_src, dst, ld, dstT, ldT, kind, fs);
         j.tile0 = m->copy_tiles;
         m->copy_tiles += qcopy_tiles(j);
         copies.push_back(j);
     };
+    // rows [r0, r0 + y) of a matrix, quantized into its row-major copy and on to dst, dstT
+    auto quant = [&](int mat, int64_t r0, int64_t y, void *dst, void *dstT, int64_t ldT, int kind) {
+        const Matrix &mt = m->mats[mat];
+        const Bucket &bk = m->buckets[m->mat_bucket[mat]];
+        uint8_t *q = bk.qflat + (mt.offset - bk.off + r0 * mt.x) * bk.qsize;
+        CopyJob j = job(q, mt.x, y, mt.x, dst, mt.x, dstT, ldT, kind, bk.qsize);
+        j.w = mt.w + r0 * mt.x;
+        j.sko = mt.sko;
+        j.q = q;
+        j.qkind = bk.qsize == 2 ? 1 : (m->ft == 2 ? 2 : 0);
+        j.tile0 = m->quant_tiles;
+        m->quant_tiles += qcopy_tiles(j);
+        quants.push_back(j);
+    };
     const int plain = fs == 2 ? QCOPY_2BYTE : QCOPY_1BYTE;
     // final layer: fp16 transposed copy of the same quantized values for the dX contraction
-    add(m->Wf, D, m->V, D, nullptr, 0, m->WfT16, m->V, m->ft == 0 ? QCOPY_E4M3_HALF : m->ft == 2 ? QCOPY_I8_HALF : QCOPY_2BYTE);
+    const int final_kind = m->ft == 0 ? QCOPY_E4M3_HALF : m->ft == 2 ? QCOPY_I8_HALF : QCOPY_2BYTE;
+    add(m->Wf, D, m->V, D, nullptr, 0, m->WfT16, m->V, final_kind);
+    quant(0, 0, m->mats[0].y, nullptr, nullptr, 0, QCOPY_2BYTE);
+    quant(1, 0, m->V, nullptr, m->WfT16, m->V, final_kind);
     for (Layer &ly : m->layers) {
         const int W = ly.wide, n = ly.ncat;
         auto qsrc = [&](int mat) {
@@ -836,24 +858,34 @@ int build_post_quantize(ts2_model *m)
             const int E = m->E, X = m->X;
             for (int e = 0; e < E; ++e) {
                 uint8_t *cat = (uint8_t *)ly.Wcat + (size_t)e * 2 * X * D * fs, *catT = (uint8_t *)ly.WcatT + (size_t)e * D * 2 * X * fs;
+                uint8_t *con = (uint8_t *)ly.Wc + (size_t)e * D * X * fs, *conT = (uint8_t *)ly.WcT + (size_t)e * X * D * fs;
                 add(qsrc(ly.mat0) + (size_t)e * X * D * fs, D, X, D, cat, D, catT, 2 * X, plain);
                 add(qsrc(ly.mat0 + 1) + (size_t)e * X * D * fs, D, X, D, cat + (size_t)X * D * fs, D, catT + (size_t)X * fs, 2 * X, plain);
-                add(qsrc(ly.mat0 + 2) + (size_t)e * D * X * fs, X, D, X, (uint8_t *)ly.Wc + (size_t)e * D * X * fs, X,
-                    (uint8_t *)ly.WcT + (size_t)e * X * D * fs, D, plain);
+                add(qsrc(ly.mat0 + 2) + (size_t)e * D * X * fs, X, D, X, con, X, conT, D, plain);
+                quant(ly.mat0, (int64_t)e * X, X, cat, catT, 2 * X, plain);
+                quant(ly.mat0 + 1, (int64_t)e * X, X, cat + (size_t)X * D * fs, catT + (size_t)X * fs, 2 * X, plain);
+                quant(ly.mat0 + 2, (int64_t)e * D, D, con, conT, D, plain);
             }
             add(qsrc(ly.mat0 + 3), D, E, D, ly.Wsel, D, ly.WselT, m->epad, plain);
+            quant(ly.mat0 + 3, 0, E, ly.Wsel, ly.WselT, m->epad, plain);
             scales.push_back({ly.fwd_col, ly.bwd_row_e, m->skos + ly.mat0, X, 2, SCALES_MOE});
             continue;
         }
         // the concatenated block [n W][D] transposes in one pass: its row blocks become the column blocks of WcatT
         add(ly.Wcat, D, (int64_t)n * W, D, nullptr, 0, ly.WcatT, (int64_t)n * W, plain);
         add(ly.Wc, W, D, W, nullptr, 0, ly.WcT, D, plain);
+        for (int j = 0; j < n; ++j)
+            quant(ly.mat0 + j, 0, W, nullptr, (uint8_t *)ly.WcatT + (size_t)j * W * fs, (int64_t)n * W, plain);
+        quant(ly.mat0 + n, 0, D, nullptr, ly.WcT, D, plain);
         // forward column scales: matrices followed by a normalisation (Q, V, Expand) and the gates use the unit-RMS
         // matrix q/32 (GetDataNoScale), K carries its matrix scale; dW rows of Q, K, V / Expand are divided by theirs
         scales.push_back({ly.fwd_col, ly.bwd_row, m->skos + ly.mat0, W, n, ly.type == TS2_LAYER_ATT ? SCALES_ATT : SCALES_FFN});
     }
     m->n_copies = (int)copies.size();
+    m->n_quants = (int)quants.size();
     m->n_scales = (int)scales.size();
+    M_TRY(dalloc(m, &m->d_quants, quants.size()));
+    TS2_CUDA(cudaMemcpyAsync(m->d_quants, quants.data(), quants.size() * sizeof(CopyJob), cudaMemcpyHostToDevice, m->stream));
     M_TRY(dalloc(m, &m->d_copies, copies.size()));
     M_TRY(dalloc(m, &m->d_scales, scales.size() + 1));
     TS2_CUDA(cudaMemcpyAsync(m->d_copies, copies.data(), copies.size() * sizeof(CopyJob), cudaMemcpyHostToDevice, m->stream));
@@ -865,10 +897,12 @@ int build_post_quantize(ts2_model *m)
 // transposed copies, per-expert layouts and scale vectors from the row-major quantized matrices and their scales
 int post_quantize(ts2_model *m)
 {
-    Ctx c = ctx_of(m);
-    M_TRY(qcopy(c, m->d_copies, m->n_copies, m->copy_tiles));
-    M_TRY(layer_scales(c, m->d_scales, m->n_scales, sqrtf(1.0f / m->D) / (m->s_act * 32.f)));
-    return TS2_OK;
+    return qcopy(ctx_of(m), m->d_copies, m->n_copies, m->copy_tiles, m->d_scales, m->n_scales, sqrtf(1.0f / m->D) / (m->s_act * 32.f));
+}
+// the same and the quantized matrices themselves from the weights (a rank that holds all of them)
+int quantize_all(ts2_model *m)
+{
+    return qcopy(ctx_of(m), m->d_quants, m->n_quants, m->quant_tiles, m->d_scales, m->n_scales, sqrtf(1.0f / m->D) / (m->s_act * 32.f));
 }
 
 // Requantisation of the whole model on this rank alone (creation, ts2_set_params): matrix scales, quantized copies
@@ -877,9 +911,7 @@ int requantize_all(ts2_model *m)
     Ctx c = ctx_of(m);
     M_TRY(opt_update(c, m->d_segs_full, m->nseg_full, m->nitems_full, nullptr, nullptr, nullptr, nullptr, m->w_flat, m->roww2));
     M_TRY(opt_sko(c, m->d_optmats, (int)m->mats.size(), m->roww2, m->skos, -1.f));
-    M_TRY(opt_quantize(c, m->d_segs_full, m->nseg_full, m->nitems_full, m->w_flat, m->skos));
-    M_TRY(post_quantize(m));
-    return TS2_OK;
+    return quantize_all(m);
 }
 
 int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const float *bias)
@@ -1737,6 +1769,8 @@ int apply(ts2_model *m, const ts2_training_step *step)
     if (dp)
         M_NCCL(ncclAllReduce(m->roww2, m->roww2, (size_t)m->n_rows_total, ncclDouble, ncclSum, m->comm, m->stream));
     M_TRY(opt_sko(c, m->d_optmats, n_mats, m->roww2, m->skos, step->disp_decay));
+    if (!dp)
+        return quantize_all(m);
     M_TRY(opt_quantize(c, m->d_segs_shard, m->nseg_shard, m->nitems_shard, m->w_flat, m->skos));
     if (dp) {
         M_NCCL(ncclGroupStart());
