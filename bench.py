@@ -420,7 +420,7 @@ def main():
     for i in range(args.steps):
         model.set_batch(batches[i % len(batches)])
         model.backprop(train_step, apply=True)
-        loss = model.avg_train_err()  # device -> host read, waits for the step
+        loss = model.avg_train_err()  # device -> host read, waits for the forward pass
         e2e_losses.append(loss)
     e2e_ms = model.timer_end()
     barrier()

@@ -193,14 +193,17 @@ int ts2_wait(ts2_model *m);
 int ts2_set_wait_limit(ts2_model *m, double seconds);
 /* IModelInstance::ComputeScore, src/gpt/compute/model.h:39: mean log p(target) (natural log) */
 int ts2_forward_score(ts2_model *m, float *out_score);
-/* IModel::GetAvrgTrainErr, src/gpt/compute/model.h:55: mean -log p(target) of the last backprop */
+/* IModel::GetAvrgTrainErr, src/gpt/compute/model.h:55: mean -log p(target) of the last backprop.
+ * Waits for its forward pass; the backward pass and the update may still be running (ts2_wait waits for those, and reports what
+ * goes wrong in them, as does every later call that waits). */
 int ts2_avg_train_err(ts2_model *m, float *out_err);
 
 /* IModel::GetParams / SetParams, src/gpt/compute/model.h:48-49.  what selects
  * the per-matrix tensor: master weights, momentum (Grad1), or the raw fp32
  * weight gradient of the last ts2_backprop (the tap the parity tests read:
  * the tensor the reference hands to HostApplyDelta,
- * src/gpt/compute/cpu_util.h:86-95). */
+ * src/gpt/compute/cpu_util.h:86-95).  The values are those after everything queued before; weights and momentum of a large
+ * model leave matrix by matrix as the running step updates them. */
 #define TS2_PARAM_WEIGHTS 0
 #define TS2_PARAM_MOMENTUM 1
 #define TS2_PARAM_GRADIENT 2

@@ -235,10 +235,10 @@ struct OptMat {
     int row_disp_size, grow0;
     float *row_disp, *sum_weight;
 };
-int opt_row_sum2(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const float *grad, float *rowsum);
+int opt_row_sum2(const Ctx &c, const OptSeg *segs, int nseg, int item0, int nitems, const float *grad, float *rowsum);
 int opt_disp(const Ctx &c, const OptMat *mats, int n_mats, const float *rowsum, float disp_decay, float *row_scale);
 // step == nullptr: no update, only the per-row sums of squares of the weights
-int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const float *grad, const float *row_scale,
+int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int item0, int nitems, const float *grad, const float *row_scale,
                const ts2_training_step *step, float *avg, float *w, double *roww2);
 // disp_decay: the step's, or negative when no step was applied
 int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos, float disp_decay);

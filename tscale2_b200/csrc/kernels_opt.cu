@@ -22,6 +22,7 @@ static constexpr int THREADS = WARPS * 32;
 // AddGradientKernel -> ConvertMatrixKernel of the reference (agpu_cuda.cu:32-134, agpu_cuda.cuh:63-101) by five
 // launches per step over everything a rank owns.
 
+// The launches below take a run of segments and the work items [item0, item0 + nitems) they hold.
 // binary search: the segment that holds work item `item`
 __device__ __forceinline__ int find_seg(const OptSeg *__restrict__ segs, int nseg, int item)
 {
@@ -45,12 +46,12 @@ __device__ __forceinline__ void seg_row_cols(const OptSeg &sg, int r, long long 
     base = sg.flat_off + row_begin;
 }
 
-__global__ void opt_row_sum2_kernel(const OptSeg *__restrict__ segs, int nseg, int nitems, const float *__restrict__ grad,
+__global__ void opt_row_sum2_kernel(const OptSeg *__restrict__ segs, int nseg, int item0, int nitems, const float *__restrict__ grad,
                                     float *__restrict__ rowsum)
 {
     grid_dep_wait();
     const int lane = threadIdx.x & 31;
-    for (int item = blockIdx.x * WARPS + (threadIdx.x >> 5); item < nitems; item += gridDim.x * WARPS) {
+    for (int item = item0 + blockIdx.x * WARPS + (threadIdx.x >> 5); item < item0 + nitems; item += gridDim.x * WARPS) {
         const OptSeg sg = segs[find_seg(segs, nseg, item)];
         const int r = sg.row0 + (item - sg.item0);
         long long base;
@@ -119,13 +120,13 @@ __global__ void opt_disp_kernel(const OptMat *__restrict__ mats, const float *__
 
 // AddGradientKernel on the rows of the range (UPDATE) and the sum of squares of the (new) weights per row part
 template <bool UPDATE>
-__global__ void opt_update_kernel(const OptSeg *__restrict__ segs, int nseg, int nitems, const float *__restrict__ grad,
+__global__ void opt_update_kernel(const OptSeg *__restrict__ segs, int nseg, int item0, int nitems, const float *__restrict__ grad,
                                   const float *__restrict__ row_scale, ts2_training_step step, float *__restrict__ avg,
                                   float *__restrict__ w, double *__restrict__ roww2)
 {
     grid_dep_wait();
     const int lane = threadIdx.x & 31;
-    for (int item = blockIdx.x * WARPS + (threadIdx.x >> 5); item < nitems; item += gridDim.x * WARPS) {
+    for (int item = item0 + blockIdx.x * WARPS + (threadIdx.x >> 5); item < item0 + nitems; item += gridDim.x * WARPS) {
         const OptSeg sg = segs[find_seg(segs, nseg, item)];
         const int r = sg.row0 + (item - sg.item0);
         long long base;
@@ -239,11 +240,11 @@ static int opt_grid(const Ctx &c, int nitems)
     return (int)std::max<long long>(1, std::min<long long>(ceil_div(nitems, WARPS), (long long)sm_count(c.device) * 8));
 }
 
-int opt_row_sum2(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const float *grad, float *rowsum)
+int opt_row_sum2(const Ctx &c, const OptSeg *segs, int nseg, int item0, int nitems, const float *grad, float *rowsum)
 {
     if (nitems <= 0)
         return TS2_OK;
-    TS2_LAUNCH((opt_row_sum2_kernel), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, nitems, grad, rowsum);
+    TS2_LAUNCH((opt_row_sum2_kernel), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, item0, nitems, grad, rowsum);
     return TS2_OK;
 }
 
@@ -253,16 +254,16 @@ int opt_disp(const Ctx &c, const OptMat *mats, int n_mats, const float *rowsum, 
     return TS2_OK;
 }
 
-int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const float *grad, const float *row_scale,
+int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int item0, int nitems, const float *grad, const float *row_scale,
                const ts2_training_step *step, float *avg, float *w, double *roww2)
 {
     if (nitems <= 0)
         return TS2_OK;
     if (step)
-        TS2_LAUNCH((opt_update_kernel<true>), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, nitems, grad, row_scale, *step, avg,
+        TS2_LAUNCH((opt_update_kernel<true>), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, item0, nitems, grad, row_scale, *step, avg,
                    w, roww2);
     else
-        TS2_LAUNCH((opt_update_kernel<false>), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, nitems, nullptr, nullptr,
+        TS2_LAUNCH((opt_update_kernel<false>), opt_grid(c, nitems), THREADS, 0, c.stream, segs, nseg, item0, nitems, nullptr, nullptr,
                    ts2_training_step(), nullptr, w, roww2);
     return TS2_OK;
 }

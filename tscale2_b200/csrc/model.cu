@@ -25,6 +25,7 @@
 namespace ts2 {
 const char *global_error();
 
+static constexpr size_t UPDATE_GROUP_ELEMS = (size_t)16 << 20; // see build_update_groups()
 static const float LOG2F = 0.693147f; // LOG2, model_dim.h:16
 
 struct Matrix {
@@ -126,6 +127,12 @@ struct BatchDev {
     int next_slot = 0;
 };
 
+// Matrices [mat0, mat1) that are updated together as soon as the backward pass has their gradients
+struct UpdateGroup {
+    int mat0 = 0, mat1 = 0;
+    cudaEvent_t done = nullptr; // their weights and momentum are those of the last applied step
+};
+
 } // namespace ts2
 
 using namespace ts2;
@@ -150,6 +157,12 @@ struct ts2_model {
     OptMat *d_optmats = nullptr;
     OptSeg *d_segs_full = nullptr, *d_segs_shard = nullptr;
     int nseg_full = 0, nitems_full = 0, nseg_shard = 0, nitems_shard = 0;
+    // One GPU, large models: in the order in which the backward pass completes them.  Small models are updated in one go after
+    // it (empty).
+    std::vector<UpdateGroup> update_groups;
+    const ts2_training_step *step_in_backward = nullptr; // of the ts2_backprop call that is queuing its backward pass, if it applies
+    cudaEvent_t ev_loss = nullptr;      // the training error of the last ts2_backprop is known
+    cudaStream_t read_stream = nullptr; // what is read back while the step goes on
     CopyJob *d_copies = nullptr, *d_quants = nullptr; // what post_quantize and quantize_all do
     ScaleJob *d_scales = nullptr;
     int n_copies = 0, copy_tiles = 0, n_quants = 0, quant_tiles = 0, n_scales = 0;
@@ -369,8 +382,8 @@ Ctx ctx_of(ts2_model *m)
 size_t fast_size(const ts2_model *m) { return m->ft == 1 ? 2 : 1; }
 
 // C = epilogue(A[M][K] . B[N][K]^T), K contiguous in both
-int gemm_tn(ts2_model *m, int kind, int64_t M, int64_t N, int64_t K, const void *A, int64_t lda, const void *B, int64_t ldb, void *C,
-            int64_t ldc, const Epilogue &epi)
+GemmArgs tn_args(ts2_model *m, int kind, int64_t M, int64_t N, int64_t K, const void *A, int64_t lda, const void *B, int64_t ldb, void *C,
+                 int64_t ldc, const Epilogue &epi)
 {
     GemmArgs a;
     a.device = m->device;
@@ -383,25 +396,27 @@ int gemm_tn(ts2_model *m, int kind, int64_t M, int64_t N, int64_t K, const void 
     a.tag = m->gemm_tag;
     a.workspace = m->workspace;
     a.workspace_bytes = m->workspace_bytes;
-    return gemm(a);
+    return a;
+}
+int gemm_tn(ts2_model *m, int kind, int64_t M, int64_t N, int64_t K, const void *A, int64_t lda, const void *B, int64_t ldb, void *C,
+            int64_t ldc, const Epilogue &epi)
+{
+    return gemm(tn_args(m, kind, M, N, K, A, lda, B, ldb, C, ldc, epi));
 }
 
 // dW[Mo][Ni] = epilogue(dY[T][Mo]^T . X[T][Ni]), both token-major
+GemmArgs dw_args(ts2_model *m, int kind, int64_t Mo, int64_t Ni, int64_t T, const void *dY, int64_t ldy, const void *X, int64_t ldx, float *dW,
+                 const Epilogue &epi)
+{
+    GemmArgs a = tn_args(m, kind, Mo, Ni, T, dY, ldy, X, ldx, dW, Ni, epi);
+    a.mn_major = true;
+    a.tag = m->gemm_tag == GEMM_TAG_FINAL ? GEMM_TAG_FINAL : GEMM_TAG_DW;
+    return a;
+}
 int gemm_dw(ts2_model *m, int kind, int64_t Mo, int64_t Ni, int64_t T, const void *dY, int64_t ldy, const void *X, int64_t ldx, float *dW,
             const Epilogue &epi)
 {
-    GemmArgs a;
-    a.device = m->device;
-    a.stream = m->stream;
-    a.kind = kind;
-    a.mn_major = true;
-    a.M = Mo, a.N = Ni, a.K = T;
-    a.A = dY, a.lda = ldy, a.B = X, a.ldb = ldx, a.C = dW, a.ldc = Ni;
-    a.epi = epi;
-    a.tag = m->gemm_tag == GEMM_TAG_FINAL ? GEMM_TAG_FINAL : GEMM_TAG_DW;
-    a.workspace = m->workspace;
-    a.workspace_bytes = m->workspace_bytes;
-    return gemm(a);
+    return gemm(dw_args(m, kind, Mo, Ni, T, dY, ldy, X, ldx, dW, epi));
 }
 
 // rows of A are expert-sorted: every 128-row tile reads the weights of its expert (B has E * N rows)
@@ -909,9 +924,36 @@ int quantize_all(ts2_model *m)
 int requantize_all(ts2_model *m)
 {
     Ctx c = ctx_of(m);
-    M_TRY(opt_update(c, m->d_segs_full, m->nseg_full, m->nitems_full, nullptr, nullptr, nullptr, nullptr, m->w_flat, m->roww2));
+    M_TRY(opt_update(c, m->d_segs_full, m->nseg_full, 0, m->nitems_full, nullptr, nullptr, nullptr, nullptr, m->w_flat, m->roww2));
     M_TRY(opt_sko(c, m->d_optmats, (int)m->mats.size(), m->roww2, m->skos, -1.f));
     return quantize_all(m);
+}
+
+// Final layer, runs of layers from the last one down, embedding.  The weights of a group are final before the layers below it have
+// their gradients, so ts2_get_params copies them meanwhile (dim 2048, 4 blocks, 8 x 4096 tokens: step and export 147 -> 124 ms).
+// A group has at least UPDATE_GROUP_ELEMS elements: its four launches then take 20 us and more.  A model of less than two groups
+// is updated in one go: its export takes 1 ms or less.
+int build_update_groups(ts2_model *m)
+{
+    if (m->flat_elems < 2 * UPDATE_GROUP_ELEMS)
+        return TS2_OK;
+    auto elems = [&](int m0, int m1) { return (m1 < (int)m->mats.size() ? m->mats[m1].offset : m->flat_elems) - m->mats[m0].offset; };
+    auto add = [&](int m0, int m1) {
+        UpdateGroup g;
+        g.mat0 = m0, g.mat1 = m1;
+        m->update_groups.push_back(g);
+    };
+    add(1, 2);
+    int end = (int)m->mats.size();
+    for (int l = m->L - 1; l >= 0; --l)
+        if (l == 0 || elems(m->layers[l].mat0, end) >= UPDATE_GROUP_ELEMS) {
+            add(m->layers[l].mat0, end);
+            end = m->layers[l].mat0;
+        }
+    add(0, 1);
+    for (UpdateGroup &g : m->update_groups)
+        TS2_CUDA(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming));
+    return TS2_OK;
 }
 
 int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const float *bias)
@@ -1220,6 +1262,7 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
         m->nseg_shard = m->nseg_full;
         m->nitems_shard = m->nitems_full;
     }
+    M_TRY(build_update_groups(m));
     M_TRY(build_post_quantize(m));
     M_TRY(requantize_all(m));
     TS2_CUDA(cudaStreamSynchronize(m->stream));
@@ -1442,6 +1485,33 @@ static int reduce_matrices(ts2_model *m, int m0, int m1)
     return TS2_OK;
 }
 
+// Gradient apply of the matrices [m0, m1) on one GPU: row sums, dispersion, update, matrix scales
+int update_matrices(ts2_model *m, const ts2_training_step *step, int m0, int m1)
+{
+    Ctx c = ctx_of(m);
+    const OptSeg *segs = m->d_segs_full + m0; // a segment per matrix
+    const OptMat *mats = m->d_optmats + m0;
+    const int n = m1 - m0, item0 = m->mat_grow0[m0], items = (m1 < (int)m->mats.size() ? m->mat_grow0[m1] : m->n_rows_total) - item0;
+    M_TRY(opt_row_sum2(c, segs, n, item0, items, m->grad_flat, m->rowsum));
+    M_TRY(opt_disp(c, mats, n, m->rowsum, step->disp_decay, m->row_scale));
+    M_TRY(opt_update(c, segs, n, item0, items, m->grad_flat, m->row_scale, step, m->avg_flat, m->w_flat, m->roww2));
+    return opt_sko(c, mats, n, m->roww2, m->skos + m0, step->disp_decay);
+}
+
+// The gradient of the matrices from m0 on is complete: applies the update groups that start there (a step that applies, one GPU).
+// Nothing of this step reads these weights any more.
+int gradients_complete(ts2_model *m, int m0)
+{
+    if (!m->step_in_backward)
+        return TS2_OK;
+    for (UpdateGroup &g : m->update_groups)
+        if (g.mat0 == m0) {
+            M_TRY(update_matrices(m, m->step_in_backward, g.mat0, g.mat1));
+            TS2_CUDA(cudaEventRecord(g.done, m->stream));
+        }
+    return TS2_OK;
+}
+
 AttBwdPlan att_plan(const ts2_model *m, const Layer &ly)
 {
     AttBwdPlan p = m->att_bwd;
@@ -1449,6 +1519,25 @@ AttBwdPlan att_plan(const ts2_model *m, const Layer &ly)
     if (!m->batch.ds_fits[ly.att_type])
         p.ds = nullptr;
     return p;
+}
+
+// Last step of a dense layer's backward pass: dn (scale-free) = dcat . (q_cat / 32) * sqrt(1 / D), the layer's weight
+// gradient from the same dcat, and the backward of the normalisation, which adds to the state gradient.
+int input_gradient(ts2_model *m, int l, const GemmArgs &dn, const GemmArgs *dw_cat)
+{
+    const Layer &ly = m->layers[l];
+    const int T = m->batch.node_count, D = m->D;
+    M_TRY(gemm(dn));
+    TRACE("dn", l, m->dn, (size_t)T * D * 4, TR_F32);
+    if (dw_cat) {
+        M_TRY(gemm(*dw_cat));
+        TRACE("dW_cat", l, m->mats[ly.mat0].grad, (size_t)dw_cat->M * D * 4, TR_F32);
+    }
+    M_TRY(reduce_matrices(m, ly.mat0, l + 1 < m->L ? m->layers[l + 1].mat0 : (int)m->mats.size()));
+    M_TRY(tilenorm_backward(ctx_of(m), m->states[l], m->dn, m->fscale, 1.f, T, D, m->g, true, m->absmax + l, m->health + l, m->step_no));
+    TRACE("g", l, m->g, (size_t)T * D * 4, TR_F32);
+    M_TRY(tap_gradient(m, l));
+    return gradients_complete(m, ly.mat0);
 }
 
 // Backward pass of one dense layer in the int8 pipeline (the reference's default build: FWD / BWD_MATMUL_TYPE =
@@ -1504,18 +1593,15 @@ int backward_dense_int8(ts2_model *m, int l)
     e4.alpha = sqrtf(1.0f / D) / 32.f;
     e4.row_scale = m->dcat_rs;
     e4.out_kind = TS2_OUT_F32;
-    M_TRY(gemm_tn(m, KIND_I8, T, D, C, m->dcat, C, ly.WcatT, C, m->dn, D, e4));
-    TRACE("dn", l, m->dn, (size_t)T * D * 4, TR_F32);
-    if (tune_layers) {
+    if (tune_layers)
         M_TRY(i8_to_half(c, ly.n_fast, (size_t)T * D, m->x16));
-        Epilogue e5;
-        e5.alpha = 1.f / m->s_act;
-        e5.dyn_scale = m->fscale;
-        e5.row_scale = ly.bwd_row;
-        e5.out_kind = m->dense_dw_out();
-        M_TRY(gemm_dw(m, KIND_F16, C, D, T, m->dcat16, C, m->x16, D, m->mats[ly.mat0].grad, e5));
-        TRACE("dW_cat", l, m->mats[ly.mat0].grad, (size_t)C * D * 4, TR_F32);
-    }
+    Epilogue e5;
+    e5.alpha = 1.f / m->s_act;
+    e5.dyn_scale = m->fscale;
+    e5.row_scale = ly.bwd_row;
+    e5.out_kind = m->dense_dw_out();
+    const GemmArgs dw_cat = dw_args(m, KIND_F16, C, D, T, m->dcat16, C, m->x16, D, m->mats[ly.mat0].grad, e5);
+    M_TRY(input_gradient(m, l, tn_args(m, KIND_I8, T, D, C, m->dcat, C, ly.WcatT, C, m->dn, D, e4), tune_layers ? &dw_cat : nullptr));
     return TS2_OK;
 }
 
@@ -1549,8 +1635,10 @@ int backward(ts2_model *m)
     const BatchDev &b = m->batch;
     const bool tune_layers = !(m->descr.flags & TS2_MPF_DISABLE_TUNE_LAYERS);
     M_TRY(final_layer(m, true));
+    TS2_CUDA(cudaEventRecord(m->ev_loss, m->stream)); // see ts2_avg_train_err
     m->gemm_tag = GEMM_TAG_DX;
     M_TRY(reduce_matrices(m, 1, 2));
+    M_TRY(gradients_complete(m, 1));
     M_TRY(tilenorm_backward(c, m->states[L], m->dn, nullptr, 1.f, T, D, m->g, false, m->absmax + L, m->health + L, m->step_no));
     TRACE("g", L, m->g, (size_t)T * D * 4, TR_F32);
     M_TRY(tap_gradient(m, L));
@@ -1649,11 +1737,13 @@ int backward(ts2_model *m)
             M_TRY(tilenorm_backward(c, m->states[l], m->dn, m->fscale, 1.f, T, D, m->g, true, m->absmax + l, m->health + l, m->step_no));
             TRACE("g", l, m->g, (size_t)T * D * 4, TR_F32);
             M_TRY(tap_gradient(m, l));
+            M_TRY(gradients_complete(m, ly.mat0));
             continue;
         }
         if (m->ft == 2) {
             M_TRY(backward_dense_int8(m, l));
-        } else {
+            continue;
+        }
         // g_fast = g * 2^k; fscale = sqrt(D/W) * sko_c / 2^k turns the scale-free intermediate gradients
         // below into true ones
         M_TRY(cast_grad(c, m->g, (size_t)T * D, m->absmax + l + 1, m->g_fast, m->ginv, sqrtf((float)D / (float)W), mc.sko, m->fscale));
@@ -1706,27 +1796,17 @@ int backward(ts2_model *m)
             M_TRY(ffn_act_backward(c, m->drg, ly.cat16, ly.cat16, 2 * W, ly.wscale, T, W, m->dcat));
         }
         TRACE("dcat", l, m->dcat, (size_t)T * C * fsz, fsz == 2 ? TR_F16 : TR_RAW);
-        // dn (scale-free) = dcat . (q_cat/32) * sqrt(1/D)
         Epilogue e4;
         e4.alpha = sqrtf(1.0f / D) / 32.f;
         e4.out_kind = TS2_OUT_F32;
-        M_TRY(gemm_tn(m, m->kind, T, D, C, m->dcat, C, ly.WcatT, C, m->dn, D, e4));
-        TRACE("dn", l, m->dn, (size_t)T * D * 4, TR_F32);
-        if (tune_layers) {
-            // dWcat = dcat^T . n * fscale, rows of matrices that are followed by a normalisation divided by sko
-            Epilogue e5;
-            e5.alpha = 1.f / m->s_act;
-            e5.dyn_scale = m->fscale;
-            e5.row_scale = ly.bwd_row;
-            e5.out_kind = m->dense_dw_out();
-            M_TRY(gemm_dw(m, m->kind, C, D, T, m->dcat, C, ly.n_fast, D, m->mats[ly.mat0].grad, e5));
-            TRACE("dW_cat", l, m->mats[ly.mat0].grad, (size_t)C * D * 4, TR_F32);
-        }
-        }
-        M_TRY(reduce_matrices(m, ly.mat0, l + 1 < L ? m->layers[l + 1].mat0 : (int)m->mats.size()));
-        M_TRY(tilenorm_backward(c, m->states[l], m->dn, m->fscale, 1.f, T, D, m->g, true, m->absmax + l, m->health + l, m->step_no));
-        TRACE("g", l, m->g, (size_t)T * D * 4, TR_F32);
-        M_TRY(tap_gradient(m, l));
+        // dWcat = dcat^T . n * fscale, rows of matrices that are followed by a normalisation divided by sko
+        Epilogue e5;
+        e5.alpha = 1.f / m->s_act;
+        e5.dyn_scale = m->fscale;
+        e5.row_scale = ly.bwd_row;
+        e5.out_kind = m->dense_dw_out();
+        const GemmArgs dw_cat = dw_args(m, m->kind, C, D, T, m->dcat, C, ly.n_fast, D, m->mats[ly.mat0].grad, e5);
+        M_TRY(input_gradient(m, l, tn_args(m, m->kind, T, D, C, m->dcat, C, ly.WcatT, C, m->dn, D, e4), tune_layers ? &dw_cat : nullptr));
     }
     if (!(m->descr.flags & TS2_MPF_DISABLE_TUNE_EMBED)) {
         if (!m->batch.ix_sorted) {
@@ -1736,7 +1816,7 @@ int backward(ts2_model *m)
         M_TRY(embed_backward_indexed(c, m->g, b.ix, D, m->mats[0].grad));
     }
     M_TRY(reduce_matrices(m, 0, 1));
-    return TS2_OK;
+    return gradients_complete(m, 0);
 }
 
 // Optimizer + requantisation of this rank's parts (everything without data parallelism).  Per-row sums of squares
@@ -1746,47 +1826,43 @@ int backward(ts2_model *m)
 int apply(ts2_model *m, const ts2_training_step *step)
 {
     Ctx c = ctx_of(m);
-    const bool dp = m->comm && m->world > 1;
     const int n_mats = (int)m->mats.size();
-    if (dp) {
-        if (!m->reduce_in_backward) { // gradients accumulated by calls that did not apply: exchange them now
-            m->reduce_in_backward = true;
-            for (const Bucket &bk : m->buckets)
-                M_TRY(reduce_matrices(m, bk.mat0, bk.mat1));
-            m->reduce_in_backward = false;
-        }
-        TS2_CUDA(cudaEventRecord(m->ev_reduced, m->comm_stream));
-        TS2_CUDA(cudaStreamWaitEvent(m->stream, m->ev_reduced, 0));
-        TS2_CUDA(cudaMemsetAsync(m->rowsum, 0, (size_t)m->n_rows_total * 4, m->stream));
-        TS2_CUDA(cudaMemsetAsync(m->roww2, 0, (size_t)m->n_rows_total * 8, m->stream));
-    }
-    M_TRY(opt_row_sum2(c, m->d_segs_shard, m->nseg_shard, m->nitems_shard, m->grad_flat, m->rowsum));
-    if (dp)
-        M_NCCL(ncclAllReduce(m->rowsum, m->rowsum, (size_t)m->n_rows_total, ncclFloat, ncclSum, m->comm, m->stream));
-    M_TRY(opt_disp(c, m->d_optmats, n_mats, m->rowsum, step->disp_decay, m->row_scale));
-    M_TRY(opt_update(c, m->d_segs_shard, m->nseg_shard, m->nitems_shard, m->grad_flat, m->row_scale, step, m->avg_flat, m->w_flat,
-                     m->roww2));
-    if (dp)
-        M_NCCL(ncclAllReduce(m->roww2, m->roww2, (size_t)m->n_rows_total, ncclDouble, ncclSum, m->comm, m->stream));
-    M_TRY(opt_sko(c, m->d_optmats, n_mats, m->roww2, m->skos, step->disp_decay));
-    if (!dp)
+    if (!(m->comm && m->world > 1)) {
+        if (m->update_groups.empty())
+            M_TRY(update_matrices(m, step, 0, n_mats));
         return quantize_all(m);
-    M_TRY(opt_quantize(c, m->d_segs_shard, m->nseg_shard, m->nitems_shard, m->w_flat, m->skos));
-    if (dp) {
-        M_NCCL(ncclGroupStart());
-        for (const Bucket &bk : m->buckets) {
-            if (bk.owner_only)
-                continue; // a rank only reads the quantized weights of its own experts
-            const size_t part = bk.elems / m->world * bk.qsize;
-            ncclResult_t r = ncclAllGather(bk.qflat + part * m->rank, bk.qflat, part, ncclUint8, m->comm, m->stream);
-            if (r != ncclSuccess) {
-                ncclGroupEnd();
-                return mfail(m, fail(TS2_ERR_COMM, "ncclAllGather failed: %s", ncclGetErrorString(r)));
-            }
-        }
-        M_NCCL(ncclGroupEnd());
-        m->master_stale = true;
     }
+    if (!m->reduce_in_backward) { // gradients accumulated by calls that did not apply: exchange them now
+        m->reduce_in_backward = true;
+        for (const Bucket &bk : m->buckets)
+            M_TRY(reduce_matrices(m, bk.mat0, bk.mat1));
+        m->reduce_in_backward = false;
+    }
+    TS2_CUDA(cudaEventRecord(m->ev_reduced, m->comm_stream));
+    TS2_CUDA(cudaStreamWaitEvent(m->stream, m->ev_reduced, 0));
+    TS2_CUDA(cudaMemsetAsync(m->rowsum, 0, (size_t)m->n_rows_total * 4, m->stream));
+    TS2_CUDA(cudaMemsetAsync(m->roww2, 0, (size_t)m->n_rows_total * 8, m->stream));
+    M_TRY(opt_row_sum2(c, m->d_segs_shard, m->nseg_shard, 0, m->nitems_shard, m->grad_flat, m->rowsum));
+    M_NCCL(ncclAllReduce(m->rowsum, m->rowsum, (size_t)m->n_rows_total, ncclFloat, ncclSum, m->comm, m->stream));
+    M_TRY(opt_disp(c, m->d_optmats, n_mats, m->rowsum, step->disp_decay, m->row_scale));
+    M_TRY(opt_update(c, m->d_segs_shard, m->nseg_shard, 0, m->nitems_shard, m->grad_flat, m->row_scale, step, m->avg_flat, m->w_flat,
+                     m->roww2));
+    M_NCCL(ncclAllReduce(m->roww2, m->roww2, (size_t)m->n_rows_total, ncclDouble, ncclSum, m->comm, m->stream));
+    M_TRY(opt_sko(c, m->d_optmats, n_mats, m->roww2, m->skos, step->disp_decay));
+    M_TRY(opt_quantize(c, m->d_segs_shard, m->nseg_shard, m->nitems_shard, m->w_flat, m->skos));
+    M_NCCL(ncclGroupStart());
+    for (const Bucket &bk : m->buckets) {
+        if (bk.owner_only)
+            continue; // a rank only reads the quantized weights of its own experts
+        const size_t part = bk.elems / m->world * bk.qsize;
+        ncclResult_t r = ncclAllGather(bk.qflat + part * m->rank, bk.qflat, part, ncclUint8, m->comm, m->stream);
+        if (r != ncclSuccess) {
+            ncclGroupEnd();
+            return mfail(m, fail(TS2_ERR_COMM, "ncclAllGather failed: %s", ncclGetErrorString(r)));
+        }
+    }
+    M_NCCL(ncclGroupEnd());
+    m->master_stale = true;
     M_TRY(post_quantize(m));
     return TS2_OK;
 }
@@ -1901,14 +1977,15 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
 }
 
 // what the device found wrong with a batch, if anything; clears the record
-int report_batch_status(ts2_model *m)
+int report_batch_status(ts2_model *m, cudaStream_t stream)
 {
     int *h = m->report->batch;
     if (h[0] == BATCH_OK)
         return TS2_OK;
     const int code = h[0], where = h[1], d0 = h[2], d1 = h[3];
     h[0] = BATCH_OK;
-    cudaMemsetAsync(m->batch.status, 0, 16, m->stream);
+    cudaMemsetAsync(m->batch.status, 0, 16, stream);
+    cudaStreamSynchronize(stream); // the stream is idle: a later batch, on another stream, finds the record cleared
     switch (code) {
     case BATCH_BAD_SPAN_PTR:
         return fail(TS2_ERR_INVALID_ARG, "batch: span_ptr of node %d is malformed (offset %d, count %d)", where, d0, d1);
@@ -1938,7 +2015,7 @@ int wait_stream(ts2_model *m, const float *scalar = nullptr, float *value = null
     m->unreported = false;
     if (m->report->device_status | m->report->static_status)
         M_TRY(collect_device_status(m->device)); // clears the words and reports them
-    M_TRY(report_batch_status(m));
+    M_TRY(report_batch_status(m, m->stream));
     if (value)
         *value = m->report->scalar;
     return TS2_OK;
@@ -2007,6 +2084,8 @@ int ts2_create(const ts2_model_descr *descr, const ts2_matrix_view *mats, int n_
     cudaEventCreate(&m->ev_t0);
     cudaEventCreate(&m->ev_t1);
     cudaEventCreateWithFlags(&m->ev_grads, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&m->ev_loss, cudaEventDisableTiming);
+    cudaStreamCreateWithFlags(&m->read_stream, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&m->ev_reduced, cudaEventDisableTiming);
     rc = build_model(m, mats, n_mats, bias);
     if (rc != TS2_OK) {
@@ -2053,6 +2132,13 @@ void ts2_destroy(ts2_model *m)
     for (cudaEvent_t e : m->batch.slot_ev)
         if (e)
             cudaEventDestroy(e);
+    for (UpdateGroup &g : m->update_groups)
+        if (g.done)
+            cudaEventDestroy(g.done);
+    if (m->ev_loss)
+        cudaEventDestroy(m->ev_loss);
+    if (m->read_stream)
+        cudaStreamDestroy(m->read_stream);
     if (m->ev_start)
         cudaEventDestroy(m->ev_start);
     if (m->ev_stop)
@@ -2138,9 +2224,12 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
         M_TRY(clear_gradient(m));
     M_TRY(forward(m));
     // an accumulated gradient of earlier calls sits in the same buffer: the per-layer sums below then cover it too
-    m->reduce_in_backward = add_to_model == TS2_GRADIENT_APPLY && m->comm && m->world > 1;
+    const bool dp = m->comm && m->world > 1;
+    m->reduce_in_backward = add_to_model == TS2_GRADIENT_APPLY && dp;
+    m->step_in_backward = add_to_model == TS2_GRADIENT_APPLY && !dp ? step : nullptr;
     const int brc = backward(m);
     m->reduce_in_backward = false;
+    m->step_in_backward = nullptr;
     if (brc != TS2_OK)
         return brc;
     m->grads_dirty = true;
@@ -2200,14 +2289,22 @@ int ts2_forward_score(ts2_model *m, float *out_score)
     return TS2_OK;
 }
 
+// The error is known when the forward pass and the final layer are through: the call waits for that and not for the backward
+// pass and the update behind it, so that the host prepares the next batch, or fetches weights as they are updated, meanwhile.
 int ts2_avg_train_err(ts2_model *m, float *out_err)
 {
     if (!m || !out_err)
         return fail(TS2_ERR_INVALID_ARG, "null argument");
     TS2_CUDA(cudaSetDevice(m->device));
-    float s = 0;
-    M_TRY(wait_stream(m, m->logp, &s));
-    *out_err = m->last_targets ? -s / m->last_targets : 0.f;
+    Ctx c = ctx_of(m);
+    c.stream = m->read_stream;
+    TS2_CUDA(cudaStreamWaitEvent(m->read_stream, m->ev_loss, 0));
+    M_TRY(queue_report(c, m->batch.status, m->logp, m->report));
+    M_TRY(poll_until(m, [&] { return cudaStreamQuery(m->read_stream); }));
+    if (m->report->device_status | m->report->static_status)
+        M_TRY(wait_stream(m)); // the step went wrong: reported when it is over
+    M_TRY(report_batch_status(m, m->read_stream));
+    *out_err = m->last_targets ? -m->report->scalar / m->last_targets : 0.f;
     return TS2_OK;
 }
 
@@ -2216,12 +2313,11 @@ int ts2_get_params(ts2_model *m, int what, ts2_matrix_view *mats_out, int n_mats
     if (!m || !mats_out || n_mats != (int)m->mats.size())
         return fail(TS2_ERR_INVALID_ARG, "bad arguments to ts2_get_params");
     TS2_CUDA(cudaSetDevice(m->device));
-    if (what != TS2_PARAM_GRADIENT)
-        M_TRY(sync_master(m));
-    M_TRY(wait_stream(m));
     for (int i = 0; i < n_mats; ++i)
         if (mats_out[i].data && (mats_out[i].x_size != m->mats[i].x || mats_out[i].y_size != m->mats[i].y))
             return mfail(m, fail(TS2_ERR_INVALID_ARG, "matrix %d: shape mismatch", i));
+    if (what != TS2_PARAM_GRADIENT)
+        M_TRY(sync_master(m));
     // Matrices that follow one another on both sides leave in one copy, all copies are queued before any is waited for.
     // A copy stays inside one page-locked range: neighbours in address may be allocations (or registrations) of their own,
     // or pageable, and a copy across such a border is not a valid one.
@@ -2231,26 +2327,45 @@ int ts2_get_params(ts2_model *m, int what, ts2_matrix_view *mats_out, int n_mats
     cudaError_t err = cudaSuccess;
     auto flush = [&]() {
         if (run && err == cudaSuccess)
-            err = cudaMemcpyAsync(dst0, src0, run * 4, cudaMemcpyDeviceToHost, m->stream);
+            err = cudaMemcpyAsync(dst0, src0, run * 4, cudaMemcpyDeviceToHost, m->read_stream);
         run = 0;
     };
-    for (int i = 0; i < n_mats; ++i) {
-        Matrix &mt = m->mats[i];
-        if (!mats_out[i].data)
-            continue;
-        const float *src = what == TS2_PARAM_WEIGHTS ? mt.w : what == TS2_PARAM_MOMENTUM ? mt.avg : mt.grad;
-        const size_t n = (size_t)mt.x * mt.y;
-        if (run && (src != src0 + run || mats_out[i].data != dst0 + run || !one_pinned_range(dst0, (run + n) * 4)))
-            flush();
-        if (!run) {
-            src0 = src;
-            dst0 = mats_out[i].data;
+    auto fetch = [&](int m0, int m1) {
+        for (int i = m0; i < m1; ++i) {
+            Matrix &mt = m->mats[i];
+            if (!mats_out[i].data)
+                continue;
+            const float *src = what == TS2_PARAM_WEIGHTS ? mt.w : what == TS2_PARAM_MOMENTUM ? mt.avg : mt.grad;
+            const size_t n = (size_t)mt.x * mt.y;
+            if (run && (src != src0 + run || mats_out[i].data != dst0 + run || !one_pinned_range(dst0, (run + n) * 4)))
+                flush();
+            if (!run) {
+                src0 = src;
+                dst0 = mats_out[i].data;
+            }
+            run += n;
         }
-        run += n;
+        flush();
+    };
+    // Weights and momentum leave as soon as their group is updated, while the backward pass goes on below it: the copies of a
+    // large model take as long as a step and more (437 M parameters 32 ms).  A copy is queued only when its source is ready, so
+    // none waits on the device for a step that does not end.
+    int rc = TS2_OK;
+    const bool dp = m->comm && m->world > 1;
+    if (what != TS2_PARAM_GRADIENT && !dp && !m->update_groups.empty()) {
+        for (UpdateGroup &g : m->update_groups) {
+            if ((rc = poll_until(m, [&] { return cudaEventQuery(g.done); })) != TS2_OK)
+                break;
+            fetch(g.mat0, g.mat1);
+        }
+        if (rc == TS2_OK)
+            rc = wait_stream(m);
+    } else if ((rc = wait_stream(m)) == TS2_OK) {
+        fetch(0, n_mats);
     }
-    flush();
-    // the steps are over (wait_stream): only these copies remain, and none may still be on its way when the call returns
-    const cudaError_t done = cudaStreamSynchronize(m->stream);
+    // none of the copies may still be on its way when the call returns
+    const cudaError_t done = cudaStreamSynchronize(m->read_stream);
+    M_TRY(rc);
     TS2_CUDA(err);
     TS2_CUDA(done);
     return TS2_OK;
