@@ -16,12 +16,6 @@ struct Ctx {
     float s_act = 16.f; // quantization scale of normalized activations (1 for fp16)
 };
 
-// ---- kernels_elem.cu ---------------------------------------------------------------
-// state0[t] = sum over the node's labels of +-E[label] * (sko/32)   (ComputeEmbedding, cpu_transformer.cpp:66-90)
-// zero: n_zero words that the step accumulates into later, cleared by the way (its first launch)
-int embed_forward(const Ctx &c, const __half *embed, const float *sko, const uint32_t *label_arr, const uint32_t *label_ptr, int T,
-                  int D, float *state, unsigned *zero, int n_zero, float *zero_scalar);
-
 // ---- kernels_batch.cu: batch preparation on the device -------------------------------
 // codes of the batch status record {code, where, detail, detail}; 0 = the batch was well formed
 enum {
@@ -59,7 +53,23 @@ struct LabelIndex {
     uint32_t n = 0;
     int sorted = 0; // which of key[] / val[] holds the sorted entries
 };
-// every table of a batch: the kernels above, or, for a small batch, one launch that also sorts the inverse index (*sorted)
+// ---- kernels_elem.cu ---------------------------------------------------------------
+// state0[t] = sum over the node's labels of +-E[label] * (sko/32)   (ComputeEmbedding, cpu_transformer.cpp:66-90)
+// n_fast, n16: its tile normalisation, as tilenorm_forward writes it
+// What else a step's first launch does: zero: n_zero words that the step accumulates into; clear: n_clear floats (a multiple of
+// 4) of the gradient; sort: an inverse index of at most LABEL_RANK_MAX entries, from its buffer 0 into buffer 1
+struct StepStart {
+    unsigned *zero = nullptr;
+    int n_zero = 0;
+    float *zero_scalar = nullptr;
+    float *clear = nullptr;
+    size_t n_clear = 0;
+    const LabelIndex *sort = nullptr;
+};
+int embed_forward(const Ctx &c, const __half *embed, const float *sko, const uint32_t *label_arr, const uint32_t *label_ptr, int T,
+                  int D, float *state, void *n_fast, __half *n16, const StepStart &start);
+
+// every table of a batch: the kernels above, or, for a small batch, one launch; the inverse index is left unsorted
 struct BatchTables {
     int T, V, n_targets;
     uint32_t n_labels, label_count;
@@ -72,7 +82,7 @@ struct BatchSpans {
     int n_spans;
     int *start, *finish, *rev_first, *rev_last;
 };
-int batch_prepare(const Ctx &c, const BatchTables &b, const BatchSpans *att, int n_types, LabelIndex &ix, bool *sorted);
+int batch_prepare(const Ctx &c, const BatchTables &b, const BatchSpans *att, int n_types, LabelIndex &ix);
 size_t label_index_hist_elems(size_t label_cap);
 size_t label_index_partial_elems(int device, size_t label_cap, int D);
 // validates label_arr / label_ptr in place (bad labels become label 0, label_ptr is clamped to n_labels) and writes the
@@ -208,9 +218,12 @@ int moe_act_forward(const Ctx &c, const __half *cat, const int *token_of, const 
                     float *wscale, void *rg);
 int moe_act_backward(const Ctx &c, const __half *drg, const __half *cat, const __half *what, const float *wscale, const int *token_of,
                      const float *weight_of, int rows, int X, void *dcat, float *dmoe_part);
-// out[t] = (in ? in[t] : out[t]) + sum_j y[slot_of[t*k+j]]
-int moe_combine(const Ctx &c, const float *y, const int *slot_of, int T, int k, int D, const float *in, float *out);
-int moe_combine_half(const Ctx &c, const __half *y, const int *slot_of, int T, int k, int D, const float *in, float *out);
+// out[t] = in[t] + sum_j y[slot_of[t*k+j]], y fp32 or fp16; n_fast, n16: its tile normalisation, as tilenorm_forward writes it
+int moe_combine(const Ctx &c, const void *y, bool y16, const int *slot_of, int T, int k, int D, const float *in, float *out, void *n_fast,
+                __half *n16);
+// the same sum over the gradients of a layer's input, dn[t] + sum_j y[slot_of[t*k+j]], and tilenorm_backward of it, added to g
+int moe_combine_backward(const Ctx &c, const void *y, bool y16, const int *slot_of, int T, int k, int D, const float *dn, const float *x,
+                         const float *dyn, float *g, unsigned *absmax, unsigned *health, unsigned step_no);
 int moe_router_backward(const Ctx &c, const float *dmoe_part, int tiles, const int *ids, const float *weights, const int *slot_of, int T,
                         int k, int E, int ld, void *dl);
 

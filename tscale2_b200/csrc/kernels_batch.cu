@@ -14,6 +14,7 @@
 // span, no target) so that the kernels that follow stay inside their buffers, and the first one is recorded in a
 // status record that the host reads when it next waits for the stream.
 #include "kernels.cuh"
+#include "label_rank.cuh"
 
 namespace ts2 {
 namespace {
@@ -344,10 +345,11 @@ __global__ void __launch_bounds__(1024) exclusive_scan_kernel(uint32_t *__restri
 }
 
 // ---- a small batch in one launch -----------------------------------------------------------
-// Up to SB_MAX nodes and labels everything above is work for one block per table: block 0 validates the labels and sorts
-// the inverse index (a bitonic sort of (label, position) pairs: positions differ, so it is stable), block 1 fills the
-// targets, block 2 + a the spans of attention type a.  The launches above took 45 us of a 512-token step, mostly
-// latency between them; this takes 12.
+// Up to SB_MAX nodes and labels everything above but the order of the index is work for one block per table: block 0
+// validates the labels, block 1 fills the targets, block 2 + a the spans of attention type a.  The launches above took 45 us
+// of a 512-token step, mostly latency between them.  The index is put in order by blocks of the step's first kernel
+// (embed_forward, label_rank.cuh), and not at all for a batch that is only scored: as a bitonic sort in block 0 it made up a
+// third of this kernel's time (9.7 -> 6.9 us).
 constexpr int SB_MAX = 4096, SB_TYPES = 8, SB_THREADS = 1024, SB_PER = SB_MAX / SB_THREADS;
 struct SmallBatch {
     int T, V, n_targets;
@@ -365,15 +367,13 @@ struct SmallBatch {
 __global__ void __launch_bounds__(SB_THREADS) small_batch_kernel(const SmallBatch p)
 {
     grid_dep_wait();
-    __shared__ unsigned long long pairs[SB_MAX]; // block 0: label << 32 | position; span blocks: run_max and suf_min
+    __shared__ int run_max[SB_MAX], suf_min[SB_MAX];
     __shared__ int w_max[32], w_min[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = p.T;
     if (blockIdx.x == 0) {
         const uint32_t n = p.n_labels;
-        for (uint32_t k = tid; k < n; k += SB_THREADS) { // entries that no node owns count as label 0 of node 0
-            pairs[k] = k;
-            p.val[k] = 0;
-        }
+        for (uint32_t k = tid; k < n; k += SB_THREADS) // entries that no node owns count as label 0 of node 0
+            p.key[k] = p.val[k] = 0;
         __syncthreads();
         for (int t = tid; t < T; t += SB_THREADS) {
             uint32_t p0 = p.label_ptr[t], p1 = p.label_ptr[t + 1];
@@ -390,44 +390,13 @@ __global__ void __launch_bounds__(SB_THREADS) small_batch_kernel(const SmallBatc
                     label = 0;
                     p.label_arr[k] = raw & TS2_LABEL_NEGATIVE;
                 }
-                pairs[k] = (unsigned long long)label << 32 | k;
+                p.key[k] = label;
                 p.val[k] = (uint32_t)t | (raw & TS2_LABEL_NEGATIVE);
             }
         }
-        uint32_t n2 = 64;
-        while (n2 < n)
-            n2 *= 2;
-        for (uint32_t k = n + tid; k < n2; k += SB_THREADS)
-            pairs[k] = ~0ull;
         __syncthreads();
         for (int t = tid; t <= T; t += SB_THREADS)
             p.label_ptr[t] = min(p.label_ptr[t], n);
-        for (uint32_t k = 2; k <= n2; k <<= 1)
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t i = tid; i < n2 / 2; i += SB_THREADS) {
-                    const uint32_t a = 2 * i - (i & (j - 1)), b = a + j;
-                    const unsigned long long x = pairs[a], y = pairs[b];
-                    if ((x > y) == ((a & k) == 0)) {
-                        pairs[a] = y;
-                        pairs[b] = x;
-                    }
-                }
-                // up to a distance of 32 a warp's 32 exchanges stay inside 64 entries of its own
-                if (j > 32 || (j == 1 && k >= 64))
-                    __syncthreads();
-                else
-                    __syncwarp();
-            }
-        uint32_t v[SB_PER];
-        int c = 0;
-        for (uint32_t k = tid; k < n; k += SB_THREADS)
-            v[c++] = p.val[(uint32_t)pairs[k]];
-        __syncthreads();
-        c = 0;
-        for (uint32_t k = tid; k < n; k += SB_THREADS) {
-            p.key[k] = (uint32_t)(pairs[k] >> 32);
-            p.val[k] = v[c++];
-        }
         return;
     }
     if (blockIdx.x == 1) {
@@ -444,7 +413,6 @@ __global__ void __launch_bounds__(SB_THREADS) small_batch_kernel(const SmallBatc
         return;
     }
     const auto &at = p.att[blockIdx.x - 2];
-    int *run_max = (int *)pairs, *suf_min = run_max + SB_MAX;
     // a thread takes SB_PER consecutive nodes: its own prefix maximum and suffix minimum, then the warp's, then the block's
     int mx[SB_PER], mn[SB_PER], t0 = tid * SB_PER;
 #pragma unroll
@@ -697,10 +665,9 @@ static bool batch_prepare_small(const BatchTables &b, int n_types)
     return b.T <= SB_MAX && b.n_labels <= (uint32_t)SB_MAX && n_types <= SB_TYPES;
 }
 
-int batch_prepare(const Ctx &c, const BatchTables &b, const BatchSpans *att, int n_types, LabelIndex &ix, bool *sorted)
+int batch_prepare(const Ctx &c, const BatchTables &b, const BatchSpans *att, int n_types, LabelIndex &ix)
 {
-    *sorted = batch_prepare_small(b, n_types);
-    if (!*sorted) {
+    if (!batch_prepare_small(b, n_types)) {
         if (int rc = label_index_entries(c, b.label_arr, b.label_ptr, b.T, b.n_labels, b.label_count, ix, b.status))
             return rc;
         for (int a = 0; a < n_types; ++a)
@@ -759,10 +726,22 @@ int label_index_entries(const Ctx &c, uint32_t *label_arr, uint32_t *label_ptr, 
     return TS2_OK;
 }
 
+__global__ void __launch_bounds__(LABEL_RANK_THREADS) label_rank_kernel(const uint32_t *__restrict__ key, const uint32_t *__restrict__ val, uint32_t n,
+                                                                        uint32_t *__restrict__ key_out, uint32_t *__restrict__ val_out)
+{
+    grid_dep_wait();
+    label_rank(key, val, n, key_out, val_out, blockIdx.x);
+}
+
 int label_index_sort(const Ctx &c, uint32_t label_count, LabelIndex &ix)
 {
     if (ix.n == 0)
         return TS2_OK;
+    if (ix.n <= LABEL_RANK_MAX) {
+        TS2_LAUNCH((label_rank_kernel), label_rank_blocks(ix.n), LABEL_RANK_THREADS, 0, c.stream, ix.key[0], ix.val[0], ix.n, ix.key[1], ix.val[1]);
+        ix.sorted = 1;
+        return TS2_OK;
+    }
     int bits = 1;
     while (bits < 31 && (1u << bits) < label_count)
         ++bits;

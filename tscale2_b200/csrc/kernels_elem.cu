@@ -5,6 +5,7 @@
 // strides over (row, tile) pairs; reductions are warp shuffles.
 #include "kernels.cuh"
 #include "row_math.cuh"
+#include "label_rank.cuh"
 
 namespace ts2 {
 
@@ -42,21 +43,43 @@ static int grid_for(const Ctx &c, K kernel, long long warp_items)
          item += gridDim.x * WARPS)
 
 // ---------------------------------------------------------------------------------
+static_assert(THREADS == LABEL_RANK_THREADS, "blocks of embed_forward_kernel");
+struct EmbedStart { // see StepStart
+    int blocks; // the blocks from here on put the inverse label index in order
+    unsigned *zero;
+    int n_zero;
+    float *zero_scalar;
+    float4 *clear;
+    size_t n_clear4;
+    const uint32_t *key, *val;
+    uint32_t *key_out, *val_out, n_labels;
+};
+
+// one warp per (node, 128 columns); the first layer's normalisation runs on the sum in registers
+template <int FT>
 __global__ void embed_forward_kernel(const __half *__restrict__ embed, const float *__restrict__ sko,
                                      const uint32_t *__restrict__ label_arr, const uint32_t *__restrict__ label_ptr, int T, int D,
-                                     float *__restrict__ state, unsigned *__restrict__ zero, int n_zero, float *__restrict__ zero_scalar)
+                                     float *__restrict__ state, float s_act, void *__restrict__ n_fast, __half *__restrict__ n16,
+                                     const EmbedStart st)
 {
     grid_dep_wait();
-    if (blockIdx.x == 0) {
-        for (int i = threadIdx.x; i < n_zero; i += THREADS)
-            zero[i] = 0u;
-        if (threadIdx.x == 0)
-            *zero_scalar = 0.f;
+    if ((int)blockIdx.x >= st.blocks) {
+        label_rank(st.key, st.val, st.n_labels, st.key_out, st.val_out, blockIdx.x - st.blocks);
+        return;
     }
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < st.n_zero; i += THREADS)
+            st.zero[i] = 0u;
+        if (threadIdx.x == 0)
+            *st.zero_scalar = 0.f;
+    }
+    for (size_t i = (size_t)blockIdx.x * THREADS + threadIdx.x; i < st.n_clear4; i += (size_t)st.blocks * THREADS)
+        st.clear[i] = make_float4(0, 0, 0, 0);
     const int tiles = D / TILE;
     const float scale = __ldg(sko) * (1.f / 32);
-    WARP_ITEM_LOOP((long long)T * tiles)
-    {
+    const int lane = threadIdx.x & 31;
+    const unsigned total = (unsigned)((long long)T * tiles);
+    for (unsigned item = blockIdx.x * WARPS + (threadIdx.x >> 5); item < total; item += st.blocks * WARPS) {
         const int t = (int)(item / tiles), off = (int)(item % tiles) * TILE + lane * 4;
         float4 acc = make_float4(0, 0, 0, 0);
         for (uint32_t k = label_ptr[t]; k < label_ptr[t + 1]; ++k) {
@@ -70,16 +93,42 @@ __global__ void embed_forward_kernel(const __half *__restrict__ embed, const flo
             acc.z += (e.z * scale) * w;
             acc.w += (e.w * scale) * w;
         }
-        *(float4 *)(state + (size_t)t * D + off) = acc;
+        const size_t at = (size_t)t * D + off;
+        *(float4 *)(state + at) = acc;
+        const float4 nv = scale4(acc, tile_scale(warp_sum(dot4(acc, acc))));
+        Fast<FT>::store4(n_fast, at, scale4(nv, s_act));
+        if (n16)
+            store_half4(n16 + at, nv);
     }
 }
 
 int embed_forward(const Ctx &c, const __half *embed, const float *sko, const uint32_t *label_arr, const uint32_t *label_ptr, int T,
-                  int D, float *state, unsigned *zero, int n_zero, float *zero_scalar)
+                  int D, float *state, void *n_fast, __half *n16, const StepStart &start)
 {
-    TS2_LAUNCH((embed_forward_kernel), grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream, embed, sko, label_arr, label_ptr, T,
-               D, state,
-               zero, n_zero, zero_scalar);
+    EmbedStart st;
+    st.blocks = grid_for(c, (long long)T * (D / TILE));
+    st.zero = start.zero, st.n_zero = start.n_zero, st.zero_scalar = start.zero_scalar;
+    st.clear = (float4 *)start.clear, st.n_clear4 = start.n_clear / 4;
+    if (st.n_clear4) // a few short texts over a large vocabulary: the clearing wants the whole device
+        st.blocks = std::max(st.blocks, (int)std::min<size_t>(ceil_div(st.n_clear4, 4 * THREADS), (size_t)sm_count(c.device) * 8));
+    st.key = st.val = nullptr;
+    st.key_out = st.val_out = nullptr;
+    st.n_labels = 0;
+    int grid = st.blocks;
+    if (start.sort && start.sort->n) {
+        const LabelIndex &ix = *start.sort;
+        st.key = ix.key[0], st.val = ix.val[0], st.key_out = ix.key[1], st.val_out = ix.val[1], st.n_labels = ix.n;
+        grid += label_rank_blocks(ix.n);
+    }
+#define TS2_EMBED(FT_) \
+    TS2_LAUNCH((embed_forward_kernel<FT_>), grid, THREADS, 0, c.stream, embed, sko, label_arr, label_ptr, T, D, state, c.s_act, n_fast, n16, st)
+    if (c.ft == 0)
+        TS2_EMBED(0);
+    else if (c.ft == 1)
+        TS2_EMBED(1);
+    else
+        TS2_EMBED(2);
+#undef TS2_EMBED
     return TS2_OK;
 }
 

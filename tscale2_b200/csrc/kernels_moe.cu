@@ -10,7 +10,7 @@
 // padded to a multiple of 128 rows so that every 128-row tile of a contraction belongs to one expert.
 // Slot order inside a segment is token order (stable), so the tables are deterministic.
 #include "kernels.cuh"
-#include "fast_types.cuh"
+#include "row_math.cuh"
 
 namespace ts2 {
 
@@ -463,9 +463,29 @@ int moe_act_backward(const Ctx &c, const __half *drg, const __half *cat, const _
 }
 
 // ---------------------------------------------------------------------------------------
-// out[t] = (in ? in[t] : out[t]) + sum over the token's choices of y[slot]   (fp32 rows of width D)
-__global__ void moe_combine_kernel(const float *__restrict__ y, const int *__restrict__ slot_of, int T, int k, int D,
-                                   const float *__restrict__ in, float *__restrict__ out)
+// sums over a token's choices, one warp per (token, 128 columns).  The row-wise step that follows runs on the sum in
+// registers: by itself it read the sum back (32768 tokens x 1024, e4m3: combine 74 and normalisation 32 -> 101 us; combine 74 and
+// the normalisation's backward 75 -> 122 us).
+template <typename YT>
+__device__ __forceinline__ float4 moe_sum4(const float *__restrict__ base, const YT *__restrict__ y, const int *__restrict__ slot_of, size_t t,
+                                           int k, int D, int off)
+{
+    float4 acc = *(const float4 *)(base + t * D + off);
+    for (int j = 0; j < k; ++j) {
+        const YT *src = y + (size_t)slot_of[t * k + j] * D + off;
+        float4 v;
+        if constexpr (sizeof(YT) == 2)
+            v = load_half4(src);
+        else
+            v = *(const float4 *)src;
+        acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+    }
+    return acc;
+}
+
+template <int FT, typename YT>
+__global__ void moe_combine_kernel(const YT *__restrict__ y, const int *__restrict__ slot_of, int T, int k, int D, const float *__restrict__ in,
+                                   float *__restrict__ out, float s_act, void *__restrict__ n_fast, __half *__restrict__ n16)
 {
     grid_dep_wait();
     const int tiles = D / TILE;
@@ -473,43 +493,69 @@ __global__ void moe_combine_kernel(const float *__restrict__ y, const int *__res
     {
         const size_t t = item / tiles;
         const int off = (item % tiles) * TILE + lane * 4;
-        float4 acc = *(const float4 *)((in ? in : out) + t * D + off);
-        for (int j = 0; j < k; ++j) {
-            const float4 v = *(const float4 *)(y + (size_t)slot_of[t * k + j] * D + off);
-            acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
-        }
-        *(float4 *)(out + t * D + off) = acc;
+        const float4 v = moe_sum4(in, y, slot_of, t, k, D, off);
+        *(float4 *)(out + t * D + off) = v;
+        const float4 nv = scale4(v, tile_scale(warp_sum(dot4(v, v))));
+        Fast<FT>::store4(n_fast, t * D + off, scale4(nv, s_act));
+        if (n16)
+            store_half4(n16 + t * D + off, nv);
     }
 }
 
-// the same sum over fp16 rows (expert parallel: results come back from the experts' owners as fp16)
-__global__ void moe_combine_half_kernel(const __half *__restrict__ y, const int *__restrict__ slot_of, int T, int k, int D,
-                                        const float *__restrict__ in, float *__restrict__ out)
+int moe_combine(const Ctx &c, const void *y, bool y16, const int *slot_of, int T, int k, int D, const float *in, float *out, void *n_fast,
+                __half *n16)
 {
-    grid_dep_wait();
-    const int tiles = D / TILE;
-    WARP_ITEM_LOOP((long long)T * tiles)
-    {
-        const size_t t = item / tiles;
-        const int off = (item % tiles) * TILE + lane * 4;
-        float4 acc = *(const float4 *)((in ? in : out) + t * D + off);
-        for (int j = 0; j < k; ++j) {
-            const float4 v = load_half4(y + (size_t)slot_of[t * k + j] * D + off);
-            acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
-        }
-        *(float4 *)(out + t * D + off) = acc;
-    }
-}
-
-int moe_combine_half(const Ctx &c, const __half *y, const int *slot_of, int T, int k, int D, const float *in, float *out)
-{
-    TS2_LAUNCH((moe_combine_half_kernel), grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream, y, slot_of, T, k, D, in, out);
+    const int grid = grid_for(c, (long long)T * (D / TILE));
+    if (y16)
+        TS2_LAUNCH((moe_combine_kernel<0, __half>), grid, THREADS, 0, c.stream, (const __half *)y, slot_of, T, k, D, in, out, c.s_act, n_fast, n16);
+    else if (c.ft == 0)
+        TS2_LAUNCH((moe_combine_kernel<0, float>), grid, THREADS, 0, c.stream, (const float *)y, slot_of, T, k, D, in, out, c.s_act, n_fast, n16);
+    else
+        TS2_LAUNCH((moe_combine_kernel<1, float>), grid, THREADS, 0, c.stream, (const float *)y, slot_of, T, k, D, in, out, c.s_act, n_fast, n16);
     return TS2_OK;
 }
 
-int moe_combine(const Ctx &c, const float *y, const int *slot_of, int T, int k, int D, const float *in, float *out)
+template <typename YT>
+__global__ void moe_combine_backward_kernel(const YT *__restrict__ y, const int *__restrict__ slot_of, int T, int k, int D,
+                                            const float *__restrict__ dn, const float *__restrict__ x, const float *__restrict__ dyn,
+                                            float *__restrict__ g, unsigned *__restrict__ absmax, unsigned *__restrict__ health, unsigned step_no)
 {
-    TS2_LAUNCH((moe_combine_kernel), grid_for(c, (long long)T * (D / TILE)), THREADS, 0, c.stream, y, slot_of, T, k, D, in, out);
+    grid_dep_wait();
+    const int tiles = D / TILE;
+    const float a = __ldg(dyn);
+    float mx = 0.f;
+    WARP_ITEM_LOOP((long long)T * tiles)
+    {
+        const size_t t = item / tiles;
+        const int off = (item % tiles) * TILE + lane * 4;
+        const float4 xv = *(const float4 *)(x + t * D + off), o = *(const float4 *)(g + t * D + off);
+        const float4 r = tilenorm_backward4(xv, scale4(moe_sum4(dn, y, slot_of, t, k, D, off), a));
+        const float4 v = make_float4(o.x + r.x, o.y + r.y, o.z + r.z, o.w + r.w);
+        *(float4 *)(g + t * D + off) = v;
+        mx = absmax4(mx, v);
+    }
+    __shared__ float block_max[WARPS];
+    mx = warp_max(mx);
+    if ((threadIdx.x & 31) == 0)
+        block_max[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < WARPS; ++i)
+            mx = fmaxf(mx, block_max[i]);
+        absmax_report(mx, absmax, health, step_no);
+    }
+}
+
+int moe_combine_backward(const Ctx &c, const void *y, bool y16, const int *slot_of, int T, int k, int D, const float *dn, const float *x,
+                         const float *dyn, float *g, unsigned *absmax, unsigned *health, unsigned step_no)
+{
+    const int grid = grid_for(c, (long long)T * (D / TILE));
+    if (y16)
+        TS2_LAUNCH((moe_combine_backward_kernel<__half>), grid, THREADS, 0, c.stream, (const __half *)y, slot_of, T, k, D, dn, x, dyn, g, absmax,
+                   health, step_no);
+    else
+        TS2_LAUNCH((moe_combine_backward_kernel<float>), grid, THREADS, 0, c.stream, (const float *)y, slot_of, T, k, D, dn, x, dyn, g, absmax,
+                   health, step_no);
     return TS2_OK;
 }
 

@@ -12,8 +12,9 @@
 //     is also the message of the data-parallel all-reduce.
 // Scale bookkeeping follows the CPU formulas of the reference (cpu_util.cpp, layer_att.cu:368-482,
 // layer_ffn.cu:190-248); see the comments at each contraction.
-#include "gemm.cuh"
+#include "gemm_row.cuh"
 #include "kernels.cuh"
+#include "label_rank.cuh"
 #include <nccl.h>
 #include <vector>
 #include <cmath>
@@ -114,6 +115,7 @@ struct BatchDev {
     int *target = nullptr;
     std::vector<int *> span_start, span_finish, rev_first, rev_last;
     std::vector<void *> att_layout; // per attention type, see AttBwdPlan
+    std::vector<bool> layout_ready; // per attention type: made at the first backward pass of the batch (scoring does without)
     std::vector<bool> ds_fits;      // per attention type: the batch's score gradients fit the model's buffer
     int *scan_tmp = nullptr; // batch_scan_tmp_elems(max_nodes)
     int *status = nullptr;   // {code, where, detail, detail}: the first malformed element seen since it was last reported
@@ -1196,6 +1198,7 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
     b.rev_first.resize(na);
     b.rev_last.resize(na);
     b.att_layout.resize(na);
+    b.layout_ready.assign(na, false);
     b.ds_fits.assign(na, true);
     for (int a = 0; a < na; ++a) {
         M_TRY(dalloc(m, &b.span_start[a], (size_t)T));
@@ -1287,20 +1290,45 @@ int trace(ts2_model *m, const char *name, int layer, const void *p, size_t bytes
 }
 #define TRACE(name, layer, p, bytes, kind) M_TRY(trace(m, name, layer, p, bytes, kind))
 
+// where the normalised state at layer boundary l goes: the next layer's operand, or the final layer's two
+RowOp norm_op(const ts2_model *m, int l)
+{
+    RowOp op;
+    op.form = ROW_NORM;
+    op.s_act = m->s_act;
+    op.n_fast = l < m->L ? m->layers[l].n_fast : m->nF_fast;
+    op.n16 = l < m->L ? nullptr : m->nF16;
+    return op;
+}
+
 // ---- forward -------------------------------------------------------------------------
-int forward(ts2_model *m)
+// train: a backward pass follows
+int forward(ts2_model *m, bool train)
 {
     Ctx c = ctx_of(m);
     const int T = m->batch.node_count, D = m->D, H = m->H;
-    const BatchDev &b = m->batch;
+    BatchDev &b = m->batch;
     const size_t fsz = fast_size(m);
     m->gemm_tag = GEMM_TAG_FWD;
-    M_TRY(embed_forward(c, m->embed16, m->mats[0].sko, b.label_arr, b.label_ptr, T, D, m->states[0], m->absmax, m->L + 2, m->logp));
+    const RowOp first = norm_op(m, 0);
+    StepStart start;
+    start.zero = m->absmax, start.n_zero = m->L + 2, start.zero_scalar = m->logp;
+    if (train) {
+        if (!m->grads_dirty)
+            start.clear = m->grad_flat + m->buckets[0].off, start.n_clear = m->buckets[0].elems;
+        if (!b.ix_sorted && b.ix.n <= LABEL_RANK_MAX && !(m->descr.flags & TS2_MPF_DISABLE_TUNE_EMBED))
+            start.sort = &b.ix;
+    }
+    M_TRY(embed_forward(c, m->embed16, m->mats[0].sko, b.label_arr, b.label_ptr, T, D, m->states[0], first.n_fast, first.n16, start));
+    if (start.sort) {
+        b.ix.sorted = 1;
+        b.ix_sorted = true;
+    }
     TRACE("state", 0, m->states[0], (size_t)T * D * 4, TR_F32);
     for (int l = 0; l < m->L; ++l) {
         Layer &ly = m->layers[l];
         const int W = ly.wide, C = ly.ncat * W;
-        M_TRY(tilenorm_forward(c, m->states[l], T, D, ly.n_fast, nullptr));
+        const RowOp norm = norm_op(m, l + 1); // every layer writes the normalised form of the state it leaves
         TRACE("n_fast", l, ly.n_fast, (size_t)T * D * fsz, fsz == 2 ? TR_F16 : TR_RAW);
         if (ly.type == TS2_LAYER_MOE) {
             // TMoELayer::ComputeForward, layer_moe.cu:459-486, on expert-sorted rows
@@ -1358,13 +1386,8 @@ int forward(ts2_model *m)
                     M_TRY(ep_exchange_peer(m, ly, false, ts2_model::PB_MOE_Y, m->own_y, yb, false));
                 else
                     M_TRY(ep_exchange(m, ly, false, m->own_y, m->moe_y, yb, false));
-                if (y16)
-                    M_TRY(moe_combine_half(c, (const __half *)m->own_y, ly.slot_of, T, K, D, m->states[l], m->states[l + 1]));
-                else
-                    M_TRY(moe_combine(c, m->own_y, ly.slot_of, T, K, D, m->states[l], m->states[l + 1]));
-            } else {
-                M_TRY(moe_combine(c, m->moe_y, ly.slot_of, T, K, D, m->states[l], m->states[l + 1]));
             }
+            M_TRY(moe_combine(c, m->ep ? m->own_y : m->moe_y, y16, ly.slot_of, T, K, D, m->states[l], m->states[l + 1], norm.n_fast, norm.n16));
             TRACE("state", l + 1, m->states[l + 1], (size_t)T * D * 4, TR_F32);
             continue;
         }
@@ -1405,10 +1428,11 @@ int forward(ts2_model *m)
         e2.dyn_scale = m->mats[ly.mat0 + ly.ncat].sko;
         e2.out_kind = TS2_OUT_F32_ADD;
         e2.c_in = m->states[l];
-        M_TRY(gemm_tn(m, m->kind, T, D, W, ly.rg, W, ly.Wc, W, m->states[l + 1], D, e2));
+        GemmArgs out = tn_args(m, m->kind, T, D, W, ly.rg, W, ly.Wc, W, m->states[l + 1], D, e2);
+        M_TRY(gemm(out));
+        M_TRY(tilenorm_forward(c, m->states[l + 1], T, D, norm.n_fast, norm.n16));
         TRACE("state", l + 1, m->states[l + 1], (size_t)T * D * 4, TR_F32);
     }
-    M_TRY(tilenorm_forward(c, m->states[m->L], T, D, m->nF_fast, m->nF16));
     TRACE("nF16", -1, m->nF16, (size_t)T * D * 2, TR_F16);
     return TS2_OK;
 }
@@ -1423,12 +1447,12 @@ int final_layer(ts2_model *m, bool backward)
     const float gs = (1.f / LOG2F) * LOG2F;                // CalcFinalLayerMult() * LOG2, cpu_transformer.cpp:159
     const bool tune_final = !(m->descr.flags & TS2_MPF_DISABLE_TUNE_FINAL_LAYER);
     m->gemm_tag = GEMM_TAG_FINAL;
+    Epilogue e;
+    e.alpha = sqrtf(1.0f / D) / (m->s_act * 32.f) * (1.f / LOG2F); // MulForward scale * CalcFinalLayerMult()
+    e.dyn_scale = m->mats[1].sko;
+    e.out_kind = TS2_OUT_F16;
     for (int r0 = 0; r0 < T; r0 += m->chunk) {
         const int rows = std::min(m->chunk, T - r0);
-        Epilogue e;
-        e.alpha = sqrtf(1.0f / D) / (m->s_act * 32.f) * (1.f / LOG2F); // MulForward scale * CalcFinalLayerMult()
-        e.dyn_scale = m->mats[1].sko;
-        e.out_kind = TS2_OUT_F16;
         M_TRY(gemm_tn(m, m->kind, rows, V, D, (const uint8_t *)m->nF_fast + (size_t)r0 * D * fs, D, m->Wf, D, m->logits, V, e));
         TRACE("logits", r0 / m->chunk, m->logits, (size_t)rows * V * 2, TR_F16);
         M_TRY(softmax_ce(c, m->logits, rows, V, m->has_bias ? m->bias : nullptr, m->batch.target + r0, gscale, m->logp, backward));
@@ -1440,15 +1464,16 @@ int final_layer(ts2_model *m, bool backward)
         ex.alpha = sqrtf(1.0f / D) / 32.f * gs / gscale;
         ex.dyn_scale = m->mats[1].sko;
         ex.out_kind = TS2_OUT_F32;
-        M_TRY(gemm_tn(m, KIND_F16, rows, D, V, m->logits, V, m->WfT16, V, m->dn + (size_t)r0 * D, D, ex));
+        const GemmArgs dx = tn_args(m, KIND_F16, rows, D, V, m->logits, V, m->WfT16, V, m->dn + (size_t)r0 * D, D, ex);
+        // dWf += g^T . nF   (SumRankOne, cpu_transformer.cpp:168)
+        Epilogue ew;
+        ew.alpha = gs / gscale;
+        ew.out_kind = m->grads_dirty || r0 ? TS2_OUT_F32_ADD : TS2_OUT_F32;
+        const GemmArgs dw = dw_args(m, KIND_F16, V, D, rows, m->logits, V, m->nF16 + (size_t)r0 * D, D, m->mats[1].grad, ew);
+        M_TRY(gemm(dx));
         TRACE("dnF", r0 / m->chunk, m->dn + (size_t)r0 * D, (size_t)rows * D * 4, TR_F32);
-        if (tune_final) {
-            // dWf += g^T . nF   (SumRankOne, cpu_transformer.cpp:168)
-            Epilogue ew;
-            ew.alpha = gs / gscale;
-            ew.out_kind = m->grads_dirty || r0 ? TS2_OUT_F32_ADD : TS2_OUT_F32;
-            M_TRY(gemm_dw(m, KIND_F16, V, D, rows, m->logits, V, m->nF16 + (size_t)r0 * D, D, m->mats[1].grad, ew));
-        }
+        if (tune_final)
+            M_TRY(gemm(dw));
     }
     if (backward && tune_final)
         TRACE("dW_final", -1, m->mats[1].grad, (size_t)V * D * 4, TR_F32);
@@ -1605,8 +1630,9 @@ int backward_dense_int8(ts2_model *m, int l)
     return TS2_OK;
 }
 
-// Zeroes what an accumulation adds to from its first call on: the embedding (only the rows of the batch's labels are
-// written), expert matrices (an expert without rows is not), and what the model's flags keep from being written at all.
+// Zeroes what an accumulation adds to from its first call on, the embedding aside (only the rows of the batch's labels are
+// written; the step's first kernel clears it): expert matrices (an expert without rows is not), and what the model's flags keep
+// from being written at all.
 // The rest, most of the bytes, is overwritten by its first dW contraction.
 int clear_gradient(ts2_model *m)
 {
@@ -1614,7 +1640,7 @@ int clear_gradient(ts2_model *m)
     size_t lo = 0, hi = 0; // adjacent buckets go together
     for (size_t b = 0; b <= m->buckets.size(); ++b) {
         const bool end = b == m->buckets.size();
-        if (!end && !(b == 0 || m->buckets[b].expert_matrix || !(b == 1 ? tune_final : tune_layers)))
+        if (!end && (b == 0 || !(m->buckets[b].expert_matrix || !(b == 1 ? tune_final : tune_layers))))
             continue;
         if (end || m->buckets[b].off != hi) {
             if (hi > lo)
@@ -1632,10 +1658,17 @@ int backward(ts2_model *m)
 {
     Ctx c = ctx_of(m);
     const int T = m->batch.node_count, D = m->D, H = m->H, L = m->L;
-    const BatchDev &b = m->batch;
+    BatchDev &b = m->batch;
     const bool tune_layers = !(m->descr.flags & TS2_MPF_DISABLE_TUNE_LAYERS);
     M_TRY(final_layer(m, true));
     TS2_CUDA(cudaEventRecord(m->ev_loss, m->stream)); // see ts2_avg_train_err
+    for (const Layer &ly : m->layers) {
+        const int a = ly.att_type;
+        if (ly.type != TS2_LAYER_ATT || b.layout_ready[a])
+            continue;
+        M_TRY(att_layout(c, b.span_start[a], b.span_finish[a], b.rev_first[a], b.rev_last[a], T, b.att_layout[a]));
+        b.layout_ready[a] = true;
+    }
     m->gemm_tag = GEMM_TAG_DX;
     M_TRY(reduce_matrices(m, 1, 2));
     M_TRY(gradients_complete(m, 1));
@@ -1715,12 +1748,6 @@ int backward(ts2_model *m)
                     M_TRY(ep_exchange_peer(m, ly, false, ts2_model::PB_MOE_Y, m->own_y, yb, false));
                 else
                     M_TRY(ep_exchange(m, ly, false, m->own_y, m->moe_y, yb, false));
-                if (y16)
-                    M_TRY(moe_combine_half(c, (const __half *)m->own_y, ly.slot_of, T, K, D, nullptr, m->dn));
-                else
-                    M_TRY(moe_combine(c, m->own_y, ly.slot_of, T, K, D, nullptr, m->dn));
-            } else {
-                M_TRY(moe_combine(c, m->moe_y, ly.slot_of, T, K, D, nullptr, m->dn));
             }
             if (tune_layers && xrows) {
                 Epilogue e5;
@@ -1734,7 +1761,9 @@ int backward(ts2_model *m)
                                      m->mats[ly.mat0 + 1].grad, (int64_t)X * D, e5));
             }
             M_TRY(reduce_matrices(m, ly.mat0, l + 1 < L ? m->layers[l + 1].mat0 : (int)m->mats.size()));
-            M_TRY(tilenorm_backward(c, m->states[l], m->dn, m->fscale, 1.f, T, D, m->g, true, m->absmax + l, m->health + l, m->step_no));
+            const float *y = m->ep ? m->own_y : m->moe_y;
+            M_TRY(moe_combine_backward(c, y, y16, ly.slot_of, T, K, D, m->dn, m->states[l], m->fscale, m->g, m->absmax + l, m->health + l,
+                                       m->step_no));
             TRACE("g", l, m->g, (size_t)T * D * 4, TR_F32);
             M_TRY(tap_gradient(m, l));
             M_TRY(gradients_complete(m, ly.mat0));
@@ -1963,9 +1992,10 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
         const int *raw = (const int *)b.raw;
         spans[a] = {raw + o_ptr[a], raw + o_start[a], raw + o_finish[a], n_spans[a], b.span_start[a], b.span_finish[a], b.rev_first[a], b.rev_last[a]};
     }
-    M_TRY(batch_prepare(c, bt, spans.data(), na, b.ix, &b.ix_sorted));
+    M_TRY(batch_prepare(c, bt, spans.data(), na, b.ix));
+    b.ix_sorted = false;
     for (int a = 0; a < na; ++a) {
-        M_TRY(att_layout(c, b.span_start[a], b.span_finish[a], b.rev_first[a], b.rev_last[a], T, b.att_layout[a]));
+        b.layout_ready[a] = false;
         // a big batch: count what its own spans need (a pass over them on the host, beside the step that is running)
         b.ds_fits[a] = m->att_bwd.ds && (att_ds_bytes(T, nullptr, nullptr, nullptr) * m->H <= m->att_bwd.ds_bytes ||
                                          att_ds_bytes(T, nd->att[a].span_ptr, nd->att[a].span_start, nd->att[a].span_finish) * m->H <=
@@ -2222,7 +2252,7 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
     }
     if (!m->grads_dirty)
         M_TRY(clear_gradient(m));
-    M_TRY(forward(m));
+    M_TRY(forward(m, true));
     // an accumulated gradient of earlier calls sits in the same buffer: the per-layer sums below then cover it too
     const bool dp = m->comm && m->world > 1;
     m->reduce_in_backward = add_to_model == TS2_GRADIENT_APPLY && dp;
@@ -2275,7 +2305,7 @@ int ts2_forward_score(ts2_model *m, float *out_score)
     m->trace_on = false;
     float *const step_slot = m->logp;
     m->logp = m->logp_ring + ts2_model::LOSS_RING; // the last training step's slot stays readable
-    int rc = forward(m);
+    int rc = forward(m, false);
     if (rc == TS2_OK)
         rc = final_layer(m, false);
     float *const score_slot = m->logp;
