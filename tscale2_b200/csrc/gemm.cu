@@ -18,12 +18,14 @@
 // Fp16MatMul (src/lib/cuda/cuda_fp16.cuh:49-164), and, because the dW operands are read
 // token-major through MN-major shared-memory descriptors, also the per-step transposes
 // (src/gpt/compute/matmul_fwdbwd.cuh:149-162,169-280).
+#include "gemm_row.cuh"
 #include "gemm_params.cuh"
 #include "fast_types.cuh"
 #include <cuda.h>
 #include <vector>
 #include <type_traits>
 #include <mutex>
+#include <algorithm>
 
 namespace ts2 {
 
@@ -810,7 +812,7 @@ int make_tensor_map(::CUtensorMap_st *tm, const void *base, int es, int64_t inne
 
 static int elem_size(int kind) { return (kind == KIND_F16 || kind == KIND_BF16) ? 2 : 1; }
 
-static uint32_t instr_desc(int kind, bool mn, int bm, int bn)
+uint32_t gemm_instr_desc(int kind, bool mn, int bm, int bn)
 {
     uint32_t c_fmt, ab_fmt;
     switch (kind) {
@@ -943,6 +945,14 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
 bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N)
 {
     return kind == KIND_E4M3 && !dynamic_units() && N % 128 == 0 && (N % 256 == 0 || N > 512) && ceil_div(M, 2 * BM) * ceil_div(N, 256) >= sm_count(device) / 2;
+}
+
+bool gemm_takes_row(int device, int kind, int64_t M, int64_t N, int64_t K, int form)
+{
+    if (K <= 0 || N % 128 || form == ROW_PLAIN)
+        return false;
+    const Plan pl = make_plan(device, kind, false, M, N, K, form == ROW_NORM ? FORM_ADD : FORM_F32);
+    return pl.pair() && pl.splits == 1;
 }
 
 size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int out_kind)
@@ -1081,6 +1091,27 @@ static cudaEvent_t pooled_event()
     return e;
 }
 
+GemmTimed gemm_timed_begin(cudaStream_t stream)
+{
+    GemmTimed t;
+    std::lock_guard<std::mutex> lk(g_time_mu);
+    if (g_time_on) {
+        t.a = pooled_event();
+        t.b = pooled_event();
+        cudaEventRecord(t.a, stream);
+    }
+    return t;
+}
+
+void gemm_timed_end(const GemmTimed &t, cudaStream_t stream, double flops, double bytes, int tag)
+{
+    if (!t.a)
+        return;
+    cudaEventRecord(t.b, stream);
+    std::lock_guard<std::mutex> lk(g_time_mu);
+    g_timed.push_back({t.a, t.b, flops, bytes, tag});
+}
+
 template <int BM_, int BN>
 static int reduce_splits(const GemmArgs &a, const Plan &pl, const GemmParams &p)
 {
@@ -1146,6 +1177,12 @@ int gemm(const GemmArgs &a)
                     a.ldc != bwd_ld || !(gate_bwd ? a.epi.bwd_dscale && a.epi.bwd_dout : a.epi.act_scale != nullptr) ||
                     (((uintptr_t)a.epi.bwd_wg | (uintptr_t)a.epi.bwd_o | (uintptr_t)a.epi.bwd_dout) & 15) || !pl.pair() || pl.splits != 1))
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of the activation's backward form");
+    const RowOp *const op = a.epi.row;
+    const bool norm_bwd = op && op->form == ROW_NORM_BWD, norm = op && op->form == ROW_NORM;
+    if (op && (!(norm || norm_bwd) || !pl.pair() || pl.splits != 1 || a.N % 128 || a.mn_major || a.group_mode || a.ldc != a.N ||
+               a.epi.col_scale || (!norm_bwd && a.epi.row_scale) ||
+               a.epi.out_kind != (norm_bwd ? TS2_OUT_F32 : TS2_OUT_F32_ADD)))
+        return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of a row-wise epilogue");
     const size_t room = a.workspace ? a.workspace_bytes : 0;
     if (pl.workspace() > room) {
         // The fastest plan splits outputs that others leave whole (2048 x 1280 from 16384 tokens): without scratch for it the
@@ -1179,7 +1216,7 @@ int gemm(const GemmArgs &a)
     p.splits = pl.splits;
     p.k_blocks = pl.k_blocks;
     p.kb_per_split = pl.kb_per_split;
-    p.idesc = instr_desc(a.kind, a.mn_major, pl.bm, pl.bn);
+    p.idesc = gemm_instr_desc(a.kind, a.mn_major, pl.bm, pl.bn);
     p.C = a.C;
     p.ldc = a.ldc;
     p.alpha = a.epi.alpha;
@@ -1220,12 +1257,24 @@ int gemm(const GemmArgs &a)
                 rc = make_tmap(&tmCin, a.epi.bwd_wg, 2, bwd_ld, a.M, bwd_ld, 32);
             if (gate_bwd && rc == TS2_OK && (rc = make_tmap(&tmX, a.epi.bwd_o, 2, a.N, a.M, a.N, 32)) == TS2_OK)
                 rc = make_tmap(&tmY, a.epi.bwd_dout, 2, a.N, a.M, a.N, 32);
+        } else if (norm_bwd) {
+            if ((rc = make_tmap(&tmC, op->g, 4, a.N, a.M, a.N, 32)) == TS2_OK && (rc = make_tmap(&tmX, op->x, 4, a.N, a.M, a.N, 32)) == TS2_OK)
+                tmCin = tmC;
+            p.norm_add = op->add;
+            p.norm_dyn = op->dyn;
+            p.norm_absmax = op->absmax, p.norm_health = op->health, p.norm_step = op->step_no;
         } else if (pl.splits > 1)
             rc = make_tmap(&tmC, a.workspace, 4, pl.bn, (int64_t)pl.m_tiles * pl.n_tiles * pl.splits * pl.bm, pl.bn, 32);
         else
             rc = make_tmap(&tmC, a.C, out_es, a.N, a.M, a.ldc, 32, paired ? 64 : STAGE_ROW_BYTES);
         if (rc == TS2_OK && pl.splits == 1 && a.epi.out_kind == TS2_OUT_F32_ADD)
             rc = make_tmap(&tmCin, p.c_in, 4, a.N, a.M, a.ldc, 32);
+        if (norm && rc == TS2_OK) {
+            if ((rc = make_tmap(&tmX, op->n_fast, es, a.N, a.M, a.N, 32)) == TS2_OK && op->n16)
+                rc = make_tmap(&tmY, op->n16, 2, a.N, a.M, a.N, 32);
+            p.norm16 = op->n16 != nullptr;
+            p.act_mult = op->s_act;
+        }
         if (rc != TS2_OK)
             return rc;
     } else if (pl.splits == 1 && a.group_mode != 2) {
@@ -1234,19 +1283,7 @@ int gemm(const GemmArgs &a)
         p.tma_store = 1;
     }
 
-    cudaEvent_t ea = nullptr, eb = nullptr;
-    bool timed;
-    {
-        std::lock_guard<std::mutex> lk(g_time_mu);
-        timed = g_time_on;
-        if (timed) {
-            ea = pooled_event();
-            eb = pooled_event();
-        }
-    }
-    if (timed)
-        cudaEventRecord(ea, a.stream);
-
+    const GemmTimed timed = gemm_timed_begin(a.stream);
     const int mma = (a.kind == KIND_E4M3) ? 0 : (a.kind == KIND_I8 ? 2 : 1);
 #define TS2_GEMM_CASE(BN_, ES_, MMA_, MN_)                                   \
     if (pl.bn == BN_ && es == ES_ && mma == MMA_ && a.mn_major == MN_)       \
@@ -1255,7 +1292,7 @@ int gemm(const GemmArgs &a)
     if (pl.pair()) {
         const int sms = std::max(2, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)) & ~1;
         const bool out16 = pl.splits == 1 && (a.epi.out_kind == TS2_OUT_F16 || a.epi.out_kind == TS2_OUT_BF16);
-        const PairForm form = gate_bwd ? P_GATE_BWD : act_bwd ? P_ACT_BWD : paired ? P_GATED : out16 ? P_16 : P_F32;
+        const PairForm form = norm_bwd ? P_NORM_BWD : norm ? P_NORM : gate_bwd ? P_GATE_BWD : act_bwd ? P_ACT_BWD : paired ? P_GATED : out16 ? P_16 : P_F32;
         rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, form, std::min(pl.grid, sms), tmA, tmB, tmC, tmCin, tmX, tmY, p);
         if (rc == TS2_OK && pl.splits > 1)
             rc = reduce_splits<2 * BM, 256>(a, pl, p);
@@ -1287,15 +1324,12 @@ int gemm(const GemmArgs &a)
 #undef TS2_GEMM_CASE
     if (rc == TS2_ERR_UNSUPPORTED)
         return fail(rc, "gemm: unsupported configuration");
-    if (timed) {
-        cudaEventRecord(eb, a.stream);
-        std::lock_guard<std::mutex> lk(g_time_mu);
-        // algorithmic bytes: both operands once, the output once, the residual input of the accumulate form once
-        const double mn = (double)a.M * (double)a.N;
-        const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + (gate_bwd ? mn * 7 : act_bwd ? mn * 6 : mn * out_es) +
-                             (a.epi.out_kind == TS2_OUT_F32_ADD ? mn * 4 : 0);
-        g_timed.push_back({ea, eb, 2.0 * mn * (double)a.K, bytes, a.tag});
-    }
+    // algorithmic bytes: both operands once, the output once, the residual input of the accumulate form once
+    const double mn = (double)a.M * (double)a.N;
+    const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + (gate_bwd ? mn * 7 : act_bwd ? mn * 6 : norm_bwd ? mn * 12 : mn * out_es) +
+                         (norm ? mn * (es + (op->n16 ? 2 : 0)) : 0) +
+                         (a.epi.out_kind == TS2_OUT_F32_ADD ? mn * 4 : 0);
+    gemm_timed_end(timed, a.stream, 2.0 * mn * (double)a.K, bytes, a.tag);
     return rc;
 }
 
@@ -1412,7 +1446,7 @@ extern "C" int ts2_gemm_dw_noalloc(int device, void *stream, int prec, int out_k
     p.splits = pl.splits;
     p.k_blocks = pl.k_blocks;
     p.kb_per_split = pl.kb_per_split;
-    p.idesc = instr_desc(kind, true, BM, pl.bn);
+    p.idesc = gemm_instr_desc(kind, true, BM, pl.bn);
     p.C = dW;
     p.ldc = in_dim;
     p.alpha = alpha;

@@ -9,6 +9,8 @@ namespace ts2 {
 
 enum GemmKind { KIND_E4M3 = 0, KIND_F16 = 1, KIND_I8 = 2, KIND_BF16 = 3 };
 
+struct RowOp;
+
 struct Epilogue {
     float alpha = 1.f;
     const float *dyn_scale = nullptr;  // device scalar multiplied in (loss-scale bookkeeping)
@@ -38,6 +40,9 @@ struct Epilogue {
     const void *bwd_wg = nullptr, *bwd_o = nullptr;
     void *bwd_dout = nullptr;
     float *bwd_dscale = nullptr;
+    // The row-wise step that follows (gemm_row.cuh), where gemm_takes_row() says so: ROW_NORM behind the accumulate form and
+    // ROW_NORM_BWD behind the plain one.
+    const RowOp *row = nullptr;
 };
 
 struct GemmArgs {
@@ -75,6 +80,9 @@ void gemm_plan(int device, int kind, bool mn_major, int64_t M, int64_t N, int64_
                int *splits);
 // whether the epilogue can apply the backward of the gated activation (Epilogue::bwd_wg) to a product of this shape
 bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N);
+
+// whether the epilogue can apply Epilogue::row of this form (RowForm) to a product of this shape
+bool gemm_takes_row(int device, int kind, int64_t M, int64_t N, int64_t K, int form);
 
 // 2-D TMA descriptor over a row-major [rows][ld] array of es-byte elements: box = row_bytes (128 or 64, swizzled alike) x
 // box_rows, out-of-range elements read as zero

@@ -17,7 +17,7 @@
 // Units (tile, K split) are assigned statically to clusters.  Every wait is bounded, as in gemm.cu; a CTA leaves only
 // after a cluster barrier, so no barrier or copy of its peer can still refer to it.
 #include "gemm_params.cuh"
-#include "fast_types.cuh"
+#include "row_math.cuh"
 
 namespace ts2 {
 
@@ -27,6 +27,7 @@ constexpr int PM = 256, PN = 256; // the pair's tile
 constexpr int P_HALF_BYTES = 128 * STAGE_ROW_BYTES; // a CTA's half of either operand, one K block
 constexpr int P_STAGE_BYTES = 2 * P_HALF_BYTES;
 constexpr int P_THREADS = 320, P_THREADS_16 = 576;
+constexpr bool epi8(int form) { return form == P_F32 || form == P_NORM || form == P_NORM_BWD; } // 8 epilogue warps, else 16
 constexpr bool is_bwd(int form) { return form == P_ACT_BWD || form == P_GATE_BWD; }
 // shared memory of a form: ring, epilogue staging, barriers, alignment slack
 template <int FORM>
@@ -122,9 +123,9 @@ __device__ __forceinline__ PairUnit pair_unit(const GemmParams &p, int u)
 // 16-byte piece c of row r of a 32 x 128 byte block in the 128-byte swizzle
 __device__ __forceinline__ uint32_t piece(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
-// FORM of the epilogue (PairForm): 8 epilogue warps in P_F32, 16 in the others
+// FORM of the epilogue (PairForm)
 template <int ES, int MMA, bool MN, int FORM>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_THREADS : P_THREADS_16, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(epi8(FORM) ? P_THREADS : P_THREADS_16, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmCin,
                      const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmParams p)
@@ -132,7 +133,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
     constexpr int ELEMS_PER_ROW = STAGE_ROW_BYTES / ES;
     constexpr int UMMA_K = 32 / ES, K_STEPS = 4, BK = ELEMS_PER_ROW;
     constexpr bool GATED = FORM == P_GATED;
-    constexpr int EPI_WARPS = FORM == P_F32 ? 8 : 16;
+    constexpr int EPI_WARPS = epi8(FORM) ? 8 : 16;
     constexpr int P_STAGES = PairSmem<FORM>::STAGES, P_STG_OFF = PairSmem<FORM>::STG_OFF, P_BAR_OFF = PairSmem<FORM>::BAR_OFF;
 
     extern __shared__ uint8_t pair_smem[];
@@ -645,6 +646,228 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FORM == P_F32 ? P_TH
                 if (acc == 0)
                     acc_phase ^= 1;
             }
+        } else if constexpr (FORM == P_NORM || FORM == P_NORM_BWD) {
+            // The row-wise step behind a layer's last contraction: a thread has the 128 columns of a normalisation tile of its
+            // row, 32 at a time through the warp's three staging buffers.  A buffer is taken again when all stores but the most
+            // recent one have read theirs: `cur` holds the block that was fetched ahead, `prev` was stored from last, the third
+            // one is free.
+            // P_NORM: C = c_in + product, and its tile normalisation, which as a kernel of its own read C back (65536 x 768,
+            // e4m3: contraction 121 and normalisation 48 -> 138 us).  P_NORM_BWD: the product d (scale-free, times dyn_scale2) is the gradient of the normalised x; the
+            // accumulator is read twice, beside x for the two sums over the tile and beside g for the result; the product
+            // used to go through memory (65536 x 768, e4m3: contraction 239 and normalisation 114 -> 277 us).
+            constexpr bool BWD = FORM == P_NORM_BWD;
+            const int half = ew >> 2;
+            uint8_t *const stg = smem + P_STG_OFF + ew * (3 * 4096);
+            const uint32_t cin_bar = cin0 + 8 * 3 * ew;
+            int cur = 0, prev = 2;
+            uint32_t cin_phase = 0; // one bit per buffer
+            auto fetch = [&](const CUtensorMap *tm, int u, int b, int to) {
+                if (lane == 0) {
+                    const PairUnit un = pair_unit(p, u);
+                    mbar_arrive_expect_tx(cin_bar + 8 * to, 4096);
+                    tma_load_2d(smem_u32(stg + to * 4096), tm, cin_bar + 8 * to, un.n0 + half * 128 + b * 32, un.m0 + (int)rank * 128 + quarter * 32);
+                }
+            };
+            const CUtensorMap *const first_in = BWD ? &tmX : &tmCin;
+            if (first < units)
+                fetch(first_in, first, 0, 0);
+            bool ok = true;
+            float mx = 0.f;
+            for (int u = first; u < units; u += step) {
+                const PairUnit un = pair_unit(p, u);
+                const int m0 = un.m0 + (int)rank * 128, col = un.n0 + half * 128;
+                const bool inside = col < p.N;
+                ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag));
+                if (!ok)
+                    break;
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * PN + half * 128;
+                auto value = [&](uint32_t r) { return (MMA == 2) ? (float)(int)r : __uint_as_float(r); };
+                auto release = [&]() { // the accumulator is read: the next tile may have it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive_cluster(map_to_leader(tempty0 + 8 * acc));
+                };
+                // the block that was fetched ahead is in `cur`; the one after it goes into the free buffer
+                auto landed = [&](const CUtensorMap *tm, int nu, int nb) {
+                    const int free_buf = 3 - cur - prev;
+                    if (lane == 0)
+                        bulk_wait_read<1>();
+                    if (nu < units)
+                        fetch(tm, nu, nb, free_buf);
+                    const bool got = __all_sync(0xffffffffu, mbar_wait(cin_bar + 8 * cur, (cin_phase >> cur) & 1, abort_flag));
+                    cin_phase ^= 1u << cur;
+                    return got;
+                };
+                auto stored = [&](const CUtensorMap *tm, int x) { // the block in `cur` leaves; a group is committed also for a clipped one
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (inside)
+                            tma_store_2d(tm, smem_u32(stg + cur * 4096), x, m0 + quarter * 32);
+                        bulk_commit();
+                    }
+                    const int next = 3 - cur - prev;
+                    prev = cur;
+                    cur = next;
+                };
+                float keep[4][32], sum2 = 0.f;
+                if constexpr (!BWD) {
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        uint32_t r[32];
+                        tmem_ld32(taddr + b * 32, r);
+                        tmem_ld_wait();
+                        if (b == 3)
+                            release();
+                        if (!(ok = landed(&tmCin, b < 3 ? u : u + step, (b + 1) & 3)))
+                            break;
+                        uint8_t *blk = stg + cur * 4096;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            float4 *q = (float4 *)(blk + piece(lane, i));
+                            const float4 c = *q;
+                            const float4 o = make_float4(c.x + value(r[4 * i]) * alpha, c.y + value(r[4 * i + 1]) * alpha, c.z + value(r[4 * i + 2]) * alpha,
+                                                         c.w + value(r[4 * i + 3]) * alpha);
+                            *q = o;
+                            sum2 += dot4(o, o);
+                            keep[b][4 * i] = o.x, keep[b][4 * i + 1] = o.y, keep[b][4 * i + 2] = o.z, keep[b][4 * i + 3] = o.w;
+                        }
+                        stored(&tmC, col + b * 32);
+                    }
+                    if (!ok)
+                        break;
+                    // `cur` now holds the next tile's first block (or nothing): the normalised rows leave from the free buffer
+                    const float scale = tile_scale(sum2), mult = p.act_mult;
+                    auto leave = [&](const CUtensorMap *tm, int x, auto words) { // words(i): 16-byte piece i of this row
+                        const int buf = 3 - cur - prev;
+                        if (lane == 0)
+                            bulk_wait_read<1>();
+                        __syncwarp();
+                        uint8_t *blk = stg + buf * 4096;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            *(uint4 *)(blk + piece(lane, i)) = words(i);
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (inside)
+                                tma_store_2d(tm, smem_u32(blk), x, m0 + quarter * 32);
+                            bulk_commit();
+                        }
+                        prev = buf;
+                    };
+                    auto half8 = [&](const float *v, float s) {
+                        float f[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            f[j] = v[j] * scale * s;
+                        return make_uint4(bits_from_h2(sat_half2(f[0], f[1])), bits_from_h2(sat_half2(f[2], f[3])), bits_from_h2(sat_half2(f[4], f[5])),
+                                          bits_from_h2(sat_half2(f[6], f[7])));
+                    };
+                    if constexpr (MMA == 1) {
+#pragma unroll
+                        for (int hb = 0; hb < 2; ++hb)
+                            leave(&tmX, col + hb * 64, [&](int i) { return half8(&keep[2 * hb + (i >> 2)][(i & 3) * 8], mult); });
+                    } else {
+                        leave(&tmX, col, [&](int i) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float *v = &keep[i >> 1][(i & 1) * 16 + 4 * j];
+                                const float4 f = scale4(scale4(make_float4(v[0], v[1], v[2], v[3]), scale), mult);
+                                if (MMA == 0) {
+                                    __nv_fp8x4_e4m3 pk(f);
+                                    w[j] = pk.__x;
+                                } else {
+                                    w[j] = sat_i8(f.x) | (sat_i8(f.y) << 8) | (sat_i8(f.z) << 16) | (sat_i8(f.w) << 24);
+                                }
+                            }
+                            return make_uint4(w[0], w[1], w[2], w[3]);
+                        });
+                    }
+                    if (p.norm16) {
+#pragma unroll
+                        for (int hb = 0; hb < 2; ++hb)
+                            leave(&tmY, col + hb * 64, [&](int i) { return half8(&keep[2 * hb + (i >> 2)][(i & 3) * 8], 1.f); });
+                    }
+                } else {
+                    float dp = 0.f;
+                    const float rs = p.row_scale && m0 + row_in_cta < p.M ? alpha * __ldg(p.row_scale + m0 + row_in_cta) : alpha;
+                    const float dyn = p.norm_dyn ? __ldg(p.norm_dyn) : 1.f;
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) { // x beside the product: both sums over the tile
+                        uint32_t r[32];
+                        tmem_ld32(taddr + b * 32, r);
+                        tmem_ld_wait();
+                        if (!(ok = landed(b < 3 ? &tmX : &tmCin, u, (b + 1) & 3)))
+                            break;
+                        const uint8_t *blk = stg + cur * 4096;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const float4 x = *(const float4 *)(blk + piece(lane, i));
+                            const float4 d = scale4(make_float4(value(r[4 * i]) * rs, value(r[4 * i + 1]) * rs, value(r[4 * i + 2]) * rs, value(r[4 * i + 3]) * rs), dyn);
+                            sum2 += dot4(x, x);
+                            dp += dot4(x, d);
+                            keep[b][4 * i] = x.x, keep[b][4 * i + 1] = x.y, keep[b][4 * i + 2] = x.z, keep[b][4 * i + 3] = x.w;
+                        }
+                        // nothing leaves from this buffer: every lane has read its row.  An empty group keeps the count of those that
+                        // may still be reading.
+                        __syncwarp();
+                        if (lane == 0)
+                            bulk_commit();
+                        const int next = 3 - cur - prev;
+                        prev = cur;
+                        cur = next;
+                    }
+                    if (!ok)
+                        break;
+                    const float sigma = sum2 != 0.f ? dp / sum2 : 0.f, scale = sum2 != 0.f ? sqrtf(128.f / sum2) : 0.f;
+                    const bool row_in = m0 + row_in_cta < p.M && inside;
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) { // g beside it once more
+                        uint32_t r[32];
+                        tmem_ld32(taddr + b * 32, r);
+                        tmem_ld_wait();
+                        if (b == 3)
+                            release();
+                        if (!(ok = landed(b < 3 ? &tmCin : &tmX, b < 3 ? u : u + step, (b + 1) & 3)))
+                            break;
+                        uint8_t *blk = stg + cur * 4096;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            float4 *q = (float4 *)(blk + piece(lane, i));
+                            const float4 g = p.norm_add ? *q : make_float4(0, 0, 0, 0);
+                            const float4 d = scale4(make_float4(value(r[4 * i]) * rs, value(r[4 * i + 1]) * rs, value(r[4 * i + 2]) * rs, value(r[4 * i + 3]) * rs), dyn);
+                            const float *x = &keep[b][4 * i];
+                            const float4 o = make_float4(g.x + scale * (d.x - x[0] * sigma), g.y + scale * (d.y - x[1] * sigma),
+                                                         g.z + scale * (d.z - x[2] * sigma), g.w + scale * (d.w - x[3] * sigma));
+                            *q = o;
+                            if (row_in)
+                                mx = absmax4(mx, o);
+                        }
+                        stored(&tmC, col + b * 32);
+                    }
+                    if (!ok)
+                        break;
+                }
+                acc ^= 1;
+                if (acc == 0)
+                    acc_phase ^= 1;
+            }
+            if constexpr (BWD) {
+                mx = warp_max(mx);
+                if (ok && lane == 0 && first < units)
+                    absmax_report(mx, p.norm_absmax, p.norm_health, p.norm_step);
+            }
+            // abort path: a block may still be on its way into this CTA's shared memory
+            if (!ok && lane == 0) {
+                long long t0 = clock64();
+                for (int i = 0; i < 3; ++i)
+                    while (!mbar_try_wait(cin_bar + 8 * i, (cin_phase >> i) & 1) && clock64() - t0 < 200000000ll) {
+                    }
+            }
         } else {
             // The two warps of a quarter take 128 columns each, in 4 blocks of 32 rows x 32 columns.  Blocks go through the
             // warp's three staging buffers in turn; before a buffer is refilled all stores but the two most recent must have
@@ -789,7 +1012,7 @@ int launch_pair(int device, cudaStream_t stream, int grid, const CUtensorMap &tm
         TS2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<FORM>::TOTAL));
         configured[device & 15] = true;
     }
-    TS2_LAUNCH((kern), grid, FORM == P_F32 ? P_THREADS : P_THREADS_16, PairSmem<FORM>::TOTAL, stream, tmA, tmB, tmC, tmCin, tmX, tmY, p);
+    TS2_LAUNCH((kern), grid, epi8(FORM) ? P_THREADS : P_THREADS_16, PairSmem<FORM>::TOTAL, stream, tmA, tmB, tmC, tmCin, tmX, tmY, p);
     return TS2_OK;
 }
 
@@ -806,6 +1029,8 @@ int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, 
     TS2_PAIR_CASE(ES_, MMA_, false, P_F32)     \
     TS2_PAIR_CASE(ES_, MMA_, false, P_16)      \
     TS2_PAIR_CASE(ES_, MMA_, false, P_GATED)   \
+    TS2_PAIR_CASE(ES_, MMA_, false, P_NORM)    \
+    TS2_PAIR_CASE(ES_, MMA_, false, P_NORM_BWD) \
     TS2_PAIR_CASE(ES_, MMA_, true, P_F32)      \
     TS2_PAIR_CASE(ES_, MMA_, true, P_16)
     TS2_PAIR_CASES(1, 0)

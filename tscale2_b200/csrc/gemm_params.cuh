@@ -44,17 +44,31 @@ struct GemmParams {
     float act_mult = 1.f;
     int act_kind = 0; // format of act_out: 0 e4m3, 1 fp16, 2 int8
     float *bwd_dscale = nullptr; // backward of the attention gate (see Epilogue)
+    // tile normalisation behind the product, or its backward (see Epilogue)
+    int norm16 = 0, norm_add = 0;
+    const float *norm_dyn = nullptr;
+    unsigned *norm_absmax = nullptr, *norm_health = nullptr;
+    unsigned norm_step = 0;
 };
 
 // Forms of the epilogue of gemm_pair.cu: fp32 output, accumulate form and partial tiles; fp16 / bf16 output; gated
-// activation; its backward; backward of the attention gate (see Epilogue)
-enum PairForm { P_F32, P_16, P_GATED, P_ACT_BWD, P_GATE_BWD };
+// activation; its backward; backward of the attention gate; residual input + tile normalisation; backward of the latter;
+enum PairForm { P_F32, P_16, P_GATED, P_ACT_BWD, P_GATE_BWD, P_NORM, P_NORM_BWD };
 // gemm_pair.cu: the contraction on pairs of CTAs (tiles of 256 x 256).  tmB's box is 128 rows (K-major) or one K block
 // (token-major); tmC's and tmCin's are 32 rows x 128 bytes (P_GATED: tmC 32 x 64 bytes).  grid: CTAs, an even number.
 // P_ACT_BWD: tmC 32 rows x 64 bytes, tmCin [wide | gate] in 32 rows x 128; P_GATE_BWD: the same, and tmX: o, tmY: dout, both
-// 32 rows x 128; tmX, tmY otherwise unused
+// 32 rows x 128; P_NORM: tmX: n_fast, tmY: n16; P_NORM_BWD: tmX: x, tmCin and tmC: g; tmX, tmY otherwise unused
 int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, PairForm form, int grid, const CUtensorMap &tmA,
                      const CUtensorMap &tmB, const CUtensorMap &tmC, const CUtensorMap &tmCin, const CUtensorMap &tmX, const CUtensorMap &tmY,
                      const GemmParams &p);
+
+// instruction descriptor of a contraction on bm x bn tiles
+uint32_t gemm_instr_desc(int kind, bool mn, int bm, int bn);
+// timing statistics (gemm_timing_enable): events around a launch, null where they are off
+struct GemmTimed {
+    cudaEvent_t a = nullptr, b = nullptr;
+};
+GemmTimed gemm_timed_begin(cudaStream_t stream);
+void gemm_timed_end(const GemmTimed &t, cudaStream_t stream, double flops, double bytes, int tag);
 
 } // namespace ts2

@@ -1300,6 +1300,20 @@ RowOp norm_op(const ts2_model *m, int l)
     op.n16 = l < m->L ? nullptr : m->nF16;
     return op;
 }
+// the backward of the normalisation at layer boundary l behind the contraction that gives its gradient
+RowOp norm_backward_op(const ts2_model *m, int l, const float *dyn)
+{
+    RowOp op;
+    op.form = ROW_NORM_BWD;
+    op.x = m->states[l];
+    op.dyn = dyn;
+    op.g = m->g;
+    op.add = l < m->L;
+    op.absmax = m->absmax + l;
+    op.health = m->health + l;
+    op.step_no = m->step_no;
+    return op;
+}
 
 // ---- forward -------------------------------------------------------------------------
 // train: a backward pass follows
@@ -1429,8 +1443,11 @@ int forward(ts2_model *m, bool train)
         e2.out_kind = TS2_OUT_F32_ADD;
         e2.c_in = m->states[l];
         GemmArgs out = tn_args(m, m->kind, T, D, W, ly.rg, W, ly.Wc, W, m->states[l + 1], D, e2);
+        const bool fused = gemm_takes_row(m->device, m->kind, T, D, W, ROW_NORM);
+        out.epi.row = fused ? &norm : nullptr;
         M_TRY(gemm(out));
-        M_TRY(tilenorm_forward(c, m->states[l + 1], T, D, norm.n_fast, norm.n16));
+        if (!fused)
+            M_TRY(tilenorm_forward(c, m->states[l + 1], T, D, norm.n_fast, norm.n16));
         TRACE("state", l + 1, m->states[l + 1], (size_t)T * D * 4, TR_F32);
     }
     TRACE("nF16", -1, m->nF16, (size_t)T * D * 2, TR_F16);
@@ -1547,19 +1564,29 @@ AttBwdPlan att_plan(const ts2_model *m, const Layer &ly)
 }
 
 // Last step of a dense layer's backward pass: dn (scale-free) = dcat . (q_cat / 32) * sqrt(1 / D), the layer's weight
-// gradient from the same dcat, and the backward of the normalisation, which adds to the state gradient.
+// gradient from the same dcat, and the backward of the normalisation, which adds to the state gradient: in the epilogue where
+// pairs take the product, dn then never reaches memory (a traced step has it all the same).
 int input_gradient(ts2_model *m, int l, const GemmArgs &dn, const GemmArgs *dw_cat)
 {
     const Layer &ly = m->layers[l];
     const int T = m->batch.node_count, D = m->D;
-    M_TRY(gemm(dn));
+    const bool fused = gemm_takes_row(m->device, dn.kind, dn.M, dn.N, dn.K, ROW_NORM_BWD);
+    const RowOp op = norm_backward_op(m, l, m->fscale);
+    if (!fused || m->trace_on)
+        M_TRY(gemm(dn));
     TRACE("dn", l, m->dn, (size_t)T * D * 4, TR_F32);
+    if (fused) {
+        GemmArgs a = dn;
+        a.epi.row = &op;
+        M_TRY(gemm(a));
+    }
     if (dw_cat) {
         M_TRY(gemm(*dw_cat));
         TRACE("dW_cat", l, m->mats[ly.mat0].grad, (size_t)dw_cat->M * D * 4, TR_F32);
     }
     M_TRY(reduce_matrices(m, ly.mat0, l + 1 < m->L ? m->layers[l + 1].mat0 : (int)m->mats.size()));
-    M_TRY(tilenorm_backward(ctx_of(m), m->states[l], m->dn, m->fscale, 1.f, T, D, m->g, true, m->absmax + l, m->health + l, m->step_no));
+    if (!fused)
+        M_TRY(tilenorm_backward(ctx_of(m), m->states[l], m->dn, m->fscale, 1.f, T, D, m->g, true, m->absmax + l, m->health + l, m->step_no));
     TRACE("g", l, m->g, (size_t)T * D * 4, TR_F32);
     M_TRY(tap_gradient(m, l));
     return gradients_complete(m, ly.mat0);

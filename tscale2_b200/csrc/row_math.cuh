@@ -1,4 +1,5 @@
-// Arithmetic that the row-wise kernels share (kernels_elem.cu, kernels_att.cu), on values in registers.  A warp holds 128 consecutive columns of a row, four to a lane; in the functions on
+// Arithmetic of the row-wise kernels, on values in registers: the kernels that run it on tensors in memory
+// (kernels_elem.cu, kernels_att.cu) and the contractions whose epilogue runs it on their own product (gemm_pair.cu) share it.  A warp holds 128 consecutive columns of a row, four to a lane; in the functions on
 // eight values half a warp does.
 #pragma once
 #include "fast_types.cuh"
