@@ -148,3 +148,18 @@ def test_row_steps_of_a_training_step(prec, T, D, H, F, seq):
     # a traced step is otherwise the same step
     for a, b in zip(m.plain, m.model.get_gradients()):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", [capi.PREC_FP8, capi.PREC_F16, capi.PREC_INT8])
+@pytest.mark.parametrize("T,vocab,bias", [(5003, 4128, True), (8192, 2080, False), (40, 1024, True)])
+def test_score_without_logits_in_memory(prec, T, vocab, bias):
+    """Scoring keeps the logits on the chip where its contraction runs on pairs; the training step rounds them to fp16 (2^-11 of
+    values of a few units, averaged over T nodes).  Vocabularies that end inside a tile and inside a warp's 64 columns."""
+    spec = host.ModelSpec(dim=256, head_count=1, ffn_tiles=2, vocab=vocab, attention_widths=[32], precision=prec).add_blocks(1)
+    rng = np.random.default_rng(vocab)
+    model = Model(spec, host.init_weights(spec, 2), T, bias=rng.standard_normal(vocab).astype(np.float32) * 2 if bias else None)
+    batch = host.Batch(rng.integers(0, vocab, (1, T + 1)), spec.attention_widths)
+    model.set_batch(batch)
+    score = model.compute_score()
+    model.backprop(host.training_step(rate=0.0))
+    assert abs(score + model.avg_train_err()) < 2e-4

@@ -949,9 +949,9 @@ bool gemm_takes_act_backward(int device, int kind, int64_t M, int64_t N)
 
 bool gemm_takes_row(int device, int kind, int64_t M, int64_t N, int64_t K, int form)
 {
-    if (K <= 0 || N % 128 || form == ROW_PLAIN)
+    if (K <= 0 || N % (form == ROW_LSE ? 32 : 128) || form == ROW_PLAIN)
         return false;
-    const Plan pl = make_plan(device, kind, false, M, N, K, form == ROW_NORM ? FORM_ADD : FORM_F32);
+    const Plan pl = make_plan(device, kind, false, M, N, K, form == ROW_NORM ? FORM_ADD : form == ROW_NORM_BWD ? FORM_F32 : FORM_16);
     return pl.pair() && pl.splits == 1;
 }
 
@@ -1178,10 +1178,10 @@ int gemm(const GemmArgs &a)
                     (((uintptr_t)a.epi.bwd_wg | (uintptr_t)a.epi.bwd_o | (uintptr_t)a.epi.bwd_dout) & 15) || !pl.pair() || pl.splits != 1))
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of the activation's backward form");
     const RowOp *const op = a.epi.row;
-    const bool norm_bwd = op && op->form == ROW_NORM_BWD, norm = op && op->form == ROW_NORM;
-    if (op && (!(norm || norm_bwd) || !pl.pair() || pl.splits != 1 || a.N % 128 || a.mn_major || a.group_mode || a.ldc != a.N ||
-               a.epi.col_scale || (!norm_bwd && a.epi.row_scale) ||
-               a.epi.out_kind != (norm_bwd ? TS2_OUT_F32 : TS2_OUT_F32_ADD)))
+    const bool norm_bwd = op && op->form == ROW_NORM_BWD, norm = op && op->form == ROW_NORM, lse = op && op->form == ROW_LSE;
+    if (op && (!(norm || norm_bwd || lse) || !pl.pair() || pl.splits != 1 || (!lse && a.N % 128) || a.mn_major || a.group_mode || a.ldc != a.N ||
+               a.epi.col_scale || (!norm_bwd && a.epi.row_scale) || ((uintptr_t)op->bias & 15) ||
+               a.epi.out_kind != (norm_bwd ? TS2_OUT_F32 : lse ? TS2_OUT_F16 : TS2_OUT_F32_ADD)))
         return fail(TS2_ERR_INVALID_ARG, "gemm: bad arguments of a row-wise epilogue");
     const size_t room = a.workspace ? a.workspace_bytes : 0;
     if (pl.workspace() > room) {
@@ -1263,6 +1263,12 @@ int gemm(const GemmArgs &a)
             p.norm_add = op->add;
             p.norm_dyn = op->dyn;
             p.norm_absmax = op->absmax, p.norm_health = op->health, p.norm_step = op->step_no;
+        } else if (lse) {
+            rc = TS2_OK; // nothing leaves by TMA
+            p.lse_bias = op->bias;
+            p.lse_target = op->target;
+            p.lse_partial = op->partial;
+            p.lse_logit = op->target_logit;
         } else if (pl.splits > 1)
             rc = make_tmap(&tmC, a.workspace, 4, pl.bn, (int64_t)pl.m_tiles * pl.n_tiles * pl.splits * pl.bm, pl.bn, 32);
         else
@@ -1292,7 +1298,7 @@ int gemm(const GemmArgs &a)
     if (pl.pair()) {
         const int sms = std::max(2, sm_count(a.device) - g_reserved_sms.load(std::memory_order_relaxed)) & ~1;
         const bool out16 = pl.splits == 1 && (a.epi.out_kind == TS2_OUT_F16 || a.epi.out_kind == TS2_OUT_BF16);
-        const PairForm form = norm_bwd ? P_NORM_BWD : norm ? P_NORM : gate_bwd ? P_GATE_BWD : act_bwd ? P_ACT_BWD : paired ? P_GATED : out16 ? P_16 : P_F32;
+        const PairForm form = norm_bwd ? P_NORM_BWD : norm ? P_NORM : lse ? P_LSE : gate_bwd ? P_GATE_BWD : act_bwd ? P_ACT_BWD : paired ? P_GATED : out16 ? P_16 : P_F32;
         rc = gemm_pair_launch(a.device, a.stream, es, mma, a.mn_major, form, std::min(pl.grid, sms), tmA, tmB, tmC, tmCin, tmX, tmY, p);
         if (rc == TS2_OK && pl.splits > 1)
             rc = reduce_splits<2 * BM, 256>(a, pl, p);
@@ -1326,7 +1332,7 @@ int gemm(const GemmArgs &a)
         return fail(rc, "gemm: unsupported configuration");
     // algorithmic bytes: both operands once, the output once, the residual input of the accumulate form once
     const double mn = (double)a.M * (double)a.N;
-    const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + (gate_bwd ? mn * 7 : act_bwd ? mn * 6 : norm_bwd ? mn * 12 : mn * out_es) +
+    const double bytes = ((double)a.M + (double)a.N) * (double)a.K * es + (gate_bwd ? mn * 7 : act_bwd ? mn * 6 : norm_bwd ? mn * 12 : lse ? mn / 8 : mn * out_es) +
                          (norm ? mn * (es + (op->n16 ? 2 : 0)) : 0) +
                          (a.epi.out_kind == TS2_OUT_F32_ADD ? mn * 4 : 0);
     gemm_timed_end(timed, a.stream, 2.0 * mn * (double)a.K, bytes, a.tag);

@@ -40,8 +40,8 @@ struct Epilogue {
     const void *bwd_wg = nullptr, *bwd_o = nullptr;
     void *bwd_dout = nullptr;
     float *bwd_dscale = nullptr;
-    // The row-wise step that follows (gemm_row.cuh), where gemm_takes_row() says so: ROW_NORM behind the accumulate form and
-    // ROW_NORM_BWD behind the plain one.
+    // The row-wise step that follows (gemm_row.cuh), where gemm_takes_row() says so: ROW_NORM behind the accumulate form,
+    // ROW_NORM_BWD behind the plain one, ROW_LSE in place of fp16 output.
     const RowOp *row = nullptr;
 };
 

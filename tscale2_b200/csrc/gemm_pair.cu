@@ -577,6 +577,67 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(epi8(FORM) ? P_THREA
                 while (!mbar_try_wait(in_bar, in_phase) && clock64() - t0 < 200000000ll) {
                 }
             }
+        } else if constexpr (FORM == P_LSE) {
+            // Scoring: nothing of the logits leaves the chip but each row's maximum and sum per 64 columns (an eighth of a percent
+            // of their bytes) and the target's logit.  12000 x 50304 logits x 768, fp16: 700 us and 26 for the sum over the partial
+            // results, where logits in memory (2.4 GB written and read) took 790 and 320.
+            const int part = ew >> 2;
+            for (int u = first; u < units; u += step) {
+                const PairUnit un = pair_unit(p, u);
+                const long long row = un.m0 + (int)rank * 128 + row_in_cta;
+                const int col = un.n0 + part * 64;
+                const int target = row < p.M ? p.lse_target[row] - col : -1; // 0 .. 63: in this thread's columns
+                if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag)))
+                    break;
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * PN + part * 64;
+                float v[64], mx = -INFINITY;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + h * 32, r);
+                    tmem_ld_wait();
+                    if (h == 1) { // the accumulator is read: the next tile may have it
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0)
+                            mbar_arrive_cluster(map_to_leader(tempty0 + 8 * acc));
+                    }
+                    const bool cols = col + h * 32 < p.N; // N is a multiple of 32
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float4 b = p.lse_bias && cols ? __ldg((const float4 *)(p.lse_bias + col + h * 32) + i) : make_float4(0, 0, 0, 0);
+                        auto val = [&](int k) { return (MMA == 2) ? (float)(int)r[4 * i + k] : __uint_as_float(r[4 * i + k]); };
+                        float *o = v + 32 * h + 4 * i;
+                        o[0] = cols ? fmaf(val(0), alpha, b.x) : -INFINITY;
+                        o[1] = cols ? fmaf(val(1), alpha, b.y) : -INFINITY;
+                        o[2] = cols ? fmaf(val(2), alpha, b.z) : -INFINITY;
+                        o[3] = cols ? fmaf(val(3), alpha, b.w) : -INFINITY;
+                        mx = fmaxf(mx, fmaxf(fmaxf(o[0], o[1]), fmaxf(o[2], o[3])));
+                    }
+                }
+                if (__any_sync(0xffffffffu, (unsigned)target < 64u)) { // one tile in a hundred or so
+                    float x = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 64; ++i)
+                        x = i == target ? v[i] : x;
+                    if ((unsigned)target < 64u)
+                        p.lse_logit[row] = x;
+                }
+                float s4[4] = {0.f, 0.f, 0.f, 0.f};
+                const float ref = mx == -INFINITY ? 0.f : mx;
+#pragma unroll
+                for (int i = 0; i < 64; ++i) {
+                    float e;
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v[i] - ref));
+                    s4[i & 3] += e;
+                }
+                if (row < p.M)
+                    p.lse_partial[(size_t)(un.nt * 4 + part) * p.M + row] = make_float2(mx, (s4[0] + s4[1]) + (s4[2] + s4[3]));
+                acc ^= 1;
+                if (acc == 0)
+                    acc_phase ^= 1;
+            }
         } else if constexpr (FORM == P_16) {
             // Sixteen warps, four per lane quarter, 64 columns of the tile each: one block of 32 rows x 128 bytes in the 128-byte
             // swizzle and one store per tile.  With eight warps a tile of K = 768 took 3.6 us, 2.6 of them its main loop and
@@ -1030,6 +1091,7 @@ int gemm_pair_launch(int device, cudaStream_t stream, int es, int mma, bool mn, 
     TS2_PAIR_CASE(ES_, MMA_, false, P_16)      \
     TS2_PAIR_CASE(ES_, MMA_, false, P_GATED)   \
     TS2_PAIR_CASE(ES_, MMA_, false, P_NORM)    \
+    TS2_PAIR_CASE(ES_, MMA_, false, P_LSE)     \
     TS2_PAIR_CASE(ES_, MMA_, false, P_NORM_BWD) \
     TS2_PAIR_CASE(ES_, MMA_, true, P_F32)      \
     TS2_PAIR_CASE(ES_, MMA_, true, P_16)

@@ -49,11 +49,17 @@ struct GemmParams {
     const float *norm_dyn = nullptr;
     unsigned *norm_absmax = nullptr, *norm_health = nullptr;
     unsigned norm_step = 0;
+    // log-sum-exp of the row
+    const float *lse_bias = nullptr;
+    const int *lse_target = nullptr;
+    float2 *lse_partial = nullptr;
+    float *lse_logit = nullptr;
 };
 
 // Forms of the epilogue of gemm_pair.cu: fp32 output, accumulate form and partial tiles; fp16 / bf16 output; gated
 // activation; its backward; backward of the attention gate; residual input + tile normalisation; backward of the latter;
-enum PairForm { P_F32, P_16, P_GATED, P_ACT_BWD, P_GATE_BWD, P_NORM, P_NORM_BWD };
+// log-sum-exp of the row
+enum PairForm { P_F32, P_16, P_GATED, P_ACT_BWD, P_GATE_BWD, P_NORM, P_NORM_BWD, P_LSE };
 // gemm_pair.cu: the contraction on pairs of CTAs (tiles of 256 x 256).  tmB's box is 128 rows (K-major) or one K block
 // (token-major); tmC's and tmCin's are 32 rows x 128 bytes (P_GATED: tmC 32 x 64 bytes).  grid: CTAs, an even number.
 // P_ACT_BWD: tmC 32 rows x 64 bytes, tmCin [wide | gate] in 32 rows x 128; P_GATE_BWD: the same, and tmX: o, tmY: dout, both

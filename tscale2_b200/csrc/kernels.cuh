@@ -138,6 +138,10 @@ int checksum(const Ctx &c, const void *p, size_t bytes, int kind, unsigned long 
 int softmax_ce(const Ctx &c, __half *logits, int rows, int V, const float *bias, const int *target, float gscale, float *logp_sum,
                bool write_grad);
 
+// logp_sum += log p(target) over the rows with a target, from what a contraction with ROW_LSE left (gemm_row.cuh): n partial
+// results per row
+int softmax_from_partials(const Ctx &c, const float2 *partial, int n, const float *target_logit, const int *target, int rows, float *logp_sum);
+
 // ---- kernels_att.cu ----------------------------------------------------------------
 // qkvg [T][4Q] fp16 -> q = rope(tilenorm_h(Q)), k = rope(K), v = tilenorm_h(V), each [T][Q] fp16;
 // qscale, vscale [T][H]   (TAttLayer::ComputeForward, layer_att.cu:384-394)

@@ -999,4 +999,47 @@ int softmax_ce(const Ctx &c, __half *logits, int rows, int V, const float *bias,
     return TS2_OK;
 }
 
+// 32 rows a block, lane = row: a warp takes every eighth partial result (coalesced: they lie [partial][row]), keeping maximum
+// and sum as it goes; the eight warps' results meet in shared memory.
+__global__ void __launch_bounds__(THREADS) softmax_from_partials_kernel(const float2 *__restrict__ partial, int n, const float *__restrict__ target_logit,
+                                                                        const int *__restrict__ target, int rows, float *__restrict__ logp_sum)
+{
+    grid_dep_wait();
+    __shared__ float2 part_s[WARPS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
+    auto merge = [](float2 a, float2 b) {
+        const float m = fmaxf(a.x, b.x);
+        if (m == -INFINITY)
+            return a;
+        return make_float2(m, a.y * exp2f(a.x - m) + b.y * exp2f(b.x - m));
+    };
+    float2 acc = make_float2(-INFINITY, 0.f);
+    if (row < rows)
+        for (int i0 = w; i0 < n; i0 += WARPS * 4) {
+            float2 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                v[u] = i0 + u * WARPS < n ? partial[(size_t)(i0 + u * WARPS) * rows + row] : make_float2(-INFINITY, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                acc = merge(acc, v[u]);
+        }
+    part_s[w][lane] = acc;
+    __syncthreads();
+    if (w == 0) {
+        for (int i = 1; i < WARPS; ++i)
+            acc = merge(acc, part_s[i][lane]);
+        const float logp = row < rows && target[row] >= 0 ? (target_logit[row] - acc.x) * 0.69314718f - logf(acc.y) : 0.f;
+        const float sum = warp_sum(logp);
+        if (lane == 0)
+            atomicAdd(logp_sum, sum);
+    }
+}
+
+int softmax_from_partials(const Ctx &c, const float2 *partial, int n, const float *target_logit, const int *target, int rows, float *logp_sum)
+{
+    TS2_LAUNCH((softmax_from_partials_kernel), (int)ceil_div(rows, 32), THREADS, 0, c.stream, partial, n, target_logit, target, rows, logp_sum);
+    return TS2_OK;
+}
+
 } // namespace ts2

@@ -1454,6 +1454,34 @@ int forward(ts2_model *m, bool train)
     return TS2_OK;
 }
 
+// Scoring without logits in memory (see ROW_LSE): the buffer of a chunk's logits holds the partial results of many times as many
+// nodes.  *done: false where the contraction's tiles do not carry that.
+int score_rows(ts2_model *m, const Epilogue &logits, bool *done)
+{
+    Ctx c = ctx_of(m);
+    const int T = m->batch.node_count, D = m->D, V = m->V, n = 4 * (int)ceil_div(V, 256);
+    const size_t fs = fast_size(m);
+    const size_t room = (size_t)m->chunk * V * sizeof(__half) / (n * sizeof(float2) + sizeof(float)); // nodes
+    const int most = (int)(room >= (size_t)T ? T : room / 256 * 256);
+    *done = most > 0;
+    for (int r0 = 0; r0 < T && *done; r0 += most) // whatever is left in the last one
+        *done = gemm_takes_row(m->device, m->kind, std::min(most, T - r0), V, D, ROW_LSE);
+    for (int r0 = 0; r0 < T && *done; r0 += most) {
+        const int rows = std::min(most, T - r0);
+        RowOp op;
+        op.form = ROW_LSE;
+        op.bias = m->has_bias ? m->bias : nullptr;
+        op.target = m->batch.target + r0;
+        op.partial = (float2 *)m->logits;
+        op.target_logit = (float *)(op.partial + (size_t)n * rows);
+        GemmArgs a = tn_args(m, m->kind, rows, V, D, (const uint8_t *)m->nF_fast + (size_t)r0 * D * fs, D, m->Wf, D, m->logits, V, logits);
+        a.epi.row = &op;
+        M_TRY(gemm(a));
+        M_TRY(softmax_from_partials(c, op.partial, n, op.target_logit, op.target, rows, m->logp));
+    }
+    return TS2_OK;
+}
+
 // logits of nodes [r0, r0+rows) -> softmax; with backward: dnF rows and the final-layer gradient
 int final_layer(ts2_model *m, bool backward)
 {
@@ -1468,6 +1496,12 @@ int final_layer(ts2_model *m, bool backward)
     e.alpha = sqrtf(1.0f / D) / (m->s_act * 32.f) * (1.f / LOG2F); // MulForward scale * CalcFinalLayerMult()
     e.dyn_scale = m->mats[1].sko;
     e.out_kind = TS2_OUT_F16;
+    if (!backward) {
+        bool done = false;
+        M_TRY(score_rows(m, e, &done));
+        if (done)
+            return TS2_OK;
+    }
     for (int r0 = 0; r0 < T; r0 += m->chunk) {
         const int rows = std::min(m->chunk, T - r0);
         M_TRY(gemm_tn(m, m->kind, rows, V, D, (const uint8_t *)m->nF_fast + (size_t)r0 * D * fs, D, m->Wf, D, m->logits, V, e));
