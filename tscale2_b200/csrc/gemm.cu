@@ -892,7 +892,8 @@ static bool dynamic_units()
 // dW 4096 x 256 from 512 tokens 8.6 -> 6.5, dW 768 x 3072 from 4000 tokens 20.6 -> 17.7; pairs: 65536 x 768 x 1536 e4m3
 // with residual input 142 -> 112, 32768 x 2048 x 2048 211 -> 152, dX + dW of 16384 x 4096 x 4096 482 -> 466.  A unit keeps
 // at least 4 K blocks, and split units stay within two waves, which bounds the scratch (ts2_create reserves as much).
-static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int form, int group_mode = 0, int groups = 1)
+static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int form, int group_mode = 0, int groups = 1,
+                      double *time = nullptr)
 {
     Plan best;
     double best_t = 1e30;
@@ -934,6 +935,8 @@ static Plan make_plan(int device, int kind, bool mn, int64_t M, int64_t N, int64
             }
         }
     }
+    if (time)
+        *time = best_t;
     return best;
 }
 
@@ -953,6 +956,20 @@ bool gemm_takes_row(int device, int kind, int64_t M, int64_t N, int64_t K, int f
         return false;
     const Plan pl = make_plan(device, kind, false, M, N, K, form == ROW_NORM ? FORM_ADD : form == ROW_NORM_BWD ? FORM_F32 : FORM_16);
     return pl.pair() && pl.splits == 1;
+}
+
+// The row kernel takes a contraction and the backward of a normalisation where its time is below the other kernels' for the
+// contraction alone and what the normalisation costs by itself: a launch and the traffic of the product (where pairs carry it
+// in their epilogue, neither).
+bool gemm_row_takes(int device, int kind, int64_t M, int64_t N, int64_t K)
+{
+    if (N % 128 || K <= 0 || dynamic_units())
+        return false;
+    double other = 0;
+    int splits;
+    const Plan pl = make_plan(device, kind, false, M, N, K, FORM_F32, 0, 1, &other);
+    const double saved = pl.pair() && pl.splits == 1 ? 0 : 3.0 + (double)M * N * 8 / 6e6;
+    return gemm_row_plan(device, kind, M, N, K, &splits) < other + saved;
 }
 
 size_t gemm_workspace_bytes(int device, int kind, bool mn, int64_t M, int64_t N, int64_t K, int out_kind)

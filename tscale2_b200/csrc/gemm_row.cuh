@@ -4,7 +4,8 @@
 
 namespace ts2 {
 
-// What pairs of CTAs make of their product (Epilogue::row; widths are multiples of 128 but in the last form)
+// What becomes of the product, 128 columns of a row at a time (widths are multiples of 128 in all forms but the first and the
+// last).  The row kernel (gemm_row.cu) has the first and the third, pairs of CTAs (Epilogue::row) all but the first.
 enum RowForm {
     ROW_PLAIN = 0, // Epilogue::out_kind, as any contraction
     ROW_NORM,      // C = c_in + product (fp32); n_fast = tile normalisation of C, n16 optionally (tilenorm_forward)
@@ -29,5 +30,20 @@ struct RowOp {
     float2 *partial = nullptr;
     float *target_logit = nullptr;
 };
+
+// First contraction (K contiguous in both operands) with its row step, and optionally a second one beside it in the same
+// launch: token-major operands, ROW_PLAIN, independent of the first.
+struct RowGemm {
+    GemmArgs a;
+    RowOp op;
+    const GemmArgs *second = nullptr;
+};
+// K split and estimated time (us) of one contraction in this kernel
+double gemm_row_plan(int device, int kind, int64_t M, int64_t N, int64_t K, int *splits);
+// whether gemm_row() is the faster way for this shape and the backward of a normalisation behind it
+bool gemm_row_takes(int device, int kind, int64_t M, int64_t N, int64_t K);
+// whether the second contraction fits beside the first
+bool gemm_row_takes_pair(int device, const GemmArgs &a, const GemmArgs &second);
+int gemm_row(const RowGemm &r);
 
 } // namespace ts2

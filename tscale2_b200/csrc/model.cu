@@ -421,6 +421,18 @@ int gemm_dw(ts2_model *m, int kind, int64_t Mo, int64_t Ni, int64_t T, const voi
     return gemm(dw_args(m, kind, Mo, Ni, T, dY, ldy, X, ldx, dW, epi));
 }
 
+// a contraction and its row-wise step in one launch (where gemm_row_takes() its shape), and dw, if there is one, beside it, or
+// after it if the launch has no room
+int row_step(const GemmArgs &a, const RowOp &op, const GemmArgs *dw = nullptr)
+{
+    RowGemm r;
+    r.a = a;
+    r.op = op;
+    r.second = dw && gemm_row_takes_pair(a.device, a, *dw) ? dw : nullptr;
+    const int rc = gemm_row(r);
+    return rc == TS2_OK && dw && !r.second ? gemm(*dw) : rc;
+}
+
 // rows of A are expert-sorted: every 128-row tile reads the weights of its expert (B has E * N rows)
 int gemm_rows_grouped(ts2_model *m, const Layer &ly, int64_t rows, int64_t N, int64_t K, const void *A, int64_t lda, const void *B,
                       int64_t ldb, void *C, int64_t ldc, const Epilogue &epi)
@@ -1454,6 +1466,12 @@ int forward(ts2_model *m, bool train)
     return TS2_OK;
 }
 
+// whether the final layer's dX goes on through the backward of the last normalisation (a batch of one chunk and few tiles)
+bool final_row_step(const ts2_model *m)
+{
+    return m->batch.node_count <= m->chunk && gemm_row_takes(m->device, KIND_F16, m->batch.node_count, m->D, m->V);
+}
+
 // Scoring without logits in memory (see ROW_LSE): the buffer of a chunk's logits holds the partial results of many times as many
 // nodes.  *done: false where the contraction's tiles do not carry that.
 int score_rows(ts2_model *m, const Epilogue &logits, bool *done)
@@ -1521,9 +1539,13 @@ int final_layer(ts2_model *m, bool backward)
         ew.alpha = gs / gscale;
         ew.out_kind = m->grads_dirty || r0 ? TS2_OUT_F32_ADD : TS2_OUT_F32;
         const GemmArgs dw = dw_args(m, KIND_F16, V, D, rows, m->logits, V, m->nF16 + (size_t)r0 * D, D, m->mats[1].grad, ew);
-        M_TRY(gemm(dx));
+        const bool row = final_row_step(m);
+        if (!row || m->trace_on)
+            M_TRY(gemm(dx));
         TRACE("dnF", r0 / m->chunk, m->dn + (size_t)r0 * D, (size_t)rows * D * 4, TR_F32);
-        if (tune_final)
+        if (row)
+            M_TRY(row_step(dx, norm_backward_op(m, m->L, nullptr), tune_final ? &dw : nullptr));
+        else if (tune_final)
             M_TRY(gemm(dw));
     }
     if (backward && tune_final)
@@ -1598,15 +1620,17 @@ AttBwdPlan att_plan(const ts2_model *m, const Layer &ly)
 }
 
 // Last step of a dense layer's backward pass: dn (scale-free) = dcat . (q_cat / 32) * sqrt(1 / D), the layer's weight
-// gradient from the same dcat, and the backward of the normalisation, which adds to the state gradient: in the epilogue where
-// pairs take the product, dn then never reaches memory (a traced step has it all the same).
+// gradient from the same dcat, and the backward of the normalisation, which adds to the state gradient.  Few tiles: one
+// launch for all of it; many: the normalisation's in the epilogue; dn then never reaches memory (a traced step has it all
+// the same).
 int input_gradient(ts2_model *m, int l, const GemmArgs &dn, const GemmArgs *dw_cat)
 {
     const Layer &ly = m->layers[l];
     const int T = m->batch.node_count, D = m->D;
-    const bool fused = gemm_takes_row(m->device, dn.kind, dn.M, dn.N, dn.K, ROW_NORM_BWD);
+    const bool row = gemm_row_takes(m->device, dn.kind, dn.M, dn.N, dn.K);
+    const bool fused = !row && gemm_takes_row(m->device, dn.kind, dn.M, dn.N, dn.K, ROW_NORM_BWD);
     const RowOp op = norm_backward_op(m, l, m->fscale);
-    if (!fused || m->trace_on)
+    if (!(row || fused) || m->trace_on)
         M_TRY(gemm(dn));
     TRACE("dn", l, m->dn, (size_t)T * D * 4, TR_F32);
     if (fused) {
@@ -1614,12 +1638,14 @@ int input_gradient(ts2_model *m, int l, const GemmArgs &dn, const GemmArgs *dw_c
         a.epi.row = &op;
         M_TRY(gemm(a));
     }
-    if (dw_cat) {
+    if (row)
+        M_TRY(row_step(dn, op, dw_cat));
+    else if (dw_cat)
         M_TRY(gemm(*dw_cat));
+    if (dw_cat)
         TRACE("dW_cat", l, m->mats[ly.mat0].grad, (size_t)dw_cat->M * D * 4, TR_F32);
-    }
     M_TRY(reduce_matrices(m, ly.mat0, l + 1 < m->L ? m->layers[l + 1].mat0 : (int)m->mats.size()));
-    if (!fused)
+    if (!(row || fused))
         M_TRY(tilenorm_backward(ctx_of(m), m->states[l], m->dn, m->fscale, 1.f, T, D, m->g, true, m->absmax + l, m->health + l, m->step_no));
     TRACE("g", l, m->g, (size_t)T * D * 4, TR_F32);
     M_TRY(tap_gradient(m, l));
@@ -1733,7 +1759,8 @@ int backward(ts2_model *m)
     m->gemm_tag = GEMM_TAG_DX;
     M_TRY(reduce_matrices(m, 1, 2));
     M_TRY(gradients_complete(m, 1));
-    M_TRY(tilenorm_backward(c, m->states[L], m->dn, nullptr, 1.f, T, D, m->g, false, m->absmax + L, m->health + L, m->step_no));
+    if (!final_row_step(m))
+        M_TRY(tilenorm_backward(c, m->states[L], m->dn, nullptr, 1.f, T, D, m->g, false, m->absmax + L, m->health + L, m->step_no));
     TRACE("g", L, m->g, (size_t)T * D * 4, TR_F32);
     M_TRY(tap_gradient(m, L));
     const size_t fsz = fast_size(m);

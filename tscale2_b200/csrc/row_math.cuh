@@ -1,5 +1,6 @@
 // Arithmetic of the row-wise kernels, on values in registers: the kernels that run it on tensors in memory
-// (kernels_elem.cu, kernels_att.cu) and the contractions whose epilogue runs it on their own product (gemm_pair.cu) share it.  A warp holds 128 consecutive columns of a row, four to a lane; in the functions on
+// (kernels_elem.cu, kernels_att.cu) and the contractions whose epilogue runs it on their own product (gemm_row.cu, gemm_pair.cu)
+// share it.  A warp holds 128 consecutive columns of a row, four to a lane; in the functions on
 // eight values half a warp does.
 #pragma once
 #include "fast_types.cuh"
