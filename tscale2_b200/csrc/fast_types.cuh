@@ -144,26 +144,13 @@ __device__ __forceinline__ float tile_scale(float sum2) { return sum2 == 0.f ? 0
 // Weight encoder of the reference's CPU path for e4m3 (ConvertToFp8e4m3,
 // src/gpt/model_params/sse_utils.h:161-204): round half away from zero on the 4th
 // mantissa bit, values below 2^-7 become 0, saturate to +-448.  Bit-exact with it.
-__device__ __forceinline__ uint8_t encode_e4m3_weight(float v)
+// In integers: the fourth mantissa bit, added to itself, carries into the bits that are kept and on into the exponent, as the
+// reference's addition in fp32 does (the same byte for every one of the 2^32 arguments; -inf and NaN give 0x7e there too).
+__device__ __forceinline__ uint32_t encode_e4m3_weight(float v)
 {
-    uint32_t bits = __float_as_uint(v);
-    float f0 = __uint_as_float(bits & 0xFF800000u), f1 = __uint_as_float(bits & 0xFF880000u);
-    v = __fadd_rn(v, __fsub_rn(f1, f0));
-    bits = __float_as_uint(v);
-    int sign = bits >> 31;
-    int exponent = (int)((bits & 0x7F800000u) >> 23) - 120;
-    int mantissa = (bits & 0x007FFFFFu) >> 20;
-    int fp8 = (sign << 7) | (exponent << 3) | mantissa;
-    if (exponent > 15)
-        fp8 = (sign << 7) | 0x7f;
-    if (exponent < 0)
-        fp8 = 0;
-    fp8 &= 0xff;
-    if (fp8 == 0xff)
-        fp8 = 0xfe;
-    if (fp8 == 0x7f)
-        fp8 = 0x7e;
-    return (uint8_t)fp8;
+    const uint32_t bits = __float_as_uint(v), mag = bits & 0x7fffffffu;
+    const int code = min((int)((mag + (mag & 0x00080000u)) >> 20) - (120 << 3), 126);
+    return code < 0 ? 0u : (uint32_t)code | (mag < 0x7f800000u ? (bits >> 24) & 0x80u : 0u);
 }
 
 } // namespace ts2

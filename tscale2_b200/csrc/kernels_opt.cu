@@ -201,9 +201,7 @@ __device__ __forceinline__ uint2 quantize4(float4 v, int kind)
     if (kind == 2) // int8: nearest even, saturating (PackFloatToInt8, src/gpt/model_params/sse_utils.h:56-78)
         return make_uint2(sat_i8(v.x) | (sat_i8(v.y) << 8) | (sat_i8(v.z) << 16) | (sat_i8(v.w) << 24), 0u);
     if (kind == 0)
-        return make_uint2((uint32_t)encode_e4m3_weight(v.x) | ((uint32_t)encode_e4m3_weight(v.y) << 8) | ((uint32_t)encode_e4m3_weight(v.z) << 16) |
-                              ((uint32_t)encode_e4m3_weight(v.w) << 24),
-                          0u);
+        return make_uint2(encode_e4m3_weight(v.x) | (encode_e4m3_weight(v.y) << 8) | (encode_e4m3_weight(v.z) << 16) | (encode_e4m3_weight(v.w) << 24), 0u);
     const __half h0 = __float2half_rn(v.x), h1 = __float2half_rn(v.y), h2 = __float2half_rn(v.z), h3 = __float2half_rn(v.w);
     return make_uint2((uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16),
                       (uint32_t)__half_as_ushort(h2) | ((uint32_t)__half_as_ushort(h3) << 16));
@@ -284,9 +282,13 @@ int opt_quantize(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const f
 
 // Copies of quantized blocks into another row-major place and / or their transpose, all of a model's in one launch, from
 // the quantized values, or (CopyJob::w) from the weights themselves, which are quantized on the way: one launch and one pass
-// less where this rank holds whole matrices (124 M parameters 350 + 155 -> 494 us, 437 M 642 + 350 -> 947).  A tile is 128 bytes of 128 rows (64 rows of 2-byte values): it comes in as 16-byte vectors, lies in shared
+// less where this rank holds whole matrices (124 M parameters 350 + 155 -> 494 us, 437 M 642 + 350 -> 947).  A tile is 128
+// bytes of 128 rows (64 rows of 2-byte values): it comes in as 16-byte vectors, lies in shared
 // memory with its 16-byte pieces rotated by the row group (so that both the vector writes and the word reads of eight
 // row groups are free of bank conflicts), is transposed in registers by byte permutes and leaves in 16-byte vectors.
+// A small model's launch is one tile per CTA, a chain of latencies: the search for the tile's job is one load per 32 jobs.
+// Four rows a thread are in flight; eight cost a third of the resident blocks and gain nothing (3272 against 3257 us for eight
+// steps of a 4 M parameter model, 67.3 against 67.5 ms for one of 437 M).
 // Bound by its bytes (read once, written once or twice): 4 transposes of [16384 x 2048] bytes and their like took 52 us
 // each with 32 x 32 byte tiles (1.3 TB/s) and a launch of their own; an expert layer of 32 experts was 97 launches.
 __device__ __forceinline__ void transpose4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t (&c)[4])
@@ -342,14 +344,11 @@ __global__ void __launch_bounds__(256) qcopy_kernel(const CopyJob *__restrict__ 
         return;
     }
     for (int tile = blockIdx.x; tile < tiles; tile += blocks) {
-        int lo = 0, hi = n_jobs - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (jobs[mid].tile0 <= tile)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
+        // the last job that starts at or before the tile: a warp counts them, 32 a load
+        int lo = -1;
+#pragma unroll 4
+        for (int j = 0; j < n_jobs; j += 32)
+            lo += __popc(__ballot_sync(0xffffffffu, j + (tid & 31) < n_jobs && jobs[j + (tid & 31)].tile0 <= tile));
         const CopyJob jb = jobs[lo];
         const int two = jb.kind == QCOPY_2BYTE, rows = two ? 64 : 128, shift = two ? 3 : 4;
         const int t = tile - jb.tile0, tx = t % jb.tiles_x, y0 = (t / jb.tiles_x) * rows;

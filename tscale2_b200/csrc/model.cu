@@ -944,7 +944,7 @@ int requantize_all(ts2_model *m)
 }
 
 // Final layer, runs of layers from the last one down, embedding.  The weights of a group are final before the layers below it have
-// their gradients, so ts2_get_params copies them meanwhile (dim 2048, 4 blocks, 8 x 4096 tokens: step and export 147 -> 124 ms).
+// their gradients, so ts2_get_params copies them meanwhile (dim 2048, 4 blocks, 8 x 4096 tokens: step and export 147 -> 126 ms).
 // A group has at least UPDATE_GROUP_ELEMS elements: its four launches then take 20 us and more.  A model of less than two groups
 // is updated in one go: its export takes 1 ms or less.
 int build_update_groups(ts2_model *m)
