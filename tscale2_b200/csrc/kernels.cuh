@@ -31,7 +31,7 @@ enum {
 // what the host wants to know when it waits, in pinned host memory
 struct HostReport {
     int32_t device_status, static_status; // the device's status words (common.cuh)
-    int batch[4];                         // {code, where, detail, detail} of the first malformed batch element
+    int batch[2][4];                      // the batch status records: {code, where, detail, detail} of the first malformed element
     float scalar;
 };
 int queue_report(const Ctx &c, const int *batch_status, const float *scalar, HostReport *report);

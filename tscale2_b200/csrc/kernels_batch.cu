@@ -38,8 +38,9 @@ __global__ void report_kernel(const int32_t *device_status, const int32_t *stati
     grid_dep_wait();
     report->device_status = device_status ? *device_status : 0;
     report->static_status = static_status ? *static_status : 0;
-    for (int i = 0; i < 4; ++i)
-        report->batch[i] = batch_status[i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        report->batch[i / 4][i % 4] = batch_status[i];
     report->scalar = scalar ? *scalar : 0.f;
 }
 

@@ -118,7 +118,12 @@ struct BatchDev {
     std::vector<bool> layout_ready; // per attention type: made at the first backward pass of the batch (scoring does without)
     std::vector<bool> ds_fits;      // per attention type: the batch's score gradients fit the model's buffer
     int *scan_tmp = nullptr; // batch_scan_tmp_elems(max_nodes)
-    int *status = nullptr;   // {code, where, detail, detail}: the first malformed element seen since it was last reported
+    // Two records {code, where, detail, detail}: the first malformed element seen since the last report.  A batch is checked into
+    // the one that the last step's batch did not use, so that ts2_avg_train_err reads a record that nothing writes any more.
+    int *status = nullptr;
+    int record = 0, step_record = 0; // of the current batch; of the batch of the last ts2_backprop
+    int set_no = 0, record_since[2] = {0, 0}; // batches so far; the first one that went into a record since the last report
+    int *record_of(int r) const { return status + 4 * r; }
     LabelIndex ix;
     bool ix_sorted = false;
     size_t label_cap = 0;
@@ -164,7 +169,7 @@ struct ts2_model {
     std::vector<UpdateGroup> update_groups;
     const ts2_training_step *step_in_backward = nullptr; // of the ts2_backprop call that is queuing its backward pass, if it applies
     cudaEvent_t ev_loss = nullptr;      // the training error of the last ts2_backprop is known
-    cudaStream_t read_stream = nullptr; // what is read back while the step goes on
+    cudaStream_t read_stream = nullptr; // what is read back while the step goes on; nothing on it waits for another stream
     CopyJob *d_copies = nullptr, *d_quants = nullptr; // what post_quantize and quantize_all do
     ScaleJob *d_scales = nullptr;
     int n_copies = 0, copy_tiles = 0, n_quants = 0, quant_tiles = 0, n_scales = 0;
@@ -237,6 +242,7 @@ struct ts2_model {
     void *pinned = nullptr;
     size_t pinned_bytes = 0;
     HostReport *report = nullptr;  // pinned; written by the kernel that every wait queues (queue_report)
+    HostReport *read_report = nullptr; // the same for read_stream
     bool unreported = false;       // work was queued since the last wait
     double wait_limit_s = 120;     // wall time after which a wait gives up (poll_until)
     bool grads_dirty = false; // the flat gradient holds an accumulated, not yet applied gradient
@@ -1220,18 +1226,19 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
         M_TRY(dalloc(m, (uint8_t **)&b.att_layout[a], att_layout_bytes(T)));
     }
     M_TRY(dalloc(m, &b.scan_tmp, batch_scan_tmp_elems(T)));
-    M_TRY(dalloc(m, &b.status, 4));
-    TS2_CUDA(cudaMemsetAsync(b.status, 0, 16, m->stream));
+    M_TRY(dalloc(m, &b.status, 8));
+    TS2_CUDA(cudaMemsetAsync(b.status, 0, 32, m->stream));
     for (int i = 0; i < 2; ++i) {
         M_TRY(dalloc(m, &b.ix.key[i], b.label_cap));
         M_TRY(dalloc(m, &b.ix.val[i], b.label_cap));
     }
     M_TRY(dalloc(m, &b.ix.hist, label_index_hist_elems(b.label_cap)));
     M_TRY(dalloc(m, &b.ix.partial, label_index_partial_elems(m->device, b.label_cap, D)));
-    m->pinned_bytes = 2 * b.raw_cap * 4 + sizeof(HostReport);
+    m->pinned_bytes = 2 * b.raw_cap * 4 + 2 * sizeof(HostReport);
     TS2_CUDA(cudaMallocHost(&m->pinned, m->pinned_bytes));
     m->report = (HostReport *)((uint32_t *)m->pinned + 2 * b.raw_cap);
-    memset(m->report, 0, sizeof(HostReport));
+    m->read_report = m->report + 1;
+    memset(m->report, 0, 2 * sizeof(HostReport));
     for (int i = 0; i < 2; ++i)
         TS2_CUDA(cudaEventCreateWithFlags(&b.slot_ev[i], cudaEventDisableTiming));
 
@@ -2074,7 +2081,11 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
     bt.n_labels = b.n_labels, bt.label_count = (uint32_t)m->descr.label_count;
     bt.label_arr = b.label_arr, bt.label_ptr = b.label_ptr;
     bt.target_node = (const int *)b.raw + o_tnode, bt.target_id = (const int *)b.raw + o_tid;
-    bt.target = b.target, bt.scan_tmp = b.scan_tmp, bt.status = b.status;
+    b.record = b.step_record ^ 1;
+    ++b.set_no;
+    if (!b.record_since[b.record])
+        b.record_since[b.record] = b.set_no;
+    bt.target = b.target, bt.scan_tmp = b.scan_tmp, bt.status = b.record_of(b.record);
     std::vector<BatchSpans> spans(na);
     for (int a = 0; a < na; ++a) {
         const int *raw = (const int *)b.raw;
@@ -2094,16 +2105,18 @@ int stage_batch(ts2_model *m, const ts2_batch_nodes *nd)
     return TS2_OK;
 }
 
-// what the device found wrong with a batch, if anything; clears the record
-int report_batch_status(ts2_model *m, cudaStream_t stream)
+// what the device found wrong with a batch, if anything; clears the records (m->stream is idle and was just reported)
+int report_batch_status(ts2_model *m)
 {
-    int *h = m->report->batch;
+    BatchDev &b = m->batch;
+    const int first = b.record_since[1] && (!b.record_since[0] || b.record_since[1] < b.record_since[0]); // the one in use for longer
+    const int *h = m->report->batch[m->report->batch[first][0] != BATCH_OK ? first : first ^ 1];
+    b.record_since[0] = b.record_since[1] = 0;
     if (h[0] == BATCH_OK)
         return TS2_OK;
     const int code = h[0], where = h[1], d0 = h[2], d1 = h[3];
-    h[0] = BATCH_OK;
-    cudaMemsetAsync(m->batch.status, 0, 16, stream);
-    cudaStreamSynchronize(stream); // the stream is idle: a later batch, on another stream, finds the record cleared
+    memset(m->report->batch, 0, sizeof(m->report->batch));
+    cudaMemsetAsync(b.status, 0, 32, m->stream);
     switch (code) {
     case BATCH_BAD_SPAN_PTR:
         return fail(TS2_ERR_INVALID_ARG, "batch: span_ptr of node %d is malformed (offset %d, count %d)", where, d0, d1);
@@ -2133,7 +2146,7 @@ int wait_stream(ts2_model *m, const float *scalar = nullptr, float *value = null
     m->unreported = false;
     if (m->report->device_status | m->report->static_status)
         M_TRY(collect_device_status(m->device)); // clears the words and reports them
-    M_TRY(report_batch_status(m, m->stream));
+    M_TRY(report_batch_status(m));
     if (value)
         *value = m->report->scalar;
     return TS2_OK;
@@ -2331,6 +2344,7 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
     TS2_CUDA(cudaSetDevice(m->device));
     m->unreported = true;
     TS2_CUDA(cudaEventRecord(m->ev_start, m->stream));
+    m->batch.step_record = m->batch.record;
     ++m->step_no;
     m->logp = m->logp_ring + m->step_no % ts2_model::LOSS_RING; // final_layer() clears and fills this step's slot
     m->ring_targets[m->step_no % ts2_model::LOSS_RING] = m->batch.target_count;
@@ -2409,20 +2423,24 @@ int ts2_forward_score(ts2_model *m, float *out_score)
 
 // The error is known when the forward pass and the final layer are through: the call waits for that and not for the backward
 // pass and the update behind it, so that the host prepares the next batch, or fetches weights as they are updated, meanwhile.
+// The host waits for the event and queues the read then: a call that gives up leaves nothing behind that a later one, with
+// another limit, would have to wait for.
 int ts2_avg_train_err(ts2_model *m, float *out_err)
 {
     if (!m || !out_err)
         return fail(TS2_ERR_INVALID_ARG, "null argument");
     TS2_CUDA(cudaSetDevice(m->device));
+    M_TRY(poll_until(m, [&] { return cudaEventQuery(m->ev_loss); }));
     Ctx c = ctx_of(m);
     c.stream = m->read_stream;
-    TS2_CUDA(cudaStreamWaitEvent(m->read_stream, m->ev_loss, 0));
-    M_TRY(queue_report(c, m->batch.status, m->logp, m->report));
+    const HostReport &r = *m->read_report;
+    M_TRY(queue_report(c, m->batch.status, m->logp, m->read_report));
     M_TRY(poll_until(m, [&] { return cudaStreamQuery(m->read_stream); }));
-    if (m->report->device_status | m->report->static_status)
-        M_TRY(wait_stream(m)); // the step went wrong: reported when it is over
-    M_TRY(report_batch_status(m, m->read_stream));
-    *out_err = m->last_targets ? -m->report->scalar / m->last_targets : 0.f;
+    // Something went wrong, with the step or its batch: reported when the step is over.  The other record is not looked at: the
+    // check of a batch that was set since may be writing it.
+    if (r.device_status | r.static_status | r.batch[m->batch.step_record][0])
+        M_TRY(wait_stream(m));
+    *out_err = m->last_targets ? -r.scalar / m->last_targets : 0.f;
     return TS2_OK;
 }
 
