@@ -203,7 +203,9 @@ int ts2_avg_train_err(ts2_model *m, float *out_err);
  * weight gradient of the last ts2_backprop (the tap the parity tests read:
  * the tensor the reference hands to HostApplyDelta,
  * src/gpt/compute/cpu_util.h:86-95).  The values are those after everything queued before; weights and momentum of a large
- * model leave matrix by matrix as the running step updates them. */
+ * model leave matrix by matrix as the running step updates them.  A call that fails because the step's batch was malformed or
+ * its forward pass went wrong leaves the arrays as they were.  Where the failure arises later (a wait that runs out in the
+ * backward pass, the time limit, a batch set since), some of them may hold the matrices of a large model after the step. */
 #define TS2_PARAM_WEIGHTS 0
 #define TS2_PARAM_MOMENTUM 1
 #define TS2_PARAM_GRADIENT 2

@@ -169,7 +169,8 @@ struct ts2_model {
     std::vector<UpdateGroup> update_groups;
     const ts2_training_step *step_in_backward = nullptr; // of the ts2_backprop call that is queuing its backward pass, if it applies
     cudaEvent_t ev_loss = nullptr;      // the training error of the last ts2_backprop is known
-    cudaStream_t read_stream = nullptr; // what is read back while the step goes on; nothing on it waits for another stream
+    // What is read back while the step goes on, and weights that leave; nothing on either waits for another stream
+    cudaStream_t read_stream = nullptr, export_stream = nullptr;
     CopyJob *d_copies = nullptr, *d_quants = nullptr; // what post_quantize and quantize_all do
     ScaleJob *d_scales = nullptr;
     int n_copies = 0, copy_tiles = 0, n_quants = 0, quant_tiles = 0, n_scales = 0;
@@ -2152,6 +2153,15 @@ int wait_stream(ts2_model *m, const float *scalar = nullptr, float *value = null
     return TS2_OK;
 }
 
+// what wait_stream would report as things stand, and a scalar, into m->read_report, beside the running step
+int read_beside(ts2_model *m, const float *scalar)
+{
+    Ctx c = ctx_of(m);
+    c.stream = m->read_stream;
+    M_TRY(queue_report(c, m->batch.status, scalar, m->read_report));
+    return poll_until(m, [&] { return cudaStreamQuery(m->read_stream); });
+}
+
 } // namespace
 
 // ---------------------------------------------------------------------------------------
@@ -2217,6 +2227,7 @@ int ts2_create(const ts2_model_descr *descr, const ts2_matrix_view *mats, int n_
     cudaEventCreateWithFlags(&m->ev_grads, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&m->ev_loss, cudaEventDisableTiming);
     cudaStreamCreateWithFlags(&m->read_stream, cudaStreamNonBlocking);
+    cudaStreamCreateWithFlags(&m->export_stream, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&m->ev_reduced, cudaEventDisableTiming);
     rc = build_model(m, mats, n_mats, bias);
     if (rc != TS2_OK) {
@@ -2270,6 +2281,8 @@ void ts2_destroy(ts2_model *m)
         cudaEventDestroy(m->ev_loss);
     if (m->read_stream)
         cudaStreamDestroy(m->read_stream);
+    if (m->export_stream)
+        cudaStreamDestroy(m->export_stream);
     if (m->ev_start)
         cudaEventDestroy(m->ev_start);
     if (m->ev_stop)
@@ -2431,11 +2444,8 @@ int ts2_avg_train_err(ts2_model *m, float *out_err)
         return fail(TS2_ERR_INVALID_ARG, "null argument");
     TS2_CUDA(cudaSetDevice(m->device));
     M_TRY(poll_until(m, [&] { return cudaEventQuery(m->ev_loss); }));
-    Ctx c = ctx_of(m);
-    c.stream = m->read_stream;
+    M_TRY(read_beside(m, m->logp));
     const HostReport &r = *m->read_report;
-    M_TRY(queue_report(c, m->batch.status, m->logp, m->read_report));
-    M_TRY(poll_until(m, [&] { return cudaStreamQuery(m->read_stream); }));
     // Something went wrong, with the step or its batch: reported when the step is over.  The other record is not looked at: the
     // check of a batch that was set since may be writing it.
     if (r.device_status | r.static_status | r.batch[m->batch.step_record][0])
@@ -2463,7 +2473,7 @@ int ts2_get_params(ts2_model *m, int what, ts2_matrix_view *mats_out, int n_mats
     cudaError_t err = cudaSuccess;
     auto flush = [&]() {
         if (run && err == cudaSuccess)
-            err = cudaMemcpyAsync(dst0, src0, run * 4, cudaMemcpyDeviceToHost, m->read_stream);
+            err = cudaMemcpyAsync(dst0, src0, run * 4, cudaMemcpyDeviceToHost, m->export_stream);
         run = 0;
     };
     auto fetch = [&](int m0, int m1) {
@@ -2485,25 +2495,31 @@ int ts2_get_params(ts2_model *m, int what, ts2_matrix_view *mats_out, int n_mats
     };
     // Weights and momentum leave as soon as their group is updated, while the backward pass goes on below it: the copies of a
     // large model take as long as a step and more (437 M parameters 32 ms).  A copy is queued only when its source is ready, so
-    // none waits on the device for a step that does not end.
+    // none waits on the device for a step that does not end, and only while nothing is known to be wrong (8 us a group, beside the
+    // copies of the one before): what wait_stream would report leaves the caller's arrays alone.
     int rc = TS2_OK;
-    const bool dp = m->comm && m->world > 1;
-    if (what != TS2_PARAM_GRADIENT && !dp && !m->update_groups.empty()) {
-        for (UpdateGroup &g : m->update_groups) {
-            if ((rc = poll_until(m, [&] { return cudaEventQuery(g.done); })) != TS2_OK)
-                break;
-            fetch(g.mat0, g.mat1);
-        }
-        if (rc == TS2_OK)
-            rc = wait_stream(m);
-    } else if ((rc = wait_stream(m)) == TS2_OK) {
-        fetch(0, n_mats);
+    size_t done = 0; // groups fetched
+    const bool dp = m->comm && m->world > 1, grouped = what != TS2_PARAM_GRADIENT && !dp && !m->update_groups.empty();
+    for (; grouped && done < m->update_groups.size(); ++done) {
+        const UpdateGroup &g = m->update_groups[done];
+        if ((rc = poll_until(m, [&] { return cudaEventQuery(g.done); })) != TS2_OK || (rc = read_beside(m, nullptr)) != TS2_OK)
+            break;
+        const HostReport &r = *m->read_report;
+        if (r.device_status | r.static_status | r.batch[0][0] | r.batch[1][0])
+            break;
+        fetch(g.mat0, g.mat1);
     }
+    if (rc == TS2_OK)
+        rc = wait_stream(m);
+    if (rc == TS2_OK && !grouped)
+        fetch(0, n_mats);
+    for (; rc == TS2_OK && grouped && done < m->update_groups.size(); ++done) // what was wrong was not this model's
+        fetch(m->update_groups[done].mat0, m->update_groups[done].mat1);
     // none of the copies may still be on its way when the call returns
-    const cudaError_t done = cudaStreamSynchronize(m->read_stream);
+    const cudaError_t copied = cudaStreamSynchronize(m->export_stream);
     M_TRY(rc);
     TS2_CUDA(err);
-    TS2_CUDA(done);
+    TS2_CUDA(copied);
     return TS2_OK;
 }
 
