@@ -169,7 +169,7 @@ struct ts2_model {
     std::vector<UpdateGroup> update_groups;
     const ts2_training_step *step_in_backward = nullptr; // of the ts2_backprop call that is queuing its backward pass, if it applies
     cudaEvent_t ev_loss = nullptr;      // the training error of the last ts2_backprop is known
-    // What is read back while the step goes on, and weights that leave; nothing on either waits for another stream
+    // What is read back while the step goes on; weights that leave (queued when they are ready: nothing there waits for another stream)
     cudaStream_t read_stream = nullptr, export_stream = nullptr;
     CopyJob *d_copies = nullptr, *d_quants = nullptr; // what post_quantize and quantize_all do
     ScaleJob *d_scales = nullptr;
@@ -2436,14 +2436,14 @@ int ts2_forward_score(ts2_model *m, float *out_score)
 
 // The error is known when the forward pass and the final layer are through: the call waits for that and not for the backward
 // pass and the update behind it, so that the host prepares the next batch, or fetches weights as they are updated, meanwhile.
-// The host waits for the event and queues the read then: a call that gives up leaves nothing behind that a later one, with
-// another limit, would have to wait for.
+// The read waits for the event on the device: a host that waits first and queues then is 8 us later.  After a call that gave up it
+// is still queued, on a stream that is only ever waited for with the limit.
 int ts2_avg_train_err(ts2_model *m, float *out_err)
 {
     if (!m || !out_err)
         return fail(TS2_ERR_INVALID_ARG, "null argument");
     TS2_CUDA(cudaSetDevice(m->device));
-    M_TRY(poll_until(m, [&] { return cudaEventQuery(m->ev_loss); }));
+    TS2_CUDA(cudaStreamWaitEvent(m->read_stream, m->ev_loss, 0));
     M_TRY(read_beside(m, m->logp));
     const HostReport &r = *m->read_report;
     // Something went wrong, with the step or its batch: reported when the step is over.  The other record is not looked at: the
