@@ -96,6 +96,8 @@ def _declare(lib):
         "ts2_backprop": (i32, [vp, P(TrainingStep), i32]),
         "ts2_wait": (i32, [vp]),
         "ts2_set_wait_limit": (i32, [vp, C.c_double]),
+        "ts2_selftest_fail_backward": (i32, [vp, i32]),
+        "ts2_selftest_update_groups": (i32, [vp, C.c_int64, C.POINTER(i32)]),
         "ts2_forward_score": (i32, [vp, P(f32)]),
         "ts2_avg_train_err": (i32, [vp, P(f32)]),
         "ts2_get_params": (i32, [vp, i32, P(MatrixView), i32]),

@@ -137,7 +137,8 @@ struct BatchDev {
 // Matrices [mat0, mat1) that are updated together as soon as the backward pass has their gradients
 struct UpdateGroup {
     int mat0 = 0, mat1 = 0;
-    cudaEvent_t done = nullptr; // their weights and momentum are those of the last applied step
+    cudaEvent_t ready = nullptr; // the gradients of the step that is being queued are complete
+    cudaEvent_t done = nullptr;  // weights and momentum are those of the last applied step
 };
 
 } // namespace ts2
@@ -167,7 +168,8 @@ struct ts2_model {
     // One GPU, large models: in the order in which the backward pass completes them.  Small models are updated in one go after
     // it (empty).
     std::vector<UpdateGroup> update_groups;
-    const ts2_training_step *step_in_backward = nullptr; // of the ts2_backprop call that is queuing its backward pass, if it applies
+    bool groups_in_backward = false; // the backward pass that is being queued is followed by apply(), which updates in groups
+    cudaStream_t update_stream = nullptr;
     cudaEvent_t ev_loss = nullptr;      // the training error of the last ts2_backprop is known
     // What is read back while the step goes on; weights that leave (queued when they are ready: nothing there waits for another stream)
     cudaStream_t read_stream = nullptr, export_stream = nullptr;
@@ -271,6 +273,7 @@ struct ts2_model {
     float last_ms = 0;
     bool timing_valid = false;
     int last_targets = 0;
+    int fail_layer = -1; // self-test: the next backward pass ends in an error where it comes to this layer
     // data parallel
     ncclComm_t comm = nullptr;
     int rank = 0, world = 1;
@@ -950,13 +953,26 @@ int requantize_all(ts2_model *m)
     return quantize_all(m);
 }
 
-// Final layer, runs of layers from the last one down, embedding.  The weights of a group are final before the layers below it have
-// their gradients, so ts2_get_params copies them meanwhile (dim 2048, 4 blocks, 8 x 4096 tokens: step and export 147 -> 126 ms).
-// A group has at least UPDATE_GROUP_ELEMS elements: its four launches then take 20 us and more.  A model of less than two groups
-// is updated in one go: its export takes 1 ms or less.
-int build_update_groups(ts2_model *m)
+void drop_update_groups(ts2_model *m)
 {
-    if (m->flat_elems < 2 * UPDATE_GROUP_ELEMS)
+    for (UpdateGroup &g : m->update_groups)
+        for (cudaEvent_t e : {g.ready, g.done})
+            if (e)
+                cudaEventDestroy(e);
+    m->update_groups.clear();
+}
+
+// Final layer, runs of layers from the last one down, embedding.  The weights of a group are final before the layers below it have
+// their gradients, so ts2_get_params copies them meanwhile (dim 2048, 4 blocks, 8 x 4096 tokens: step and export 147 -> 122 ms).
+// A group has at least group_elems elements: its four launches then take 20 us and more.  A model of less than two groups is
+// updated in one go: its export takes 1 ms or less.
+// The groups run on a stream of their own.  Two launches of a group are a block per matrix, 15 to 27 us that in the main stream
+// only delayed the backward pass of models with many parameters and few tokens.  A step that no export follows, in one go /
+// groups in the main stream / as they are: 317 M parameters, 500 tokens 4.13 / 4.33 / 4.08 ms; 180 M, 300 tokens 2.70 / 2.77 / 2.71;
+// 113 M with experts, 500 tokens 1.84 / 1.88 / 1.77; 57 M, 256 tokens 0.706 / 0.723 / 0.700; 233 M, 4000 tokens 7.76 / 7.87 / 7.74.
+int build_update_groups(ts2_model *m, size_t group_elems)
+{
+    if (m->flat_elems < 2 * group_elems)
         return TS2_OK;
     auto elems = [&](int m0, int m1) { return (m1 < (int)m->mats.size() ? m->mats[m1].offset : m->flat_elems) - m->mats[m0].offset; };
     auto add = [&](int m0, int m1) {
@@ -967,13 +983,15 @@ int build_update_groups(ts2_model *m)
     add(1, 2);
     int end = (int)m->mats.size();
     for (int l = m->L - 1; l >= 0; --l)
-        if (l == 0 || elems(m->layers[l].mat0, end) >= UPDATE_GROUP_ELEMS) {
+        if (l == 0 || elems(m->layers[l].mat0, end) >= group_elems) {
             add(m->layers[l].mat0, end);
             end = m->layers[l].mat0;
         }
     add(0, 1);
-    for (UpdateGroup &g : m->update_groups)
+    for (UpdateGroup &g : m->update_groups) {
+        TS2_CUDA(cudaEventCreateWithFlags(&g.ready, cudaEventDisableTiming));
         TS2_CUDA(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming));
+    }
     return TS2_OK;
 }
 
@@ -1285,7 +1303,7 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
         m->nseg_shard = m->nseg_full;
         m->nitems_shard = m->nitems_full;
     }
-    M_TRY(build_update_groups(m));
+    M_TRY(build_update_groups(m, UPDATE_GROUP_ELEMS));
     M_TRY(build_post_quantize(m));
     M_TRY(requantize_all(m));
     TS2_CUDA(cudaStreamSynchronize(m->stream));
@@ -1592,9 +1610,10 @@ static int reduce_matrices(ts2_model *m, int m0, int m1)
 }
 
 // Gradient apply of the matrices [m0, m1) on one GPU: row sums, dispersion, update, matrix scales
-int update_matrices(ts2_model *m, const ts2_training_step *step, int m0, int m1)
+int update_matrices(ts2_model *m, const ts2_training_step *step, int m0, int m1, cudaStream_t stream)
 {
     Ctx c = ctx_of(m);
+    c.stream = stream;
     const OptSeg *segs = m->d_segs_full + m0; // a segment per matrix
     const OptMat *mats = m->d_optmats + m0;
     const int n = m1 - m0, item0 = m->mat_grow0[m0], items = (m1 < (int)m->mats.size() ? m->mat_grow0[m1] : m->n_rows_total) - item0;
@@ -1604,17 +1623,14 @@ int update_matrices(ts2_model *m, const ts2_training_step *step, int m0, int m1)
     return opt_sko(c, mats, n, m->roww2, m->skos + m0, step->disp_decay);
 }
 
-// The gradient of the matrices from m0 on is complete: applies the update groups that start there (a step that applies, one GPU).
-// Nothing of this step reads these weights any more.
+// The gradient of the matrices from m0 on is complete, and nothing of this step reads these weights any more: apply() may
+// update the groups that start there from here on
 int gradients_complete(ts2_model *m, int m0)
 {
-    if (!m->step_in_backward)
-        return TS2_OK;
-    for (UpdateGroup &g : m->update_groups)
-        if (g.mat0 == m0) {
-            M_TRY(update_matrices(m, m->step_in_backward, g.mat0, g.mat1));
-            TS2_CUDA(cudaEventRecord(g.done, m->stream));
-        }
+    if (m->groups_in_backward)
+        for (const UpdateGroup &g : m->update_groups)
+            if (g.mat0 == m0)
+                TS2_CUDA(cudaEventRecord(g.ready, m->stream));
     return TS2_OK;
 }
 
@@ -1773,6 +1789,10 @@ int backward(ts2_model *m)
     M_TRY(tap_gradient(m, L));
     const size_t fsz = fast_size(m);
     for (int l = L - 1; l >= 0; --l) {
+        if (l == m->fail_layer) {
+            m->fail_layer = -1;
+            return mfail(m, fail(TS2_ERR_UNSUPPORTED, "self-test: the backward pass ends at layer %d", l));
+        }
         Layer &ly = m->layers[l];
         const int W = ly.wide, C = ly.ncat * W;
         Matrix &mc = m->mats[ly.mat0 + ly.ncat];
@@ -1954,7 +1974,16 @@ int apply(ts2_model *m, const ts2_training_step *step)
     const int n_mats = (int)m->mats.size();
     if (!(m->comm && m->world > 1)) {
         if (m->update_groups.empty())
-            M_TRY(update_matrices(m, step, 0, n_mats));
+            M_TRY(update_matrices(m, step, 0, n_mats, m->stream));
+        // Queued when the whole backward pass is, so that a step that fails while it is being queued has changed no weight; on a
+        // stream of their own, so that they run beside what is left of it.
+        for (const UpdateGroup &g : m->update_groups) {
+            TS2_CUDA(cudaStreamWaitEvent(m->update_stream, g.ready, 0));
+            M_TRY(update_matrices(m, step, g.mat0, g.mat1, m->update_stream));
+            TS2_CUDA(cudaEventRecord(g.done, m->update_stream));
+        }
+        if (!m->update_groups.empty())
+            TS2_CUDA(cudaStreamWaitEvent(m->stream, m->update_groups.back().done, 0));
         return quantize_all(m);
     }
     if (!m->reduce_in_backward) { // gradients accumulated by calls that did not apply: exchange them now
@@ -2228,6 +2257,7 @@ int ts2_create(const ts2_model_descr *descr, const ts2_matrix_view *mats, int n_
     cudaEventCreateWithFlags(&m->ev_loss, cudaEventDisableTiming);
     cudaStreamCreateWithFlags(&m->read_stream, cudaStreamNonBlocking);
     cudaStreamCreateWithFlags(&m->export_stream, cudaStreamNonBlocking);
+    cudaStreamCreateWithFlags(&m->update_stream, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&m->ev_reduced, cudaEventDisableTiming);
     rc = build_model(m, mats, n_mats, bias);
     if (rc != TS2_OK) {
@@ -2274,15 +2304,15 @@ void ts2_destroy(ts2_model *m)
     for (cudaEvent_t e : m->batch.slot_ev)
         if (e)
             cudaEventDestroy(e);
-    for (UpdateGroup &g : m->update_groups)
-        if (g.done)
-            cudaEventDestroy(g.done);
+    drop_update_groups(m);
     if (m->ev_loss)
         cudaEventDestroy(m->ev_loss);
     if (m->read_stream)
         cudaStreamDestroy(m->read_stream);
     if (m->export_stream)
         cudaStreamDestroy(m->export_stream);
+    if (m->update_stream)
+        cudaStreamDestroy(m->update_stream);
     if (m->ev_start)
         cudaEventDestroy(m->ev_start);
     if (m->ev_stop)
@@ -2371,10 +2401,9 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
     // an accumulated gradient of earlier calls sits in the same buffer: the per-layer sums below then cover it too
     const bool dp = m->comm && m->world > 1;
     m->reduce_in_backward = add_to_model == TS2_GRADIENT_APPLY && dp;
-    m->step_in_backward = add_to_model == TS2_GRADIENT_APPLY && !dp ? step : nullptr;
+    m->groups_in_backward = add_to_model == TS2_GRADIENT_APPLY && !dp;
     const int brc = backward(m);
-    m->reduce_in_backward = false;
-    m->step_in_backward = nullptr;
+    m->reduce_in_backward = m->groups_in_backward = false;
     if (brc != TS2_OK)
         return brc;
     m->grads_dirty = true;
@@ -2389,6 +2418,27 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
     }
     TS2_CUDA(cudaEventRecord(m->ev_stop, m->stream));
     m->timing_valid = true;
+    return TS2_OK;
+}
+
+int ts2_selftest_fail_backward(ts2_model *m, int layer)
+{
+    if (!m || layer < 0 || layer >= m->L)
+        return fail(TS2_ERR_INVALID_ARG, "ts2_selftest_fail_backward: pass a model and one of its layers");
+    m->fail_layer = layer;
+    return TS2_OK;
+}
+
+int ts2_selftest_update_groups(ts2_model *m, int64_t group_elems, int *groups)
+{
+    if (!m || group_elems <= 0)
+        return fail(TS2_ERR_INVALID_ARG, "ts2_selftest_update_groups: pass a model and a number of elements");
+    TS2_CUDA(cudaSetDevice(m->device));
+    M_TRY(wait_stream(m));
+    drop_update_groups(m);
+    M_TRY(build_update_groups(m, (size_t)group_elems));
+    if (groups)
+        *groups = (int)m->update_groups.size();
     return TS2_OK;
 }
 
