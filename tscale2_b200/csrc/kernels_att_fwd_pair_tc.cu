@@ -1,6 +1,7 @@
 // Attention forward for many nodes (head width 128, sm_100a): a CTA works on two blocks of 128 nodes of a head at a time.
 // Same operands, results and rules as kernels_att_tc.cu (the zero "sink" vector is the initial state m = 0, l = 1; O is
-// rescaled only where a row's maximum grew by more than 8), without its form that also applies the gate.
+// rescaled only where a row's maximum grew by more than 8), without its form that also applies the gate: the operator call
+// (ts2_attention_forward) asks the rule below, the gated forward of training and scoring stays with the other kernel.
 //
 //   warp 0       TMA producer; draws the work items (pair of blocks, head) from a counter and finds their key ranges
 //   warp 1       TMEM owner and MMA issuer: S_i = Q_i . K^T (128 x 128), O_i += P_i . V with P_i from tensor memory
@@ -503,7 +504,8 @@ __global__ void __launch_bounds__(FP_THREADS, 1)
 } // namespace
 
 // Long causal sequences that start on tiles.  Whole calls, one block per CTA and two CTAs an SM (kernels_att_tc.cu) -> pairs, us:
-//   4 x 4096 x 16 heads 418 -> 359, 4 x 4096 x 7 234 -> 206, 2 x 4096 x 14 235 -> 200, 4 x 3072 x 16 270 -> 243;
+//   4 x 4096 x 16 heads 418 -> 359, 4 x 4096 x 7 234 -> 206, 2 x 4096 x 14 235 -> 200; 3072 nodes, the shortest, 4 x 3072 x 16
+//   forward and backward 907 -> 876, 4 x 3072 x 10 628 -> 616;
 //   spans of 1024 keys on average (8 x 2048 x 16) 252 -> 253, shorter ones lose (16 x 1024 x 12 141 -> 147): an item's start and
 //   end, which a second CTA on the SM hides;
 //   sequences that start inside a tile 4 x 3000 x 16 296 -> 296, 5 x 3333 x 9 282 -> 296: more tiles need the mask, and a pair waits
@@ -521,7 +523,7 @@ bool attention_forward_takes_pairs(int device, const int *span_start, const int 
                 return false;
             keys += span_finish[t] - span_start[t] + 1;
         }
-    return keys >= 1536ll * T;
+    return 2 * keys >= 3071ll * T; // what a causal sequence of 3072 nodes has
 }
 
 int attention_forward_pair_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
