@@ -425,7 +425,7 @@ int ts2_attention_forward(int device, void *stream, int variant, const void *q, 
     int *d = spans.d;
     if (variant == 2 && attention_forward_takes_pairs(device, span_start, span_finish, T, head_count, alibi_slope)) {
         TS2_CUDA(cudaMemsetAsync(d + 2 * (size_t)T, 0, 8, c.stream));
-        return attention_forward_pair_tc(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count, alibi_slope,
+        return attention_forward_pair_tc(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,
                                          (__half *)o, lse, d + 2 * (size_t)T);
     }
     int rc = variant == 2 ? attention_forward_tc(c, (const __half *)q, (const __half *)k, (const __half *)v, d, d + T, T, head_count,

@@ -194,7 +194,7 @@ int attention_forward_tc(const Ctx &c, const __half *q, const __half *k, const _
 // the tcgen05 form on pairs of 128-node blocks and when it is the faster one (spans on the host); counter: two zero words, left at zero
 bool attention_forward_takes_pairs(int device, const int *span_start, const int *span_finish, int T, int H, float slope);
 int attention_forward_pair_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
-                              int T, int H, float slope, __half *o, float *lse, int *counter);
+                              int T, int H, __half *o, float *lse, int *counter);
 int attention_forward_rowwise(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start,
                               const int *span_finish, int T, int H, float slope, __half *o, float *lse);
 int attention_backward_rowwise(const Ctx &c, const __half *q, const __half *k, const __half *v, const __half *dout, const float *lse,

@@ -34,7 +34,6 @@ constexpr int FP_ITEMS = 4; // slots of the item ring
 
 struct FwdPairParams {
     int T, H, n_pairs;
-    float slope;
     const int *span_start, *span_finish;
     float *lse;
     int *counter; // {next item, finished CTAs}, zero between launches (the last CTA resets them)
@@ -329,7 +328,7 @@ __global__ void __launch_bounds__(FP_THREADS, 1)
         const int grp = (warp - 4) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16, tS = tmem + grp * 128 + lane_addr, tO = tmem + 256 + grp * 128 + lane_addr;
         const uint32_t s_full = s_full0 + 8 * grp, p_full = p_full0 + 8 * grp, o_full = o_full0 + 8 * grp, o_free = o_free0 + 8 * grp;
-        const float ds = att_dot_scale_tc(), slope = p.slope;
+        const float ds = att_dot_scale_tc();
         uint8_t *const stg = smem + FP_STG_OFF + (warp - 4) * 4096, *const srow = stg + lane * 128;
         uint32_t s_phase = 0, o_phase = 0;
         bool ok = true;
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(FP_THREADS, 1)
                     tmem_ld32(tS + c * 32, s[c]);
                 tmem_ld_wait();
                 const int key0 = k * TC_BM;
-                const bool plain = slope == 0.f && __all_sync(0xffffffffu, key0 >= st_row && key0 + TC_BM - 1 <= fi_row);
+                const bool plain = __all_sync(0xffffffffu, key0 >= st_row && key0 + TC_BM - 1 <= fi_row);
                 float mx;
                 if (plain) { // the scores stay raw products and the scale rides in the exponent's fma
                     float r4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -372,14 +371,12 @@ __global__ void __launch_bounds__(FP_THREADS, 1)
                     mx = fmaxf(fmaxf(r4[0], r4[1]), fmaxf(r4[2], r4[3])) * ds;
                 } else {
                     float r4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-                    const float base = slope * (float)(t - key0);
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
                             const int key = key0 + c * 32 + i;
-                            float x = fmaf(__uint_as_float(s[c][i]), ds, fmaf(slope, (float)(c * 32 + i), -base));
-                            x = (key >= st_row && key <= fi_row) ? x : -INFINITY;
+                            const float x = (key >= st_row && key <= fi_row) ? __uint_as_float(s[c][i]) * ds : -INFINITY;
                             s[c][i] = __float_as_uint(x);
                             r4[i & 3] = fmaxf(r4[i & 3], x);
                         }
@@ -527,7 +524,7 @@ bool attention_forward_takes_pairs(int device, const int *span_start, const int 
 }
 
 int attention_forward_pair_tc(const Ctx &c, const __half *q, const __half *k, const __half *v, const int *span_start, const int *span_finish,
-                              int T, int H, float slope, __half *o, float *lse, int *counter)
+                              int T, int H, __half *o, float *lse, int *counter)
 {
     static bool configured[16] = {};
     if (!configured[c.device & 15]) {
@@ -544,7 +541,6 @@ int attention_forward_pair_tc(const Ctx &c, const __half *q, const __half *k, co
     p.T = T;
     p.H = H;
     p.n_pairs = (int)ceil_div(T, 2 * TC_BM);
-    p.slope = slope;
     p.span_start = span_start;
     p.span_finish = span_finish;
     p.lse = lse;
