@@ -37,10 +37,11 @@ struct RowProblem {
     int M, N, n_tiles, tiles, splits, k_blocks, kb_per_split;
     uint32_t idesc;
     float alpha;
-    const float *dyn_scale, *dyn_scale2, *row_scale, *col_scale, *c_in;
-    void *C;
+    const float *dyn_scale, *dyn_scale2, *row_scale;
+    // second problem: C = (c_in or nothing) + product
+    const float *c_in;
+    float *C;
     long long ldc;
-    int out_kind;
 };
 struct RowParams {
     RowProblem pr[2];
@@ -233,35 +234,26 @@ __global__ void __launch_bounds__(R_THREADS, 2)
             alpha *= __ldg(pr.dyn_scale);
         if (pr.dyn_scale2)
             alpha *= __ldg(pr.dyn_scale2);
-        auto product = [&](int r, int c) { // columns c .. c + 3 of row r, summed over the cluster in rank order
-            const uint32_t at = tile_addr + (uint32_t)(r * R_PITCH + c) * 4;
-            if (splits == 1)
-                return *(const float4 *)(tile_s + r * R_PITCH + c);
+        auto times = [](float4 v, float f) { // rounded: no part of an fma with what it is added to
+            return make_float4(__fmul_rn(v.x, f), __fmul_rn(v.y, f), __fmul_rn(v.z, f), __fmul_rn(v.w, f));
+        };
+        auto product = [&](int r, int c) { // columns c .. c + 3 of row r, summed over the cluster in rank order, with the scales applied
             float4 s = make_float4(0, 0, 0, 0);
-            for (int sp = 0; sp < splits; ++sp) {
-                const float4 v = ld_cluster4(at, sp);
-                s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
-            }
-            return s;
+            if (splits == 1)
+                s = *(const float4 *)(tile_s + r * R_PITCH + c);
+            else
+                for (int sp = 0; sp < splits; ++sp) {
+                    const float4 v = ld_cluster4(tile_addr + (uint32_t)(r * R_PITCH + c) * 4, sp);
+                    s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+                }
+            return times(s, alpha * (pr.row_scale ? __ldg(pr.row_scale + m0 + r) : 1.f));
         };
-        // with the scales applied, as the plain epilogues do
-        auto scaled = [&](int r, int c, float4 cs, bool cols) {
-            float4 v = product(r, c);
-            const float rs = alpha * (pr.row_scale ? __ldg(pr.row_scale + m0 + r) : 1.f);
-            if (cols)
-                return make_float4(v.x * (rs * cs.x), v.y * (rs * cs.y), v.z * (rs * cs.z), v.w * (rs * cs.w));
-            return scale4(v, rs);
-        };
-        const int c = lane * 4, col = n0 + c, form = second ? (int)ROW_PLAIN : p.op.form;
-        const bool cols = pr.col_scale && col < pr.N;
-        const float4 cs = cols ? __ldg((const float4 *)(pr.col_scale + col)) : make_float4(1, 1, 1, 1);
-        const RowOp &op = p.op;
-        switch (form) {
-        case ROW_PLAIN:
+        const int c = lane * 4, col = n0 + c;
+        if (second) {
             if (col < pr.N)
                 for_rows(r0, rm, [&](int r, int n) {
                     float4 in[R_ROWS];
-                    if (pr.out_kind == TS2_OUT_F32_ADD)
+                    if (pr.c_in)
 #pragma unroll
                         for (int i = 0; i < R_ROWS; ++i)
                             if (i < n)
@@ -270,22 +262,14 @@ __global__ void __launch_bounds__(R_THREADS, 2)
                     for (int i = 0; i < R_ROWS; ++i) {
                         if (i >= n)
                             break;
-                        float4 v = scaled(r + i, c, cs, cols);
-                        const long long at = (m0 + r + i) * pr.ldc + col;
-                        if (pr.out_kind == TS2_OUT_F32_ADD)
+                        float4 v = product(r + i, c);
+                        if (pr.c_in)
                             v = make_float4(in[i].x + v.x, in[i].y + v.y, in[i].z + v.z, in[i].w + v.w);
-                        if (pr.out_kind == TS2_OUT_F16) {
-                            store_half4((__half *)pr.C + at, v);
-                        } else if (pr.out_kind == TS2_OUT_BF16) {
-                            const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-                            *(uint2 *)((__nv_bfloat16 *)pr.C + at) = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
-                        } else {
-                            *(float4 *)((float *)pr.C + at) = v;
-                        }
+                        *(float4 *)(pr.C + (m0 + r + i) * pr.ldc + col) = v;
                     }
                 });
-            break;
-        case ROW_NORM_BWD: {
+        } else {
+            const RowOp &op = p.op;
             const float a = op.dyn ? __ldg(op.dyn) : 1.f;
             float mx = 0.f;
             for_rows(r0, rm, [&](int r, int n) {
@@ -300,7 +284,10 @@ __global__ void __launch_bounds__(R_THREADS, 2)
                 for (int i = 0; i < R_ROWS; ++i) {
                     if (i >= n)
                         break;
-                    const float4 d = tilenorm_backward4(xv[i], scale4(scaled(r + i, c, cs, cols), a));
+                    const float4 x = xv[i], dn = times(product(r + i, c), a);
+                    // the sum's order spelled out: the compiler's own choice follows from what stands around it
+                    const float xd = fmaf(x.w, dn.w, fmaf(x.z, dn.z, fmaf(x.y, dn.y, __fmul_rn(x.x, dn.x))));
+                    const float4 d = tilenorm_backward4(x, dn, xd);
                     const float4 g = make_float4(gv[i].x + d.x, gv[i].y + d.y, gv[i].z + d.z, gv[i].w + d.w);
                     *(float4 *)(op.g + (long long)(m0 + r + i) * pr.N + col) = g;
                     mx = absmax4(mx, g);
@@ -309,8 +296,6 @@ __global__ void __launch_bounds__(R_THREADS, 2)
             mx = warp_max(mx);
             if (lane == 0 && r0 < rm)
                 absmax_report(mx, op.absmax, op.health, op.step_no);
-            break;
-        }
         }
     }
     __syncwarp();
@@ -336,11 +321,9 @@ RowProblem row_problem(const GemmArgs &a, int splits)
     p.dyn_scale = a.epi.dyn_scale;
     p.dyn_scale2 = a.epi.dyn_scale2;
     p.row_scale = a.epi.row_scale;
-    p.col_scale = a.epi.col_scale;
-    p.c_in = a.epi.c_in ? a.epi.c_in : (const float *)a.C;
-    p.C = a.C;
+    p.c_in = a.epi.out_kind != TS2_OUT_F32_ADD ? nullptr : a.epi.c_in ? a.epi.c_in : (const float *)a.C;
+    p.C = (float *)a.C;
     p.ldc = a.ldc;
-    p.out_kind = a.epi.out_kind;
     return p;
 }
 
@@ -426,29 +409,26 @@ bool gemm_row_takes_pair(int device, const GemmArgs &a, const GemmArgs &b)
 int gemm_row(const RowGemm &r)
 {
     const GemmArgs &a = r.a;
-    const GemmArgs *const list[2] = {a.M > 0 ? &a : nullptr, r.second};
-    const GemmArgs &any = list[0] ? a : *r.second;
+    const GemmArgs *const list[2] = {&a, r.second};
     double flops = 0, bytes = 0;
     for (const GemmArgs *g : list) {
         if (!g)
             continue;
-        const int out_es = g->epi.out_kind == TS2_OUT_F32 || g->epi.out_kind == TS2_OUT_F32_ADD ? 4 : 2;
-        if (g->M <= 0 || g->N <= 0 || g->K <= 0 || g->N % 32 || g->mn_major != (g == r.second) || g->group_mode || g->epi.pair_stride ||
-            g->epi.bwd_wg || g->kind == KIND_BF16 || ((uintptr_t)g->C & 15) || ((g->ldc * out_es) & 15) ||
-            ((uintptr_t)g->epi.col_scale & 15) || (g == &a && r.op.form != ROW_PLAIN && g->N % 128))
+        const bool add = g->epi.out_kind == TS2_OUT_F32_ADD;
+        if (g->M <= 0 || g->N <= 0 || g->K <= 0 || g->mn_major != (g == r.second) || g->group_mode || g->epi.pair_stride || g->epi.bwd_wg ||
+            g->kind == KIND_BF16 || g->epi.col_scale || (g->epi.out_kind != TS2_OUT_F32 && !add) ||
+            (g == &a ? r.op.form != ROW_NORM_BWD || add || g->N % 128 : g->N % 32 || ((uintptr_t)g->C & 15) || ((g->ldc * 4) & 15)))
             return fail(TS2_ERR_INVALID_ARG, "gemm_row: bad arguments");
         flops += 2.0 * g->M * g->N * g->K;
-        bytes += ((double)g->M + g->N) * g->K * (g->kind == KIND_F16 ? 2 : 1) + (double)g->M * g->N * (g->epi.out_kind == TS2_OUT_F32_ADD ? 8 : out_es);
+        bytes += ((double)g->M + g->N) * g->K * (g->kind == KIND_F16 ? 2 : 1) + (double)g->M * g->N * (add ? 8 : 4);
     }
-    TS2_CUDA(cudaSetDevice(any.device));
+    TS2_CUDA(cudaSetDevice(a.device));
     RowParams p;
     CUtensorMap tm[4];
-    int rc, s[2] = {1, 1}, cluster = 1;
-    const long long slots = 2 * sm_count(any.device);
-    for (int i = 0; i < 2; ++i)
-        if (list[i])
-            gemm_row_plan(any.device, list[i]->kind, list[i]->M, list[i]->N, list[i]->K, &s[i]);
-    if (list[0] && list[1]) {
+    int rc, s[2] = {1, 1};
+    const long long slots = 2 * sm_count(a.device);
+    gemm_row_plan(a.device, a.kind, a.M, a.N, a.K, &s[0]);
+    if (r.second) {
         // one cluster size for the launch: the first contraction, which the next kernel waits for, has its choice as far as
         // both stay within one wave; the second takes the same or none
         const long long t1 = ceil_div(a.M, BM) * ceil_div(a.N, R_BN), t2 = ceil_div(r.second->M, BM) * ceil_div(r.second->N, R_BN);
@@ -457,10 +437,10 @@ int gemm_row(const RowGemm &r)
             s[0] /= 2;
         s[1] = s[0] > 1 && (t1 + t2) * s[0] <= slots / 2 && (int)ceil_div(k2, ceil_div(k2, s[0])) == s[0] && k2 >= 4 * s[0] ? s[0] : 1;
     }
-    cluster = std::max(s[0], s[1]);
+    const int cluster = s[0]; // s[1] is the same or 1
     int grid = 0;
     for (int i = 0; i < 2; ++i) {
-        const GemmArgs &g = list[i] ? *list[i] : any;
+        const GemmArgs &g = list[i] ? *list[i] : a;
         p.pr[i] = row_problem(g, s[i]);
         if ((rc = row_maps(g, &tm[2 * i], &tm[2 * i + 1])) != TS2_OK)
             return rc;
@@ -470,22 +450,20 @@ int gemm_row(const RowGemm &r)
             p.first2 = grid;
     }
     p.op = r.op;
-    p.status = device_status_word(any.device);
+    p.status = device_status_word(a.device);
     if (!p.status)
         return fail(TS2_ERR_CUDA, "gemm: no device status word");
-    const GemmTimed timed = gemm_timed_begin(any.stream);
-    const int k1 = a.M > 0 ? a.kind : r.second->kind, k2 = r.second ? r.second->kind : a.kind;
+    const GemmTimed timed = gemm_timed_begin(a.stream);
+    const int k1 = a.kind, k2 = r.second ? r.second->kind : k1 == KIND_I8 ? KIND_F16 : k1; // of none: any that is built
     if (k1 == KIND_E4M3 && k2 == KIND_E4M3)
-        rc = launch_row<0, 0>(any.device, any.stream, grid, cluster, tm, p);
+        rc = launch_row<0, 0>(a.device, a.stream, grid, cluster, tm, p);
     else if (k1 == KIND_F16 && k2 == KIND_F16)
-        rc = launch_row<1, 1>(any.device, any.stream, grid, cluster, tm, p);
+        rc = launch_row<1, 1>(a.device, a.stream, grid, cluster, tm, p);
     else if (k1 == KIND_I8 && k2 == KIND_F16)
-        rc = launch_row<2, 1>(any.device, any.stream, grid, cluster, tm, p);
-    else if (k1 == KIND_I8 && k2 == KIND_I8)
-        rc = launch_row<2, 2>(any.device, any.stream, grid, cluster, tm, p);
+        rc = launch_row<2, 1>(a.device, a.stream, grid, cluster, tm, p);
     else
         return fail(TS2_ERR_UNSUPPORTED, "gemm_row: unsupported pair of operand formats");
-    gemm_timed_end(timed, any.stream, flops, bytes, any.tag);
+    gemm_timed_end(timed, a.stream, flops, bytes, a.tag);
     return rc;
 }
 

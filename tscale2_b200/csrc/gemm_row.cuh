@@ -5,7 +5,7 @@
 namespace ts2 {
 
 // What becomes of the product, 128 columns of a row at a time (widths are multiples of 128 in all forms but the first and the
-// last).  The row kernel (gemm_row.cu) has the first and the third, pairs of CTAs (Epilogue::row) all but the first.
+// last).  The row kernel (gemm_row.cu) has the third, pairs of CTAs (Epilogue::row) all but the first.
 enum RowForm {
     ROW_PLAIN = 0, // Epilogue::out_kind, as any contraction
     ROW_NORM,      // C = c_in + product (fp32); n_fast = tile normalisation of C, n16 optionally (tilenorm_forward)
@@ -31,8 +31,8 @@ struct RowOp {
     float *target_logit = nullptr;
 };
 
-// First contraction (K contiguous in both operands) with its row step, and optionally a second one beside it in the same
-// launch: token-major operands, ROW_PLAIN, independent of the first.
+// First contraction (K contiguous in both operands) with ROW_NORM_BWD behind it, and optionally a second one beside it in the same
+// launch: token-major operands, fp32 output or added to it, independent of the first.
 struct RowGemm {
     GemmArgs a;
     RowOp op;

@@ -8,16 +8,17 @@
 namespace ts2 {
 
 // ---- tile normalisation ---------------------------------------------------------
-// gradient of the raw values x from the gradient d of the normalised ones (whole warp)
-__device__ __forceinline__ float4 tilenorm_backward4(float4 x, float4 d)
+// gradient of the raw values x from the gradient d of the normalised ones (whole warp); xd: the lane's part of x . d
+__device__ __forceinline__ float4 tilenorm_backward4(float4 x, float4 d, float xd)
 {
     const float sum2 = warp_sum(dot4(x, x));
-    const float dp = warp_sum(dot4(x, d));
+    const float dp = warp_sum(xd);
     if (sum2 == 0.f)
         return make_float4(0, 0, 0, 0);
     const float sigma = dp / sum2, scale = sqrtf(128.f / sum2);
     return make_float4(scale * (d.x - x.x * sigma), scale * (d.y - x.y * sigma), scale * (d.z - x.z * sigma), scale * (d.w - x.w * sigma));
 }
+__device__ __forceinline__ float4 tilenorm_backward4(float4 x, float4 d) { return tilenorm_backward4(x, d, dot4(x, d)); }
 // running |maximum| of a gradient; fmaxf drops a NaN operand: a NaN turns it into inf instead
 __device__ __forceinline__ float absmax4(float m, float4 r)
 {
