@@ -188,9 +188,11 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model);
 /* Self-tests.  The first makes the next ts2_backprop fail (TS2_ERR_UNSUPPORTED) while it queues its backward pass, where that comes
  * to `layer`: such a call leaves weights, momentum and scales as they were, and the step can be repeated.  The second sets from how
  * many elements on matrices are updated as a group beside the backward pass (a model of less than twice as many is updated in one
- * go; the results are the same bits) and tells the number of groups (may be NULL). */
+ * go; the results are the same bits) and tells the number of groups (may be NULL).  The third sets how many nodes (a multiple of
+ * 256; 0: as many as there is room for) ts2_forward_score takes through the final layer at a time. */
 int ts2_selftest_fail_backward(ts2_model *m, int layer);
 int ts2_selftest_update_groups(ts2_model *m, int64_t group_elems, int *groups);
+int ts2_selftest_score_part(ts2_model *m, int nodes);
 /* IModel::WaitAllCompute, src/gpt/compute/model.h:54 — bounded wait */
 int ts2_wait(ts2_model *m);
 /* Wall time after which a call that waits for the device (ts2_wait and everything that reads results, and ts2_set_batch

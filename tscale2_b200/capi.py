@@ -98,6 +98,7 @@ def _declare(lib):
         "ts2_set_wait_limit": (i32, [vp, C.c_double]),
         "ts2_selftest_fail_backward": (i32, [vp, i32]),
         "ts2_selftest_update_groups": (i32, [vp, C.c_int64, C.POINTER(i32)]),
+        "ts2_selftest_score_part": (i32, [vp, i32]),
         "ts2_forward_score": (i32, [vp, P(f32)]),
         "ts2_avg_train_err": (i32, [vp, P(f32)]),
         "ts2_get_params": (i32, [vp, i32, P(MatrixView), i32]),

@@ -273,7 +273,9 @@ struct ts2_model {
     float last_ms = 0;
     bool timing_valid = false;
     int last_targets = 0;
-    int fail_layer = -1; // self-test: the next backward pass ends in an error where it comes to this layer
+    // self-tests: the next backward pass ends in an error where it comes to this layer; nodes that are scored at a time (0: as many as
+    // there is room for)
+    int fail_layer = -1, score_part = 0;
     // data parallel
     ncclComm_t comm = nullptr;
     int rank = 0, world = 1;
@@ -1506,7 +1508,7 @@ int score_rows(ts2_model *m, const Epilogue &logits, bool *done)
     const int T = m->batch.node_count, D = m->D, V = m->V, n = 4 * (int)ceil_div(V, 256);
     const size_t fs = fast_size(m);
     const size_t room = (size_t)m->chunk * V * sizeof(__half) / (n * sizeof(float2) + sizeof(float)); // nodes
-    const int most = (int)(room >= (size_t)T ? T : room / 256 * 256);
+    const int fit = (int)(room >= (size_t)T ? T : room / 256 * 256), most = m->score_part ? std::min(m->score_part, fit) : fit;
     *done = most > 0;
     for (int r0 = 0; r0 < T && *done; r0 += most) // whatever is left in the last one
         *done = gemm_takes_row(m->device, m->kind, std::min(most, T - r0), V, D, ROW_LSE);
@@ -2426,6 +2428,14 @@ int ts2_selftest_fail_backward(ts2_model *m, int layer)
     if (!m || layer < 0 || layer >= m->L)
         return fail(TS2_ERR_INVALID_ARG, "ts2_selftest_fail_backward: pass a model and one of its layers");
     m->fail_layer = layer;
+    return TS2_OK;
+}
+
+int ts2_selftest_score_part(ts2_model *m, int nodes)
+{
+    if (!m || nodes < 0 || nodes % 256)
+        return fail(TS2_ERR_INVALID_ARG, "ts2_selftest_score_part: pass a model and a multiple of 256 nodes");
+    m->score_part = nodes;
     return TS2_OK;
 }
 
