@@ -25,7 +25,7 @@ def forward(lib, variant, q, k, v, seq, H):
     return o.download(q.shape, np.float16), lse.download((T, H), np.float32)
 
 
-@pytest.mark.parametrize("seq,pairs", [(3072, True), (2816, False)])
+@pytest.mark.parametrize("seq,pairs", [(3072, True), (2816, False), (4096, True), (3200, False), (3073, False)])
 def test_the_border(seq, pairs):
     """One sequence alone has too few work items and runs on the other kernel, whose sums come in another order: four of them give
     the same bits only if they run there too."""
