@@ -75,3 +75,18 @@ def test_no_time_left_leaves_the_arrays_alone():
     model.wait()
     for a, b in zip(out, model.get_weights()):
         assert np.array_equal(a, b)
+
+
+def test_a_later_batch_that_is_known_to_be_malformed():
+    spec, model, good, bad = a_model()
+    flat, out = arrays(spec, True)
+    views = host.matrix_views(out)
+    model.set_batch(good)
+    model.backprop(host.training_step(rate=0.01))
+    model.set_batch(bad)
+    torch.cuda.synchronize()  # it is checked by now
+    assert model.lib.ts2_get_params(model.h, capi.PARAM_WEIGHTS, views, len(out)) == capi.TS2_ERR_INVALID_ARG
+    assert (flat == 7.5).all()
+    model._check(model.lib.ts2_get_params(model.h, capi.PARAM_WEIGHTS, views, len(out)))  # reported: the step's weights are there
+    for a, b in zip(out, model.get_weights()):
+        assert np.array_equal(a, b)

@@ -258,7 +258,14 @@ int opt_disp(const Ctx &c, const OptMat *mats, int n_mats, const float *rowsum, 
 int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int item0, int nitems, const float *grad, const float *row_scale,
                const ts2_training_step *step, float *avg, float *w, double *roww2);
 // disp_decay: the step's, or negative when no step was applied
-int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos, float disp_decay);
+// wrong (pinned memory, optional): not zero if the device's status words or the batch records hold anything by then
+struct WrongSoFar {
+    const int32_t *device_status = nullptr, *static_status = nullptr;
+    const int *batch_status = nullptr;
+    int *out = nullptr;
+};
+int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos, float disp_decay, const int *batch_status = nullptr,
+            int *wrong = nullptr);
 int opt_quantize(const Ctx &c, const OptSeg *segs, int nseg, int nitems, const float *w, const float *skos);
 // copy (dst) and / or transposed copy (dstT) of a block of quantized values [y][x], x a multiple of 128; pitches in bytes
 enum { QCOPY_1BYTE = 0, QCOPY_E4M3_HALF = 1, QCOPY_I8_HALF = 2, QCOPY_2BYTE = 3 }; // _HALF: the transpose is widened to fp16

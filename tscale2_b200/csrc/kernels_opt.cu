@@ -172,9 +172,13 @@ __global__ void opt_update_kernel(const OptSeg *__restrict__ segs, int nseg, int
 
 // one block per matrix: sko = sqrt(sum of squares / (x y)), rows summed in a fixed order
 // (disp_decay >= 0: a step was applied, the weight of the dispersion average moves on)
-__global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__restrict__ roww2, float *__restrict__ skos, float disp_decay)
+__global__ void opt_sko_kernel(const OptMat *__restrict__ mats, const double *__restrict__ roww2, float *__restrict__ skos, float disp_decay,
+                               const WrongSoFar wrong)
 {
     grid_dep_wait();
+    if (wrong.out && blockIdx.x == 0 && threadIdx.x == 0)
+        *wrong.out = (wrong.device_status ? *wrong.device_status : 0) | (wrong.static_status ? *wrong.static_status : 0) |
+                     wrong.batch_status[0] | wrong.batch_status[4];
     __shared__ double red[32];
     const OptMat mt = mats[blockIdx.x];
     double s = 0.0;
@@ -266,9 +270,14 @@ int opt_update(const Ctx &c, const OptSeg *segs, int nseg, int item0, int nitems
     return TS2_OK;
 }
 
-int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos, float disp_decay)
+int opt_sko(const Ctx &c, const OptMat *mats, int n_mats, const double *roww2, float *skos, float disp_decay, const int *batch_status, int *wrong)
 {
-    TS2_LAUNCH((opt_sko_kernel), n_mats, 1024, 0, c.stream, mats, roww2, skos, disp_decay);
+    WrongSoFar w;
+    if (wrong) {
+        w.device_status = device_status_word(c.device), w.static_status = static_status_word_if_ready(c.device);
+        w.batch_status = batch_status, w.out = wrong;
+    }
+    TS2_LAUNCH((opt_sko_kernel), n_mats, 1024, 0, c.stream, mats, roww2, skos, disp_decay, w);
     return TS2_OK;
 }
 

@@ -139,6 +139,7 @@ struct UpdateGroup {
     int mat0 = 0, mat1 = 0;
     cudaEvent_t ready = nullptr; // the gradients of the step that is being queued are complete
     cudaEvent_t done = nullptr;  // weights and momentum are those of the last applied step
+    int *wrong = nullptr;        // pinned: whether something was known by then to have gone wrong
 };
 
 } // namespace ts2
@@ -246,6 +247,8 @@ struct ts2_model {
     size_t pinned_bytes = 0;
     HostReport *report = nullptr;  // pinned; written by the kernel that every wait queues (queue_report)
     HostReport *read_report = nullptr; // the same for read_stream
+    int *wrong = nullptr;          // pinned, a word per update group
+    bool applied_last = false;     // an applied step is the last thing that was queued
     bool unreported = false;       // work was queued since the last wait
     double wait_limit_s = 120;     // wall time after which a wait gives up (poll_until)
     bool grads_dirty = false; // the flat gradient holds an accumulated, not yet applied gradient
@@ -980,6 +983,7 @@ int build_update_groups(ts2_model *m, size_t group_elems)
     auto add = [&](int m0, int m1) {
         UpdateGroup g;
         g.mat0 = m0, g.mat1 = m1;
+        g.wrong = m->wrong + m->update_groups.size();
         m->update_groups.push_back(g);
     };
     add(1, 2);
@@ -1255,11 +1259,13 @@ int build_model(ts2_model *m, const ts2_matrix_view *mats, int n_mats, const flo
     }
     M_TRY(dalloc(m, &b.ix.hist, label_index_hist_elems(b.label_cap)));
     M_TRY(dalloc(m, &b.ix.partial, label_index_partial_elems(m->device, b.label_cap, D)));
-    m->pinned_bytes = 2 * b.raw_cap * 4 + 2 * sizeof(HostReport);
+    const size_t max_groups = (size_t)m->L + 2;
+    m->pinned_bytes = 2 * b.raw_cap * 4 + 2 * sizeof(HostReport) + max_groups * sizeof(int);
     TS2_CUDA(cudaMallocHost(&m->pinned, m->pinned_bytes));
     m->report = (HostReport *)((uint32_t *)m->pinned + 2 * b.raw_cap);
     m->read_report = m->report + 1;
-    memset(m->report, 0, 2 * sizeof(HostReport));
+    m->wrong = (int *)(m->report + 2);
+    memset(m->report, 0, 2 * sizeof(HostReport) + max_groups * sizeof(int));
     for (int i = 0; i < 2; ++i)
         TS2_CUDA(cudaEventCreateWithFlags(&b.slot_ev[i], cudaEventDisableTiming));
 
@@ -1612,7 +1618,7 @@ static int reduce_matrices(ts2_model *m, int m0, int m1)
 }
 
 // Gradient apply of the matrices [m0, m1) on one GPU: row sums, dispersion, update, matrix scales
-int update_matrices(ts2_model *m, const ts2_training_step *step, int m0, int m1, cudaStream_t stream)
+int update_matrices(ts2_model *m, const ts2_training_step *step, int m0, int m1, cudaStream_t stream, int *wrong = nullptr)
 {
     Ctx c = ctx_of(m);
     c.stream = stream;
@@ -1622,7 +1628,7 @@ int update_matrices(ts2_model *m, const ts2_training_step *step, int m0, int m1,
     M_TRY(opt_row_sum2(c, segs, n, item0, items, m->grad_flat, m->rowsum));
     M_TRY(opt_disp(c, mats, n, m->rowsum, step->disp_decay, m->row_scale));
     M_TRY(opt_update(c, segs, n, item0, items, m->grad_flat, m->row_scale, step, m->avg_flat, m->w_flat, m->roww2));
-    return opt_sko(c, mats, n, m->roww2, m->skos + m0, step->disp_decay);
+    return opt_sko(c, mats, n, m->roww2, m->skos + m0, step->disp_decay, m->batch.status, wrong);
 }
 
 // The gradient of the matrices from m0 on is complete, and nothing of this step reads these weights any more: apply() may
@@ -1981,7 +1987,7 @@ int apply(ts2_model *m, const ts2_training_step *step)
         // stream of their own, so that they run beside what is left of it.
         for (const UpdateGroup &g : m->update_groups) {
             TS2_CUDA(cudaStreamWaitEvent(m->update_stream, g.ready, 0));
-            M_TRY(update_matrices(m, step, g.mat0, g.mat1, m->update_stream));
+            M_TRY(update_matrices(m, step, g.mat0, g.mat1, m->update_stream, g.wrong));
             TS2_CUDA(cudaEventRecord(g.done, m->update_stream));
         }
         if (!m->update_groups.empty())
@@ -2351,6 +2357,7 @@ int ts2_set_batch(ts2_model *m, const ts2_batch_nodes *nodes)
     if (m->unreported && cudaStreamQuery(m->stream) == cudaSuccess)
         M_TRY(wait_stream(m));
     m->unreported = true;
+    m->applied_last = false;
     M_TRY(stage_batch(m, nodes));
     return TS2_OK;
 }
@@ -2388,6 +2395,7 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
         return mfail(m, fail(TS2_ERR_INVALID_ARG, "ts2_backprop before ts2_set_batch"));
     TS2_CUDA(cudaSetDevice(m->device));
     m->unreported = true;
+    m->applied_last = false;
     TS2_CUDA(cudaEventRecord(m->ev_start, m->stream));
     m->batch.step_record = m->batch.record;
     ++m->step_no;
@@ -2417,6 +2425,7 @@ int ts2_backprop(ts2_model *m, const ts2_training_step *step, int add_to_model)
         if (arc != TS2_OK)
             return arc;
         m->grads_dirty = false;
+        m->applied_last = true;
     }
     TS2_CUDA(cudaEventRecord(m->ev_stop, m->stream));
     m->timing_valid = true;
@@ -2555,17 +2564,20 @@ int ts2_get_params(ts2_model *m, int what, ts2_matrix_view *mats_out, int n_mats
     };
     // Weights and momentum leave as soon as their group is updated, while the backward pass goes on below it: the copies of a
     // large model take as long as a step and more (437 M parameters 32 ms).  A copy is queued only when its source is ready, so
-    // none waits on the device for a step that does not end, and only while nothing is known to be wrong (8 us a group, beside the
-    // copies of the one before): what wait_stream would report leaves the caller's arrays alone.
+    // none waits on the device for a step that does not end, and only while nothing is known to be wrong: what wait_stream would
+    // report leaves the caller's arrays alone.  The group's last launch notes that down (a launch for it alone waits until a
+    // contraction gives an SM free: 0.3 ms before the first group of that model leaves); where more was queued behind the step,
+    // the records are read once more.
     int rc = TS2_OK;
     size_t done = 0; // groups fetched
     const bool dp = m->comm && m->world > 1, grouped = what != TS2_PARAM_GRADIENT && !dp && !m->update_groups.empty();
     for (; grouped && done < m->update_groups.size(); ++done) {
         const UpdateGroup &g = m->update_groups[done];
-        if ((rc = poll_until(m, [&] { return cudaEventQuery(g.done); })) != TS2_OK || (rc = read_beside(m, nullptr)) != TS2_OK)
+        if ((rc = poll_until(m, [&] { return cudaEventQuery(g.done); })) != TS2_OK || *(volatile int *)g.wrong ||
+            (!m->applied_last && (rc = read_beside(m, nullptr)) != TS2_OK))
             break;
         const HostReport &r = *m->read_report;
-        if (r.device_status | r.static_status | r.batch[0][0] | r.batch[1][0])
+        if (!m->applied_last && (r.device_status | r.static_status | r.batch[0][0] | r.batch[1][0]))
             break;
         fetch(g.mat0, g.mat1);
     }
