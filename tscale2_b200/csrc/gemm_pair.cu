@@ -580,7 +580,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(epi8(FORM) ? P_THREA
         } else if constexpr (FORM == P_LSE) {
             // Scoring: nothing of the logits leaves the chip but each row's maximum and sum per 64 columns (an eighth of a percent
             // of their bytes) and the target's logit.  12000 x 50304 logits x 768, fp16: 700 us and 26 for the sum over the partial
-            // results, where logits in memory (2.4 GB written and read) took 790 and 320.
+            // results, where logits in memory (2.4 GB written and read) took 790 and 320.  18 warps leave 96 registers
+            // a thread: 44 bytes spilled, 56 loaded.
             const int part = ew >> 2;
             for (int u = first; u < units; u += step) {
                 const PairUnit un = pair_unit(p, u);
@@ -713,9 +714,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(epi8(FORM) ? P_THREA
             // recent one have read theirs: `cur` holds the block that was fetched ahead, `prev` was stored from last, the third
             // one is free.
             // P_NORM: C = c_in + product, and its tile normalisation, which as a kernel of its own read C back (65536 x 768,
-            // e4m3: contraction 121 and normalisation 48 -> 138 us).  P_NORM_BWD: the product d (scale-free, times dyn_scale2) is the gradient of the normalised x; the
-            // accumulator is read twice, beside x for the two sums over the tile and beside g for the result; the product
-            // used to go through memory (65536 x 768, e4m3: contraction 239 and normalisation 114 -> 277 us).
+            // e4m3: contraction 121 and normalisation 48 -> 138 us).  P_NORM_BWD: the product d (scale-free, times dyn_scale2) is
+            // the gradient of the normalised x; the accumulator is read twice, beside x for the two sums over the tile and beside
+            // g for the result; the product used to go through memory (65536 x 768, e4m3: contraction 239 and normalisation 114
+            // -> 277 us).
+            // What bounds both: 128 values a thread stay in registers from one pass to the next, and ten warps leave 168 registers
+            // a thread: they spill (stored / loaded bytes a thread, e4m3: 332 / 396, backward 152 / 340; fp16 452 / 552).  0.52 GB in
+            // 115 us and 1.05 GB in 277 are 4.5 and 3.8 TB/s.
             constexpr bool BWD = FORM == P_NORM_BWD;
             const int half = ew >> 2;
             uint8_t *const stg = smem + P_STG_OFF + ew * (3 * 4096);

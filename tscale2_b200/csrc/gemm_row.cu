@@ -10,7 +10,8 @@
 //  * the product lies in shared memory row by row, a warp takes a whole 128-column row, four columns a lane, as the
 //    normalisation's own kernel does with rows in memory, with the same arithmetic (row_math.cuh);
 //  * the weight gradient, independent of both, takes further CTAs of the launch.
-// Two blocks of dim 256 with 4 x 128 tokens, 8 steps, fp16: 3.08 -> 2.80 ms; with 3 x 100 tokens, e4m3: 2.74 -> 2.43 ms.
+// Two blocks of dim 256, 8 steps of 4 x 128 tokens and an export, fp16: 3.56 -> 3.24 ms; 8 batches of 3 x 100 tokens, two steps and an
+// export, e4m3: 3.22 -> 2.86 ms.
 // The other row-wise steps of a layer (residual + normalisation, split of Q | K | V, backward of gate and activation) ran here
 // as well and gained nothing: their products have a short K and so few CTAs that a launch over all SMs is as fast.  A launch with
 // clusters takes about 2 us more than one without.
